@@ -707,8 +707,10 @@ static void op_release(Op* op) {
   op->ws.clear();
   for (int p = 0; p < 2; p++) {
     dev_free(op->links[p], op->stream);
+    dev_free(op->links_fx[p], op->stream);
     dev_free(op->nbr[p], op->stream);
   }
+  dev_free(op->fx_field, op->stream);
   dev_free(op->d_err, op->stream);
   dev_free(op->d_partial, op->stream);
   dev_free(op->d_result, op->stream);
@@ -807,6 +809,7 @@ static int op_create(int kind, const int dims[4], int Ls, double mass, double M5
 
 int op_import_gauge_dev(Op* op, const double* U_dev) {
   for (int p = 0; p < 2; p++) GB_TRY(launch_double_store(op, U_dev, p));
+  GB_TRY(fx_import_links(op));
   GB_CHECK_CUDA(cudaStreamSynchronize(op->stream));
   op->gauge_loaded = true;
   return GB_OK;

@@ -1,0 +1,494 @@
+// gb_dhop_fx.cu -- the FP64 hopping term in 64-bit fixed-point arithmetic (gb_fx64.cuh).
+//
+// The same sum as gb_dhop.cu's dhop_kernel<double> (DhopEO / DhopOE and their daggers,
+// WilsonKernelsImplementation.h:113-163) on the same FP64 fields.  What bounds that kernel is
+// the FP64 pipe, 2 lanes per clock and SM for 860 operations per output site.  Here:
+//   fx_convert_kernel     the input checkerboard as integers with one exponent per 5D site: a
+//                         pass over the field (22 us for 75 MB in, 77 MB out, at HBM rate).
+//                         Converting inside the legs, eight times per site, took 1700 of 6200
+//                         instructions per output site and was slower for every Moebius size
+//   dhop_fx_kernel        projections, SU(3) products and sums over legs and spins as exact
+//                         integer arithmetic, each result rounded to a double once; 1728 wide
+//                         multiply-adds (32 lanes per clock and SM) of 4600 instructions per
+//                         output site.  The multiply-add pipe is its bound (70 % busy); four
+//                         CTAs of 128 threads at 128 registers beat three at 168
+//   dhop_fx_split_kernel  the same with a site's directions over four warps
+// DhopEO, dhop_kernel<double> -> these: 16^4 x 16 820 -> 185 us, 16^4 x 12 599 -> 153 us,
+// 24^3 x 32 x 12 right-hand sides 3847 -> 955 us, Wilson 24^3 x 32 345 -> 138 us, 8^4 33 -> 12 us.
+//
+// A site whose values the fixed-point range does not hold (infinities, NaN, magnitudes outside
+// 2^(fx::kEmin - 1023) .. 2^(fx::kEmax - 1022)) is marked, and the outputs next to it are
+// computed by fx_site_fp64 in FP64.
+//
+// Links: fixed-point copies made at the gauge import, in one of two layouts.
+//   slots in CTAs   [x_cb][leg][9] int4, staged per CTA in shared memory by TMA bulk copies, one
+//                   1168-byte slot per site (the padding keeps a warp's sites on distinct
+//                   banks): many slots share a site's links
+//   sites in lanes  [leg][9][x_cb] int4, read coalesced by each thread, below 8 slots per site:
+//                   staging 1152 bytes for each few threads would leave an SM one or two CTAs
+#include <cmath>
+
+#include "gb_dhop_site.cuh"
+#include "gb_fx64.cuh"
+
+namespace gb {
+namespace {
+
+struct FxParams {
+  const void* in[2];    // [z]: the checkerboards of a full-lattice Dhop, one per blockIdx.z
+  longlong2* fxin[2];   // their fixed-point copies: 12 planes, then an exponent per 5D site
+  int* exps[2];
+  void* out[2];
+  const int4* links[2];
+  const double* links_d[2];  // the FP64 links, for sites that leave the fixed-point range
+  const int* nbr[2];
+  int64_t n4h;
+  size_t n5;
+  int L5, L5a, L5c, k4;  // as DhopParams (gb_dhop.cu)
+  int link_exp;          // k of gb_fx64.cuh
+  int dag;
+  int* err;
+};
+
+constexpr int kFxLinkStride = 73;  // int4 per staged site: 72 and one of padding
+// Up to this many output sites in a launch the split kernel takes the slots-in-CTAs layout too:
+// equal at 32768 sites (8^3 x 16 x 8: 22.3 against 22.7 us), 15.5 against 19.3 us at 16384, and
+// 232 against 185 us at 524288, where the shared staging of the links counts.
+constexpr int64_t kFxSplitSites = 40000;
+
+// f of the leg's two-spinor h = (1 + S gamma_MU) f as integers
+template <int MU, int S>
+__device__ __forceinline__ void fx_project(const longlong2 (&f)[12], long long (&hr)[6], long long (&hi)[6]) {
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    const longlong2 f0 = f[c], f1 = f[3 + c], f2 = f[6 + c], f3 = f[9 + c];
+    if (MU == 0) {
+      hr[c] = f0.x - S * f3.y; hi[c] = f0.y + S * f3.x;
+      hr[3 + c] = f1.x - S * f2.y; hi[3 + c] = f1.y + S * f2.x;
+    } else if (MU == 1) {
+      hr[c] = f0.x - S * f3.x; hi[c] = f0.y - S * f3.y;
+      hr[3 + c] = f1.x + S * f2.x; hi[3 + c] = f1.y + S * f2.y;
+    } else if (MU == 2) {
+      hr[c] = f0.x - S * f2.y; hi[c] = f0.y + S * f2.x;
+      hr[3 + c] = f1.x + S * f3.y; hi[3 + c] = f1.y - S * f3.x;
+    } else {
+      hr[c] = f0.x + S * f2.x; hi[c] = f0.y + S * f2.y;
+      hr[3 + c] = f1.x + S * f3.x; hi[3 + c] = f1.y + S * f3.y;
+    }
+  }
+}
+
+struct FxAcc {
+  long long re[12], im[12];
+};
+
+// acc += u on spins 0, 1 and, on spins 2, 3, the phases of accumRecon{X,Y,Z,T}p times u
+template <int MU>
+__device__ __forceinline__ void fx_reconstruct(FxAcc& acc, const long long (&ur)[6], const long long (&ui)[6]) {
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    acc.re[a] += ur[a]; acc.im[a] += ui[a];
+    acc.re[3 + a] += ur[3 + a]; acc.im[3 + a] += ui[3 + a];
+    if (MU == 0) {
+      acc.re[6 + a] += ui[3 + a]; acc.im[6 + a] -= ur[3 + a];
+      acc.re[9 + a] += ui[a]; acc.im[9 + a] -= ur[a];
+    } else if (MU == 1) {
+      acc.re[6 + a] += ur[3 + a]; acc.im[6 + a] += ui[3 + a];
+      acc.re[9 + a] -= ur[a]; acc.im[9 + a] -= ui[a];
+    } else if (MU == 2) {
+      acc.re[6 + a] += ui[a]; acc.im[6 + a] -= ur[a];
+      acc.re[9 + a] -= ui[3 + a]; acc.im[9 + a] += ur[3 + a];
+    } else {
+      acc.re[6 + a] += ur[a]; acc.im[6 + a] += ui[a];
+      acc.re[9 + a] += ur[3 + a]; acc.im[9 + a] += ui[3 + a];
+    }
+  }
+}
+
+// One leg; pl selects the direction and the sign S of its projector (2 mu + (S > 0)), the same
+// for the whole grid, so its switches do not diverge.  The leg is a loop body: unrolled over
+// the eight legs the code would not fit the instruction cache.
+__device__ __forceinline__ void fx_leg(int pl, const longlong2* __restrict__ in, size_t n5, size_t i, int sh,
+                                       const int4* U, size_t ustride, FxAcc& acc) {
+  int hrh[6], hrl[6], hih[6], hil[6];
+  {
+    longlong2 f[12];
+#pragma unroll
+    for (int k = 0; k < 12; k++) f[k] = __ldg(in + size_t(k) * n5 + i);
+    long long hr[6], hi[6];
+    switch (pl) {
+      case 0: fx_project<0, -1>(f, hr, hi); break;
+      case 1: fx_project<0, 1>(f, hr, hi); break;
+      case 2: fx_project<1, -1>(f, hr, hi); break;
+      case 3: fx_project<1, 1>(f, hr, hi); break;
+      case 4: fx_project<2, -1>(f, hr, hi); break;
+      case 5: fx_project<2, 1>(f, hr, hi); break;
+      case 6: fx_project<3, -1>(f, hr, hi); break;
+      default: fx_project<3, 1>(f, hr, hi); break;
+    }
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+      fx::split(hr[k] >> sh, hrh[k], hrl[k]);
+      fx::split(hi[k] >> sh, hih[k], hil[k]);
+      fx::opaque(hrh[k]); fx::opaque(hrl[k]); fx::opaque(hih[k]); fx::opaque(hil[k]);
+    }
+  }
+  long long ur[6], ui[6];
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    long long rh[2], rm[2], ih[2], im[2];
+#pragma unroll
+    for (int b = 0; b < 3; b++) {
+      const int4 w = U[size_t(a * 3 + b) * ustride];
+      int nh = -w.z, nl = -w.w;
+      fx::opaque(nh); fx::opaque(nl);
+#pragma unroll
+      for (int sp = 0; sp < 2; sp++) {
+        const int k = sp * 3 + b;
+        rh[sp] = fx::mad(w.x, hrh[k], b == 0 ? fx::kStartHh : rh[sp]);
+        rm[sp] = fx::mad(w.x, hrl[k], b == 0 ? fx::kStartMid : rm[sp]);
+        rm[sp] = fx::mad(w.y, hrh[k], rm[sp]);
+        rh[sp] = fx::mad(nh, hih[k], rh[sp]);
+        rm[sp] = fx::mad(nh, hil[k], rm[sp]);
+        rm[sp] = fx::mad(nl, hih[k], rm[sp]);
+        ih[sp] = fx::mad(w.x, hih[k], b == 0 ? fx::kStartHh : ih[sp]);
+        im[sp] = fx::mad(w.x, hil[k], b == 0 ? fx::kStartMid : im[sp]);
+        im[sp] = fx::mad(w.y, hih[k], im[sp]);
+        ih[sp] = fx::mad(w.z, hrh[k], ih[sp]);
+        im[sp] = fx::mad(w.z, hrl[k], im[sp]);
+        im[sp] = fx::mad(w.w, hrh[k], im[sp]);
+      }
+    }
+#pragma unroll
+    for (int sp = 0; sp < 2; sp++) {
+      ur[sp * 3 + a] = fx::join(rh[sp], rm[sp]);
+      ui[sp * 3 + a] = fx::join(ih[sp], im[sp]);
+    }
+  }
+  switch (pl >> 1) {
+    case 0: fx_reconstruct<0>(acc, ur, ui); break;
+    case 1: fx_reconstruct<1>(acc, ur, ui); break;
+    case 2: fx_reconstruct<2>(acc, ur, ui); break;
+    default: fx_reconstruct<3>(acc, ur, ui); break;
+  }
+}
+
+// The FP64 sum of one site, straight to the output.
+template <bool DAG, int LEG>
+__device__ __forceinline__ void fp64_leg(const double2* in, const double* links, const int* nbr, size_t n5, int L5,
+                                         int64_t x, int s, Spinor<double>& acc) {
+  constexpr int MU = LEG & 3;
+  constexpr int S = (LEG < 4 ? -1 : 1) * (DAG ? -1 : 1);
+  Spinor<double> f;
+  SpinorIO<double>::load(in, nullptr, n5, size_t(nbr[x * 8 + LEG]) * L5 + s, f);
+  double hr[6], hi[6], ur[6], ui[6];
+  project<MU, S>(f, hr, hi);
+  su3_mul<double>(links + (size_t(x) * 8 + LEG) * 18, hr, hi, ur, ui);
+  reconstruct<MU, S, LEG == 0>(acc, ur, ui);
+}
+template <bool DAG>
+__device__ __forceinline__ void fp64_legs(const double2* in, const double* links, const int* nbr, size_t n5, int L5,
+                                          int64_t x, int s, Spinor<double>& acc) {
+  fp64_leg<DAG, 0>(in, links, nbr, n5, L5, x, s, acc);
+  fp64_leg<DAG, 1>(in, links, nbr, n5, L5, x, s, acc);
+  fp64_leg<DAG, 2>(in, links, nbr, n5, L5, x, s, acc);
+  fp64_leg<DAG, 3>(in, links, nbr, n5, L5, x, s, acc);
+  fp64_leg<DAG, 4>(in, links, nbr, n5, L5, x, s, acc);
+  fp64_leg<DAG, 5>(in, links, nbr, n5, L5, x, s, acc);
+  fp64_leg<DAG, 6>(in, links, nbr, n5, L5, x, s, acc);
+  fp64_leg<DAG, 7>(in, links, nbr, n5, L5, x, s, acc);
+}
+__device__ __noinline__ void fx_site_fp64(const double2* in, double2* out, const double* links, const int* nbr, size_t n5,
+                                          int L5, int64_t x, int s, int dag) {
+  Spinor<double> acc;
+  if (dag) fp64_legs<true>(in, links, nbr, n5, L5, x, s, acc);
+  else fp64_legs<false>(in, links, nbr, n5, L5, x, s, acc);
+  SpinorIO<double>::store(out, nullptr, n5, size_t(x) * L5 + s, acc);
+}
+
+// the integer (units of 2^e) as a double, rounded once; 0 stays 0
+__device__ __forceinline__ double fx_value(long long v, int e) {
+  const double d = __ll2double_rn(v);
+  return v == 0 ? 0.0 : __hiloint2double(__double2hiint(d) + (e << 20), __double2loint(d));
+}
+
+// the largest exponent of a site's eight neighbours (kBad is above every other)
+__device__ __forceinline__ int fx_site_exponent(const int* exps, const int* nbr, int L5, int64_t x, int s) {
+  const int4* nb = reinterpret_cast<const int4*>(nbr + x * 8);
+  const int4 a = __ldg(nb), b = __ldg(nb + 1);
+  const int* e = exps + s;
+  const int e0 = max(__ldg(e + size_t(a.x) * L5), __ldg(e + size_t(a.y) * L5));
+  const int e1 = max(__ldg(e + size_t(a.z) * L5), __ldg(e + size_t(a.w) * L5));
+  const int e2 = max(__ldg(e + size_t(b.x) * L5), __ldg(e + size_t(b.y) * L5));
+  const int e3 = max(__ldg(e + size_t(b.z) * L5), __ldg(e + size_t(b.w) * L5));
+  return max(max(e0, e1), max(e2, e3));
+}
+
+__device__ __forceinline__ void fx_negate_lower(FxAcc& acc) {
+#pragma unroll
+  for (int k = 6; k < 12; k++) { acc.re[k] = -acc.re[k]; acc.im[k] = -acc.im[k]; }
+}
+
+// The legs [leg0, leg0 + n) and [leg0 + 4, leg0 + 4 + n) of one site, in units of Ea.  Spins 2,
+// 3 are summed without the legs' sign S and negated after the forward legs.
+__device__ __forceinline__ void fx_legs(const FxParams& p, const longlong2* in, const int* exps, const int* nbr,
+                                        const int4* U, size_t ustride, int64_t x, int s, int leg0, int n, int Ea,
+                                        FxAcc& acc) {
+#pragma unroll
+  for (int k = 0; k < 12; k++) { acc.re[k] = 0; acc.im[k] = 0; }
+#pragma unroll 1
+  for (int m = 0; m < 2 * n; m++) {
+    if (m == n) fx_negate_lower(acc);
+    const int leg = m < n ? leg0 + m : leg0 + 4 + m - n;
+    const size_t j = size_t(__ldg(nbr + x * 8 + leg)) * p.L5 + s;
+    fx_leg(2 * (leg & 3) + ((leg >= 4) != (p.dag != 0) ? 1 : 0), in, p.n5, j, min(Ea - __ldg(exps + j), 63),
+           U + size_t(leg) * 9 * ustride, ustride, acc);
+  }
+  if (p.dag) fx_negate_lower(acc);
+}
+
+// zeros into the padding slots of an odd right-hand-side count
+__device__ __forceinline__ void fx_pad(const FxParams& p, double2* out, int64_t x, int s) {
+  if (s != 0 || p.L5a == p.L5) return;
+  Spinor<double> zero;
+#pragma unroll
+  for (int k = 0; k < 12; k++) { zero.re[k] = 0.0; zero.im[k] = 0.0; }
+  for (int z = p.L5a; z < p.L5; z++) SpinorIO<double>::store(out, nullptr, p.n5, size_t(x) * p.L5 + z, zero);
+}
+
+// The fixed-point copy of one checkerboard of a field (both with blockIdx.z), one thread per 5D
+// site.  A pass of its own: each site is read by eight outputs, and converting it eight times
+// there took more instructions than the SU(3) products.
+__global__ void __launch_bounds__(256) fx_convert_kernel(const __grid_constant__ FxParams p) {
+  const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= p.n5) return;
+  const double2* in = static_cast<const double2*>(p.in[blockIdx.z]);
+  longlong2* out = p.fxin[blockIdx.z];
+  Spinor<double> f;
+  SpinorIO<double>::load(in, nullptr, p.n5, i, f);
+  uint32_t amax = 0, low = 0;
+#pragma unroll
+  for (int k = 0; k < 12; k++) {
+    amax = max(amax, max(uint32_t(__double2hiint(f.re[k])) & 0x7fffffffu, uint32_t(__double2hiint(f.im[k])) & 0x7fffffffu));
+    low |= uint32_t(__double2loint(f.re[k])) | uint32_t(__double2loint(f.im[k]));
+  }
+  int E = int(amax >> 20);
+  const bool zero = (amax | low) == 0, ok = E >= fx::kEmin && E <= fx::kEmax;
+  p.exps[blockIdx.z][i] = zero ? 0 : ok ? E : fx::kBad;
+  E = ok ? E : fx::kEmax;  // values of zero and marked sites: zeros, or not read
+#pragma unroll
+  for (int k = 0; k < 12; k++) {
+    longlong2 v;
+    v.x = fx::from_words(uint32_t(__double2hiint(f.re[k])), uint32_t(__double2loint(f.re[k])), E);
+    v.y = fx::from_words(uint32_t(__double2hiint(f.im[k])), uint32_t(__double2loint(f.im[k])), E);
+    out[size_t(k) * p.n5 + i] = v;
+  }
+}
+
+__global__ void __launch_bounds__(128, 4) dhop_fx_kernel(const __grid_constant__ FxParams p) {
+  extern __shared__ __align__(128) unsigned char dyn_smem[];
+  int4* slink = reinterpret_cast<int4*>(dyn_smem);  // k4 * kFxLinkStride
+  __shared__ __align__(8) uint64_t bar;
+  const int side = blockIdx.z;
+  const double2* in = static_cast<const double2*>(p.in[side]);
+  double2* out = static_cast<double2*>(p.out[side]);
+  const int* nbr = p.nbr[side];
+  const int* exps = p.exps[side];
+  const int t = threadIdx.x;
+  const int64_t x0 = int64_t(blockIdx.x) * p.k4;
+  const int nsite = int(min(int64_t(p.k4), p.n4h - x0));
+  const int j = t / p.L5c;
+  const int s = int(blockIdx.y) * p.L5c + (t - j * p.L5c);
+  if (t == 0) mbar_init(&bar, 1);
+  __syncthreads();
+  if (t == 0) {
+    mbar_expect_tx(&bar, uint32_t(nsite) * 1152u);
+    for (int k = 0; k < nsite; k++) bulk_g2s(slink + k * kFxLinkStride, p.links[side] + (x0 + k) * 72, 1152u, &bar);
+  }
+  if (!mbar_wait_bounded(&bar, 0)) {  // every thread waits; the error flag as in gb_dhop.cu
+    atomicExch(p.err, 1);
+    return;
+  }
+  if (j >= nsite || s >= p.L5a) return;
+  const int64_t x = x0 + j;
+  fx_pad(p, out, x, s);
+  const int Ea = fx_site_exponent(exps, nbr, p.L5, x, s);
+  if (Ea == fx::kBad) {
+    fx_site_fp64(in, out, p.links_d[side], nbr, p.n5, p.L5, x, s, p.dag);
+    return;
+  }
+  FxAcc acc;
+  fx_legs(p, p.fxin[side], exps, nbr, slink + j * kFxLinkStride, 1, x, s, 0, 4, Ea, acc);
+  const int e = fx::result_exponent(Ea, p.link_exp);
+  const size_t i = size_t(x) * p.L5 + s;
+#pragma unroll
+  for (int k = 0; k < 12; k++) out[size_t(k) * p.n5 + i] = make_double2(fx_value(acc.re[k], e), fx_value(acc.im[k], e));
+}
+
+// Four warps share 32 output sites, one direction (its forward and backward leg) each, and add
+// their integer sums through shared memory: exactly, so the result does not depend on which
+// kernel ran.  A site is a chain of about 4600 instructions for one thread: with few sites that
+// chain is the launch's time (8^4: 12.4 us, one thread per site 20.0), and with sites in lanes
+// the extra warps keep more of the links' 1152 bytes per site in flight (24^3 x 32: 138 us, one
+// thread per site 153).  SOA: the links' sites-in-lanes layout.
+template <bool SOA>
+__global__ void __launch_bounds__(128, 4) dhop_fx_split_kernel(const __grid_constant__ FxParams p) {
+  __shared__ long long part[4][24][32];
+  const int side = blockIdx.z;
+  const int lane = threadIdx.x & 31, mu = threadIdx.x >> 5;
+  const double2* in = static_cast<const double2*>(p.in[side]);
+  double2* out = static_cast<double2*>(p.out[side]);
+  const int* nbr = p.nbr[side];
+  const int* exps = p.exps[side];
+  const int64_t g = int64_t(blockIdx.x) * 32 + lane;
+  const bool active = g < p.n4h * p.L5a;
+  const int64_t x = active ? g / p.L5a : 0;
+  const int s = active ? int(g - x * p.L5a) : 0;
+  const int Ea = fx_site_exponent(exps, nbr, p.L5, x, s);
+  if (Ea != fx::kBad) {
+    FxAcc acc;
+    fx_legs(p, p.fxin[side], exps, nbr, SOA ? p.links[side] + x : p.links[side] + x * 72, SOA ? size_t(p.n4h) : size_t(1),
+            x, s, mu, 1, Ea, acc);
+#pragma unroll
+    for (int k = 0; k < 12; k++) { part[mu][2 * k][lane] = acc.re[k]; part[mu][2 * k + 1][lane] = acc.im[k]; }
+  }
+  __syncthreads();
+  if (!active) return;
+  if (mu == 0) fx_pad(p, out, x, s);
+  if (Ea == fx::kBad) {
+    if (mu == 0) fx_site_fp64(in, out, p.links_d[side], nbr, p.n5, p.L5, x, s, p.dag);
+    return;
+  }
+  const int e = fx::result_exponent(Ea, p.link_exp);
+  const size_t i = size_t(x) * p.L5 + s;
+#pragma unroll
+  for (int m = 0; m < 3; m++) {  // warp mu finishes components 3 mu .. 3 mu + 2
+    const int k = 3 * mu + m;
+    long long v[2];
+#pragma unroll
+    for (int c = 0; c < 2; c++)
+      v[c] = (part[0][2 * k + c][lane] + part[1][2 * k + c][lane]) + (part[2][2 * k + c][lane] + part[3][2 * k + c][lane]);
+    out[size_t(k) * p.n5 + i] = make_double2(fx_value(v[0], e), fx_value(v[1], e));
+  }
+}
+
+// the largest row sum of absolute values over one parity's links, as the bits of a float
+// rounded up (infinity for anything not finite)
+__global__ void __launch_bounds__(256) fx_row_sum_kernel(const double* links, size_t rows, unsigned* out) {
+  float m = 0.f;
+  for (size_t r = size_t(blockIdx.x) * blockDim.x + threadIdx.x; r < rows; r += size_t(gridDim.x) * blockDim.x) {
+    double s = 0.0;
+#pragma unroll
+    for (int e = 0; e < 6; e++) s += fabs(links[r * 6 + e]);
+    const float f = __double2float_ru(s);
+    m = f <= 3.0e38f ? fmaxf(m, f) : __int_as_float(0x7f800000);
+    if (!(f <= 3.0e38f)) break;
+  }
+  m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
+  if ((threadIdx.x & 31) == 0) atomicMax(out, __float_as_uint(m));
+}
+
+// fixed-point copy of one parity's links (k = exponent), AoS [x][leg][9] or SoA [leg][9][x]
+__global__ void __launch_bounds__(256) fx_links_kernel(const double* links, int4* out, int64_t n4h, int k, int soa) {
+  const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (t >= size_t(n4h) * 72) return;
+  int4 w;
+  fx::split_link(__double2ll_rn(ldexp(links[2 * t], 61 - k)), w.x, w.y);
+  fx::split_link(__double2ll_rn(ldexp(links[2 * t + 1], 61 - k)), w.z, w.w);
+  const size_t x = t / 72, e = t - x * 72;
+  out[soa ? e * size_t(n4h) + x : t] = w;
+}
+
+}  // namespace
+
+// Operators whose FP64 hopping term runs in fixed point: the native FP64 arithmetic stays for
+// 12-real links (rebuilt per CTA in FP64) and GB_FLAG_DF64 chooses its own.
+bool fx_wanted(const Op* op) { return op->prec == GB_F64 && !op->recon12 && !op->df64; }
+
+// The links' layout: sites in lanes below 8 slots per site (a CTA of 128 threads then stages 16
+// sites at most, 18.7 KB, and four CTAs stay resident).
+static bool fx_soa(const Op* op) { return op->Ls * op->nrhs_user < 8; }
+
+// Fixed-point copies of op->links, and the scratch of fx_convert_kernel (both checkerboards of
+// a field and their exponents): allocated here so that a launch allocates nothing.  Links that
+// are all zero, not finite or of extreme magnitude, and a device without the memory, leave
+// op->fx_ready off and the hopping term on the FP64 kernel.
+int fx_import_links(Op* op) {
+  op->fx_ready = false;
+  if (!fx_wanted(op)) return GB_OK;
+  unsigned* d_max = reinterpret_cast<unsigned*>(op->d_result);
+  GB_CHECK_CUDA(cudaMemsetAsync(d_max, 0, sizeof(unsigned), op->stream));
+  for (int p = 0; p < 2; p++)
+    fx_row_sum_kernel<<<kRedBlocks, 256, 0, op->stream>>>(static_cast<const double*>(op->links[p]), size_t(op->half4) * 24,
+                                                          d_max);
+  GB_CHECK_CUDA(cudaGetLastError());
+  GB_CHECK_CUDA(cudaMemcpyAsync(op->h_result, d_max, sizeof(float), cudaMemcpyDeviceToHost, op->stream));
+  GB_CHECK_CUDA(cudaStreamSynchronize(op->stream));
+  const float top = *reinterpret_cast<const float*>(op->h_result);
+  if (!(top > 1e-9f && top < 1e9f)) return GB_OK;
+  int k = -32;
+  while (double(top) > 1.5 * std::ldexp(1.0, k)) k++;
+  op->fx_exp = k;
+  const size_t n = size_t(op->half4) * 72;
+  const size_t field = op->n5() * 2 * (12 * sizeof(longlong2) + sizeof(int));
+  void** bufs[3] = {&op->links_fx[0], &op->links_fx[1], &op->fx_field};
+  for (int i = 0; i < 3; i++) {
+    if (*bufs[i]) continue;  // kept from an earlier import
+    if (cudaMallocAsync(bufs[i], i < 2 ? n * sizeof(int4) : field, op->stream) != cudaSuccess) {
+      cudaGetLastError();
+      for (int j = 0; j < i; j++) {
+        cudaFreeAsync(*bufs[j], op->stream);
+        *bufs[j] = nullptr;
+      }
+      *bufs[i] = nullptr;
+      return GB_OK;
+    }
+  }
+  for (int p = 0; p < 2; p++)
+    fx_links_kernel<<<unsigned((n + 255) / 256), 256, 0, op->stream>>>(static_cast<const double*>(op->links[p]),
+                                                                       static_cast<int4*>(op->links_fx[p]), op->half4, k,
+                                                                       fx_soa(op) ? 1 : 0);
+  GB_CHECK_CUDA(cudaGetLastError());
+  op->fx_ready = true;
+  return GB_OK;
+}
+
+int launch_dhop_fx(Op* op, HalfView in, HalfView out, int out_parity, const HalfView* in2, const HalfView* out2, int dag) {
+  FxParams p;
+  const HalfView* ins[2] = {&in, in2};
+  const HalfView* outs[2] = {&out, out2};
+  for (int z = 0; z < 2; z++) {
+    const int par = z ? 1 - out_parity : out_parity;
+    p.in[z] = ins[z] ? ins[z]->data : nullptr;
+    p.out[z] = outs[z] ? outs[z]->data : nullptr;
+    p.links[z] = static_cast<const int4*>(op->links_fx[par]);
+    p.links_d[z] = static_cast<const double*>(op->links[par]);
+    p.nbr[z] = op->nbr[par];
+    p.fxin[z] = static_cast<longlong2*>(op->fx_field) + size_t(z) * 12 * op->n5();
+    p.exps[z] = reinterpret_cast<int*>(static_cast<longlong2*>(op->fx_field) + 24 * op->n5()) + size_t(z) * op->n5();
+  }
+  p.n4h = op->half4;
+  p.n5 = op->n5();
+  p.L5 = op->L5;
+  p.L5a = op->Ls * op->nrhs_user;
+  p.link_exp = op->fx_exp;
+  p.dag = dag;
+  p.err = op->d_err;
+  fx_convert_kernel<<<dim3(unsigned((p.n5 + 255) / 256), 1, in2 ? 2u : 1u), 256, 0, op->stream>>>(p);
+  const bool soa = fx_soa(op);
+  if (soa || p.n4h * p.L5a * (in2 ? 2 : 1) <= kFxSplitSites) {
+    const dim3 grid(unsigned((p.n4h * p.L5a + 31) / 32), 1, in2 ? 2u : 1u);
+    if (soa) dhop_fx_split_kernel<true><<<grid, 128, 0, op->stream>>>(p);
+    else dhop_fx_split_kernel<false><<<grid, 128, 0, op->stream>>>(p);
+  } else {
+    p.L5c = p.L5a > 128 ? 128 : p.L5a;
+    p.k4 = 128 / p.L5c;
+    const dim3 grid(unsigned((p.n4h + p.k4 - 1) / p.k4), unsigned((p.L5a + p.L5c - 1) / p.L5c), in2 ? 2u : 1u);
+    const unsigned threads = unsigned((p.k4 * p.L5c + 31) / 32 * 32);
+    dhop_fx_kernel<<<grid, threads, size_t(p.k4) * kFxLinkStride * sizeof(int4), op->stream>>>(p);
+  }
+  GB_CHECK_CUDA(cudaGetLastError());
+  return GB_OK;
+}
+
+}  // namespace gb

@@ -79,6 +79,12 @@ struct Op {
 
   void* links[2] = {nullptr, nullptr};  // per output parity
   int* nbr[2] = {nullptr, nullptr};
+  // fixed-point copies of FP64 links for the hopping term (gb_dhop_fx.cu): made at the gauge
+  // import, with the exponent of their units; fx_ready is off where the FP64 kernel is used
+  void* links_fx[2] = {nullptr, nullptr};
+  void* fx_field = nullptr;  // the input field of a launch in fixed point
+  int fx_exp = 0;
+  bool fx_ready = false;
   int* d_err = nullptr;                 // device error flag of bounded waits
   // Set when the host finds d_err raised.  A Dhop CTA whose bounded wait for its TMA copy
   // gave up returns while that copy may still be writing into shared memory that the
@@ -179,6 +185,11 @@ int launch_dhop_mooee(Op* op, HalfView in, HalfView x5, HalfView out, int out_pa
                       const double* diag, const double* upper, int* parts);
 // CTAs of one single-checkerboard launch of the FP32 / FP16 Dhop kernel
 size_t dhop_pair_ctas(const Op* op);
+// FP64 hopping term in fixed point (gb_dhop_fx.cu): whether an operator takes it, the link
+// copies, and one launch (in2, out2: the second checkerboard of a full-lattice Dhop)
+bool fx_wanted(const Op* op);
+int fx_import_links(Op* op);
+int launch_dhop_fx(Op* op, HalfView in, HalfView out, int out_parity, const HalfView* in2, const HalfView* out2, int dag);
 int launch_dhop_full(Op* op, HalfView in_odd, HalfView out_even, HalfView in_even, HalfView out_odd, int dag);
 // force term of the output parity's sites into mat (FP64 canonical gauge layout, indexed
 // by x_cb when half_out, else by the lexicographic site); A has the output parity

@@ -187,8 +187,10 @@ size_t request_bytes(const gb_request& r, int nsrc) {
   for (int k = 0; k < 4; k++) vol *= r.dims[k];
   const int64_t n5 = vol / 2 * r.Ls * (nsrc + ((r.Ls * nsrc) & 1));
   const size_t lo = r.inner_precision == GB_F16 ? 52 : 96;
-  const size_t per_site4 = 1152 + 576 + 64 + 576;  // FP64 + FP32 links, neighbours, FP64 gauge staging
-  return size_t(vol) * per_site4 + size_t(n5) * (26 * 192 + 12 * lo);
+  // FP64 + fixed-point + FP32 links, neighbours, FP64 gauge staging
+  const size_t per_site4 = 1152 + 1152 + 576 + 64 + 576;
+  // work fields, and both checkerboards of the FP64 hopping term's fixed-point input
+  return size_t(vol) * per_site4 + size_t(n5) * (26 * 192 + 2 * 196 + 12 * lo);
 }
 
 // work of one CG iteration (the shortest-first key): 4D volume x Ls x sources

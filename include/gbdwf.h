@@ -74,9 +74,10 @@ int gb_device_count(int* n);
  * phases (+1 / -1), else GB_ERR_UNSUPPORTED.
  * GB_FLAG_DF64 (GB_F64 operators with 18-real links, else GB_ERR_UNSUPPORTED): the hopping
  * term computes in double-float arithmetic (pairs of floats, about 48 significant bits:
- * relative L2 error near 5e-15 per application) on the FP32 pipes instead of the FP64
- * pipe, which on GB300 runs at 1/64 of the FP32 rate; fields stay FP64.  Every other
- * FP64 kernel is unchanged.
+ * relative L2 error near 5e-15 per application); fields stay FP64.  Every other FP64 kernel
+ * is unchanged.  Without the flag the FP64 hopping term sums exact fixed-point products and
+ * rounds each result to a double once (error below IEEE double arithmetic's), which is
+ * faster; the flag remains for callers that chose its arithmetic.
  */
 #define GB_FLAG_RECON12 1u
 #define GB_FLAG_DF64 2u
