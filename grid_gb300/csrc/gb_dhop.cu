@@ -862,8 +862,17 @@ int launch_dhop_full(Op* op, HalfView in_odd, HalfView out_even, HalfView in_eve
 // WilsonImpl::InsertForce5D (WilsonImpl.h:193-238).  For each output site x and direction
 // mu:  mat[x][mu]_ab = sum_s sum_spin Bt(x,s)_{spin,a} conj(A(x,s)_{spin,b}),
 // Bt = (1 -+ gamma_mu) U~_mu(x) B(x + mu) -- the forward leg of Dhop (dag: of Dhop^dag).
-// One thread per (x, mu) walks the L5 slots (all right-hand sides are summed), so the sum
-// has a fixed order; the result is FP64 in the canonical gauge layout.
+// All right-hand sides are summed, in a fixed order; the result is FP64 in the canonical gauge
+// layout.
+//
+// Spins 2, 3 of Bt are phases of spins 0, 1, and the same phases on A make its projection, so
+//   mat = U~ W,  W_cb = sum_s sum_{j = 0,1} h_{j,c} conj(g_{j,b}),
+// h and g the two-spinors of B(x + mu) and A(x): per s 72 FP64 multiply-adds (and 24 projection
+// additions) where the four-spinor outer product with the link inside the sum took 216.
+// FP64 issue bounds it (2 lanes per clock and SM): MDeriv at 16^4 x 12 FP64 7014 -> 707 us, of
+// which Meooe5D is 80.  A warp takes one direction of 32 / G sites;
+// G lanes share a site, each walking every G-th of its s, and a CTA's four warps are the
+// four directions of the same sites, which read A once from HBM and three times from L1.
 // =======================================================================================
 struct DerivParams {
   const void* A;
@@ -880,45 +889,97 @@ struct DerivParams {
   DhopParams geo;  // L, sgn, parity (for the 12-real link rebuild and the site index)
 };
 
-template <class T, bool DAG, int MU, bool RECON>
-__device__ __forceinline__ void deriv_site(const DerivParams& q, int64_t x) {
+// w += h conj(g)^T over both spins of the two-spinors
+template <class R>
+__device__ __forceinline__ void deriv_outer(const R (&hr)[6], const R (&hi)[6], const R (&gr)[6], const R (&gi)[6],
+                                            double (&wr)[9], double (&wi)[9]) {
+#pragma unroll
+  for (int j = 0; j < 2; j++)
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+#pragma unroll
+      for (int b = 0; b < 3; b++) {
+        const double xr = hr[j * 3 + c], xi = hi[j * 3 + c], yr = gr[j * 3 + b], yi = gi[j * 3 + b];
+        wr[c * 3 + b] = fma(xr, yr, fma(xi, yi, wr[c * 3 + b]));
+        wi[c * 3 + b] = fma(xi, yr, fma(-xr, yi, wi[c * 3 + b]));
+      }
+}
+
+// lane g of G of one site: every G-th 16-byte vector along s (FP64 one s, FP32 a pair)
+template <class T, int MU, int S, int G>
+__device__ __forceinline__ void deriv_site(const DerivParams& q, int64_t x, int64_t nb, int g, double (&wr)[9],
+                                           double (&wi)[9]) {
+  if constexpr (sizeof(T) == 8) {
+    for (int s = g; s < q.L5; s += G) {
+      double hr[6], hi[6], gr[6], gi[6];
+      Spinor<double> f;
+      SpinorIO<double>::load(q.B, nullptr, q.n5, size_t(nb) * q.L5 + s, f);
+      project<MU, S>(f, hr, hi);
+      SpinorIO<double>::load(q.A, nullptr, q.n5, size_t(x) * q.L5 + s, f);
+      project<MU, S>(f, gr, gi);
+      deriv_outer<double>(hr, hi, gr, gi, wr, wi);
+    }
+  } else {
+    const int hl = q.L5 >> 1;
+    for (int sp = g; sp < hl; sp += G) {
+      float2 hr[6], hi[6], gr[6], gi[6];
+      Pair12 f;
+      PairIO<float>::load(q.B, nullptr, q.n5 >> 1, size_t(nb) * hl + sp, f);
+      project2<MU, S>(f, hr, hi);
+      PairIO<float>::load(q.A, nullptr, q.n5 >> 1, size_t(x) * hl + sp, f);
+      project2<MU, S>(f, gr, gi);
+#pragma unroll
+      for (int l = 0; l < 2; l++) {
+        float xr[6], xi[6], yr[6], yi[6];
+#pragma unroll
+        for (int k = 0; k < 6; k++) {
+          xr[k] = l ? hr[k].y : hr[k].x; xi[k] = l ? hi[k].y : hi[k].x;
+          yr[k] = l ? gr[k].y : gr[k].x; yi[k] = l ? gi[k].y : gi[k].x;
+        }
+        deriv_outer<float>(xr, xi, yr, yi, wr, wi);
+      }
+    }
+  }
+}
+
+template <class T, bool DAG, bool RECON, int G>
+__global__ void __launch_bounds__(128) deriv_kernel(const DerivParams q) {
   using R = typename Arith<T>::type;
   constexpr int S = DAG ? 1 : -1;
+  const int mu = threadIdx.y, g = threadIdx.x % G;
+  const int64_t x = int64_t(blockIdx.x) * (32 / G) + threadIdx.x / G;
+  const bool active = x < q.n4h;
+  double wr[9], wi[9];
+#pragma unroll
+  for (int e = 0; e < 9; e++) { wr[e] = 0; wi[e] = 0; }
+  if (active) {
+    const int64_t nb = q.nbr[size_t(x) * 8 + mu];
+    switch (mu) {
+      case 0: deriv_site<T, 0, S, G>(q, x, nb, g, wr, wi); break;
+      case 1: deriv_site<T, 1, S, G>(q, x, nb, g, wr, wi); break;
+      case 2: deriv_site<T, 2, S, G>(q, x, nb, g, wr, wi); break;
+      default: deriv_site<T, 3, S, G>(q, x, nb, g, wr, wi); break;
+    }
+  }
+  if (G == 2) {
+#pragma unroll
+    for (int e = 0; e < 9; e++) {
+      wr[e] += __shfl_xor_sync(0xffffffffu, wr[e], 1);
+      wi[e] += __shfl_xor_sync(0xffffffffu, wi[e], 1);
+    }
+  }
+  if (!active) return;
   R Ul[18];
   if (RECON) {
     R raw[12];
-    const R* src = static_cast<const R*>(q.links) + (size_t(x) * 8 + MU) * 12;
+    const R* src = static_cast<const R*>(q.links) + (size_t(x) * 8 + mu) * 12;
 #pragma unroll
     for (int e = 0; e < 12; e++) raw[e] = src[e];
-    expand_link12<R>(q.geo, x, MU, raw, Ul);
+    expand_link12<R>(q.geo, x, mu, raw, Ul);
   } else {
-    const R* src = static_cast<const R*>(q.links) + (size_t(x) * 8 + MU) * 18;
+    const R* src = static_cast<const R*>(q.links) + (size_t(x) * 8 + mu) * 18;
 #pragma unroll
     for (int e = 0; e < 18; e++) Ul[e] = src[e];
-  }
-  const int nb = q.nbr[size_t(x) * 8 + MU];
-  double fr[9], fi[9];
-#pragma unroll
-  for (int e = 0; e < 9; e++) { fr[e] = 0; fi[e] = 0; }
-  for (int s = 0; s < q.L5; s++) {
-    Spinor<R> b, a, bt;
-    SpinorIO<T>::load(q.B, q.Bn, q.n5, size_t(nb) * q.L5 + s, b);
-    SpinorIO<T>::load(q.A, q.An, q.n5, size_t(x) * q.L5 + s, a);
-    R hr[6], hi[6], ur[6], ui[6];
-    project<MU, S>(b, hr, hi);
-    su3_mul<R>(Ul, hr, hi, ur, ui);
-    reconstruct<MU, S, true>(bt, ur, ui);
-#pragma unroll
-    for (int ca = 0; ca < 3; ca++)
-#pragma unroll
-      for (int cb = 0; cb < 3; cb++)
-#pragma unroll
-        for (int sp = 0; sp < 4; sp++) {
-          const double br = bt.re[sp * 3 + ca], bi = bt.im[sp * 3 + ca];
-          const double ar = a.re[sp * 3 + cb], ai = a.im[sp * 3 + cb];
-          fr[ca * 3 + cb] += br * ar + bi * ai;  // b conj(a)
-          fi[ca * 3 + cb] += bi * ar - br * ai;
-        }
   }
   int64_t idx = x;
   if (!q.half_out) {  // lexicographic site of x_cb in the output parity
@@ -930,22 +991,39 @@ __device__ __forceinline__ void deriv_site(const DerivParams& q, int64_t x) {
     const int z = int(zt % q.geo.L[2]), t = int(zt / q.geo.L[2]);
     idx = row * q.geo.L[0] + 2 * xh + ((q.geo.parity + y + z + t) & 1);
   }
-  double2* o = q.mat + (size_t(idx) * 4 + MU) * 9;
+  double2* o = q.mat + (size_t(idx) * 4 + mu) * 9;
+  // the rows of U W: two lanes take row g each, then lane 0 the last
 #pragma unroll
-  for (int e = 0; e < 9; e++) o[e] = make_double2(fr[e], fi[e]);
+  for (int pass = 0; pass < (G == 2 ? 2 : 3); pass++) {
+    const int a = G == 2 ? (pass == 0 ? g : 2) : pass;
+    if (G == 2 && pass == 1 && g == 1) break;
+    double ur[3], ui[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const int e = 2 * c;
+      ur[c] = a == 0 ? Ul[e] : a == 1 ? Ul[6 + e] : Ul[12 + e];
+      ui[c] = a == 0 ? Ul[e + 1] : a == 1 ? Ul[7 + e] : Ul[13 + e];
+    }
+#pragma unroll
+    for (int b = 0; b < 3; b++) {
+      double re = 0, im = 0;
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        re = fma(ur[c], wr[c * 3 + b], fma(-ui[c], wi[c * 3 + b], re));
+        im = fma(ur[c], wi[c * 3 + b], fma(ui[c], wr[c * 3 + b], im));
+      }
+      o[a * 3 + b] = make_double2(re, im);
+    }
+  }
 }
 
+// two lanes per site halve the walk along s; one where the site has a single vector
 template <class T, bool DAG, bool RECON>
-__global__ void __launch_bounds__(128) deriv_kernel(const DerivParams q) {
-  const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (t >= q.n4h * 4) return;
-  const int64_t x = t >> 2;
-  switch (int(t & 3)) {
-    case 0: deriv_site<T, DAG, 0, RECON>(q, x); break;
-    case 1: deriv_site<T, DAG, 1, RECON>(q, x); break;
-    case 2: deriv_site<T, DAG, 2, RECON>(q, x); break;
-    default: deriv_site<T, DAG, 3, RECON>(q, x); break;
-  }
+static void deriv_go(Op* op, const DerivParams& q) {
+  const int vectors = sizeof(T) == 8 ? q.L5 : q.L5 >> 1;
+  const dim3 block(32, 4);
+  if (vectors >= 2) deriv_kernel<T, DAG, RECON, 2><<<unsigned((q.n4h + 15) / 16), block, 0, op->stream>>>(q);
+  else deriv_kernel<T, DAG, RECON, 1><<<unsigned((q.n4h + 31) / 32), block, 0, op->stream>>>(q);
 }
 
 int launch_deriv(Op* op, HalfView A, HalfView B, int out_parity, int dag, double* mat, int half_out) {
@@ -965,17 +1043,16 @@ int launch_deriv(Op* op, HalfView A, HalfView B, int out_parity, int dag, double
     q.geo.sgn[k] = op->phases[k].real() < 0 ? -1 : 1;
   }
   q.geo.parity = out_parity;
-  const unsigned blocks = unsigned((op->half4 * 4 + 127) / 128);
   const int key = (op->prec == GB_F64 ? 4 : 0) | (dag ? 2 : 0) | (op->recon12 ? 1 : 0);
   switch (key) {
-    case 0: deriv_kernel<float, false, false><<<blocks, 128, 0, op->stream>>>(q); break;
-    case 1: deriv_kernel<float, false, true><<<blocks, 128, 0, op->stream>>>(q); break;
-    case 2: deriv_kernel<float, true, false><<<blocks, 128, 0, op->stream>>>(q); break;
-    case 3: deriv_kernel<float, true, true><<<blocks, 128, 0, op->stream>>>(q); break;
-    case 4: deriv_kernel<double, false, false><<<blocks, 128, 0, op->stream>>>(q); break;
-    case 5: deriv_kernel<double, false, true><<<blocks, 128, 0, op->stream>>>(q); break;
-    case 6: deriv_kernel<double, true, false><<<blocks, 128, 0, op->stream>>>(q); break;
-    default: deriv_kernel<double, true, true><<<blocks, 128, 0, op->stream>>>(q); break;
+    case 0: deriv_go<float, false, false>(op, q); break;
+    case 1: deriv_go<float, false, true>(op, q); break;
+    case 2: deriv_go<float, true, false>(op, q); break;
+    case 3: deriv_go<float, true, true>(op, q); break;
+    case 4: deriv_go<double, false, false>(op, q); break;
+    case 5: deriv_go<double, false, true>(op, q); break;
+    case 6: deriv_go<double, true, false>(op, q); break;
+    default: deriv_go<double, true, true>(op, q); break;
   }
   GB_CHECK_CUDA(cudaGetLastError());
   return GB_OK;
