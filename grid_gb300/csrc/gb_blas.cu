@@ -502,8 +502,10 @@ template <class CR> struct Canon2;
 template <> struct Canon2<double> { using type = double2; };
 template <> struct Canon2<float> { using type = float2; };
 
-template <class T, class CR, bool IMPORT>
-__global__ void __launch_bounds__(256) layout_kernel(const GeoParams g, CR* canon, void* dev, float* devn, int parity,
+// canonical -> device planes, one thread per 5D site (its 12 reads share their lines in L1; through
+// a shared tile as the export it measured 3-20 % slower)
+template <class T, class CR>
+__global__ void __launch_bounds__(256) import_kernel(const GeoParams g, const CR* canon, void* dev, float* devn, int parity,
                                                      int canon_full) {
   using R = typename Arith<T>::type;
   using C2 = typename Canon2<CR>::type;
@@ -514,33 +516,120 @@ __global__ void __launch_bounds__(256) layout_kernel(const GeoParams g, CR* cano
   const int s5 = int(i - size_t(xcb) * g.L5);
   const int rhs = s5 / g.Ls, s = s5 - rhs * g.Ls;
   Spinor<R> f;
-  if (rhs >= g.nrhs_user) {  // the padding right-hand side: zeros, absent from the host array
-    if (IMPORT) {
-#pragma unroll
-      for (int k = 0; k < 12; k++) { f.re[k] = R(0); f.im[k] = R(0); }
-      SpinorIO<T>::store(dev, devn, n5, i, f);
-    }
-    return;
-  }
-  const int64_t c4 = canon_full ? cb_to_site(xcb, parity, g) : xcb;
-  const int64_t n4c = canon_full ? g.vol4 : g.half4;
-  C2* c = reinterpret_cast<C2*>(canon) + ((size_t(rhs) * n4c + c4) * g.Ls + s) * 12;
-  if (IMPORT) {
+  if (rhs < g.nrhs_user) {
+    const int64_t c4 = canon_full ? cb_to_site(xcb, parity, g) : xcb;
+    const int64_t n4c = canon_full ? g.vol4 : g.half4;
+    const C2* c = reinterpret_cast<const C2*>(canon) + ((size_t(rhs) * n4c + c4) * g.Ls + s) * 12;
 #pragma unroll
     for (int k = 0; k < 12; k++) {
       const C2 v = c[k];
       f.re[k] = R(v.x); f.im[k] = R(v.y);
     }
-    SpinorIO<T>::store(dev, devn, n5, i, f);
-  } else {
-    SpinorIO<T>::load(dev, devn, n5, i, f);
+  } else {  // the padding right-hand side: zeros, absent from the host array
 #pragma unroll
-    for (int k = 0; k < 12; k++) {
-      C2 v;
-      v.x = CR(f.re[k]);
-      v.y = CR(f.im[k]);
-      c[k] = v;
+    for (int k = 0; k < 12; k++) { f.re[k] = R(0); f.im[k] = R(0); }
+  }
+  SpinorIO<T>::store(dev, devn, n5, i, f);
+}
+
+// float -> double without the FP64 pipe's conversion (2 lanes per clock and SM, which at 24 per
+// site would bound the FP32 export): the widening by integer operations, subnormals by the
+// instruction
+__device__ __forceinline__ double widen(float f) {
+  const uint32_t b = __float_as_uint(f), e = (b >> 23) & 0xffu;
+  if (e - 1u >= 0xfeu && (b << 1) != 0) return double(f);  // subnormal, infinity, NaN
+  const uint32_t hi = (b & 0x80000000u) | ((b & 0x7fffffffu) >> 3);
+  return __hiloint2double(int((b << 1) == 0 ? hi : hi + 0x38000000u), int(b << 29));
+}
+// a tile value as the canonical type of the first argument
+__device__ __forceinline__ double2 canon_value(double2, double2 v) { return v; }
+__device__ __forceinline__ double2 canon_value(double2, float2 v) { return make_double2(widen(v.x), widen(v.y)); }
+__device__ __forceinline__ float2 canon_value(float2, double2 v) { return make_float2(float(v.x), float(v.y)); }
+__device__ __forceinline__ float2 canon_value(float2, float2 v) { return v; }
+
+// Device planes -> canonical: one CTA takes kLayoutSites consecutive 5D sites through a shared tile
+// [site][component] (13 complex per site: conflict-free both ways), reading along the planes and
+// writing runs of 12 complex per site, both coalesced.  A thread per site wrote 16 bytes every
+// 192 and reached 2 TB/s; HBM bounds this one (24^3 x 32, 16 right-hand sides FP32, one half:
+// 527 -> 187 us, 150 at the measured rate; 12 right-hand sides FP64, full: 828 -> 373 us).
+constexpr int kLayoutSites = 128;
+
+template <class T> struct LayoutPlanes;
+template <> struct LayoutPlanes<double> {
+  using C = double2;
+  static __device__ __forceinline__ void load(const void* dev, const float*, size_t n5, size_t i0, int ns, C* tile, float*) {
+    const double2* p = static_cast<const double2*>(dev) + i0;
+    for (int e = threadIdx.x; e < 12 * kLayoutSites; e += 256) {
+      const int k = e / kLayoutSites, j = e - k * kLayoutSites;
+      if (j < ns) tile[j * 13 + k] = __ldg(p + size_t(k) * n5 + j);
     }
+  }
+};
+template <> struct LayoutPlanes<float> {
+  using C = float2;
+  static __device__ __forceinline__ void load(const void* dev, const float*, size_t n5, size_t i0, int ns, C* tile, float*) {
+    const float4* p = static_cast<const float4*>(dev) + (i0 >> 1);
+    for (int e = threadIdx.x; e < 12 * (kLayoutSites / 2); e += 256) {
+      const int k = e / (kLayoutSites / 2), m = e - k * (kLayoutSites / 2);
+      if (2 * m < ns) {
+        const float4 v = __ldg(p + size_t(k) * (n5 >> 1) + m);
+        tile[(2 * m) * 13 + k] = make_float2(v.x, v.z);
+        tile[(2 * m + 1) * 13 + k] = make_float2(v.y, v.w);
+      }
+    }
+  }
+};
+template <> struct LayoutPlanes<__half> {
+  using C = float2;
+  static __device__ __forceinline__ void load(const void* dev, const float* norms, size_t n5, size_t i0, int ns, C* tile,
+                                              float* scale) {
+    for (int j = threadIdx.x; j < ns; j += 256) scale[j] = __ldg(norms + i0 + j);
+    __syncthreads();
+    const uint4* p = static_cast<const uint4*>(dev) + (i0 >> 1);
+    for (int e = threadIdx.x; e < 6 * (kLayoutSites / 2); e += 256) {
+      const int q = e / (kLayoutSites / 2), m = e - q * (kLayoutSites / 2);
+      if (2 * m < ns) {
+        const uint4 v = __ldg(p + size_t(q) * (n5 >> 1) + m);
+        const __half2* h = reinterpret_cast<const __half2*>(&v);
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+          const float2 re = __half22float2(h[2 * c]), im = __half22float2(h[2 * c + 1]);
+          tile[(2 * m) * 13 + 2 * q + c] = make_float2(re.x * scale[2 * m], im.x * scale[2 * m]);
+          tile[(2 * m + 1) * 13 + 2 * q + c] = make_float2(re.y * scale[2 * m + 1], im.y * scale[2 * m + 1]);
+        }
+      }
+    }
+  }
+};
+
+template <class T, class CR>
+__global__ void __launch_bounds__(256) export_kernel(const GeoParams g, CR* canon, const void* dev, const float* devn,
+                                                     int parity, int canon_full) {
+  using P = LayoutPlanes<T>;
+  using C2 = typename Canon2<CR>::type;
+  __shared__ typename P::C tile[kLayoutSites * 13];
+  __shared__ int64_t base[kLayoutSites];  // canonical index of the site's first component
+  __shared__ float scale[kLayoutSites];
+  const size_t n5 = size_t(g.half4) * g.L5;
+  const size_t i0 = size_t(blockIdx.x) * kLayoutSites;
+  const int ns = int(min(n5 - i0, size_t(kLayoutSites)));  // even, as n5 and kLayoutSites are
+  for (int j = threadIdx.x; j < ns; j += 256) {
+    const size_t i = i0 + j;
+    const int64_t xcb = int64_t(i / g.L5);
+    const int s5 = int(i - size_t(xcb) * g.L5);
+    const int rhs = s5 / g.Ls, s = s5 - rhs * g.Ls;
+    const int64_t c4 = canon_full ? cb_to_site(xcb, parity, g) : xcb;
+    const int64_t n4c = canon_full ? g.vol4 : g.half4;
+    // the padding right-hand side is absent from the canonical array
+    base[j] = rhs < g.nrhs_user ? ((rhs * n4c + c4) * g.Ls + s) * 12 : -1;
+  }
+  P::load(dev, devn, n5, i0, ns, tile, scale);
+  __syncthreads();
+  C2* c = reinterpret_cast<C2*>(canon);
+  for (int e = threadIdx.x; e < 12 * ns; e += 256) {
+    const int j = e / 12, k = e - j * 12;
+    const int64_t at = base[j];
+    if (at >= 0) c[at + k] = canon_value(C2{}, tile[j * 13 + k]);
   }
 }
 
@@ -556,27 +645,36 @@ static GeoParams geo(const Op* op) {
   return g;
 }
 
-template <class CR, bool IMPORT>
-static int layout_p(Op* op, CR* canon, HalfView v, int parity, int canon_full) {
-  GeoParams g = geo(op);
-  const size_t n5 = op->n5();
+template <class CR> static int import_p(Op* op, const CR* canon, HalfView v, int parity, int canon_full) {
+  const GeoParams g = geo(op);
+  const unsigned blocks = nblk(op->n5());
   switch (v.prec) {
-    case GB_F64: layout_kernel<double, CR, IMPORT><<<nblk(n5), 256, 0, op->stream>>>(g, canon, v.data, v.norms, parity, canon_full); break;
-    case GB_F32: layout_kernel<float, CR, IMPORT><<<nblk(n5), 256, 0, op->stream>>>(g, canon, v.data, v.norms, parity, canon_full); break;
-    case GB_F16: layout_kernel<__half, CR, IMPORT><<<nblk(n5), 256, 0, op->stream>>>(g, canon, v.data, v.norms, parity, canon_full); break;
+    case GB_F64: import_kernel<double, CR><<<blocks, 256, 0, op->stream>>>(g, canon, v.data, v.norms, parity, canon_full); break;
+    case GB_F32: import_kernel<float, CR><<<blocks, 256, 0, op->stream>>>(g, canon, v.data, v.norms, parity, canon_full); break;
+    case GB_F16: import_kernel<__half, CR><<<blocks, 256, 0, op->stream>>>(g, canon, v.data, v.norms, parity, canon_full); break;
+  }
+  GB_CHECK_CUDA(cudaGetLastError());
+  return GB_OK;
+}
+template <class CR> static int export_p(Op* op, CR* canon, HalfView v, int parity, int canon_full) {
+  const GeoParams g = geo(op);
+  const unsigned blocks = unsigned((op->n5() + kLayoutSites - 1) / kLayoutSites);
+  switch (v.prec) {
+    case GB_F64: export_kernel<double, CR><<<blocks, 256, 0, op->stream>>>(g, canon, v.data, v.norms, parity, canon_full); break;
+    case GB_F32: export_kernel<float, CR><<<blocks, 256, 0, op->stream>>>(g, canon, v.data, v.norms, parity, canon_full); break;
+    case GB_F16: export_kernel<__half, CR><<<blocks, 256, 0, op->stream>>>(g, canon, v.data, v.norms, parity, canon_full); break;
   }
   GB_CHECK_CUDA(cudaGetLastError());
   return GB_OK;
 }
 
 int launch_import_half(Op* op, const void* canon, int canon_prec, HalfView out, int parity, int canon_is_full) {
-  if (canon_prec == GB_F32)
-    return layout_p<float, true>(op, static_cast<float*>(const_cast<void*>(canon)), out, parity, canon_is_full);
-  return layout_p<double, true>(op, static_cast<double*>(const_cast<void*>(canon)), out, parity, canon_is_full);
+  if (canon_prec == GB_F32) return import_p<float>(op, static_cast<const float*>(canon), out, parity, canon_is_full);
+  return import_p<double>(op, static_cast<const double*>(canon), out, parity, canon_is_full);
 }
 int launch_export_half(Op* op, HalfView in, void* canon, int canon_prec, int parity, int canon_is_full) {
-  if (canon_prec == GB_F32) return layout_p<float, false>(op, static_cast<float*>(canon), in, parity, canon_is_full);
-  return layout_p<double, false>(op, static_cast<double*>(canon), in, parity, canon_is_full);
+  if (canon_prec == GB_F32) return export_p<float>(op, static_cast<float*>(canon), in, parity, canon_is_full);
+  return export_p<double>(op, static_cast<double*>(canon), in, parity, canon_is_full);
 }
 
 // ---------------------------------------------------------------------------------------
