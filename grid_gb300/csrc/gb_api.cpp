@@ -191,8 +191,7 @@ int field_norm2_dev(Field* f, double* d_out) {
   Op* op = f->op;
   const int g = red_parts(op, f->prec);
   const int halves = f->full() ? 2 : 1;
-  for (int h = 0; h < halves; h++)
-    GB_TRY(launch_norm2_partial(op, half_view(f, h), f->n5, op->d_partial + size_t(h) * g * op->nrhs));
+  GB_TRY(launch_norm2_partial(op, half_view(f, 0), f->n5, op->d_partial, halves));
   return launch_reduce_final(op, op->d_partial, g * halves, 1, d_out);
 }
 
@@ -200,8 +199,7 @@ int field_inner_dev(Field* a, Field* b, double* d_out) {
   Op* op = a->op;
   const int g = red_parts(op, a->prec);
   const int halves = a->full() ? 2 : 1;
-  for (int h = 0; h < halves; h++)
-    GB_TRY(launch_inner_partial(op, half_view(a, h), half_view(b, h), a->n5, op->d_partial + size_t(h) * g * op->nrhs * 2));
+  GB_TRY(launch_inner_partial(op, half_view(a, 0), half_view(b, 0), a->n5, op->d_partial, halves));
   return launch_reduce_final(op, op->d_partial, g * halves, 2, d_out);
 }
 
@@ -222,15 +220,10 @@ int field_inner(Field* a, Field* b, double* out) {
 }
 
 int field_axpby(Field* z, double a, double b, Field* x, Field* y) {
-  const int halves = z->full() ? 2 : 1;
-  for (int h = 0; h < halves; h++)
-    GB_TRY(launch_axpby(z->op, half_view(z, h), a, half_view(x, h), b, half_view(y, h), z->n5));
-  return GB_OK;
+  return launch_axpby(z->op, half_view(z, 0), a, half_view(x, 0), b, half_view(y, 0), z->n5, z->full() ? 2 : 1);
 }
 int field_scale(Field* z, double a, Field* x) {
-  const int halves = z->full() ? 2 : 1;
-  for (int h = 0; h < halves; h++) GB_TRY(launch_scale(z->op, half_view(z, h), a, half_view(x, h), z->n5));
-  return GB_OK;
+  return launch_scale(z->op, half_view(z, 0), a, half_view(x, 0), z->n5, z->full() ? 2 : 1);
 }
 int field_copy(Field* dst, Field* src) {
   if (dst == src) return GB_OK;
@@ -417,6 +410,28 @@ int op_dhop_full(Op* op, Field* in, Field* out, int dag) {
   return launch_dhop_full(op, half_view(in, 1), half_view(out, 0), half_view(in, 0), half_view(out, 1), dag);
 }
 
+// out = c0 z + c1 Dhop(in): one launch where the operator's kernel has the form, else two
+static int op_dhop_full_axpy(Op* op, Field* in, Field* z, Field* out, double c0, double c1, int dag) {
+  if (!in->full() || !out->full()) { set_error("Dhop: full fields expected"); return GB_ERR_BAD_PARITY; }
+  int done = 0;
+  const DhopAxpy a{{half_view(z, 0), half_view(z, 1)}, c0, c1};
+  GB_TRY(launch_dhop_full_axpy(op, half_view(in, 1), half_view(out, 0), half_view(in, 0), half_view(out, 1), dag, a, &done));
+  if (done) return GB_OK;
+  GB_TRY(op_dhop_full(op, in, out, dag));
+  return field_axpby(out, c1, c0, out, z);
+}
+int op_dhop_cb_axpy(Op* op, Field* in, Field* z, Field* out, double c0, double c1, int dag) {
+  if (in->full() || out->full()) { set_error("DhopEO/OE: half fields expected"); return GB_ERR_BAD_PARITY; }
+  int done = 0;
+  const int p = in->subset;
+  const DhopAxpy a{{half_view(z, 0), half_view(z, 0)}, c0, c1};
+  GB_TRY(launch_dhop_axpy(op, half_view(in, 0), half_view(out, 0), 1 - p, dag, a, &done));
+  out->subset = 1 - p;
+  if (done) return GB_OK;
+  GB_TRY(op_dhop_cb(op, in, out, dag));
+  return field_axpby(out, c1, c0, out, z);
+}
+
 int op_meooe(Op* op, Field* in, Field* out, int dag) {
   if (in->full()) { set_error("Meooe: half field expected"); return GB_ERR_BAD_PARITY; }
   if (op->kind == 0) return op_dhop_cb(op, in, out, dag);
@@ -431,6 +446,15 @@ int op_meooe(Op* op, Field* in, Field* out, int dag) {
   GB_TRY(op_dhop_cb(op, in, t, 1));
   out->subset = 1 - in->subset;
   return op_meooe5d(op, t, out, 1);
+}
+
+int op_meooe_from(Op* op, Field* in, Field* z, Field* out) {
+  if (in->full()) { set_error("Meooe: half field expected"); return GB_ERR_BAD_PARITY; }
+  if (op->kind == 0) return op_dhop_cb_axpy(op, in, z, out, 1.0, -1.0, 0);
+  Field* t;
+  GB_TRY(ws_get(op, in->subset, in->prec, WS_MEOOE_A, &t));
+  GB_TRY(op_meooe5d(op, in, t, 0));
+  return op_dhop_cb_axpy(op, t, z, out, 1.0, -1.0, 0);
 }
 
 // the per-slot chiral diagonal of a twisted-mass operator (WilsonTMFermion5D.h:82-135):
@@ -503,6 +527,13 @@ int op_mpc(Op* op, Field* in, Field* out, int dag, int* norm_parts, Field* r_upd
   if (in->subset != GB_ODD) { set_error("Mpc: odd checkerboard expected"); return GB_ERR_BAD_PARITY; }
   Field *te1, *te2, *to;
   GB_TRY(ws_get(op, GB_EVEN, in->prec, WS_MPC_E1, &te1));
+  if (op->kind == 0 && !op->tm) {
+    // Wilson: Mooee = d and MooeeInv = 1/d are numbers, which ride on the second Dhop:
+    // out = d in - (1/d) DhopOE DhopEO in
+    te1->subset = GB_EVEN;
+    GB_TRY(op_dhop_cb(op, in, te1, dag));
+    return op_dhop_cb_axpy(op, te1, in, out, op->diag_mass, -1.0 / op->diag_mass, dag);
+  }
   GB_TRY(ws_get(op, GB_EVEN, in->prec, WS_MPC_E2, &te2));
   GB_TRY(ws_get(op, GB_ODD, in->prec, WS_MPC_O, &to));
   if (col_available(op, in->prec)) {
@@ -560,9 +591,9 @@ int op_mpcdagmpc(Op* op, Field* in, Field* out) {
 int op_m(Op* op, Field* in, Field* out, int dag) {
   if (!in->full() || !out->full()) { set_error("M: full fields expected"); return GB_ERR_BAD_PARITY; }
   if (op->kind == 0) {
+    if (!op->tm) return op_dhop_full_axpy(op, in, in, out, op->diag_mass, 1.0, dag);
     GB_TRY(op_dhop_full(op, in, out, dag));
-    if (op->tm) return tm_diag(op, in, out, dag, 0, out, 1.0);  // out = Mooee in + Dhop in
-    return field_axpby(out, 1.0, op->diag_mass, out, in);
+    return tm_diag(op, in, out, dag, 0, out, 1.0);  // out = Mooee in + Dhop in
   }
   Field* Din;
   GB_TRY(ws_get(op, GB_FULL, in->prec, WS_M_DIN, &Din));
@@ -572,12 +603,10 @@ int op_m(Op* op, Field* in, Field* out, int dag) {
   coeffs_m5d_unit(op, l, d, u);
   if (!dag) {
     GB_TRY(op_meooe5d(op, in, Din, 0));            // Din = Meooe5D psi
-    GB_TRY(op_dhop_full(op, Din, t, 0));           // t = Dhop Din
-    GB_TRY(field_axpby(t, 1.0, 4.0 - op->M5, t, Din));  // t = DW Din
+    GB_TRY(op_dhop_full_axpy(op, Din, Din, t, 4.0 - op->M5, 1.0, 0));  // t = DW Din = Dhop Din + (4 - M5) Din
     return m5d_field(op, in, t, out, l, d, u, 0, in, 1.0);  // out = M5D(psi, t) + psi
   }
-  GB_TRY(op_dhop_full(op, in, t, 1));
-  GB_TRY(field_axpby(t, 1.0, 4.0 - op->M5, t, in));   // t = DW^dag psi
+  GB_TRY(op_dhop_full_axpy(op, in, in, t, 4.0 - op->M5, 1.0, 1));  // t = DW^dag psi
   GB_TRY(op_meooe5d(op, t, Din, 1));               // Din = MeooeDag5D t
   return m5d_field(op, in, Din, out, l, d, u, 1, in, 1.0);  // out = M5Ddag(psi, Din) + psi
 }
@@ -595,18 +624,17 @@ int op_mdagm(Op* op, Field* in, Field* out, Field** m_in) {
 int op_dminus(Op* op, Field* in, Field* out, int dag) {
   if (op->kind != 1) { set_error("Dminus: Moebius operators only"); return GB_ERR_UNSUPPORTED; }
   if (!in->full() || !out->full()) { set_error("Dminus: full fields expected"); return GB_ERR_BAD_PARITY; }
-  Field* t;
-  GB_TRY(ws_get(op, GB_FULL, in->prec, WS_DMINUS, &t));
-  GB_TRY(op_dhop_full(op, in, t, dag));
   if (op->zmobius) {  // chi_s = psi_s - cs_s (DW psi)_s, conj(cs_s) for the dagger
-    GB_TRY(field_axpby(t, 1.0, 4.0 - op->M5, t, in));
+    Field* t;
+    GB_TRY(ws_get(op, GB_FULL, in->prec, WS_DMINUS, &t));
+    GB_TRY(op_dhop_full_axpy(op, in, in, t, 4.0 - op->M5, 1.0, dag));
     ZCoefsHost h;
     h.e.resize(op->Ls);
     for (int s = 0; s < op->Ls; s++) h.e[s] = dag ? -std::conj(op->zcs[s]) : -op->zcs[s];
     return zcol_field(op, ZPROG_DIAG, dag, in, t, out, 0.0, h);
   }
   const double c = op->cs[0];
-  return field_axpby(out, 1.0 - c * (4.0 - op->M5), -c, in, t);
+  return op_dhop_full_axpy(op, in, in, out, 1.0 - c * (4.0 - op->M5), -c, dag);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -791,7 +819,7 @@ static int op_create(int kind, const int dims[4], int Ls, double mass, double M5
   alloc(reinterpret_cast<void**>(&op->d_partial), op->partial_doubles * sizeof(double));
   alloc(reinterpret_cast<void**>(&op->d_result), size_t(nrhs) * 8 * sizeof(double));
   alloc(reinterpret_cast<void**>(&op->d_cg), size_t(nrhs) * sizeof(CGScalars));
-  alloc(reinterpret_cast<void**>(&op->d_all_done), 4 * sizeof(int));
+  alloc(reinterpret_cast<void**>(&op->d_all_done), 8 * sizeof(int));
   if (rc == GB_OK && !(op->h_result = static_cast<double*>(pinned_get(size_t(nrhs) * 8 * sizeof(double))))) rc = GB_ERR_OOM;
   if (rc == GB_OK && !(op->h_cg = static_cast<CGScalars*>(pinned_get(size_t(nrhs) * sizeof(CGScalars) + 64)))) rc = GB_ERR_OOM;
   if (rc == GB_OK && cudaMemsetAsync(op->d_err, 0, sizeof(int), op->stream) != cudaSuccess) rc = GB_ERR_CUDA;
@@ -835,20 +863,10 @@ size_t field_host_doubles(const Field* f) {
 }
 
 int field_import_dev(Field* f, const void* dev, int canon_prec) {
-  if (f->full()) {
-    for (int p = 0; p < 2; p++) GB_TRY(launch_import_half(f->op, dev, canon_prec, half_view(f, p), p, 1));
-  } else {
-    GB_TRY(launch_import_half(f->op, dev, canon_prec, half_view(f, 0), f->subset, 0));
-  }
-  return GB_OK;
+  return launch_import(f->op, dev, canon_prec, half_view(f, 0), f->full() ? 1 : 0);
 }
 int field_export_dev(Field* f, void* dev, int canon_prec) {
-  if (f->full()) {
-    for (int p = 0; p < 2; p++) GB_TRY(launch_export_half(f->op, half_view(f, p), dev, canon_prec, p, 1));
-  } else {
-    GB_TRY(launch_export_half(f->op, half_view(f, 0), dev, canon_prec, f->subset, 0));
-  }
-  return GB_OK;
+  return launch_export(f->op, half_view(f, 0), dev, canon_prec, f->full() ? 1 : 0);
 }
 
 int check_device_error(Op* op) {
@@ -1178,9 +1196,7 @@ int gb_field_axpy_norm(gb_field_t z, double a, gb_field_t x, gb_field_t y, doubl
   z->subset = x->subset;
   const int g = red_parts(op, z->prec);
   const int halves = z->full() ? 2 : 1;
-  for (int h = 0; h < halves; h++)
-    GB_TRY(launch_axpy_norm_partial(op, half_view(z, h), a, half_view(x, h), half_view(y, h), z->n5,
-                                    op->d_partial + size_t(h) * g * op->nrhs));
+  GB_TRY(launch_axpy_norm_partial(op, half_view(z, 0), a, half_view(x, 0), half_view(y, 0), z->n5, op->d_partial, halves));
   GB_TRY(launch_reduce_final(op, op->d_partial, g * halves, 1, op->d_result));
   std::vector<double> v(op->nrhs);
   GB_TRY(fetch(op, op->d_result, v.data(), op->nrhs));

@@ -14,28 +14,21 @@ namespace gb {
 // ---------------------------------------------------------------------------------------
 // Elementwise: z = a x + b y ; copy with precision change ; zero
 // ---------------------------------------------------------------------------------------
-template <class TZ, class TX, class TY>
-__global__ void __launch_bounds__(256) axpby_kernel(void* z, float* zn, double a, const void* x, const float* xn, double b,
-                                                    const void* y, const float* yn, size_t n5, int use_y) {
-  using R = typename Arith<TZ>::type;
+// FP64 z = a x [+ b y] on the 16-byte words of one or both checkerboards.  One word per thread: a
+// site per thread (24 values at 2 FP64 lanes per clock and SM) left a small lattice on few SMs,
+// 6.0 us at 8^4 whatever the launch did.
+template <bool USE_Y>
+__global__ void __launch_bounds__(256) axpby_kernel(double2* z, double a, const double2* x, double b, const double2* y,
+                                                    size_t words) {
   const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= n5) return;
-  Spinor<typename Arith<TX>::type> fx;
-  SpinorIO<TX>::load(x, xn, n5, i, fx);
-  Spinor<R> o;
-  if (use_y) {
-    Spinor<typename Arith<TY>::type> fy;
-    SpinorIO<TY>::load(y, yn, n5, i, fy);
-#pragma unroll
-    for (int k = 0; k < 12; k++) {
-      o.re[k] = R(a) * R(fx.re[k]) + R(b) * R(fy.re[k]);
-      o.im[k] = R(a) * R(fx.im[k]) + R(b) * R(fy.im[k]);
-    }
-  } else {
-#pragma unroll
-    for (int k = 0; k < 12; k++) { o.re[k] = R(a) * R(fx.re[k]); o.im[k] = R(a) * R(fx.im[k]); }
+  if (i >= words) return;
+  const double2 v = x[i];
+  double2 o = make_double2(a * v.x, a * v.y);
+  if (USE_Y) {
+    const double2 w = y[i];
+    o = make_double2(fma(a, v.x, b * w.x), fma(a, v.y, b * w.y));
   }
-  SpinorIO<TZ>::store(z, zn, n5, i, o);
+  z[i] = o;
 }
 
 template <class TZ, class TX>
@@ -53,30 +46,31 @@ __global__ void __launch_bounds__(256) convert_kernel(void* z, float* zn, const 
 
 static inline unsigned nblk(size_t n) { return unsigned((n + 255) / 256); }
 
-template <class TZ, class TX, class TY>
-static int axpby_t(Op* op, HalfView z, double a, HalfView x, double b, HalfView y, size_t n5, int use_y) {
-  axpby_kernel<TZ, TX, TY><<<nblk(n5), 256, 0, op->stream>>>(z.data, z.norms, a, x.data, x.norms, b, y.data, y.norms,
-                                                            n5, use_y);
-  GB_CHECK_CUDA(cudaGetLastError());
-  return GB_OK;
-}
-
-int launch_axpby(Op* op, HalfView z, double a, HalfView x, double b, HalfView y, size_t n5) {
+int launch_axpby(Op* op, HalfView z, double a, HalfView x, double b, HalfView y, size_t n5, int halves) {
   if (x.prec != z.prec || y.prec != z.prec) {
     set_error("axpby: mixed precisions");
     return GB_ERR_BAD_ARG;
   }
-  if (z.prec != GB_F64) return launch_axpby_pair(op, z, a, x, b, y, n5, 1);
-  return axpby_t<double, double, double>(op, z, a, x, b, y, n5, 1);
+  if (z.prec != GB_F64) return launch_axpby_pair(op, z, a, x, b, y, n5, 1, halves);
+  const size_t words = n5 * 12 * halves;
+  axpby_kernel<true><<<nblk(words), 256, 0, op->stream>>>(static_cast<double2*>(z.data), a,
+                                                          static_cast<const double2*>(x.data), b,
+                                                          static_cast<const double2*>(y.data), words);
+  GB_CHECK_CUDA(cudaGetLastError());
+  return GB_OK;
 }
 
-int launch_scale(Op* op, HalfView z, double a, HalfView x, size_t n5) {
+int launch_scale(Op* op, HalfView z, double a, HalfView x, size_t n5, int halves) {
   if (x.prec != z.prec) {
     set_error("scale: mixed precisions");
     return GB_ERR_BAD_ARG;
   }
-  if (z.prec != GB_F64) return launch_axpby_pair(op, z, a, x, 0.0, x, n5, 0);
-  return axpby_t<double, double, double>(op, z, a, x, 0, x, n5, 0);
+  if (z.prec != GB_F64) return launch_axpby_pair(op, z, a, x, 0.0, x, n5, 0, halves);
+  const size_t words = n5 * 12 * halves;
+  axpby_kernel<false><<<nblk(words), 256, 0, op->stream>>>(static_cast<double2*>(z.data), a,
+                                                           static_cast<const double2*>(x.data), 0.0, nullptr, words);
+  GB_CHECK_CUDA(cudaGetLastError());
+  return GB_OK;
 }
 
 template <class TZ, class TX> static int convert_t(Op* op, HalfView z, HalfView x, size_t n5) {
@@ -125,6 +119,11 @@ __global__ void __launch_bounds__(256) reduce_kernel(const RedShape sh, const vo
                                                      const CGScalars* cg, size_t n5, double* partial) {
   using R = typename Arith<T>::type;
   constexpr int NV = KIND == 1 ? 2 : 1;
+  const size_t half = size_t(blockIdx.y) * n5 * 12 * sizeof(double2);  // blockIdx.y: the checkerboard
+  x = static_cast<const char*>(x) + half;
+  y = static_cast<const char*>(y) + half;
+  z = static_cast<char*>(z) + half;
+  partial += size_t(blockIdx.y) * gridDim.x * sh.nrhs * NV;
   double v[NV];
 #pragma unroll
   for (int k = 0; k < NV; k++) v[k] = 0.0;
@@ -181,6 +180,9 @@ int red_grid(Op* op, size_t n5, int* blocks, int* threads) {
     set_error("reduction: FP64 fields with L5 = %d above 256 are not supported", L5);
     return GB_ERR_UNSUPPORTED;
   }
+  // small fields: CTAs down to two warps (multiples of L5 still), so that the FP64 sums of a site
+  // per thread spread over the SMs
+  while (B > 64 && (n5 + B - 1) / B < 152 && (B / 2) % 32 == 0 && (op->nrhs == 1 || (B / 2) % L5 == 0)) B /= 2;
   size_t need = (n5 + B - 1) / B;
   int g = int(need < size_t(kRedBlocks) ? need : size_t(kRedBlocks));
   if (g < 1) g = 1;
@@ -190,13 +192,13 @@ int red_grid(Op* op, size_t n5, int* blocks, int* threads) {
 }
 
 template <class T, int KIND>
-static int reduce_t(Op* op, HalfView x, HalfView y, HalfView z, double a, size_t n5, double* partial) {
+static int reduce_t(Op* op, HalfView x, HalfView y, HalfView z, double a, size_t n5, double* partial, int halves) {
   int g, B;
   GB_TRY(red_grid(op, n5, &g, &B));
   RedShape sh{op->L5, op->Ls, op->nrhs};
   const int NV = KIND == 1 ? 2 : 1;
   size_t smem = size_t(NV) * (op->nrhs == 1 ? 32 : B) * sizeof(double);
-  reduce_kernel<T, KIND><<<g, B, smem, op->stream>>>(sh, x.data, x.norms, y.data, y.norms, z.data, z.norms, a, op->d_cg,
+  reduce_kernel<T, KIND><<<dim3(g, halves), B, smem, op->stream>>>(sh, x.data, x.norms, y.data, y.norms, z.data, z.norms, a, op->d_cg,
                                                      n5, partial);
   GB_CHECK_CUDA(cudaGetLastError());
   return GB_OK;
@@ -204,26 +206,26 @@ static int reduce_t(Op* op, HalfView x, HalfView y, HalfView z, double a, size_t
 
 // FP32 / FP16 fields reduce through the pair kernels (gb_pair.cu), whose partial count
 // red_parts() reports; FP64 through reduce_kernel
-int launch_norm2_partial(Op* op, HalfView x, size_t n5, double* partial) {
-  if (x.prec != GB_F64) return launch_reduce_pair(op, 0, x, x, x, 0.0, n5, partial);
-  return reduce_t<double, 0>(op, x, x, x, 0.0, n5, partial);
+int launch_norm2_partial(Op* op, HalfView x, size_t n5, double* partial, int halves) {
+  if (x.prec != GB_F64) return launch_reduce_pair(op, 0, x, x, x, 0.0, n5, partial, halves);
+  return reduce_t<double, 0>(op, x, x, x, 0.0, n5, partial, halves);
 }
-int launch_inner_partial(Op* op, HalfView a, HalfView b, size_t n5, double* partial) {
+int launch_inner_partial(Op* op, HalfView a, HalfView b, size_t n5, double* partial, int halves) {
   if (a.prec != b.prec) { set_error("innerProduct: mixed precisions"); return GB_ERR_BAD_ARG; }
-  if (a.prec != GB_F64) return launch_reduce_pair(op, 1, a, b, a, 0.0, n5, partial);
-  return reduce_t<double, 1>(op, a, b, a, 0.0, n5, partial);
+  if (a.prec != GB_F64) return launch_reduce_pair(op, 1, a, b, a, 0.0, n5, partial, halves);
+  return reduce_t<double, 1>(op, a, b, a, 0.0, n5, partial, halves);
 }
 // z = a x + y, |z|^2
-int launch_axpy_norm_partial(Op* op, HalfView z, double a, HalfView x, HalfView y, size_t n5, double* partial) {
+int launch_axpy_norm_partial(Op* op, HalfView z, double a, HalfView x, HalfView y, size_t n5, double* partial, int halves) {
   if (x.prec != y.prec || z.prec != x.prec) { set_error("axpy_norm: mixed precisions"); return GB_ERR_BAD_ARG; }
-  if (x.prec != GB_F64) return launch_reduce_pair(op, 2, x, y, z, a, n5, partial);
-  return reduce_t<double, 2>(op, x, y, z, a, n5, partial);
+  if (x.prec != GB_F64) return launch_reduce_pair(op, 2, x, y, z, a, n5, partial, halves);
+  return reduce_t<double, 2>(op, x, y, z, a, n5, partial, halves);
 }
 // r -= a[rhs] mmp, |r|^2: Grid's axpy_norm(r, -a, mmp, r) with the device CG scalars
-int launch_cg_r_update(Op* op, HalfView r, HalfView mmp, size_t n5, double* partial) {
+int launch_cg_r_update(Op* op, HalfView r, HalfView mmp, size_t n5, double* partial, int halves) {
   if (r.prec != mmp.prec) { set_error("CG update: mixed precisions"); return GB_ERR_BAD_ARG; }
-  if (r.prec != GB_F64) return launch_reduce_pair(op, 3, mmp, r, r, 0.0, n5, partial);
-  return reduce_t<double, 3>(op, mmp, r, r, 0.0, n5, partial);
+  if (r.prec != GB_F64) return launch_reduce_pair(op, 3, mmp, r, r, 0.0, n5, partial, halves);
+  return reduce_t<double, 3>(op, mmp, r, r, 0.0, n5, partial, halves);
 }
 
 // partial: [nparts][nrhs][nv] -> out[nrhs][nv]; one CTA per rhs, fixed summation order
@@ -283,68 +285,74 @@ __global__ void cg_init_kernel(CGScalars* cg, const double* ssq, const double* c
     if (s.done) atomicAdd(&nd, 1);
   }
   __syncthreads();
-  if (r == 0) { flags[0] = (nd == nrhs); flags[1] = 0; }
+  if (r == 0) { flags[0] = (nd == nrhs); flags[1] = 0; flags[4] = 0; }
 }
 
-// sum over b of partial[b * stride + offset] by one CTA (a power of two, at most 1024
-// threads) in a fixed order (strided per-thread sums, then a tree); every thread gets the
-// result
+// sum over b of partial[b * stride + offset] by one CTA (whole warps, at most 1024 threads) in a
+// fixed order (strided per-thread sums, then shuffles); the result is thread 0's
 __device__ double cta_sum_fixed(const double* partial, int nparts, int stride, int offset) {
-  __shared__ double sm[1024];
+  __shared__ double sm[32];
   double s = 0;
   // unrolled so that several loads are in flight before the (ordered) adds
 #pragma unroll 8
   for (int b = threadIdx.x; b < nparts; b += blockDim.x) s += partial[size_t(b) * stride + offset];
-  sm[threadIdx.x] = s;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
   __syncthreads();
-  for (int st = blockDim.x / 2; st > 0; st >>= 1) {
-    if (threadIdx.x < st) sm[threadIdx.x] += sm[threadIdx.x + st];
-    __syncthreads();
+  if (threadIdx.x < 32) {
+    s = threadIdx.x < (blockDim.x >> 5) ? sm[threadIdx.x] : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
   }
-  const double r = sm[0];
-  __syncthreads();
-  return r;
+  return s;
 }
 
-// launched with 256 threads, 1024 above 2048 partial sums (one per CTA of an FP32 Dhop):
-// the partial sums of every right-hand side are reduced by the whole CTA (a single thread
-// walking thousands of partials would take ~100 us)
+// One CTA per right-hand side (one CTA for all took 26-30 us at 12 right-hand sides), of 256
+// threads, 1024 above 2048 partial sums (one per CTA of an FP32 Dhop)
 __global__ void __launch_bounds__(1024) cg_alpha_kernel(CGScalars* cg, const double* partial, int nparts, int nrhs,
                                                        int nv) {
-  for (int r = 0; r < nrhs; r++) {
-    const double d = cta_sum_fixed(partial, nparts, nrhs * nv, r * nv);
-    if (threadIdx.x == 0) {
-      cg[r].d = d;
-      cg[r].a = cg[r].done ? 0.0 : cg[r].c / d;
-    }
+  const int r = blockIdx.x;
+  const double d = cta_sum_fixed(partial, nparts, nrhs * nv, r * nv);
+  if (threadIdx.x == 0) {
+    cg[r].d = d;
+    cg[r].a = cg[r].done ? 0.0 : cg[r].c / d;
   }
 }
 
+// flags[4] counts the CTAs that have written their right-hand side: the last one sets the flags of
+// the whole solve and leaves the count at zero
 __global__ void __launch_bounds__(1024) cg_beta_kernel(CGScalars* cg, const double* partial, int nparts, int nrhs,
                                                       int* flags) {
-  int nd = 0, nr = 0;
-  for (int r = 0; r < nrhs; r++) {
-    const double cp = cta_sum_fixed(partial, nparts, nrhs, r);
-    if (threadIdx.x == 0) {
-      CGScalars s = cg[r];
-      if (!s.done) {
-        s.cp = cp;
-        s.b = cp / s.c;
-        s.cprev = s.c;
-        s.c = cp;
-        s.iter += 1;
-        if (cp > s.maxres) s.maxres = cp;
-        if (cp <= s.rsq) s.done = 1;
-        else if (cp < s.delta * s.maxres) s.relup = 1;
-      } else {
-        s.b = 0.0;
-      }
-      cg[r] = s;
-      nd += s.done;
-      nr += (s.relup && !s.done);
-    }
+  const int r = blockIdx.x;
+  const double cp = cta_sum_fixed(partial, nparts, nrhs, r);
+  if (threadIdx.x != 0) return;
+  CGScalars s = cg[r];
+  if (!s.done) {
+    s.cp = cp;
+    s.b = cp / s.c;
+    s.cprev = s.c;
+    s.c = cp;
+    s.iter += 1;
+    if (cp > s.maxres) s.maxres = cp;
+    if (cp <= s.rsq) s.done = 1;
+    else if (cp < s.delta * s.maxres) s.relup = 1;
+  } else {
+    s.b = 0.0;
   }
-  if (threadIdx.x == 0) { flags[0] = (nd == nrhs); flags[1] = nr; }
+  cg[r] = s;
+  __threadfence();
+  if (atomicAdd(flags + 4, 1) != nrhs - 1) return;
+  __threadfence();
+  int nd = 0, nr = 0;
+  for (int k = 0; k < nrhs; k++) {
+    const int done = __ldcg(&cg[k].done), relup = __ldcg(&cg[k].relup);
+    nd += done;
+    nr += relup && !done;
+  }
+  flags[0] = nd == nrhs;
+  flags[1] = nr;
+  flags[4] = 0;
 }
 
 __global__ void cg_relup_reset_kernel(CGScalars* cg, const double* cp_true, int nrhs) {
@@ -371,7 +379,7 @@ int launch_cg_init(Op* op, const double* d_ssq, const double* d_cp, double tol, 
 // the scalar kernels reduce the per-block partial sums themselves, in a fixed order
 static inline int sum_threads(int nparts) { return nparts > 2048 ? 1024 : 256; }
 int launch_cg_alpha(Op* op, const double* partial, int nparts, int nv) {
-  cg_alpha_kernel<<<1, sum_threads(nparts), 0, op->stream>>>(op->d_cg, partial, nparts, op->nrhs, nv);
+  cg_alpha_kernel<<<op->nrhs, sum_threads(nparts), 0, op->stream>>>(op->d_cg, partial, nparts, op->nrhs, nv);
   GB_CHECK_CUDA(cudaGetLastError());
   return GB_OK;
 }
@@ -400,7 +408,7 @@ int launch_cg_loop_check(Op* op, cudaGraphConditionalHandle h) {
 }
 
 int launch_cg_beta(Op* op, const double* partial_norm, int nparts) {
-  cg_beta_kernel<<<1, sum_threads(nparts), 0, op->stream>>>(op->d_cg, partial_norm, nparts, op->nrhs, op->d_all_done);
+  cg_beta_kernel<<<op->nrhs, sum_threads(nparts), 0, op->stream>>>(op->d_cg, partial_norm, nparts, op->nrhs, op->d_all_done);
   GB_CHECK_CUDA(cudaGetLastError());
   return GB_OK;
 }
@@ -410,36 +418,29 @@ int launch_cg_relup_reset(Op* op, const double* d_cp_true) {
   return GB_OK;
 }
 
-// p = b p + r   (the second line of ConjugateGradient.h:175-183)
-template <class T>
-__global__ void __launch_bounds__(256) cg_p_kernel(const RedShape sh, void* p, float* pn, const void* r, const float* rn,
-                                                   const CGScalars* cg, size_t n5) {
-  using R = typename Arith<T>::type;
+// p = b p + r (the second line of ConjugateGradient.h:175-183) on FP64 fields; blockIdx.y: the plane,
+// over both checkerboards of a full field
+__global__ void __launch_bounds__(256) cg_p_kernel(const RedShape sh, double2* p, const double2* r, const CGScalars* cg,
+                                                   size_t n5) {
   const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n5) return;
-  const int rhs = int(i % sh.L5) / sh.Ls;
-  const R b = R(cg[rhs].b);
-  Spinor<R> fp, fr;
-  SpinorIO<T>::load(p, pn, n5, i, fp);
-  SpinorIO<T>::load(r, rn, n5, i, fr);
-#pragma unroll
-  for (int k = 0; k < 12; k++) {
-    fp.re[k] = fma(b, fp.re[k], fr.re[k]);
-    fp.im[k] = fma(b, fp.im[k], fr.im[k]);
-  }
-  SpinorIO<T>::store(p, pn, n5, i, fp);
+  const double b = cg[int(i % sh.L5) / sh.Ls].b;
+  const size_t w = size_t(blockIdx.y) * n5 + i;
+  const double2 pk = p[w], rk = r[w];
+  p[w] = make_double2(fma(b, pk.x, rk.x), fma(b, pk.y, rk.y));
 }
 
-int launch_cg_p_update(Op* op, HalfView p, HalfView r, size_t n5) {
-  if (p.prec != GB_F64) return launch_cg_p_pair(op, p, r, n5);
+int launch_cg_p_update(Op* op, HalfView p, HalfView r, size_t n5, int halves) {
+  if (p.prec != GB_F64) return launch_cg_p_pair(op, p, r, n5, halves);
   RedShape sh{op->L5, op->Ls, op->nrhs};
-  cg_p_kernel<double><<<nblk(n5), 256, 0, op->stream>>>(sh, p.data, p.norms, r.data, r.norms, op->d_cg, n5);
+  cg_p_kernel<<<dim3(nblk(n5), 12 * halves), 256, 0, op->stream>>>(sh, static_cast<double2*>(p.data),
+                                                                  static_cast<const double2*>(r.data), op->d_cg, n5);
   GB_CHECK_CUDA(cudaGetLastError());
   return GB_OK;
 }
 
 // psi += a p, then (PUPD) p = b p + r: the CG's linear combination after the residual
-// update (ConjugateGradient.h:174-183), FP64 fields
+// update (ConjugateGradient.h:174-183), FP64 fields, a word per thread as cg_p_kernel
 template <bool PUPD>
 __global__ void __launch_bounds__(256) cg_xp_kernel(const RedShape sh, double2* psi, double2* p, const double2* r,
                                                     const CGScalars* cg, size_t n5) {
@@ -447,30 +448,29 @@ __global__ void __launch_bounds__(256) cg_xp_kernel(const RedShape sh, double2* 
   if (i >= n5) return;
   const CGScalars& c = cg[int(i % sh.L5) / sh.Ls];
   const double a = c.a, b = c.b;
-#pragma unroll
-  for (int k = 0; k < 12; k++) {
-    const double2 pk = p[size_t(k) * n5 + i];
-    double2 x = psi[size_t(k) * n5 + i];
-    x.x = fma(a, pk.x, x.x);
-    x.y = fma(a, pk.y, x.y);
-    psi[size_t(k) * n5 + i] = x;
-    if (PUPD) {
-      const double2 rk = r[size_t(k) * n5 + i];
-      p[size_t(k) * n5 + i] = make_double2(fma(b, pk.x, rk.x), fma(b, pk.y, rk.y));
-    }
+  const size_t w = size_t(blockIdx.y) * n5 + i;
+  const double2 pk = p[w];
+  double2 x = psi[w];
+  x.x = fma(a, pk.x, x.x);
+  x.y = fma(a, pk.y, x.y);
+  psi[w] = x;
+  if (PUPD) {
+    const double2 rk = r[w];
+    p[w] = make_double2(fma(b, pk.x, rk.x), fma(b, pk.y, rk.y));
   }
 }
 
-int launch_cg_xp_update(Op* op, HalfView psi, HalfView p, HalfView r, size_t n5, int update_p) {
+int launch_cg_xp_update(Op* op, HalfView psi, HalfView p, HalfView r, size_t n5, int update_p, int halves) {
   if (p.prec != r.prec) { set_error("CG update: mixed precisions"); return GB_ERR_BAD_ARG; }
-  if (p.prec != GB_F64) return launch_cg_xp_pair(op, psi, p, r, n5, update_p);
+  if (p.prec != GB_F64) return launch_cg_xp_pair(op, psi, p, r, n5, update_p, halves);
   if (psi.prec != GB_F64) { set_error("CG update: FP64 fields expected"); return GB_ERR_BAD_ARG; }
   RedShape sh{op->L5, op->Ls, op->nrhs};
   auto* x = static_cast<double2*>(psi.data);
   auto* pp = static_cast<double2*>(p.data);
   auto* rr = static_cast<const double2*>(r.data);
-  if (update_p) cg_xp_kernel<true><<<nblk(n5), 256, 0, op->stream>>>(sh, x, pp, rr, op->d_cg, n5);
-  else cg_xp_kernel<false><<<nblk(n5), 256, 0, op->stream>>>(sh, x, pp, rr, op->d_cg, n5);
+  const dim3 grid(nblk(n5), 12 * halves);
+  if (update_p) cg_xp_kernel<true><<<grid, 256, 0, op->stream>>>(sh, x, pp, rr, op->d_cg, n5);
+  else cg_xp_kernel<false><<<grid, 256, 0, op->stream>>>(sh, x, pp, rr, op->d_cg, n5);
   GB_CHECK_CUDA(cudaGetLastError());
   return GB_OK;
 }
@@ -505,20 +505,22 @@ template <> struct Canon2<float> { using type = float2; };
 // canonical -> device planes, one thread per 5D site (its 12 reads share their lines in L1; through
 // a shared tile as the export it measured 3-20 % slower)
 template <class T, class CR>
-__global__ void __launch_bounds__(256) import_kernel(const GeoParams g, const CR* canon, void* dev, float* devn, int parity,
-                                                     int canon_full) {
+__global__ void __launch_bounds__(256) import_kernel(const GeoParams g, const CR* canon, void* dev, float* devn, int full) {
   using R = typename Arith<T>::type;
   using C2 = typename Canon2<CR>::type;
   const size_t n5 = size_t(g.half4) * g.L5;
   const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n5) return;
+  const int parity = blockIdx.y;
+  dev = static_cast<char*>(dev) + parity * n5 * (sizeof(T) * 24);
+  if (devn) devn += parity * n5;
   const int64_t xcb = int64_t(i / g.L5);
   const int s5 = int(i - size_t(xcb) * g.L5);
   const int rhs = s5 / g.Ls, s = s5 - rhs * g.Ls;
   Spinor<R> f;
   if (rhs < g.nrhs_user) {
-    const int64_t c4 = canon_full ? cb_to_site(xcb, parity, g) : xcb;
-    const int64_t n4c = canon_full ? g.vol4 : g.half4;
+    const int64_t c4 = full ? cb_to_site(xcb, parity, g) : xcb;
+    const int64_t n4c = full ? g.vol4 : g.half4;
     const C2* c = reinterpret_cast<const C2*>(canon) + ((size_t(rhs) * n4c + c4) * g.Ls + s) * 12;
 #pragma unroll
     for (int k = 0; k < 12; k++) {
@@ -604,13 +606,16 @@ template <> struct LayoutPlanes<__half> {
 
 template <class T, class CR>
 __global__ void __launch_bounds__(256) export_kernel(const GeoParams g, CR* canon, const void* dev, const float* devn,
-                                                     int parity, int canon_full) {
+                                                     int full) {
   using P = LayoutPlanes<T>;
   using C2 = typename Canon2<CR>::type;
   __shared__ typename P::C tile[kLayoutSites * 13];
   __shared__ int64_t base[kLayoutSites];  // canonical index of the site's first component
   __shared__ float scale[kLayoutSites];
   const size_t n5 = size_t(g.half4) * g.L5;
+  const int parity = blockIdx.y;  // with full: the checkerboard (halves follow one another)
+  dev = static_cast<const char*>(dev) + parity * n5 * (sizeof(T) * 24);
+  if (devn) devn += parity * n5;
   const size_t i0 = size_t(blockIdx.x) * kLayoutSites;
   const int ns = int(min(n5 - i0, size_t(kLayoutSites)));  // even, as n5 and kLayoutSites are
   for (int j = threadIdx.x; j < ns; j += 256) {
@@ -618,8 +623,8 @@ __global__ void __launch_bounds__(256) export_kernel(const GeoParams g, CR* cano
     const int64_t xcb = int64_t(i / g.L5);
     const int s5 = int(i - size_t(xcb) * g.L5);
     const int rhs = s5 / g.Ls, s = s5 - rhs * g.Ls;
-    const int64_t c4 = canon_full ? cb_to_site(xcb, parity, g) : xcb;
-    const int64_t n4c = canon_full ? g.vol4 : g.half4;
+    const int64_t c4 = full ? cb_to_site(xcb, parity, g) : xcb;
+    const int64_t n4c = full ? g.vol4 : g.half4;
     // the padding right-hand side is absent from the canonical array
     base[j] = rhs < g.nrhs_user ? ((rhs * n4c + c4) * g.Ls + s) * 12 : -1;
   }
@@ -645,36 +650,36 @@ static GeoParams geo(const Op* op) {
   return g;
 }
 
-template <class CR> static int import_p(Op* op, const CR* canon, HalfView v, int parity, int canon_full) {
+template <class CR> static int import_p(Op* op, const CR* canon, HalfView v, int full) {
   const GeoParams g = geo(op);
-  const unsigned blocks = nblk(op->n5());
+  const dim3 blocks(nblk(op->n5()), full ? 2 : 1);
   switch (v.prec) {
-    case GB_F64: import_kernel<double, CR><<<blocks, 256, 0, op->stream>>>(g, canon, v.data, v.norms, parity, canon_full); break;
-    case GB_F32: import_kernel<float, CR><<<blocks, 256, 0, op->stream>>>(g, canon, v.data, v.norms, parity, canon_full); break;
-    case GB_F16: import_kernel<__half, CR><<<blocks, 256, 0, op->stream>>>(g, canon, v.data, v.norms, parity, canon_full); break;
+    case GB_F64: import_kernel<double, CR><<<blocks, 256, 0, op->stream>>>(g, canon, v.data, v.norms, full); break;
+    case GB_F32: import_kernel<float, CR><<<blocks, 256, 0, op->stream>>>(g, canon, v.data, v.norms, full); break;
+    case GB_F16: import_kernel<__half, CR><<<blocks, 256, 0, op->stream>>>(g, canon, v.data, v.norms, full); break;
   }
   GB_CHECK_CUDA(cudaGetLastError());
   return GB_OK;
 }
-template <class CR> static int export_p(Op* op, CR* canon, HalfView v, int parity, int canon_full) {
+template <class CR> static int export_p(Op* op, CR* canon, HalfView v, int full) {
   const GeoParams g = geo(op);
-  const unsigned blocks = unsigned((op->n5() + kLayoutSites - 1) / kLayoutSites);
+  const dim3 blocks(unsigned((op->n5() + kLayoutSites - 1) / kLayoutSites), full ? 2 : 1);
   switch (v.prec) {
-    case GB_F64: export_kernel<double, CR><<<blocks, 256, 0, op->stream>>>(g, canon, v.data, v.norms, parity, canon_full); break;
-    case GB_F32: export_kernel<float, CR><<<blocks, 256, 0, op->stream>>>(g, canon, v.data, v.norms, parity, canon_full); break;
-    case GB_F16: export_kernel<__half, CR><<<blocks, 256, 0, op->stream>>>(g, canon, v.data, v.norms, parity, canon_full); break;
+    case GB_F64: export_kernel<double, CR><<<blocks, 256, 0, op->stream>>>(g, canon, v.data, v.norms, full); break;
+    case GB_F32: export_kernel<float, CR><<<blocks, 256, 0, op->stream>>>(g, canon, v.data, v.norms, full); break;
+    case GB_F16: export_kernel<__half, CR><<<blocks, 256, 0, op->stream>>>(g, canon, v.data, v.norms, full); break;
   }
   GB_CHECK_CUDA(cudaGetLastError());
   return GB_OK;
 }
 
-int launch_import_half(Op* op, const void* canon, int canon_prec, HalfView out, int parity, int canon_is_full) {
-  if (canon_prec == GB_F32) return import_p<float>(op, static_cast<const float*>(canon), out, parity, canon_is_full);
-  return import_p<double>(op, static_cast<const double*>(canon), out, parity, canon_is_full);
+int launch_import(Op* op, const void* canon, int canon_prec, HalfView out, int full) {
+  if (canon_prec == GB_F32) return import_p<float>(op, static_cast<const float*>(canon), out, full);
+  return import_p<double>(op, static_cast<const double*>(canon), out, full);
 }
-int launch_export_half(Op* op, HalfView in, void* canon, int canon_prec, int parity, int canon_is_full) {
-  if (canon_prec == GB_F32) return export_p<float>(op, static_cast<float*>(canon), in, parity, canon_is_full);
-  return export_p<double>(op, static_cast<double*>(canon), in, parity, canon_is_full);
+int launch_export(Op* op, HalfView in, void* canon, int canon_prec, int full) {
+  if (canon_prec == GB_F32) return export_p<float>(op, static_cast<float*>(canon), in, full);
+  return export_p<double>(op, static_cast<double*>(canon), in, full);
 }
 
 // ---------------------------------------------------------------------------------------

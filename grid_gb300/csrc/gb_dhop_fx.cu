@@ -39,6 +39,8 @@ struct FxParams {
   longlong2* fxin[2];   // their fixed-point copies: 12 planes, then an exponent per 5D site
   int* exps[2];
   void* out[2];
+  const double2* z[2];  // out = c0 z + c1 Dhop when given, else the Dhop
+  double c0, c1;
   const int4* links[2];
   const double* links_d[2];  // the FP64 links, for sites that leave the fixed-point range
   const int* nbr[2];
@@ -173,7 +175,7 @@ __device__ __forceinline__ void fx_leg(int pl, const longlong2* __restrict__ in,
   }
 }
 
-// The FP64 sum of one site, straight to the output.
+// The FP64 sum of one site, for fx_site_fp64.
 template <bool DAG, int LEG>
 __device__ __forceinline__ void fp64_leg(const double2* in, const double* links, const int* nbr, size_t n5, int L5,
                                          int64_t x, int s, Spinor<double>& acc) {
@@ -198,18 +200,39 @@ __device__ __forceinline__ void fp64_legs(const double2* in, const double* links
   fp64_leg<DAG, 6>(in, links, nbr, n5, L5, x, s, acc);
   fp64_leg<DAG, 7>(in, links, nbr, n5, L5, x, s, acc);
 }
-__device__ __noinline__ void fx_site_fp64(const double2* in, double2* out, const double* links, const int* nbr, size_t n5,
-                                          int L5, int64_t x, int s, int dag) {
-  Spinor<double> acc;
-  if (dag) fp64_legs<true>(in, links, nbr, n5, L5, x, s, acc);
-  else fp64_legs<false>(in, links, nbr, n5, L5, x, s, acc);
-  SpinorIO<double>::store(out, nullptr, n5, size_t(x) * L5 + s, acc);
+// one output component: the Dhop's value, or (AXPY) c0 z + c1 of it
+template <bool AXPY>
+__device__ __forceinline__ void fx_store(const FxParams& p, const double2* z, double2* out, size_t w, double re, double im) {
+  if (AXPY) {
+    const double2 v = __ldg(z + w);
+    re = fma(p.c1, re, p.c0 * v.x);
+    im = fma(p.c1, im, p.c0 * v.y);
+  }
+  out[w] = make_double2(re, im);
 }
 
 // the integer (units of 2^e) as a double, rounded once; 0 stays 0
 __device__ __forceinline__ double fx_value(long long v, int e) {
   const double d = __ll2double_rn(v);
   return v == 0 ? 0.0 : __hiloint2double(__double2hiint(d) + (e << 20), __double2loint(d));
+}
+
+__device__ __noinline__ void fx_site_fp64(const double2* in, double2* out, const double2* z, double c0, double c1,
+                                          const double* links, const int* nbr, size_t n5, int L5, int64_t x, int s,
+                                          int dag) {
+  Spinor<double> acc;
+  if (dag) fp64_legs<true>(in, links, nbr, n5, L5, x, s, acc);
+  else fp64_legs<false>(in, links, nbr, n5, L5, x, s, acc);
+  const size_t i = size_t(x) * L5 + s;
+#pragma unroll
+  for (int k = 0; k < 12; k++) {
+    double2 v = make_double2(acc.re[k], acc.im[k]);
+    if (z) {
+      const double2 w = z[size_t(k) * n5 + i];
+      v = make_double2(fma(c1, v.x, c0 * w.x), fma(c1, v.y, c0 * w.y));
+    }
+    out[size_t(k) * n5 + i] = v;
+  }
 }
 
 // the largest exponent of a site's eight neighbours (kBad is above every other)
@@ -285,6 +308,7 @@ __global__ void __launch_bounds__(256) fx_convert_kernel(const __grid_constant__
   }
 }
 
+template <bool AXPY>
 __global__ void __launch_bounds__(128, 4) dhop_fx_kernel(const __grid_constant__ FxParams p) {
   extern __shared__ __align__(128) unsigned char dyn_smem[];
   int4* slink = reinterpret_cast<int4*>(dyn_smem);  // k4 * kFxLinkStride
@@ -314,7 +338,7 @@ __global__ void __launch_bounds__(128, 4) dhop_fx_kernel(const __grid_constant__
   fx_pad(p, out, x, s);
   const int Ea = fx_site_exponent(exps, nbr, p.L5, x, s);
   if (Ea == fx::kBad) {
-    fx_site_fp64(in, out, p.links_d[side], nbr, p.n5, p.L5, x, s, p.dag);
+    fx_site_fp64(in, out, p.z[side], p.c0, p.c1, p.links_d[side], nbr, p.n5, p.L5, x, s, p.dag);
     return;
   }
   FxAcc acc;
@@ -322,7 +346,7 @@ __global__ void __launch_bounds__(128, 4) dhop_fx_kernel(const __grid_constant__
   const int e = fx::result_exponent(Ea, p.link_exp);
   const size_t i = size_t(x) * p.L5 + s;
 #pragma unroll
-  for (int k = 0; k < 12; k++) out[size_t(k) * p.n5 + i] = make_double2(fx_value(acc.re[k], e), fx_value(acc.im[k], e));
+  for (int k = 0; k < 12; k++) fx_store<AXPY>(p, p.z[side], out, size_t(k) * p.n5 + i, fx_value(acc.re[k], e), fx_value(acc.im[k], e));
 }
 
 // Four warps share 32 output sites, one direction (its forward and backward leg) each, and add
@@ -331,7 +355,7 @@ __global__ void __launch_bounds__(128, 4) dhop_fx_kernel(const __grid_constant__
 // chain is the launch's time (8^4: 12.4 us, one thread per site 20.0), and with sites in lanes
 // the extra warps keep more of the links' 1152 bytes per site in flight (24^3 x 32: 138 us, one
 // thread per site 153).  SOA: the links' sites-in-lanes layout.
-template <bool SOA>
+template <bool SOA, bool AXPY>
 __global__ void __launch_bounds__(128, 4) dhop_fx_split_kernel(const __grid_constant__ FxParams p) {
   __shared__ long long part[4][24][32];
   const int side = blockIdx.z;
@@ -356,7 +380,7 @@ __global__ void __launch_bounds__(128, 4) dhop_fx_split_kernel(const __grid_cons
   if (!active) return;
   if (mu == 0) fx_pad(p, out, x, s);
   if (Ea == fx::kBad) {
-    if (mu == 0) fx_site_fp64(in, out, p.links_d[side], nbr, p.n5, p.L5, x, s, p.dag);
+    if (mu == 0) fx_site_fp64(in, out, p.z[side], p.c0, p.c1, p.links_d[side], nbr, p.n5, p.L5, x, s, p.dag);
     return;
   }
   const int e = fx::result_exponent(Ea, p.link_exp);
@@ -368,7 +392,7 @@ __global__ void __launch_bounds__(128, 4) dhop_fx_split_kernel(const __grid_cons
 #pragma unroll
     for (int c = 0; c < 2; c++)
       v[c] = (part[0][2 * k + c][lane] + part[1][2 * k + c][lane]) + (part[2][2 * k + c][lane] + part[3][2 * k + c][lane]);
-    out[size_t(k) * p.n5 + i] = make_double2(fx_value(v[0], e), fx_value(v[1], e));
+    fx_store<AXPY>(p, p.z[side], out, size_t(k) * p.n5 + i, fx_value(v[0], e), fx_value(v[1], e));
   }
 }
 
@@ -453,7 +477,8 @@ int fx_import_links(Op* op) {
   return GB_OK;
 }
 
-int launch_dhop_fx(Op* op, HalfView in, HalfView out, int out_parity, const HalfView* in2, const HalfView* out2, int dag) {
+int launch_dhop_fx(Op* op, HalfView in, HalfView out, int out_parity, const HalfView* in2, const HalfView* out2, int dag,
+                   const DhopAxpy* axpy) {
   FxParams p;
   const HalfView* ins[2] = {&in, in2};
   const HalfView* outs[2] = {&out, out2};
@@ -461,6 +486,7 @@ int launch_dhop_fx(Op* op, HalfView in, HalfView out, int out_parity, const Half
     const int par = z ? 1 - out_parity : out_parity;
     p.in[z] = ins[z] ? ins[z]->data : nullptr;
     p.out[z] = outs[z] ? outs[z]->data : nullptr;
+    p.z[z] = axpy ? static_cast<const double2*>(axpy->z[z].data) : nullptr;
     p.links[z] = static_cast<const int4*>(op->links_fx[par]);
     p.links_d[z] = static_cast<const double*>(op->links[par]);
     p.nbr[z] = op->nbr[par];
@@ -471,21 +497,25 @@ int launch_dhop_fx(Op* op, HalfView in, HalfView out, int out_parity, const Half
   p.n5 = op->n5();
   p.L5 = op->L5;
   p.L5a = op->Ls * op->nrhs_user;
+  p.c0 = axpy ? axpy->c0 : 0.0;
+  p.c1 = axpy ? axpy->c1 : 1.0;
   p.link_exp = op->fx_exp;
   p.dag = dag;
   p.err = op->d_err;
   fx_convert_kernel<<<dim3(unsigned((p.n5 + 255) / 256), 1, in2 ? 2u : 1u), 256, 0, op->stream>>>(p);
   const bool soa = fx_soa(op);
+  void (*kernel)(const FxParams);
   if (soa || p.n4h * p.L5a * (in2 ? 2 : 1) <= kFxSplitSites) {
-    const dim3 grid(unsigned((p.n4h * p.L5a + 31) / 32), 1, in2 ? 2u : 1u);
-    if (soa) dhop_fx_split_kernel<true><<<grid, 128, 0, op->stream>>>(p);
-    else dhop_fx_split_kernel<false><<<grid, 128, 0, op->stream>>>(p);
+    if (soa) kernel = axpy ? dhop_fx_split_kernel<true, true> : dhop_fx_split_kernel<true, false>;
+    else kernel = axpy ? dhop_fx_split_kernel<false, true> : dhop_fx_split_kernel<false, false>;
+    kernel<<<dim3(unsigned((p.n4h * p.L5a + 31) / 32), 1, in2 ? 2u : 1u), 128, 0, op->stream>>>(p);
   } else {
+    kernel = axpy ? dhop_fx_kernel<true> : dhop_fx_kernel<false>;
     p.L5c = p.L5a > 128 ? 128 : p.L5a;
     p.k4 = 128 / p.L5c;
     const dim3 grid(unsigned((p.n4h + p.k4 - 1) / p.k4), unsigned((p.L5a + p.L5c - 1) / p.L5c), in2 ? 2u : 1u);
     const unsigned threads = unsigned((p.k4 * p.L5c + 31) / 32 * 32);
-    dhop_fx_kernel<<<grid, threads, size_t(p.k4) * kFxLinkStride * sizeof(int4), op->stream>>>(p);
+    kernel<<<grid, threads, size_t(p.k4) * kFxLinkStride * sizeof(int4), op->stream>>>(p);
   }
   GB_CHECK_CUDA(cudaGetLastError());
   return GB_OK;

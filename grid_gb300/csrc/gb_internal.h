@@ -176,6 +176,17 @@ struct HalfView {
 inline HalfView half_view(const Field* f, int parity) { return HalfView{f->half_ptr(parity), f->half_norms(parity), f->prec}; }
 
 int launch_dhop(Op* op, HalfView in, HalfView out, int out_parity, int dag);
+// out = c0 z + c1 Dhop(in) in the Dhop's own launch, z on the output's checkerboard (z[1]: the
+// second output of a full-lattice launch, whose first output is the even one).  *done = 0,
+// and nothing launched, where the operator's kernel has no such form (12-real or double-float
+// FP64 links): the caller then runs the Dhop and the axpby.
+struct DhopAxpy {
+  HalfView z[2];
+  double c0, c1;
+};
+int launch_dhop_axpy(Op* op, HalfView in, HalfView out, int out_parity, int dag, const DhopAxpy& a, int* done);
+int launch_dhop_full_axpy(Op* op, HalfView in_odd, HalfView out_even, HalfView in_even, HalfView out_odd, int dag,
+                          const DhopAxpy& a, int* done);
 // FP32 / FP16: out = M5D(x5) - DhopEO/OE(in) in one launch (M5D with the given coefficients:
 // Mooee for the end of Mpc), |out|^2 per CTA and right-hand side into op->d_partial
 // ([CTA][nrhs], the norm partials' layout) and the CTA count into *parts.  Cases: one
@@ -189,7 +200,9 @@ size_t dhop_pair_ctas(const Op* op);
 // copies, and one launch (in2, out2: the second checkerboard of a full-lattice Dhop)
 bool fx_wanted(const Op* op);
 int fx_import_links(Op* op);
-int launch_dhop_fx(Op* op, HalfView in, HalfView out, int out_parity, const HalfView* in2, const HalfView* out2, int dag);
+struct DhopAxpy;
+int launch_dhop_fx(Op* op, HalfView in, HalfView out, int out_parity, const HalfView* in2, const HalfView* out2, int dag,
+                   const DhopAxpy* axpy = nullptr);
 int launch_dhop_full(Op* op, HalfView in_odd, HalfView out_even, HalfView in_even, HalfView out_odd, int dag);
 // force term of the output parity's sites into mat (FP64 canonical gauge layout, indexed
 // by x_cb when half_out, else by the lexicographic site); A has the output parity
@@ -198,15 +211,18 @@ int launch_deriv(Op* op, HalfView A, HalfView B, int out_parity, int dag, double
 int launch_m5d(Op* op, HalfView psi, HalfView phi, HalfView chi, const double* lower, const double* diag,
                const double* upper, int dag, size_t n5);
 int launch_mooee_inv(Op* op, HalfView in, HalfView out, int dag, size_t n4);
+// The field kernels below take one checkerboard, or with halves = 2 both of a full field in one
+// launch (the views of its first, even half; the odd one follows it in memory).
 // z = a*x + b*y (host scalars); x or y may alias z
-int launch_axpby(Op* op, HalfView z, double a, HalfView x, double b, HalfView y, size_t n5);
-int launch_scale(Op* op, HalfView z, double a, HalfView x, size_t n5);
+int launch_axpby(Op* op, HalfView z, double a, HalfView x, double b, HalfView y, size_t n5, int halves = 1);
+int launch_scale(Op* op, HalfView z, double a, HalfView x, size_t n5, int halves = 1);
 int launch_copy(Op* op, HalfView dst, HalfView src, size_t n5);
 int launch_zero(Op* op, HalfView z, size_t n5);
-// reductions: per-rhs results into op->d_result; partial per half
-int launch_norm2_partial(Op* op, HalfView x, size_t n5, double* partial);
-int launch_inner_partial(Op* op, HalfView a, HalfView b, size_t n5, double* partial);
-int launch_axpy_norm_partial(Op* op, HalfView z, double a, HalfView x, HalfView y, size_t n5, double* partial);
+// reductions: partial sums per CTA, red_parts() of them per half
+int launch_norm2_partial(Op* op, HalfView x, size_t n5, double* partial, int halves = 1);
+int launch_inner_partial(Op* op, HalfView a, HalfView b, size_t n5, double* partial, int halves = 1);
+int launch_axpy_norm_partial(Op* op, HalfView z, double a, HalfView x, HalfView y, size_t n5, double* partial,
+                             int halves = 1);
 int launch_reduce_final(Op* op, const double* partial, int nparts, int nv, double* out);
 int red_grid(Op* op, size_t n5, int* blocks, int* threads);
 // pair-layout (FP32 / FP16) kernels, gb_pair.cu
@@ -218,10 +234,11 @@ int launch_m5d_pair(Op* op, HalfView psi, HalfView phi, HalfView chi, const doub
                     const double* upper, int dag, size_t n5, const HalfView* z, double zc, int* norm_parts = nullptr);
 // kind 0: |x|^2 ; 1: <x|y> ; 2: z = a x + y, |z|^2 ; 3: y -= a[rhs] x (the device CG
 // scalars), |y|^2
-int launch_reduce_pair(Op* op, int kind, HalfView x, HalfView y, HalfView z, double a, size_t n5, double* partial);
-int launch_cg_p_pair(Op* op, HalfView p, HalfView r, size_t n5);
-int launch_cg_xp_pair(Op* op, HalfView psi, HalfView p, HalfView r, size_t n5, int update_p);
-int launch_axpby_pair(Op* op, HalfView z, double a, HalfView x, double b, HalfView y, size_t n5, int use_y);
+int launch_reduce_pair(Op* op, int kind, HalfView x, HalfView y, HalfView z, double a, size_t n5, double* partial,
+                       int halves);
+int launch_cg_p_pair(Op* op, HalfView p, HalfView r, size_t n5, int halves);
+int launch_cg_xp_pair(Op* op, HalfView psi, HalfView p, HalfView r, size_t n5, int update_p, int halves);
+int launch_axpby_pair(Op* op, HalfView z, double a, HalfView x, double b, HalfView y, size_t n5, int use_y, int halves);
 // partial sums per checkerboard half that a reduction over a field of precision prec writes
 inline int red_parts(Op* op, int prec) {
   int g = 1, B = 256;
@@ -260,8 +277,10 @@ int launch_col(Op* op, int opa, int opb, int dag, HalfView x, HalfView y, HalfVi
 // layout conversion between canonical FP64 (device) and the device layout
 // canonical host layout (complex double or, with canon_prec = GB_F32, complex float) <->
 // device layout of one checkerboard half
-int launch_import_half(Op* op, const void* canon, int canon_prec, HalfView out, int parity, int canon_is_full);
-int launch_export_half(Op* op, HalfView in, void* canon, int canon_prec, int parity, int canon_is_full);
+// (full: both checkerboards of a full field, whose canonical array is lexicographic; otherwise
+// one half and its canonical array by site >> 1)
+int launch_import(Op* op, const void* canon, int canon_prec, HalfView out, int full);
+int launch_export(Op* op, HalfView in, void* canon, int canon_prec, int full);
 int launch_double_store(Op* op, const double* U_canon, int parity);
 // 4D <-> 5D surface fields (Moebius): canonical FP64 4D field in device memory
 int launch_surface_insert(Op* op, const double* c4, HalfView even, HalfView odd);
@@ -286,12 +305,12 @@ int launch_cg_init(Op* op, const double* d_ssq, const double* d_cp, double tol, 
 // partials, real part first; nv = 1: norm partials)
 int launch_cg_alpha(Op* op, const double* partial, int nparts, int nv);
 // r -= a mmp ; partial |r|^2
-int launch_cg_r_update(Op* op, HalfView r, HalfView mmp, size_t n5, double* partial);
+int launch_cg_r_update(Op* op, HalfView r, HalfView mmp, size_t n5, double* partial, int halves = 1);
 // psi += a p ; with update_p also p = b p + r
-int launch_cg_xp_update(Op* op, HalfView psi, HalfView p, HalfView r, size_t n5, int update_p);
+int launch_cg_xp_update(Op* op, HalfView psi, HalfView p, HalfView r, size_t n5, int update_p, int halves = 1);
 int launch_cg_beta(Op* op, const double* partial_norm, int nparts);
 // p = b p + r
-int launch_cg_p_update(Op* op, HalfView p, HalfView r, size_t n5);
+int launch_cg_p_update(Op* op, HalfView p, HalfView r, size_t n5, int halves = 1);
 // after a reliable update: cp = c = maxres = cp_true ; b = cp_true / cprev
 int launch_cg_relup_reset(Op* op, const double* d_cp_true);
 // the device-resident CG loop's condition: arm before a graph launch (at most max_chunks

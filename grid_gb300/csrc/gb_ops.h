@@ -45,6 +45,10 @@ int launch_m5d_z(Op* op, HalfView psi, HalfView phi, HalfView chi, const double*
 int op_meooe5d(Op* op, Field* in, Field* out, int dag);
 int op_dhop_cb(Op* op, Field* in, Field* out, int dag);
 int op_dhop_full(Op* op, Field* in, Field* out, int dag);
+// out = c0 z + c1 Dhop(in) on half fields, z on the output's checkerboard
+int op_dhop_cb_axpy(Op* op, Field* in, Field* z, Field* out, double c0, double c1, int dag);
+// out = z - Meooe in
+int op_meooe_from(Op* op, Field* in, Field* z, Field* out);
 int op_meooe(Op* op, Field* in, Field* out, int dag);
 int op_mooee(Op* op, Field* in, Field* out, int dag, Field* z, double zc, int* norm_parts = nullptr);
 int op_mooee_inv(Op* op, Field* in, Field* out, int dag);

@@ -21,6 +21,15 @@ struct PairShape {
   int L5, Ls, nrhs;
 };
 
+// the blockIdx.y-th checkerboard half of a field of np pairs per half
+template <class T> __device__ __forceinline__ void* half_at(void* p, size_t np) {
+  return static_cast<char*>(p) + size_t(blockIdx.y) * np * (sizeof(T) == 4 ? 192 : 96);
+}
+template <class T> __device__ __forceinline__ const void* half_at(const void* p, size_t np) {
+  return static_cast<const char*>(p) + size_t(blockIdx.y) * np * (sizeof(T) == 4 ? 192 : 96);
+}
+template <class N> __device__ __forceinline__ N* norms_at(N* n, size_t np) { return n ? n + size_t(blockIdx.y) * np : n; }
+
 __device__ __forceinline__ float2 fma2s(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
 // Per-rhs block sums of per-lane FP64 values.  A thread keeps one accumulator per lane; the
@@ -227,6 +236,10 @@ __global__ void __launch_bounds__(512) reduce_pair_kernel(const PairShape sh, co
                                                           const void* y, const float2* yn, void* z, float2* zn,
                                                           double a, const CGScalars* cg, size_t np, double* partial) {
   constexpr int NV = KIND == 1 ? 2 : 1;
+  x = half_at<T>(x, np); xn = norms_at(xn, np);
+  y = half_at<T>(y, np); yn = norms_at(yn, np);
+  z = half_at<T>(z, np); zn = norms_at(zn, np);
+  partial += size_t(blockIdx.y) * gridDim.x * sh.nrhs * NV;
   double v0[NV], v1[NV];
 #pragma unroll
   for (int k = 0; k < NV; k++) { v0[k] = 0.0; v1[k] = 0.0; }
@@ -295,27 +308,28 @@ int red_grid_pair(Op* op, size_t np, int* blocks, int* threads) {
 }
 
 template <class T, int KIND>
-static int reduce_pair_t(Op* op, HalfView x, HalfView y, HalfView z, double a, size_t n5, double* partial) {
+static int reduce_pair_t(Op* op, HalfView x, HalfView y, HalfView z, double a, size_t n5, double* partial, int halves) {
   int g, B;
   const size_t np = n5 >> 1;
   GB_TRY(red_grid_pair(op, np, &g, &B));
   PairShape sh{op->L5, op->Ls, op->nrhs};
   const int NV = KIND == 1 ? 2 : 1;
   const size_t smem = size_t(NV) * (op->nrhs == 1 ? 32 : 2 * B) * sizeof(double);
-  reduce_pair_kernel<T, KIND><<<g, B, smem, op->stream>>>(
+  reduce_pair_kernel<T, KIND><<<dim3(g, halves), B, smem, op->stream>>>(
       sh, x.data, reinterpret_cast<const float2*>(x.norms), y.data, reinterpret_cast<const float2*>(y.norms), z.data,
       reinterpret_cast<float2*>(z.norms), a, op->d_cg, np, partial);
   GB_CHECK_CUDA(cudaGetLastError());
   return GB_OK;
 }
 
-int launch_reduce_pair(Op* op, int kind, HalfView x, HalfView y, HalfView z, double a, size_t n5, double* partial) {
+int launch_reduce_pair(Op* op, int kind, HalfView x, HalfView y, HalfView z, double a, size_t n5, double* partial,
+                       int halves) {
   const bool h = x.prec == GB_F16;
   switch (kind) {
-    case 0: return h ? reduce_pair_t<__half, 0>(op, x, y, z, a, n5, partial) : reduce_pair_t<float, 0>(op, x, y, z, a, n5, partial);
-    case 1: return h ? reduce_pair_t<__half, 1>(op, x, y, z, a, n5, partial) : reduce_pair_t<float, 1>(op, x, y, z, a, n5, partial);
-    case 2: return h ? reduce_pair_t<__half, 2>(op, x, y, z, a, n5, partial) : reduce_pair_t<float, 2>(op, x, y, z, a, n5, partial);
-    case 3: return h ? reduce_pair_t<__half, 3>(op, x, y, z, a, n5, partial) : reduce_pair_t<float, 3>(op, x, y, z, a, n5, partial);
+    case 0: return h ? reduce_pair_t<__half, 0>(op, x, y, z, a, n5, partial, halves) : reduce_pair_t<float, 0>(op, x, y, z, a, n5, partial, halves);
+    case 1: return h ? reduce_pair_t<__half, 1>(op, x, y, z, a, n5, partial, halves) : reduce_pair_t<float, 1>(op, x, y, z, a, n5, partial, halves);
+    case 2: return h ? reduce_pair_t<__half, 2>(op, x, y, z, a, n5, partial, halves) : reduce_pair_t<float, 2>(op, x, y, z, a, n5, partial, halves);
+    case 3: return h ? reduce_pair_t<__half, 3>(op, x, y, z, a, n5, partial, halves) : reduce_pair_t<float, 3>(op, x, y, z, a, n5, partial, halves);
   }
   return GB_ERR_BAD_ARG;
 }
@@ -328,6 +342,8 @@ __global__ void __launch_bounds__(256) cg_p_pair_kernel(const PairShape sh, void
                                                         const float2* rn, const CGScalars* cg, size_t np) {
   const size_t q = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (q >= np) return;
+  p = half_at<T>(p, np); pn = norms_at(pn, np);
+  r = half_at<T>(r, np); rn = norms_at(rn, np);
   const int s5 = int((2 * q) % sh.L5);
   const float2 b = make_float2(float(cg[s5 / sh.Ls].b), float(cg[(s5 + 1) / sh.Ls].b));
   Pair12 fp, fr;
@@ -341,10 +357,10 @@ __global__ void __launch_bounds__(256) cg_p_pair_kernel(const PairShape sh, void
   PairIO<T>::store(p, pn, np, q, fp);
 }
 
-int launch_cg_p_pair(Op* op, HalfView p, HalfView r, size_t n5) {
+int launch_cg_p_pair(Op* op, HalfView p, HalfView r, size_t n5, int halves) {
   PairShape sh{op->L5, op->Ls, op->nrhs};
   const size_t np = n5 >> 1;
-  const unsigned blocks = unsigned((np + 255) / 256);
+  const dim3 blocks(unsigned((np + 255) / 256), halves);
   if (p.prec == GB_F32)
     cg_p_pair_kernel<float><<<blocks, 256, 0, op->stream>>>(sh, p.data, reinterpret_cast<float2*>(p.norms), r.data,
                                                             reinterpret_cast<const float2*>(r.norms), op->d_cg, np);
@@ -363,6 +379,9 @@ __global__ void __launch_bounds__(256) cg_xp_pair_kernel(const PairShape sh, voi
                                                          size_t np) {
   const size_t q = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (q >= np) return;
+  p = half_at<T>(p, np); pn = norms_at(pn, np);
+  r = half_at<T>(r, np); rn = norms_at(rn, np);
+  psi = half_at<TS>(psi, np); psin = norms_at(psin, np);
   const int s5 = int((2 * q) % sh.L5);
   const CGScalars& c0 = cg[s5 / sh.Ls];
   const CGScalars& c1 = cg[(s5 + 1) / sh.Ls];
@@ -390,9 +409,9 @@ __global__ void __launch_bounds__(256) cg_xp_pair_kernel(const PairShape sh, voi
 }
 
 template <class T, class TS>
-static void cg_xp_pair_go(Op* op, HalfView psi, HalfView p, HalfView r, size_t np, bool pupd) {
+static void cg_xp_pair_go(Op* op, HalfView psi, HalfView p, HalfView r, size_t np, bool pupd, int halves) {
   PairShape sh{op->L5, op->Ls, op->nrhs};
-  const unsigned blocks = unsigned((np + 255) / 256);
+  const dim3 blocks(unsigned((np + 255) / 256), halves);
   auto* psin = reinterpret_cast<float2*>(psi.norms);
   auto* pn = reinterpret_cast<float2*>(p.norms);
   auto* rn = reinterpret_cast<const float2*>(r.norms);
@@ -402,11 +421,11 @@ static void cg_xp_pair_go(Op* op, HalfView psi, HalfView p, HalfView r, size_t n
     cg_xp_pair_kernel<T, TS, false><<<blocks, 256, 0, op->stream>>>(sh, psi.data, psin, p.data, pn, r.data, rn, op->d_cg, np);
 }
 
-int launch_cg_xp_pair(Op* op, HalfView psi, HalfView p, HalfView r, size_t n5, int update_p) {
+int launch_cg_xp_pair(Op* op, HalfView psi, HalfView p, HalfView r, size_t n5, int update_p, int halves) {
   const size_t np = n5 >> 1;
-  if (p.prec == GB_F32 && psi.prec == GB_F32) cg_xp_pair_go<float, float>(op, psi, p, r, np, update_p != 0);
-  else if (p.prec == GB_F16 && psi.prec == GB_F32) cg_xp_pair_go<__half, float>(op, psi, p, r, np, update_p != 0);
-  else if (p.prec == GB_F16 && psi.prec == GB_F16) cg_xp_pair_go<__half, __half>(op, psi, p, r, np, update_p != 0);
+  if (p.prec == GB_F32 && psi.prec == GB_F32) cg_xp_pair_go<float, float>(op, psi, p, r, np, update_p != 0, halves);
+  else if (p.prec == GB_F16 && psi.prec == GB_F32) cg_xp_pair_go<__half, float>(op, psi, p, r, np, update_p != 0, halves);
+  else if (p.prec == GB_F16 && psi.prec == GB_F16) cg_xp_pair_go<__half, __half>(op, psi, p, r, np, update_p != 0, halves);
   else {
     set_error("CG update: solution precision %d with search-direction precision %d", psi.prec, p.prec);
     return GB_ERR_BAD_ARG;
@@ -421,6 +440,9 @@ __global__ void __launch_bounds__(256) axpby_pair_kernel(void* z, float2* zn, fl
                                                          int use_y) {
   const size_t q = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (q >= np) return;
+  x = half_at<T>(x, np); xn = norms_at(xn, np);
+  y = half_at<T>(y, np); yn = norms_at(yn, np);
+  z = half_at<T>(z, np); zn = norms_at(zn, np);
   Pair12 fx, o;
   PairIO<T>::load(x, xn, np, q, fx);
   const float2 a2 = make_float2(a, a);
@@ -440,9 +462,9 @@ __global__ void __launch_bounds__(256) axpby_pair_kernel(void* z, float2* zn, fl
   PairIO<T>::store(z, zn, np, q, o);
 }
 
-int launch_axpby_pair(Op* op, HalfView z, double a, HalfView x, double b, HalfView y, size_t n5, int use_y) {
+int launch_axpby_pair(Op* op, HalfView z, double a, HalfView x, double b, HalfView y, size_t n5, int use_y, int halves) {
   const size_t np = n5 >> 1;
-  const unsigned blocks = unsigned((np + 255) / 256);
+  const dim3 blocks(unsigned((np + 255) / 256), halves);
   if (z.prec == GB_F32)
     axpby_pair_kernel<float><<<blocks, 256, 0, op->stream>>>(z.data, reinterpret_cast<float2*>(z.norms), float(a), x.data,
                                                              reinterpret_cast<const float2*>(x.norms), float(b), y.data,

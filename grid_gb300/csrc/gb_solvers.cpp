@@ -43,16 +43,13 @@ Parts parts_of(Op* op, const Field* f) {
 // d = |ap|^2 (ap = M p or Mpc p) -> a
 int cg_alpha_norm(Op* op, Field* ap) {
   Parts P = parts_of(op, ap);
-  for (int h = 0; h < P.halves; h++)
-    GB_TRY(launch_norm2_partial(op, half_view(ap, h), ap->n5, op->d_partial + size_t(h) * P.g * op->nrhs));
+  GB_TRY(launch_norm2_partial(op, half_view(ap, 0), ap->n5, op->d_partial, P.halves));
   return launch_cg_alpha(op, op->d_partial, P.g * P.halves, 1);
 }
 // r -= a mmp ; cp = |r|^2 -> b
 int cg_r_update(Op* op, Field* r, Field* mmp) {
   Parts P = parts_of(op, r);
-  for (int h = 0; h < P.halves; h++)
-    GB_TRY(launch_cg_r_update(op, half_view(r, h), half_view(mmp, h), r->n5,
-                              op->d_partial + size_t(h) * P.g * op->nrhs));
+  GB_TRY(launch_cg_r_update(op, half_view(r, 0), half_view(mmp, 0), r->n5, op->d_partial, P.halves));
   return launch_cg_beta(op, op->d_partial, P.g * P.halves);
 }
 // One CG matrix step on p: A = MdagM (kind 0) or MpcDagMpc (kind 1) with d = |M p|^2
@@ -79,15 +76,10 @@ int cg_matrix_step(Op* op, int kind, Field* p, Field* mmp, Field* r) {
 }
 // psi += a p ; with update_p also p = b p + r
 int cg_xp_update(Op* op, Field* psi, Field* p, Field* r, int update_p) {
-  const int halves = p->full() ? 2 : 1;
-  for (int h = 0; h < halves; h++)
-    GB_TRY(launch_cg_xp_update(op, half_view(psi, h), half_view(p, h), half_view(r, h), p->n5, update_p));
-  return GB_OK;
+  return launch_cg_xp_update(op, half_view(psi, 0), half_view(p, 0), half_view(r, 0), p->n5, update_p, p->full() ? 2 : 1);
 }
 int cg_p_update(Op* op, Field* p, Field* r) {
-  const int halves = p->full() ? 2 : 1;
-  for (int h = 0; h < halves; h++) GB_TRY(launch_cg_p_update(op, half_view(p, h), half_view(r, h), p->n5));
-  return GB_OK;
+  return launch_cg_p_update(op, half_view(p, 0), half_view(r, 0), p->n5, p->full() ? 2 : 1);
 }
 
 // flags[0..3] = op->d_all_done (converged, reliable update wanted, chunks the last device
@@ -468,20 +460,16 @@ int schur_solve(Op* op, Op* olo, Field* src, Field* sol, const gb_cg_params* P, 
   GB_TRY(launch_copy(op, half_view(src_e, 0), half_view(src, GB_EVEN), src->n5));
   GB_TRY(launch_copy(op, half_view(src_o, 0), half_view(src, GB_ODD), src->n5));
   GB_TRY(op_mooee_inv(op, src_e, tmp, 0));
-  GB_TRY(op_meooe(op, tmp, Mtmp, 0));
-  GB_TRY(field_axpby(Mtmp, 1.0, -1.0, src_o, Mtmp));  // Mtmp = src_o - Mtmp
+  GB_TRY(op_meooe_from(op, tmp, src_o, Mtmp));  // Mtmp = src_o - Meooe MooeeInv src_e
   GB_TRY(op_mpc(op, Mtmp, src_o, 1));
   GB_TRY(field_zero(sol_o));
   sol_o->subset = GB_ODD;
   int rc = olo ? cg_reliable(op, olo, 1, src_o, sol_o, P, R) : cg_solve(op, 1, src_o, sol_o, P, R);
   if (rc != GB_OK && rc != GB_ERR_NOT_CONVERGED) return rc;
   // RedBlackSolution: sol_e = MooeeInv (src_e - Meooe sol_o)
-  GB_TRY(op_meooe(op, sol_o, tmp, 0));
-  GB_TRY(field_axpby(tmp, 1.0, -1.0, src_e, tmp));
-  GB_TRY(launch_copy(op, half_view(src_e, 0), half_view(tmp, 0), src->n5));
-  src_e->subset = GB_EVEN;
-  Field* sol_e = tmp;
-  GB_TRY(op_mooee_inv(op, src_e, sol_e, 0));
+  GB_TRY(op_meooe_from(op, sol_o, src_e, tmp));
+  Field* sol_e = src_e;
+  GB_TRY(op_mooee_inv(op, tmp, sol_e, 0));
   GB_TRY(launch_copy(op, half_view(sol, GB_EVEN), half_view(sol_e, 0), src->n5));
   GB_TRY(launch_copy(op, half_view(sol, GB_ODD), half_view(sol_o, 0), src->n5));
   if (unprec) {
