@@ -948,22 +948,6 @@ struct DerivParams {
   DhopParams geo;  // L, sgn, parity (for the 12-real link rebuild and the site index)
 };
 
-// w += h conj(g)^T over both spins of the two-spinors
-template <class R>
-__device__ __forceinline__ void deriv_outer(const R (&hr)[6], const R (&hi)[6], const R (&gr)[6], const R (&gi)[6],
-                                            double (&wr)[9], double (&wi)[9]) {
-#pragma unroll
-  for (int j = 0; j < 2; j++)
-#pragma unroll
-    for (int c = 0; c < 3; c++)
-#pragma unroll
-      for (int b = 0; b < 3; b++) {
-        const double xr = hr[j * 3 + c], xi = hi[j * 3 + c], yr = gr[j * 3 + b], yi = gi[j * 3 + b];
-        wr[c * 3 + b] = fma(xr, yr, fma(xi, yi, wr[c * 3 + b]));
-        wi[c * 3 + b] = fma(xi, yr, fma(-xr, yi, wi[c * 3 + b]));
-      }
-}
-
 // lane g of G of one site: every G-th 16-byte vector along s (FP64 one s, FP32 a pair)
 template <class T, int MU, int S, int G>
 __device__ __forceinline__ void deriv_site(const DerivParams& q, int64_t x, int64_t nb, int g, double (&wr)[9],
@@ -1040,40 +1024,8 @@ __global__ void __launch_bounds__(128) deriv_kernel(const DerivParams q) {
 #pragma unroll
     for (int e = 0; e < 18; e++) Ul[e] = src[e];
   }
-  int64_t idx = x;
-  if (!q.half_out) {  // lexicographic site of x_cb in the output parity
-    const int Lxh = q.geo.L[0] >> 1;
-    const int64_t row = x / Lxh;
-    const int xh = int(x - row * Lxh);
-    const int y = int(row % q.geo.L[1]);
-    const int64_t zt = row / q.geo.L[1];
-    const int z = int(zt % q.geo.L[2]), t = int(zt / q.geo.L[2]);
-    idx = row * q.geo.L[0] + 2 * xh + ((q.geo.parity + y + z + t) & 1);
-  }
-  double2* o = q.mat + (size_t(idx) * 4 + mu) * 9;
-  // the rows of U W: two lanes take row g each, then lane 0 the last
-#pragma unroll
-  for (int pass = 0; pass < (G == 2 ? 2 : 3); pass++) {
-    const int a = G == 2 ? (pass == 0 ? g : 2) : pass;
-    if (G == 2 && pass == 1 && g == 1) break;
-    double ur[3], ui[3];
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-      const int e = 2 * c;
-      ur[c] = a == 0 ? Ul[e] : a == 1 ? Ul[6 + e] : Ul[12 + e];
-      ui[c] = a == 0 ? Ul[e + 1] : a == 1 ? Ul[7 + e] : Ul[13 + e];
-    }
-#pragma unroll
-    for (int b = 0; b < 3; b++) {
-      double re = 0, im = 0;
-#pragma unroll
-      for (int c = 0; c < 3; c++) {
-        re = fma(ur[c], wr[c * 3 + b], fma(-ui[c], wi[c * 3 + b], re));
-        im = fma(ur[c], wi[c * 3 + b], fma(ui[c], wr[c * 3 + b], im));
-      }
-      o[a * 3 + b] = make_double2(re, im);
-    }
-  }
+  const int64_t idx = q.half_out ? x : site_of_cb(q.geo.L, q.geo.parity, x);
+  deriv_rows<G, R>(Ul, wr, wi, g, q.mat + (size_t(idx) * 4 + mu) * 9);
 }
 
 // two lanes per site halve the walk along s; one where the site has a single vector
@@ -1088,6 +1040,7 @@ static void deriv_go(Op* op, const DerivParams& q) {
 int launch_deriv(Op* op, HalfView A, HalfView B, int out_parity, int dag, double* mat, int half_out) {
   if (A.prec != op->prec || B.prec != op->prec) { set_error("DhopDeriv: field precision differs from the operator's"); return GB_ERR_BAD_ARG; }
   if (op->prec == GB_F16) { set_error("DhopDeriv: FP64 or FP32 operators"); return GB_ERR_UNSUPPORTED; }
+  if (op->fx_ready && fx_deriv_ok(op)) return launch_deriv_fx(op, A, B, out_parity, dag, mat, half_out);
   DerivParams q;
   q.A = A.data; q.An = A.norms; q.B = B.data; q.Bn = B.norms;
   q.links = op->links[out_parity];

@@ -1,5 +1,6 @@
 // gb_dhop_site.cuh -- the steps of one leg of the hopping term on a site's spinor in registers:
-// projection to a two-spinor, SU(3) product, reconstruction (Grid/qcd/spin/TwoSpinor.h:75-330).
+// projection to a two-spinor, SU(3) product, reconstruction (Grid/qcd/spin/TwoSpinor.h:75-330);
+// and of the force term built on them.
 #pragma once
 
 #include "gb_device.cuh"
@@ -83,6 +84,62 @@ __device__ __forceinline__ void su3_mul(const R* __restrict__ U, const R (&hr)[6
       ui[o + a] = xi;
     }
   }
+}
+
+// ---- force term: W += h conj(g)^T over both spins of two-spinors (W: colour c of h, b of g) ----
+template <class R>
+__device__ __forceinline__ void deriv_outer(const R (&hr)[6], const R (&hi)[6], const R (&gr)[6], const R (&gi)[6],
+                                            double (&wr)[9], double (&wi)[9]) {
+#pragma unroll
+  for (int j = 0; j < 2; j++)
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+#pragma unroll
+      for (int b = 0; b < 3; b++) {
+        const double xr = hr[j * 3 + c], xi = hi[j * 3 + c], yr = gr[j * 3 + b], yi = gi[j * 3 + b];
+        wr[c * 3 + b] = fma(xr, yr, fma(xi, yi, wr[c * 3 + b]));
+        wi[c * 3 + b] = fma(xi, yr, fma(-xr, yi, wi[c * 3 + b]));
+      }
+}
+
+// The rows of U W into o (row-major 3 x 3) by the G lanes of a site that hold W: one lane all of
+// them, or lane 0 rows 0, 2 and lane 1 row 1.
+template <int G, class R>
+__device__ __forceinline__ void deriv_rows(const R (&U)[18], const double (&wr)[9], const double (&wi)[9], int g,
+                                           double2* o) {
+#pragma unroll
+  for (int pass = 0; pass < (G == 2 ? 2 : 3); pass++) {
+    const int a = G == 2 ? (pass == 0 ? g : 2) : pass;
+    if (G == 2 && pass == 1 && g == 1) break;
+    double ur[3], ui[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const int e = 2 * c;
+      ur[c] = a == 0 ? U[e] : a == 1 ? U[6 + e] : U[12 + e];
+      ui[c] = a == 0 ? U[e + 1] : a == 1 ? U[7 + e] : U[13 + e];
+    }
+#pragma unroll
+    for (int b = 0; b < 3; b++) {
+      double re = 0, im = 0;
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        re = fma(ur[c], wr[c * 3 + b], fma(-ui[c], wi[c * 3 + b], re));
+        im = fma(ur[c], wi[c * 3 + b], fma(ui[c], wr[c * 3 + b], im));
+      }
+      o[a * 3 + b] = make_double2(re, im);
+    }
+  }
+}
+
+// the lexicographic site of x_cb on checkerboard `parity`
+__device__ __forceinline__ int64_t site_of_cb(const int (&L)[4], int parity, int64_t x) {
+  const int Lxh = L[0] >> 1;
+  const int64_t row = x / Lxh;
+  const int xh = int(x - row * Lxh);
+  const int y = int(row % L[1]);
+  const int64_t zt = row / L[1];
+  const int z = int(zt % L[2]), t = int(zt / L[2]);
+  return row * L[0] + 2 * xh + ((parity + y + z + t) & 1);
 }
 
 }  // namespace gb

@@ -207,6 +207,9 @@ int launch_dhop_full(Op* op, HalfView in_odd, HalfView out_even, HalfView in_eve
 // force term of the output parity's sites into mat (FP64 canonical gauge layout, indexed
 // by x_cb when half_out, else by the lexicographic site); A has the output parity
 int launch_deriv(Op* op, HalfView A, HalfView B, int out_parity, int dag, double* mat, int half_out);
+// the same in fixed point for FP64 operators whose fifth dimension it takes
+bool fx_deriv_ok(const Op* op);
+int launch_deriv_fx(Op* op, HalfView A, HalfView B, int out_parity, int dag, double* mat, int half_out);
 // chi = diag*phi + upper*P(-/+) psi[s+1] + lower*P(+/-) psi[s-1]   (per rhs block of Ls)
 int launch_m5d(Op* op, HalfView psi, HalfView phi, HalfView chi, const double* lower, const double* diag,
                const double* upper, int dag, size_t n5);
