@@ -116,13 +116,14 @@ struct RedShape {
 template <class T, int KIND>
 __global__ void __launch_bounds__(256) reduce_kernel(const RedShape sh, const void* x, const float* xn, const void* y,
                                                      const float* yn, void* z, float* zn, double a,
-                                                     const CGScalars* cg, size_t n5, double* partial) {
+                                                     const CGScalars* cg, size_t n5, double* partial, const CGFinish fin) {
   using R = typename Arith<T>::type;
   constexpr int NV = KIND == 1 ? 2 : 1;
   const size_t half = size_t(blockIdx.y) * n5 * 12 * sizeof(double2);  // blockIdx.y: the checkerboard
   x = static_cast<const char*>(x) + half;
   y = static_cast<const char*>(y) + half;
   z = static_cast<char*>(z) + half;
+  const double* const all = partial;
   partial += size_t(blockIdx.y) * gridDim.x * sh.nrhs * NV;
   double v[NV];
 #pragma unroll
@@ -169,6 +170,7 @@ __global__ void __launch_bounds__(256) reduce_kernel(const RedShape sh, const vo
     }
   }
   block_reduce_rhs<NV>(v, sh.L5, sh.Ls, sh.nrhs, partial);
+  if (fin.mode != CG_FINISH_NONE) cg_finish(fin, all, gridDim.x * gridDim.y, sh.nrhs, gridDim.x * gridDim.y);
 }
 
 int red_grid(Op* op, size_t n5, int* blocks, int* threads) {
@@ -192,23 +194,24 @@ int red_grid(Op* op, size_t n5, int* blocks, int* threads) {
 }
 
 template <class T, int KIND>
-static int reduce_t(Op* op, HalfView x, HalfView y, HalfView z, double a, size_t n5, double* partial, int halves) {
+static int reduce_t(Op* op, HalfView x, HalfView y, HalfView z, double a, size_t n5, double* partial, int halves,
+                    int finish = CG_FINISH_NONE) {
   int g, B;
   GB_TRY(red_grid(op, n5, &g, &B));
   RedShape sh{op->L5, op->Ls, op->nrhs};
   const int NV = KIND == 1 ? 2 : 1;
   size_t smem = size_t(NV) * (op->nrhs == 1 ? 32 : B) * sizeof(double);
   reduce_kernel<T, KIND><<<dim3(g, halves), B, smem, op->stream>>>(sh, x.data, x.norms, y.data, y.norms, z.data, z.norms, a, op->d_cg,
-                                                     n5, partial);
+                                                     n5, partial, CGFinish{op->d_cg, op->d_all_done, finish});
   GB_CHECK_CUDA(cudaGetLastError());
   return GB_OK;
 }
 
 // FP32 / FP16 fields reduce through the pair kernels (gb_pair.cu), whose partial count
 // red_parts() reports; FP64 through reduce_kernel
-int launch_norm2_partial(Op* op, HalfView x, size_t n5, double* partial, int halves) {
-  if (x.prec != GB_F64) return launch_reduce_pair(op, 0, x, x, x, 0.0, n5, partial, halves);
-  return reduce_t<double, 0>(op, x, x, x, 0.0, n5, partial, halves);
+int launch_norm2_partial(Op* op, HalfView x, size_t n5, double* partial, int halves, int finish) {
+  if (x.prec != GB_F64) return launch_reduce_pair(op, 0, x, x, x, 0.0, n5, partial, halves, finish);
+  return reduce_t<double, 0>(op, x, x, x, 0.0, n5, partial, halves, finish);
 }
 int launch_inner_partial(Op* op, HalfView a, HalfView b, size_t n5, double* partial, int halves) {
   if (a.prec != b.prec) { set_error("innerProduct: mixed precisions"); return GB_ERR_BAD_ARG; }
@@ -224,8 +227,8 @@ int launch_axpy_norm_partial(Op* op, HalfView z, double a, HalfView x, HalfView 
 // r -= a[rhs] mmp, |r|^2: Grid's axpy_norm(r, -a, mmp, r) with the device CG scalars
 int launch_cg_r_update(Op* op, HalfView r, HalfView mmp, size_t n5, double* partial, int halves) {
   if (r.prec != mmp.prec) { set_error("CG update: mixed precisions"); return GB_ERR_BAD_ARG; }
-  if (r.prec != GB_F64) return launch_reduce_pair(op, 3, mmp, r, r, 0.0, n5, partial, halves);
-  return reduce_t<double, 3>(op, mmp, r, r, 0.0, n5, partial, halves);
+  if (r.prec != GB_F64) return launch_reduce_pair(op, 3, mmp, r, r, 0.0, n5, partial, halves, CG_FINISH_BETA);
+  return reduce_t<double, 3>(op, mmp, r, r, 0.0, n5, partial, halves, CG_FINISH_BETA);
 }
 
 // partial: [nparts][nrhs][nv] -> out[nrhs][nv]; one CTA per rhs, fixed summation order
@@ -285,7 +288,7 @@ __global__ void cg_init_kernel(CGScalars* cg, const double* ssq, const double* c
     if (s.done) atomicAdd(&nd, 1);
   }
   __syncthreads();
-  if (r == 0) { flags[0] = (nd == nrhs); flags[1] = 0; flags[4] = 0; }
+  if (r == 0) { flags[0] = (nd == nrhs); flags[1] = 0; flags[kCGTicket] = 0; }
 }
 
 // sum over b of partial[b * stride + offset] by one CTA (whole warps, at most 1024 threads) in a
@@ -310,49 +313,10 @@ __device__ double cta_sum_fixed(const double* partial, int nparts, int stride, i
 
 // One CTA per right-hand side (one CTA for all took 26-30 us at 12 right-hand sides), of 256
 // threads, 1024 above 2048 partial sums (one per CTA of an FP32 Dhop)
-__global__ void __launch_bounds__(1024) cg_alpha_kernel(CGScalars* cg, const double* partial, int nparts, int nrhs,
-                                                       int nv) {
+__global__ void __launch_bounds__(1024) cg_alpha_kernel(CGScalars* cg, const double* partial, int nparts, int nrhs) {
   const int r = blockIdx.x;
-  const double d = cta_sum_fixed(partial, nparts, nrhs * nv, r * nv);
-  if (threadIdx.x == 0) {
-    cg[r].d = d;
-    cg[r].a = cg[r].done ? 0.0 : cg[r].c / d;
-  }
-}
-
-// flags[4] counts the CTAs that have written their right-hand side: the last one sets the flags of
-// the whole solve and leaves the count at zero
-__global__ void __launch_bounds__(1024) cg_beta_kernel(CGScalars* cg, const double* partial, int nparts, int nrhs,
-                                                      int* flags) {
-  const int r = blockIdx.x;
-  const double cp = cta_sum_fixed(partial, nparts, nrhs, r);
-  if (threadIdx.x != 0) return;
-  CGScalars s = cg[r];
-  if (!s.done) {
-    s.cp = cp;
-    s.b = cp / s.c;
-    s.cprev = s.c;
-    s.c = cp;
-    s.iter += 1;
-    if (cp > s.maxres) s.maxres = cp;
-    if (cp <= s.rsq) s.done = 1;
-    else if (cp < s.delta * s.maxres) s.relup = 1;
-  } else {
-    s.b = 0.0;
-  }
-  cg[r] = s;
-  __threadfence();
-  if (atomicAdd(flags + 4, 1) != nrhs - 1) return;
-  __threadfence();
-  int nd = 0, nr = 0;
-  for (int k = 0; k < nrhs; k++) {
-    const int done = __ldcg(&cg[k].done), relup = __ldcg(&cg[k].relup);
-    nd += done;
-    nr += relup && !done;
-  }
-  flags[0] = nd == nrhs;
-  flags[1] = nr;
-  flags[4] = 0;
+  const double d = cta_sum_fixed(partial, nparts, nrhs, r);
+  if (threadIdx.x == 0) cg_alpha_update(cg[r], d);
 }
 
 __global__ void cg_relup_reset_kernel(CGScalars* cg, const double* cp_true, int nrhs) {
@@ -378,15 +342,15 @@ int launch_cg_init(Op* op, const double* d_ssq, const double* d_cp, double tol, 
 }
 // the scalar kernels reduce the per-block partial sums themselves, in a fixed order
 static inline int sum_threads(int nparts) { return nparts > 2048 ? 1024 : 256; }
-int launch_cg_alpha(Op* op, const double* partial, int nparts, int nv) {
-  cg_alpha_kernel<<<op->nrhs, sum_threads(nparts), 0, op->stream>>>(op->d_cg, partial, nparts, op->nrhs, nv);
+int launch_cg_alpha(Op* op, const double* partial, int nparts) {
+  cg_alpha_kernel<<<op->nrhs, sum_threads(nparts), 0, op->stream>>>(op->d_cg, partial, nparts, op->nrhs);
   GB_CHECK_CUDA(cudaGetLastError());
   return GB_OK;
 }
 // The device-resident CG loop (a CUDA graph whose conditional WHILE node repeats a
 // captured chunk of iterations).  flags = op->d_all_done: [0] every right-hand side has
 // converged, [1] right-hand sides that want a reliable update (both written by
-// cg_beta_kernel each iteration), [2] chunks run in this launch, [3] the most chunks one
+// cg_finish each iteration), [2] chunks run in this launch, [3] the most chunks one
 // launch may run.  arm sets [2], [3] before a launch; check decides after every chunk.
 __global__ void cg_loop_arm_kernel(int* flags, int max_chunks) {
   flags[2] = 0;
@@ -407,11 +371,6 @@ int launch_cg_loop_check(Op* op, cudaGraphConditionalHandle h) {
   return GB_OK;
 }
 
-int launch_cg_beta(Op* op, const double* partial_norm, int nparts) {
-  cg_beta_kernel<<<op->nrhs, sum_threads(nparts), 0, op->stream>>>(op->d_cg, partial_norm, nparts, op->nrhs, op->d_all_done);
-  GB_CHECK_CUDA(cudaGetLastError());
-  return GB_OK;
-}
 int launch_cg_relup_reset(Op* op, const double* d_cp_true) {
   cg_relup_reset_kernel<<<1, rhs_threads(op), 0, op->stream>>>(op->d_cg, d_cp_true, op->nrhs);
   GB_CHECK_CUDA(cudaGetLastError());

@@ -53,6 +53,7 @@ struct ColParams {
   double* rpart;
   const CGScalars* cg;
   int nrhs;
+  CGFinish fin;  // RUPD: the last CTA updates the CG's b and convergence flags
 };
 
 // stage one input into the [12][Q][ST] float4 tile: FP32 copies the vectors, FP16 decodes
@@ -389,6 +390,7 @@ __global__ void __launch_bounds__(12 * kColPipeQ) col_pipe_kernel(const ColParam
       for (int q2 = t; q2 < Q; q2 += p.nrhs) s += csum[q2];
       p.rpart[size_t(blockIdx.x) * p.nrhs + t] = s;
     }
+    cg_finish(p.fin, p.rpart, gridDim.x, p.nrhs, gridDim.x);
   }
 }
 
@@ -522,6 +524,7 @@ __global__ void __launch_bounds__(12 * kColPipeQ) col_pipe_half_kernel(const Col
       for (int q2 = t; q2 < Q; q2 += p.nrhs) s += csum[q2];
       p.rpart[size_t(blockIdx.x) * p.nrhs + t] = s;
     }
+    cg_finish(p.fin, p.rpart, gridDim.x, p.nrhs, gridDim.x);
   }
 }
 
@@ -675,6 +678,7 @@ int launch_col(Op* op, int opa, int opb, int dag, HalfView x, HalfView y, HalfVi
   p.rpart = rupd ? op->d_partial : nullptr;
   p.cg = op->d_cg;
   p.nrhs = op->nrhs;
+  p.fin = CGFinish{op->d_cg, op->d_all_done, CG_FINISH_BETA};
   int* parts = rupd ? r_parts : nullptr;
   const bool half = x.prec == GB_F16;
   switch (op->Ls) {

@@ -425,4 +425,85 @@ __device__ __forceinline__ void block_reduce_rhs(const double (&v)[NV], int L5, 
   }
 }
 
+// ---------------------------------------------------------------------------------------
+// A reduction that ends with the CG's scalars: the last CTA to have written its partial sums
+// (found by a ticket in flags[kCGTicket]) adds all of them in a fixed order and updates the
+// scalars, which saves the launch of a kernel of a few microseconds that did only that.
+// ---------------------------------------------------------------------------------------
+enum { CG_FINISH_NONE = 0, CG_FINISH_ALPHA = 1, CG_FINISH_BETA = 2 };
+constexpr int kCGTicket = 5;
+struct CGFinish {
+  CGScalars* cg;
+  int* flags;  // op->d_all_done
+  int mode;
+};
+
+// True in every thread of the CTA that comes last of `ctas`; its partial sums (written by any of its
+// threads) and those of the others are then visible (read them past L1).  The ticket is back at 0.
+__device__ __forceinline__ bool last_cta(int* ticket, int ctas) {
+  __shared__ int last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(ticket, 1) == ctas - 1;
+    if (last) *ticket = 0;
+  }
+  __syncthreads();
+  if (last) __threadfence();
+  return last != 0;
+}
+
+// a = c / d (ConjugateGradient.h:160-165); a right-hand side that is done keeps a = 0
+__device__ __forceinline__ void cg_alpha_update(CGScalars& s, double d) {
+  s.d = d;
+  s.a = s.done ? 0.0 : s.c / d;
+}
+// cp = |r|^2, b = cp / c, convergence and reliable-update marks
+__device__ __forceinline__ void cg_beta_update(CGScalars& s, double cp) {
+  if (s.done) {
+    s.b = 0.0;
+    return;
+  }
+  s.cp = cp;
+  s.b = cp / s.c;
+  s.cprev = s.c;
+  s.c = cp;
+  s.iter += 1;
+  if (cp > s.maxres) s.maxres = cp;
+  if (cp <= s.rsq) s.done = 1;
+  else if (cp < s.delta * s.maxres) s.relup = 1;
+}
+
+// Called by every thread of every CTA of a reduction with partial sums [nparts][nrhs], after they are
+// written.  One (full) warp sums a right-hand side: strided sums of its lanes, then shuffles.
+__device__ __forceinline__ void cg_finish(const CGFinish& f, const double* partial, int nparts, int nrhs, int ctas) {
+  if (!last_cta(f.flags + kCGTicket, ctas)) return;
+  const int lane = threadIdx.x & 31, warps = blockDim.x >> 5, warp = threadIdx.x >> 5;
+  for (int r = warp; warp < warps && r < nrhs; r += warps) {
+    double s = 0;
+#pragma unroll 8
+    for (int b = lane; b < nparts; b += 32) s += __ldcg(partial + size_t(b) * nrhs + r);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0) {
+      CGScalars c = f.cg[r];
+      if (f.mode == CG_FINISH_ALPHA) cg_alpha_update(c, s);
+      else cg_beta_update(c, s);
+      f.cg[r] = c;
+    }
+  }
+  if (f.mode != CG_FINISH_BETA) return;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int nd = 0, nr = 0;
+    for (int k = 0; k < nrhs; k++) {
+      const int done = f.cg[k].done;
+      nd += done;
+      nr += f.cg[k].relup && !done;
+    }
+    f.flags[0] = nd == nrhs;
+    f.flags[1] = nr;
+  }
+}
+
 }  // namespace gb

@@ -222,7 +222,8 @@ int launch_scale(Op* op, HalfView z, double a, HalfView x, size_t n5, int halves
 int launch_copy(Op* op, HalfView dst, HalfView src, size_t n5);
 int launch_zero(Op* op, HalfView z, size_t n5);
 // reductions: partial sums per CTA, red_parts() of them per half
-int launch_norm2_partial(Op* op, HalfView x, size_t n5, double* partial, int halves = 1);
+// (finish: a CG_FINISH_* of gb_device.cuh, the CG scalars that the kernel's last CTA updates)
+int launch_norm2_partial(Op* op, HalfView x, size_t n5, double* partial, int halves = 1, int finish = 0);
 int launch_inner_partial(Op* op, HalfView a, HalfView b, size_t n5, double* partial, int halves = 1);
 int launch_axpy_norm_partial(Op* op, HalfView z, double a, HalfView x, HalfView y, size_t n5, double* partial,
                              int halves = 1);
@@ -238,7 +239,7 @@ int launch_m5d_pair(Op* op, HalfView psi, HalfView phi, HalfView chi, const doub
 // kind 0: |x|^2 ; 1: <x|y> ; 2: z = a x + y, |z|^2 ; 3: y -= a[rhs] x (the device CG
 // scalars), |y|^2
 int launch_reduce_pair(Op* op, int kind, HalfView x, HalfView y, HalfView z, double a, size_t n5, double* partial,
-                       int halves);
+                       int halves, int finish = 0);
 int launch_cg_p_pair(Op* op, HalfView p, HalfView r, size_t n5, int halves);
 int launch_cg_xp_pair(Op* op, HalfView psi, HalfView p, HalfView r, size_t n5, int update_p, int halves);
 int launch_axpby_pair(Op* op, HalfView z, double a, HalfView x, double b, HalfView y, size_t n5, int use_y, int halves);
@@ -272,7 +273,8 @@ int launch_zcol(Op* op, int prog, int dag, HalfView x, const HalfView* y, HalfVi
 // With r_upd (FP32 or FP16, nrhs dividing 16, the program MooeeDag - M5Ddag z that ends MpcDag)
 // the kernel does not store out: it applies the CG's residual update r -= a out (a per
 // right-hand side from op->d_cg) and writes per-CTA sums of |r|^2 [CTA][nrhs] into
-// op->d_partial, their count into *r_parts (0 when it could not fuse; out is then stored
+// op->d_partial, from which its last CTA updates the CG's b and convergence flags, and sets
+// *r_parts to their count (0 when it could not fuse; out is then stored
 // and the caller updates r).
 int launch_col(Op* op, int opa, int opb, int dag, HalfView x, HalfView y, HalfView out, double zc,
                const ColCoefsHost& h, HalfView* r_upd = nullptr, int* r_parts = nullptr);
@@ -304,14 +306,12 @@ int build_neighbours(Op* op);
 // CG kernels (gb_blas.cu)
 // init from device arrays ssq[nrhs] and cp[nrhs]
 int launch_cg_init(Op* op, const double* d_ssq, const double* d_cp, double tol, double delta);
-// a = c / d per rhs, d from partial sums [nparts][nrhs][nv] (nv = 2: inner-product
-// partials, real part first; nv = 1: norm partials)
-int launch_cg_alpha(Op* op, const double* partial, int nparts, int nv);
-// r -= a mmp ; partial |r|^2
+// a = c / d per rhs, d from the partial sums [nparts][nrhs] of a kernel that does not finish them
+int launch_cg_alpha(Op* op, const double* partial, int nparts);
+// r -= a mmp ; |r|^2 -> b and the convergence flags
 int launch_cg_r_update(Op* op, HalfView r, HalfView mmp, size_t n5, double* partial, int halves = 1);
 // psi += a p ; with update_p also p = b p + r
 int launch_cg_xp_update(Op* op, HalfView psi, HalfView p, HalfView r, size_t n5, int update_p, int halves = 1);
-int launch_cg_beta(Op* op, const double* partial_norm, int nparts);
 // p = b p + r
 int launch_cg_p_update(Op* op, HalfView p, HalfView r, size_t n5, int halves = 1);
 // after a reliable update: cp = c = maxres = cp_true ; b = cp_true / cprev

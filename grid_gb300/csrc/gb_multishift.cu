@@ -28,13 +28,13 @@ namespace gb {
 namespace {
 
 constexpr int kMaxShift = 32;
-constexpr int kMsBlocks = 1216;  // reduction CTAs (8 per SM)
+constexpr int kMsBlocks = 1216;  // CTAs of the vector kernels at most (8 per SM)
 
 struct MSState {
   double a, b, bp, c, cp, d, m0;
   int all_done, iter, frozen, pad1;  // frozen: every update done after all shifts converged
   double mass[kMaxShift], rsq[kMaxShift], z[kMaxShift][2], bs[kMaxShift], as[kMaxShift], zr[kMaxShift];
-  int iz, nshift;
+  int iz, nshift, ticket;
   int psi_upd[kMaxShift], ps_upd[kMaxShift], conv[kMaxShift], iters[kMaxShift];
 };
 
@@ -44,15 +44,17 @@ template <> struct Word<double2> {
   static __device__ __forceinline__ double2 axpby(R a, const double2& x, R b, const double2& y) {
     return make_double2(fma(a, x.x, b * y.x), fma(a, x.y, b * y.y));
   }
-  static __device__ __forceinline__ double dot(const double2& x, const double2& y) { return x.x * y.x + x.y * y.y; }
+  static __device__ __forceinline__ double dot(const double2& x, const double2& y, double s) {
+    return fma(x.x, y.x, fma(x.y, y.y, s));
+  }
 };
 template <> struct Word<float4> {
   using R = float;
   static __device__ __forceinline__ float4 axpby(R a, const float4& x, R b, const float4& y) {
     return make_float4(fmaf(a, x.x, b * y.x), fmaf(a, x.y, b * y.y), fmaf(a, x.z, b * y.z), fmaf(a, x.w, b * y.w));
   }
-  static __device__ __forceinline__ double dot(const float4& x, const float4& y) {
-    return double(x.x) * y.x + double(x.y) * y.y + double(x.z) * y.z + double(x.w) * y.w;
+  static __device__ __forceinline__ double dot(const float4& x, const float4& y, double s) {
+    return s + (double(x.x) * y.x + double(x.y) * y.y + double(x.z) * y.z + double(x.w) * y.w);
   }
 };
 
@@ -83,32 +85,115 @@ __device__ __forceinline__ void block_sum2(double a, double b, double* partial) 
   }
 }
 
-// partial: <x, y> and <x, x> (real parts)
-template <class V> __global__ void __launch_bounds__(256) ms_dot_kernel(const V* x, const V* y, size_t nw, double* partial) {
-  double s1 = 0, s2 = 0;
-  for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < nw; i += size_t(gridDim.x) * blockDim.x) {
-    const V a = x[i], b = y[i];
-    s1 += Word<V>::dot(a, b);
-    s2 += Word<V>::dot(a, a);
-  }
-  block_sum2(s1, s2, partial);
+// sum of partial[2 i + which] by the whole CTA (256 threads) in a fixed order (past L1: the last
+// CTA of a launch reads the others' sums)
+__device__ double sum_partials(const double* partial, int n, int which) {
+  __shared__ double sm[8];
+  double s = 0;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < n; i += blockDim.x) s += __ldcg(partial + 2 * i + which);
+  for (int o = 16; o; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
+  __syncthreads();
+  s = 0;
+  for (int w = 0; w < int(blockDim.x >> 5); w++) s += sm[w];
+  __syncthreads();
+  return s;
 }
 
-// r += b (mmp + m0 p); partial |r|^2
-template <class V>
-__global__ void __launch_bounds__(256) ms_r_kernel(V* r, const V* mmp, const V* p, size_t nw, const MSState* st,
+// after d = <p, A p>: d, b
+__device__ __forceinline__ void ms_mid(MSState* st, const double* partial, int nparts) {
+  const double s0 = sum_partials(partial, nparts, 0), s1 = sum_partials(partial, nparts, 1);
+  if (threadIdx.x) return;
+  if (st->all_done) {  // the update pass before this kernel applied the last psi update
+    st->frozen = 1;
+    return;
+  }
+  st->d = s0 + st->m0 * s1;
+  st->bp = st->b;
+  st->b = -st->cp / st->d;
+}
+
+// after r += b A p: c, z, bs, convergence, then the next iteration's coefficients; one lane of the
+// first warp per shift (kMaxShift = 32)
+__device__ __forceinline__ void ms_post(MSState* st, const double* partial, int nparts) {
+  const double c = sum_partials(partial, nparts, 0);
+  if (threadIdx.x >= 32) return;
+  const int s = threadIdx.x, ns = st->nshift;
+  const double b = st->b, bp = st->bp, a = st->a, cp = st->cp;
+  const int iz = 1 - st->iz, iter = st->iter + 1;
+  const bool mine = s < ns;
+  bool conv = mine ? st->conv[s] != 0 : true;
+  double bs = mine ? st->bs[s] : 0.0, znew = 1.0, zold = 1.0;
+  if (mine && s > 0) {
+    zold = st->z[s][1 - iz];
+    znew = st->z[s][iz];
+    if (!conv) {
+      const double z0 = zold, z1 = znew;
+      znew = z0 * z1 * bp / (b * a * (z1 - z0) + z1 * bp * (1.0 - (st->mass[s] - st->mass[0]) * b));
+      bs = b * znew / z0;
+    }
+  }
+  if (s == 0) bs = b;
+  if (mine) {
+    st->psi_upd[s] = !conv;  // psi_s -= bs_s ps_s in the next pass
+    if (!conv) {
+      st->iters[s] = iter;
+      // shift 0 keeps the z it was given at the set-up
+      const double z = s > 0 ? znew : st->z[0][iz];
+      if (c * z * z < st->rsq[s]) st->conv[s] = 1, conv = true;
+    }
+    st->ps_upd[s] = !conv;
+    if (s > 0) st->z[s][iz] = znew;
+    st->bs[s] = bs;
+    // next iteration's a, as, zr (ConjugateGradientMultiShift.h:196-217)
+    const double an = c / cp;
+    st->zr[s] = s > 0 ? znew : 1.0;
+    st->as[s] = s > 0 ? an * znew * bs / (zold * b) : an;
+  }
+  const bool all = __all_sync(0xffffffffu, conv);
+  if (s == 0) {
+    st->c = c;
+    st->iz = iz;
+    st->iter = iter;
+    st->all_done = all;
+    st->a = c / cp;
+    st->cp = c;
+  }
+}
+
+// partial: <x, y> and <x, x> (real parts).  MID: the last CTA to finish runs ms_mid.
+template <class V, bool MID>
+__global__ void __launch_bounds__(256) ms_dot_kernel(const V* x, const V* y, size_t nw, double* partial, MSState* st) {
+  if (MID && st->frozen) return;
+  double s1 = 0, s2 = 0;
+#pragma unroll 4
+  for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < nw; i += size_t(gridDim.x) * blockDim.x) {
+    const V a = x[i], b = y[i];
+    s1 = Word<V>::dot(a, b, s1);
+    s2 = Word<V>::dot(a, a, s2);
+  }
+  block_sum2(s1, s2, partial);
+  if (MID && last_cta(&st->ticket, gridDim.x)) ms_mid(st, partial, gridDim.x);
+}
+
+// r += b (mmp + m0 p); partial |r|^2.  POST: the last CTA to finish runs ms_post.
+template <class V, bool POST>
+__global__ void __launch_bounds__(256) ms_r_kernel(V* r, const V* mmp, const V* p, size_t nw, MSState* st,
                                                    double* partial) {
   using R = typename Word<V>::R;
   if (st->frozen) return;
   const R b = R(st->b), bm = R(st->b * st->m0);
   double s1 = 0;
+#pragma unroll 4
   for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < nw; i += size_t(gridDim.x) * blockDim.x) {
     V v = Word<V>::axpby(b, mmp[i], R(1), r[i]);
     v = Word<V>::axpby(bm, p[i], R(1), v);
     r[i] = v;
-    s1 += Word<V>::dot(v, v);
+    s1 = Word<V>::dot(v, v, s1);
   }
   block_sum2(s1, 0.0, partial);
+  if (POST && last_cta(&st->ticket, gridDim.x)) ms_post(st, partial, gridDim.x);
 }
 
 // the fused vector pass: psi_s -= bs_s ps_s (previous iteration), ps_s = zr_s r + as_s ps_s,
@@ -150,22 +235,6 @@ __global__ void __launch_bounds__(256) ms_setup_kernel(const V* src, const MSFie
   }
 }
 
-// sum of partial[2 i + which] by the whole CTA (256 threads) in a fixed order
-__device__ double sum_partials(const double* partial, int n, int which) {
-  __shared__ double sm[256];
-  double s = 0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) s += partial[2 * i + which];
-  sm[threadIdx.x] = s;
-  __syncthreads();
-  for (int st = blockDim.x / 2; st > 0; st >>= 1) {
-    if (threadIdx.x < st) sm[threadIdx.x] += sm[threadIdx.x + st];
-    __syncthreads();
-  }
-  const double r = sm[0];
-  __syncthreads();
-  return r;
-}
-
 // after the first A p: d, b, z, bs (ConjugateGradientMultiShift.h:152-176)
 __global__ void ms_init_kernel(MSState* st, const double* partial, int nparts) {
   const double s0 = sum_partials(partial, nparts, 0), s1 = sum_partials(partial, nparts, 1);
@@ -201,61 +270,6 @@ __global__ void ms_coef_kernel(MSState* st, const double* partial, int nparts) {
   st->cp = st->c;
 }
 
-// after d = <p, A p>: d, b
-__global__ void ms_mid_kernel(MSState* st, const double* partial, int nparts) {
-  if (st->frozen) return;  // uniform: read by every thread before any write
-  const double s0 = sum_partials(partial, nparts, 0), s1 = sum_partials(partial, nparts, 1);
-  if (threadIdx.x) return;
-  if (st->all_done) {  // the update pass before this kernel applied the last psi update
-    st->frozen = 1;
-    return;
-  }
-  st->d = s0 + st->m0 * s1;
-  st->bp = st->b;
-  st->b = -st->cp / st->d;
-}
-
-// after r += b A p: c, z, bs, convergence, then the next iteration's coefficients
-__global__ void ms_post_kernel(MSState* st, const double* partial, int nparts) {
-  if (st->frozen) return;
-  const double c = sum_partials(partial, nparts, 0);
-  if (threadIdx.x) return;
-  st->c = c;
-  const double b = st->b, bp = st->bp, a = st->a;
-  st->bs[0] = b;
-  const int iz = 1 - st->iz;
-  st->iz = iz;
-  st->iter++;
-  for (int s = 1; s < st->nshift; s++) {
-    if (st->conv[s]) continue;
-    const double z0 = st->z[s][1 - iz], z1 = st->z[s][iz];
-    st->z[s][iz] = z0 * z1 * bp / (b * a * (z1 - z0) + z1 * bp * (1.0 - (st->mass[s] - st->mass[0]) * b));
-    st->bs[s] = b * st->z[s][iz] / z0;
-  }
-  int all = 1;
-  for (int s = 0; s < st->nshift; s++) {
-    st->psi_upd[s] = !st->conv[s];  // psi_s -= bs_s ps_s in the next pass
-    if (!st->conv[s]) {
-      st->iters[s] = st->iter;
-      const double css = c * st->z[s][iz] * st->z[s][iz];
-      if (css < st->rsq[s]) st->conv[s] = 1;
-      else all = 0;
-    }
-    st->ps_upd[s] = !st->conv[s];
-  }
-  st->all_done = all;
-  // next iteration's a, as, zr (ConjugateGradientMultiShift.h:196-217)
-  const double an = c / st->cp;
-  st->a = an;
-  st->as[0] = an;
-  st->zr[0] = 1.0;
-  for (int s = 1; s < st->nshift; s++) {
-    st->zr[s] = st->z[s][iz];
-    st->as[s] = an * st->z[s][iz] * st->bs[s] / (st->z[s][1 - iz] * b);
-  }
-  st->cp = c;
-}
-
 struct Timer {
   std::chrono::steady_clock::time_point t0 = std::chrono::steady_clock::now();
   double seconds() const { return std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count(); }
@@ -268,30 +282,41 @@ template <class V> struct MS {
   size_t nw;
   double* partial;
   MSState* st;
+  // CTAs of the reductions: 4 words per thread before the 8 CTAs per SM are reached, because the FP64
+  // block sum at a CTA's end costs as much as several words
   unsigned blocks() const {
+    const size_t b = (nw + 1023) / 1024;
+    return unsigned(b < size_t(kMsBlocks) ? b : size_t(kMsBlocks));
+  }
+  unsigned update_blocks() const {
     const size_t b = (nw + 255) / 256;
     return unsigned(b < size_t(kMsBlocks) ? b : size_t(kMsBlocks));
   }
-  int dot(const Field* x, const Field* y) {
-    ms_dot_kernel<V><<<blocks(), 256, 0, op->stream>>>(static_cast<const V*>(x->data), static_cast<const V*>(y->data), nw,
-                                                      partial);
+  int dot(const Field* x, const Field* y, bool mid = false) {
+    const V* a = static_cast<const V*>(x->data);
+    const V* b = static_cast<const V*>(y->data);
+    if (mid) ms_dot_kernel<V, true><<<blocks(), 256, 0, op->stream>>>(a, b, nw, partial, st);
+    else ms_dot_kernel<V, false><<<blocks(), 256, 0, op->stream>>>(a, b, nw, partial, st);
     GB_CHECK_CUDA(cudaGetLastError());
     return GB_OK;
   }
-  int r_update(Field* r, const Field* mmp, const Field* p) {
-    ms_r_kernel<V><<<blocks(), 256, 0, op->stream>>>(static_cast<V*>(r->data), static_cast<const V*>(mmp->data),
-                                                    static_cast<const V*>(p->data), nw, st, partial);
+  int r_update(Field* r, const Field* mmp, const Field* p, bool post = false) {
+    V* a = static_cast<V*>(r->data);
+    const V* b = static_cast<const V*>(mmp->data);
+    const V* c = static_cast<const V*>(p->data);
+    if (post) ms_r_kernel<V, true><<<blocks(), 256, 0, op->stream>>>(a, b, c, nw, st, partial);
+    else ms_r_kernel<V, false><<<blocks(), 256, 0, op->stream>>>(a, b, c, nw, st, partial);
     GB_CHECK_CUDA(cudaGetLastError());
     return GB_OK;
   }
   int update(Field* p, const Field* r, const MSFields& f, int do_p) {
-    ms_update_kernel<V><<<blocks(), 256, 0, op->stream>>>(static_cast<V*>(p->data), static_cast<const V*>(r->data), f,
+    ms_update_kernel<V><<<update_blocks(), 256, 0, op->stream>>>(static_cast<V*>(p->data), static_cast<const V*>(r->data), f,
                                                          nw, st, do_p);
     GB_CHECK_CUDA(cudaGetLastError());
     return GB_OK;
   }
   int setup(const Field* src, const MSFields& f) {
-    ms_setup_kernel<V><<<blocks(), 256, 0, op->stream>>>(static_cast<const V*>(src->data), f, nw, st);
+    ms_setup_kernel<V><<<update_blocks(), 256, 0, op->stream>>>(static_cast<const V*>(src->data), f, nw, st);
     GB_CHECK_CUDA(cudaGetLastError());
     return GB_OK;
   }
@@ -372,10 +397,8 @@ int multishift(Op* op, int kind, Field* src, int ns, const double* shifts, const
     for (int j = 0; j < m; j++) {
       GB_TRY(ms.update(p, r, f, 1));  // psi (previous), ps, p
       GB_TRY(op_hermop(op, kind, p, mmp));
-      GB_TRY(ms.dot(p, mmp));
-      GB_TRY(ms.scalar(ms_mid_kernel));
-      GB_TRY(ms.r_update(r, mmp, p));
-      GB_TRY(ms.scalar(ms_post_kernel));
+      GB_TRY(ms.dot(p, mmp, true));
+      GB_TRY(ms.r_update(r, mmp, p, true));
     }
     k += m;
     GB_CHECK_CUDA(cudaMemcpyAsync(hst, st, sizeof(MSState), cudaMemcpyDeviceToHost, op->stream));

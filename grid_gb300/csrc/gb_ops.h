@@ -57,8 +57,8 @@ int op_mooee_inv(Op* op, Field* in, Field* out, int dag);
 // number of CTA sums written, or to 0 when it did not.
 // r_upd, r_parts (MpcDag only, for the CG): when both are non-null, the last kernel may
 // instead of storing out apply r_upd -= a out (a: the CG scalars of op) and reduce
-// |r_upd|^2 into op->d_partial ([CTA][nrhs]); *r_parts is the number of CTA sums written, or
-// 0 when it stored out and left r_upd alone
+// |r_upd|^2, from which it updates the CG's b and convergence flags; *r_parts is the number of CTA
+// sums, or 0 when it stored out and left r_upd and the scalars alone
 int op_mpc(Op* op, Field* in, Field* out, int dag, int* norm_parts = nullptr, Field* r_upd = nullptr,
            int* r_parts = nullptr);
 int op_mpcdagmpc(Op* op, Field* in, Field* out);

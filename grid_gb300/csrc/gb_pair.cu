@@ -234,11 +234,13 @@ int launch_m5d_pair(Op* op, HalfView psi, HalfView phi, HalfView chi, const doub
 template <class T, int KIND>
 __global__ void __launch_bounds__(512) reduce_pair_kernel(const PairShape sh, const void* x, const float2* xn,
                                                           const void* y, const float2* yn, void* z, float2* zn,
-                                                          double a, const CGScalars* cg, size_t np, double* partial) {
+                                                          double a, const CGScalars* cg, size_t np, double* partial,
+                                                          const CGFinish fin) {
   constexpr int NV = KIND == 1 ? 2 : 1;
   x = half_at<T>(x, np); xn = norms_at(xn, np);
   y = half_at<T>(y, np); yn = norms_at(yn, np);
   z = half_at<T>(z, np); zn = norms_at(zn, np);
+  const double* const all = partial;
   partial += size_t(blockIdx.y) * gridDim.x * sh.nrhs * NV;
   double v0[NV], v1[NV];
 #pragma unroll
@@ -286,6 +288,7 @@ __global__ void __launch_bounds__(512) reduce_pair_kernel(const PairShape sh, co
     }
   }
   block_reduce_pairs<NV>(v0, v1, sh.L5, sh.Ls, sh.nrhs, partial);
+  if (fin.mode != CG_FINISH_NONE) cg_finish(fin, all, gridDim.x * gridDim.y, sh.nrhs, gridDim.x * gridDim.y);
 }
 
 // grid of the pair reductions: blockDim a multiple of L5/2 (about 256, at most 512 for
@@ -308,7 +311,8 @@ int red_grid_pair(Op* op, size_t np, int* blocks, int* threads) {
 }
 
 template <class T, int KIND>
-static int reduce_pair_t(Op* op, HalfView x, HalfView y, HalfView z, double a, size_t n5, double* partial, int halves) {
+static int reduce_pair_t(Op* op, HalfView x, HalfView y, HalfView z, double a, size_t n5, double* partial, int halves,
+                         int finish) {
   int g, B;
   const size_t np = n5 >> 1;
   GB_TRY(red_grid_pair(op, np, &g, &B));
@@ -317,19 +321,19 @@ static int reduce_pair_t(Op* op, HalfView x, HalfView y, HalfView z, double a, s
   const size_t smem = size_t(NV) * (op->nrhs == 1 ? 32 : 2 * B) * sizeof(double);
   reduce_pair_kernel<T, KIND><<<dim3(g, halves), B, smem, op->stream>>>(
       sh, x.data, reinterpret_cast<const float2*>(x.norms), y.data, reinterpret_cast<const float2*>(y.norms), z.data,
-      reinterpret_cast<float2*>(z.norms), a, op->d_cg, np, partial);
+      reinterpret_cast<float2*>(z.norms), a, op->d_cg, np, partial, CGFinish{op->d_cg, op->d_all_done, finish});
   GB_CHECK_CUDA(cudaGetLastError());
   return GB_OK;
 }
 
 int launch_reduce_pair(Op* op, int kind, HalfView x, HalfView y, HalfView z, double a, size_t n5, double* partial,
-                       int halves) {
+                       int halves, int finish) {
   const bool h = x.prec == GB_F16;
   switch (kind) {
-    case 0: return h ? reduce_pair_t<__half, 0>(op, x, y, z, a, n5, partial, halves) : reduce_pair_t<float, 0>(op, x, y, z, a, n5, partial, halves);
-    case 1: return h ? reduce_pair_t<__half, 1>(op, x, y, z, a, n5, partial, halves) : reduce_pair_t<float, 1>(op, x, y, z, a, n5, partial, halves);
-    case 2: return h ? reduce_pair_t<__half, 2>(op, x, y, z, a, n5, partial, halves) : reduce_pair_t<float, 2>(op, x, y, z, a, n5, partial, halves);
-    case 3: return h ? reduce_pair_t<__half, 3>(op, x, y, z, a, n5, partial, halves) : reduce_pair_t<float, 3>(op, x, y, z, a, n5, partial, halves);
+    case 0: return h ? reduce_pair_t<__half, 0>(op, x, y, z, a, n5, partial, halves, finish) : reduce_pair_t<float, 0>(op, x, y, z, a, n5, partial, halves, finish);
+    case 1: return h ? reduce_pair_t<__half, 1>(op, x, y, z, a, n5, partial, halves, finish) : reduce_pair_t<float, 1>(op, x, y, z, a, n5, partial, halves, finish);
+    case 2: return h ? reduce_pair_t<__half, 2>(op, x, y, z, a, n5, partial, halves, finish) : reduce_pair_t<float, 2>(op, x, y, z, a, n5, partial, halves, finish);
+    case 3: return h ? reduce_pair_t<__half, 3>(op, x, y, z, a, n5, partial, halves, finish) : reduce_pair_t<float, 3>(op, x, y, z, a, n5, partial, halves, finish);
   }
   return GB_ERR_BAD_ARG;
 }

@@ -43,14 +43,12 @@ Parts parts_of(Op* op, const Field* f) {
 // d = |ap|^2 (ap = M p or Mpc p) -> a
 int cg_alpha_norm(Op* op, Field* ap) {
   Parts P = parts_of(op, ap);
-  GB_TRY(launch_norm2_partial(op, half_view(ap, 0), ap->n5, op->d_partial, P.halves));
-  return launch_cg_alpha(op, op->d_partial, P.g * P.halves, 1);
+  return launch_norm2_partial(op, half_view(ap, 0), ap->n5, op->d_partial, P.halves, 1 /* CG_FINISH_ALPHA */);
 }
 // r -= a mmp ; cp = |r|^2 -> b
 int cg_r_update(Op* op, Field* r, Field* mmp) {
   Parts P = parts_of(op, r);
-  GB_TRY(launch_cg_r_update(op, half_view(r, 0), half_view(mmp, 0), r->n5, op->d_partial, P.halves));
-  return launch_cg_beta(op, op->d_partial, P.g * P.halves);
+  return launch_cg_r_update(op, half_view(r, 0), half_view(mmp, 0), r->n5, op->d_partial, P.halves);
 }
 // One CG matrix step on p: A = MdagM (kind 0) or MpcDagMpc (kind 1) with d = |M p|^2
 // (|Mpc p|^2) -> a, then r -= a A p, cp = |r|^2 -> b.  For a FP32 / FP16 Moebius Schur
@@ -67,11 +65,11 @@ int cg_matrix_step(Op* op, int kind, Field* p, Field* mmp, Field* r) {
     GB_TRY(ws_get(op, GB_ODD, p->prec, WS_MPCDAGMPC, &z));
     int dparts = 0;
     GB_TRY(op_mpc(op, p, z, 0, &dparts));
-    if (dparts > 0) GB_TRY(launch_cg_alpha(op, op->d_partial, dparts, 1));
+    if (dparts > 0) GB_TRY(launch_cg_alpha(op, op->d_partial, dparts));
     else GB_TRY(cg_alpha_norm(op, z));
     GB_TRY(op_mpc(op, z, mmp, 1, nullptr, r, &rparts));
   }
-  if (rparts > 0) return launch_cg_beta(op, op->d_partial, rparts);
+  if (rparts > 0) return GB_OK;  // r, |r|^2 and b are done
   return cg_r_update(op, r, mmp);
 }
 // psi += a p ; with update_p also p = b p + r
