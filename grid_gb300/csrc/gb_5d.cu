@@ -31,8 +31,13 @@ struct M5Params {
 };
 
 template <class T, bool DAG, bool ZTERM>
-__global__ void __launch_bounds__(256) m5d_kernel(const M5Params p, const Coef5<typename Arith<T>::type> c) {
+__global__ void __launch_bounds__(256) m5d_kernel(const M5Params p0, const Coef5<typename Arith<T>::type> c) {
   using R = typename Arith<T>::type;
+  M5Params p = p0;
+  pdl_wait();
+  p.psi = after_wait(p.psi);
+  p.phi = after_wait(p.phi);
+  p.z = after_wait(p.z);
   const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= p.n5) return;
   const int s5 = int(i % p.L5);
@@ -78,7 +83,7 @@ static int launch_m5d_t(Op* op, const M5Params& p, const double* lower, const do
   Coef5<R> c;
   for (int s = 0; s < op->Ls; s++) { c.d[s] = R(diag[s]); c.u[s] = R(upper[s]); c.l[s] = R(lower[s]); }
   const unsigned blocks = unsigned((p.n5 + 255) / 256);
-  m5d_kernel<T, DAG, ZTERM><<<blocks, 256, 0, op->stream>>>(p, c);
+  launch_pdl(m5d_kernel<T, DAG, ZTERM>, blocks, 256, 0, op->stream, p, c);
   GB_CHECK_CUDA(cudaGetLastError());
   return GB_OK;
 }
@@ -155,7 +160,10 @@ template <> struct VecOps<float4> {
 // Ls with the column in registers; LS == 0: runtime Ls, the forward sweep's values are
 // re-read from the output.
 template <class V, bool DAG, int LS>
-__global__ void __launch_bounds__(256) mooee_inv_kernel(const InvParams p, const LduCoef<typename VecOps<V>::R> c) {
+__global__ void __launch_bounds__(256) mooee_inv_kernel(const InvParams p0, const LduCoef<typename VecOps<V>::R> c) {
+  InvParams p = p0;
+  pdl_wait();
+  p.in = after_wait(p.in);
   using Ops = VecOps<V>;
   using R = typename Ops::R;
   const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -255,7 +263,10 @@ __global__ void __launch_bounds__(128) mooee_inv_half_kernel(const InvParams p, 
 // of that component is Ls/2 float4 vectors (re_s, re_s+1, im_s, im_s+1), kept in
 // registers for compile-time LS (LS == 0: runtime Ls, column re-read from the output).
 template <bool DAG, int LS>
-__global__ void __launch_bounds__(256) mooee_inv_pair_kernel(const InvParams p, const LduCoef<float> c) {
+__global__ void __launch_bounds__(256) mooee_inv_pair_kernel(const InvParams p0, const LduCoef<float> c) {
+  InvParams p = p0;
+  pdl_wait();
+  p.in = after_wait(p.in);
   const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (t >= p.nq * 12) return;
   const int k = int(t / p.nq);
@@ -355,11 +366,11 @@ template <bool DAG> static int launch_inv_pair(Op* op, const InvParams& p, const
   const unsigned blocks = unsigned((n + 255) / 256);
   switch (op->Ls) {
 #define GB_INVP_CASE(L) \
-  case L: mooee_inv_pair_kernel<DAG, L><<<blocks, 256, 0, op->stream>>>(p, c); break;
+  case L: launch_pdl(mooee_inv_pair_kernel<DAG, L>, blocks, 256, 0, op->stream, p, c); break;
     GB_INVP_CASE(2) GB_INVP_CASE(4) GB_INVP_CASE(6) GB_INVP_CASE(8) GB_INVP_CASE(10) GB_INVP_CASE(12)
     GB_INVP_CASE(14) GB_INVP_CASE(16) GB_INVP_CASE(20) GB_INVP_CASE(24) GB_INVP_CASE(32)
 #undef GB_INVP_CASE
-    default: mooee_inv_pair_kernel<DAG, 0><<<blocks, 256, 0, op->stream>>>(p, c); break;
+    default: launch_pdl(mooee_inv_pair_kernel<DAG, 0>, blocks, 256, 0, op->stream, p, c); break;
   }
   GB_CHECK_CUDA(cudaGetLastError());
   return GB_OK;
@@ -371,11 +382,11 @@ static int launch_inv_v(Op* op, const InvParams& p, const LduCoef<typename VecOp
   const unsigned blocks = unsigned((n + 255) / 256);
   switch (op->Ls) {
 #define GB_INV_CASE(L) \
-  case L: mooee_inv_kernel<V, DAG, L><<<blocks, 256, 0, op->stream>>>(p, c); break;
+  case L: launch_pdl(mooee_inv_kernel<V, DAG, L>, blocks, 256, 0, op->stream, p, c); break;
     GB_INV_CASE(4) GB_INV_CASE(6) GB_INV_CASE(8) GB_INV_CASE(10) GB_INV_CASE(12) GB_INV_CASE(16)
     GB_INV_CASE(20) GB_INV_CASE(24) GB_INV_CASE(32)
 #undef GB_INV_CASE
-    default: mooee_inv_kernel<V, DAG, 0><<<blocks, 256, 0, op->stream>>>(p, c); break;
+    default: launch_pdl(mooee_inv_kernel<V, DAG, 0>, blocks, 256, 0, op->stream, p, c); break;
   }
   GB_CHECK_CUDA(cudaGetLastError());
   return GB_OK;

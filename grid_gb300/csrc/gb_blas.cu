@@ -20,6 +20,7 @@ namespace gb {
 template <bool USE_Y>
 __global__ void __launch_bounds__(256) axpby_kernel(double2* z, double a, const double2* x, double b, const double2* y,
                                                     size_t words) {
+  pdl_wait();
   const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= words) return;
   const double2 v = x[i];
@@ -53,7 +54,7 @@ int launch_axpby(Op* op, HalfView z, double a, HalfView x, double b, HalfView y,
   }
   if (z.prec != GB_F64) return launch_axpby_pair(op, z, a, x, b, y, n5, 1, halves);
   const size_t words = n5 * 12 * halves;
-  axpby_kernel<true><<<nblk(words), 256, 0, op->stream>>>(static_cast<double2*>(z.data), a,
+  launch_pdl(axpby_kernel<true>, nblk(words), 256, 0, op->stream, static_cast<double2*>(z.data), a,
                                                           static_cast<const double2*>(x.data), b,
                                                           static_cast<const double2*>(y.data), words);
   GB_CHECK_CUDA(cudaGetLastError());
@@ -67,7 +68,7 @@ int launch_scale(Op* op, HalfView z, double a, HalfView x, size_t n5, int halves
   }
   if (z.prec != GB_F64) return launch_axpby_pair(op, z, a, x, 0.0, x, n5, 0, halves);
   const size_t words = n5 * 12 * halves;
-  axpby_kernel<false><<<nblk(words), 256, 0, op->stream>>>(static_cast<double2*>(z.data), a,
+  launch_pdl(axpby_kernel<false>, nblk(words), 256, 0, op->stream, static_cast<double2*>(z.data), a,
                                                            static_cast<const double2*>(x.data), 0.0, nullptr, words);
   GB_CHECK_CUDA(cudaGetLastError());
   return GB_OK;
@@ -117,6 +118,9 @@ template <class T, int KIND>
 __global__ void __launch_bounds__(256) reduce_kernel(const RedShape sh, const void* x, const float* xn, const void* y,
                                                      const float* yn, void* z, float* zn, double a,
                                                      const CGScalars* cg, size_t n5, double* partial, const CGFinish fin) {
+  pdl_wait();
+  x = after_wait(x);
+  y = after_wait(y);
   using R = typename Arith<T>::type;
   constexpr int NV = KIND == 1 ? 2 : 1;
   const size_t half = size_t(blockIdx.y) * n5 * 12 * sizeof(double2);  // blockIdx.y: the checkerboard
@@ -201,7 +205,7 @@ static int reduce_t(Op* op, HalfView x, HalfView y, HalfView z, double a, size_t
   RedShape sh{op->L5, op->Ls, op->nrhs};
   const int NV = KIND == 1 ? 2 : 1;
   size_t smem = size_t(NV) * (op->nrhs == 1 ? 32 : B) * sizeof(double);
-  reduce_kernel<T, KIND><<<dim3(g, halves), B, smem, op->stream>>>(sh, x.data, x.norms, y.data, y.norms, z.data, z.norms, a, op->d_cg,
+  launch_pdl(reduce_kernel<T, KIND>, dim3(g, halves), B, smem, op->stream, sh, x.data, x.norms, y.data, y.norms, z.data, z.norms, a, op->d_cg,
                                                      n5, partial, CGFinish{op->d_cg, op->d_all_done, finish});
   GB_CHECK_CUDA(cudaGetLastError());
   return GB_OK;
@@ -233,6 +237,7 @@ int launch_cg_r_update(Op* op, HalfView r, HalfView mmp, size_t n5, double* part
 
 // partial: [nparts][nrhs][nv] -> out[nrhs][nv]; one CTA per rhs, fixed summation order
 __global__ void reduce_final_kernel(const double* partial, int nparts, int nrhs, int nv, double* out) {
+  pdl_wait();
   __shared__ double sm[256][2];
   const int rhs = blockIdx.x, t = threadIdx.x;
   double s0 = 0, s1 = 0;
@@ -254,7 +259,7 @@ __global__ void reduce_final_kernel(const double* partial, int nparts, int nrhs,
 }
 
 int launch_reduce_final(Op* op, const double* partial, int nparts, int nv, double* out) {
-  reduce_final_kernel<<<op->nrhs, 256, 0, op->stream>>>(partial, nparts, op->nrhs, nv, out);
+  launch_pdl(reduce_final_kernel, op->nrhs, 256, 0, op->stream, partial, nparts, op->nrhs, nv, out);
   GB_CHECK_CUDA(cudaGetLastError());
   return GB_OK;
 }
@@ -314,6 +319,7 @@ __device__ double cta_sum_fixed(const double* partial, int nparts, int stride, i
 // One CTA per right-hand side (one CTA for all took 26-30 us at 12 right-hand sides), of 256
 // threads, 1024 above 2048 partial sums (one per CTA of an FP32 Dhop)
 __global__ void __launch_bounds__(1024) cg_alpha_kernel(CGScalars* cg, const double* partial, int nparts, int nrhs) {
+  pdl_wait();
   const int r = blockIdx.x;
   const double d = cta_sum_fixed(partial, nparts, nrhs, r);
   if (threadIdx.x == 0) cg_alpha_update(cg[r], d);
@@ -343,7 +349,7 @@ int launch_cg_init(Op* op, const double* d_ssq, const double* d_cp, double tol, 
 // the scalar kernels reduce the per-block partial sums themselves, in a fixed order
 static inline int sum_threads(int nparts) { return nparts > 2048 ? 1024 : 256; }
 int launch_cg_alpha(Op* op, const double* partial, int nparts) {
-  cg_alpha_kernel<<<op->nrhs, sum_threads(nparts), 0, op->stream>>>(op->d_cg, partial, nparts, op->nrhs);
+  launch_pdl(cg_alpha_kernel, op->nrhs, sum_threads(nparts), 0, op->stream, op->d_cg, partial, nparts, op->nrhs);
   GB_CHECK_CUDA(cudaGetLastError());
   return GB_OK;
 }
@@ -381,6 +387,7 @@ int launch_cg_relup_reset(Op* op, const double* d_cp_true) {
 // over both checkerboards of a full field
 __global__ void __launch_bounds__(256) cg_p_kernel(const RedShape sh, double2* p, const double2* r, const CGScalars* cg,
                                                    size_t n5) {
+  pdl_wait();
   const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n5) return;
   const double b = cg[int(i % sh.L5) / sh.Ls].b;
@@ -392,7 +399,7 @@ __global__ void __launch_bounds__(256) cg_p_kernel(const RedShape sh, double2* p
 int launch_cg_p_update(Op* op, HalfView p, HalfView r, size_t n5, int halves) {
   if (p.prec != GB_F64) return launch_cg_p_pair(op, p, r, n5, halves);
   RedShape sh{op->L5, op->Ls, op->nrhs};
-  cg_p_kernel<<<dim3(nblk(n5), 12 * halves), 256, 0, op->stream>>>(sh, static_cast<double2*>(p.data),
+  launch_pdl(cg_p_kernel, dim3(nblk(n5), 12 * halves), 256, 0, op->stream, sh, static_cast<double2*>(p.data),
                                                                   static_cast<const double2*>(r.data), op->d_cg, n5);
   GB_CHECK_CUDA(cudaGetLastError());
   return GB_OK;
@@ -403,6 +410,7 @@ int launch_cg_p_update(Op* op, HalfView p, HalfView r, size_t n5, int halves) {
 template <bool PUPD>
 __global__ void __launch_bounds__(256) cg_xp_kernel(const RedShape sh, double2* psi, double2* p, const double2* r,
                                                     const CGScalars* cg, size_t n5) {
+  pdl_wait();
   const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n5) return;
   const CGScalars& c = cg[int(i % sh.L5) / sh.Ls];
@@ -428,8 +436,8 @@ int launch_cg_xp_update(Op* op, HalfView psi, HalfView p, HalfView r, size_t n5,
   auto* pp = static_cast<double2*>(p.data);
   auto* rr = static_cast<const double2*>(r.data);
   const dim3 grid(nblk(n5), 12 * halves);
-  if (update_p) cg_xp_kernel<true><<<grid, 256, 0, op->stream>>>(sh, x, pp, rr, op->d_cg, n5);
-  else cg_xp_kernel<false><<<grid, 256, 0, op->stream>>>(sh, x, pp, rr, op->d_cg, n5);
+  if (update_p) launch_pdl(cg_xp_kernel<true>, grid, 256, 0, op->stream, sh, x, pp, rr, op->d_cg, n5);
+  else launch_pdl(cg_xp_kernel<false>, grid, 256, 0, op->stream, sh, x, pp, rr, op->d_cg, n5);
   GB_CHECK_CUDA(cudaGetLastError());
   return GB_OK;
 }
@@ -465,6 +473,7 @@ template <> struct Canon2<float> { using type = float2; };
 // a shared tile as the export it measured 3-20 % slower)
 template <class T, class CR>
 __global__ void __launch_bounds__(256) import_kernel(const GeoParams g, const CR* canon, void* dev, float* devn, int full) {
+  pdl_wait();
   using R = typename Arith<T>::type;
   using C2 = typename Canon2<CR>::type;
   const size_t n5 = size_t(g.half4) * g.L5;
@@ -566,6 +575,9 @@ template <> struct LayoutPlanes<__half> {
 template <class T, class CR>
 __global__ void __launch_bounds__(256) export_kernel(const GeoParams g, CR* canon, const void* dev, const float* devn,
                                                      int full) {
+  pdl_wait();
+  dev = after_wait(dev);
+  devn = after_wait(devn);
   using P = LayoutPlanes<T>;
   using C2 = typename Canon2<CR>::type;
   __shared__ typename P::C tile[kLayoutSites * 13];
@@ -613,9 +625,9 @@ template <class CR> static int import_p(Op* op, const CR* canon, HalfView v, int
   const GeoParams g = geo(op);
   const dim3 blocks(nblk(op->n5()), full ? 2 : 1);
   switch (v.prec) {
-    case GB_F64: import_kernel<double, CR><<<blocks, 256, 0, op->stream>>>(g, canon, v.data, v.norms, full); break;
-    case GB_F32: import_kernel<float, CR><<<blocks, 256, 0, op->stream>>>(g, canon, v.data, v.norms, full); break;
-    case GB_F16: import_kernel<__half, CR><<<blocks, 256, 0, op->stream>>>(g, canon, v.data, v.norms, full); break;
+    case GB_F64: launch_pdl(import_kernel<double, CR>, blocks, 256, 0, op->stream, g, canon, v.data, v.norms, full); break;
+    case GB_F32: launch_pdl(import_kernel<float, CR>, blocks, 256, 0, op->stream, g, canon, v.data, v.norms, full); break;
+    case GB_F16: launch_pdl(import_kernel<__half, CR>, blocks, 256, 0, op->stream, g, canon, v.data, v.norms, full); break;
   }
   GB_CHECK_CUDA(cudaGetLastError());
   return GB_OK;
@@ -624,9 +636,9 @@ template <class CR> static int export_p(Op* op, CR* canon, HalfView v, int full)
   const GeoParams g = geo(op);
   const dim3 blocks(unsigned((op->n5() + kLayoutSites - 1) / kLayoutSites), full ? 2 : 1);
   switch (v.prec) {
-    case GB_F64: export_kernel<double, CR><<<blocks, 256, 0, op->stream>>>(g, canon, v.data, v.norms, full); break;
-    case GB_F32: export_kernel<float, CR><<<blocks, 256, 0, op->stream>>>(g, canon, v.data, v.norms, full); break;
-    case GB_F16: export_kernel<__half, CR><<<blocks, 256, 0, op->stream>>>(g, canon, v.data, v.norms, full); break;
+    case GB_F64: launch_pdl(export_kernel<double, CR>, blocks, 256, 0, op->stream, g, canon, v.data, v.norms, full); break;
+    case GB_F32: launch_pdl(export_kernel<float, CR>, blocks, 256, 0, op->stream, g, canon, v.data, v.norms, full); break;
+    case GB_F16: launch_pdl(export_kernel<__half, CR>, blocks, 256, 0, op->stream, g, canon, v.data, v.norms, full); break;
   }
   GB_CHECK_CUDA(cudaGetLastError());
   return GB_OK;

@@ -299,6 +299,7 @@ __device__ __forceinline__ void col_issue(const float4* x, float4* tile, size_t 
 
 template <int LS, bool DAG, int OPA, int OPB, bool RUPD>
 __global__ void __launch_bounds__(12 * kColPipeQ) col_pipe_kernel(const ColParams p, const ColCoef<LS> c) {
+  pdl_wait();
   constexpr int Q = kColPipeQ, H = LS / 2, ST = col_stride<LS>(), NIN = OPB != COLB_NONE ? 2 : 1;
   constexpr int TILE = 12 * Q * ST;   // float4 of one input tile
   extern __shared__ float4 col_ring[];  // [kColStages][NIN][12][Q][ST]
@@ -438,6 +439,7 @@ __device__ __forceinline__ void col_decode_half(const uint4* raw, const float* r
 // col_pipe_kernel.
 template <int LS, bool DAG, int OPA, int OPB, bool RUPD>
 __global__ void __launch_bounds__(12 * kColPipeQ) col_pipe_half_kernel(const ColParams p, const ColCoef<LS> c) {
+  pdl_wait();
   constexpr int Q = kColPipeQ, H = LS / 2, ST = col_stride<LS>(), NIN = OPB != COLB_NONE ? 2 : 1;
   constexpr int NRING = NIN + (RUPD ? 1 : 0);  // raw inputs staged per tile
   constexpr int RAW = 6 * Q * H;      // uint4 of one input's raw tile
@@ -571,7 +573,7 @@ static int col_pipe_go(Op* op, const ColParams& p, const ColCoef<LS>& c, int* r_
   size_t slots = size_t(per_sm.load()) * size_t(sms.load());
   if (RUPD && slots > size_t(2) * kRedBlocks) slots = size_t(2) * kRedBlocks;  // the partial buffer's [CTA][nrhs]
   const unsigned blocks = unsigned(ntiles < slots ? ntiles : slots);
-  col_pipe_kernel<LS, DAG, OPA, OPB, RUPD><<<blocks, 12 * kColPipeQ, smem, op->stream>>>(p, c);
+  launch_pdl(col_pipe_kernel<LS, DAG, OPA, OPB, RUPD>, blocks, 12 * kColPipeQ, smem, op->stream, p, c);
   GB_CHECK_CUDA(cudaGetLastError());
   if (r_parts) *r_parts = RUPD ? int(blocks) : 0;
   return GB_OK;
@@ -600,7 +602,7 @@ static int col_pipe_half_go(Op* op, const ColParams& p, const ColCoef<LS>& c, in
   size_t slots = size_t(per_sm.load()) * size_t(sms.load());
   if (RUPD && slots > size_t(2) * kRedBlocks) slots = size_t(2) * kRedBlocks;  // the partial buffer's [CTA][nrhs]
   const unsigned blocks = unsigned(ntiles < slots ? ntiles : slots);
-  col_pipe_half_kernel<LS, DAG, OPA, OPB, RUPD><<<blocks, 12 * Q, smem, op->stream>>>(p, c);
+  launch_pdl(col_pipe_half_kernel<LS, DAG, OPA, OPB, RUPD>, blocks, 12 * Q, smem, op->stream, p, c);
   GB_CHECK_CUDA(cudaGetLastError());
   if (r_parts) *r_parts = RUPD ? int(blocks) : 0;
   return GB_OK;

@@ -7,6 +7,7 @@
 
 #include "gb_df64.cuh"
 #include "gb_internal.h"
+#include "gb_launch.cuh"
 
 namespace gb {
 

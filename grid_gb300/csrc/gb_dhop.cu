@@ -495,7 +495,7 @@ __device__ __forceinline__ void dhop_pair_step(const DhopParams& p, const int (&
 // (p: the kernel's __grid_constant__ parameter, so the coefficient arrays are indexed in
 // the parameter bank, not copied to local memory)
 template <int MODE>
-__device__ __forceinline__ float2 dhop_mooee_epilogue(const DhopParams& p, size_t np, size_t q, int sp,
+__device__ __forceinline__ float2 dhop_mooee_epilogue(const DhopParams& p, const void* x5, size_t np, size_t q, int sp,
                                                       const Pair12& acc) {
   const int hs = p.Ls >> 1;
   const int psb = MODE == 1 ? sp : sp % hs;  // pair index within the rhs block
@@ -503,7 +503,7 @@ __device__ __forceinline__ float2 dhop_mooee_epilogue(const DhopParams& p, size_
   const size_t qb = q - psb;                 // the block's first pair
   const size_t qprev = psb == 0 ? qb + hs - 1 : q - 1;
   const size_t qnext = psb == hs - 1 ? qb : q + 1;
-  const float4* x = static_cast<const float4*>(p.x5);
+  const float4* x = static_cast<const float4*>(x5);
   float4* o = static_cast<float4*>(p.out);
   const float2 d = make_float2(p.md[s], p.md[s + 1]);
   const float2 cl = make_float2(p.ml[s], p.ml[s + 1]);
@@ -535,16 +535,16 @@ __device__ __forceinline__ float2 dhop_mooee_epilogue(const DhopParams& p, size_
 // through the FP16 encoder; returns |out|^2 as stored.  Unlike the separate launches, the
 // Dhop result is not rounded to FP16 before the subtraction.
 template <int MODE>
-__device__ __forceinline__ float2 dhop_mooee_epilogue_half(const DhopParams& p, size_t np, size_t q, int sp,
-                                                           Pair12& acc) {
+__device__ __forceinline__ float2 dhop_mooee_epilogue_half(const DhopParams& p, const void* x5, const float* x5n, size_t np,
+                                                           size_t q, int sp, Pair12& acc) {
   const int hs = p.Ls >> 1;
   const int psb = MODE == 1 ? sp : sp % hs;
   const int s = 2 * psb;
   const size_t qb = q - psb;
   const size_t qprev = psb == 0 ? qb + hs - 1 : q - 1;
   const size_t qnext = psb == hs - 1 ? qb : q + 1;
-  const uint4* x = static_cast<const uint4*>(p.x5);
-  const float2* xn = reinterpret_cast<const float2*>(p.x5_norms);
+  const uint4* x = static_cast<const uint4*>(x5);
+  const float2* xn = reinterpret_cast<const float2*>(x5n);
   const float2 ncur = __ldg(xn + q), nprv = __ldg(xn + qprev), nnxt = __ldg(xn + qnext);
   const float2 d = make_float2(p.md[s], p.md[s + 1]);
   const float2 cl = make_float2(p.ml[s], p.ml[s + 1]);
@@ -599,7 +599,7 @@ __device__ __forceinline__ void dhop_axpy_epilogue(const DhopParams& p, size_t n
 // Dhop of 138 us at 24^3 x 32 with 12 Wilson right-hand sides.
 template <class T, bool DAG, bool RECON, int MOOEE = 0>
 __global__ void __launch_bounds__(GB_DHOP_THREADS, GB_DHOP_MINB) dhop_pair_kernel(const __grid_constant__ DhopParams p0) {
-  const DhopParams p = dhop_side(p0);
+  DhopParams p = dhop_side(p0);
   extern __shared__ __align__(128) unsigned char dyn_smem[];
   float* slink = reinterpret_cast<float*>(dyn_smem);  // k4 * kLinkStride floats
   float* sraw = slink + size_t(p.k4) * kLinkStride;   // RECON: k4 * 96 floats (rows 0, 1)
@@ -632,6 +632,11 @@ __global__ void __launch_bounds__(GB_DHOP_THREADS, GB_DHOP_MINB) dhop_pair_kerne
     nb[0] = a.x; nb[1] = a.y; nb[2] = a.z; nb[3] = a.w;
     nb[4] = b.x; nb[5] = b.y; nb[6] = b.z; nb[7] = b.w;
   }
+  pdl_wait();  // the fields; links and neighbour tables were there before
+  p.in = after_wait(p.in);
+  p.in_norms = after_wait(p.in_norms);
+  p.x5 = after_wait(p.x5);
+  p.x5_norms = after_wait(p.x5_norms);
   // every thread waits for the links before it leaves.  If the bounded wait gives up,
   // the copy may still be in flight when the CTA exits: the error flag is raised and the
   // host then refuses further Dhops on this operator (Op::poisoned)
@@ -660,8 +665,8 @@ __global__ void __launch_bounds__(GB_DHOP_THREADS, GB_DHOP_MINB) dhop_pair_kerne
     if constexpr (MOOEE == 3) dhop_axpy_epilogue<T>(p, np, size_t(x0 + j) * hl + sp, acc);
     if constexpr (MOOEE == 1 || MOOEE == 2) {
       float2 n2;
-      if constexpr (sizeof(T) == 4) n2 = dhop_mooee_epilogue<MOOEE>(p0, np, size_t(x0 + j) * hl + sp, sp, acc);
-      else n2 = dhop_mooee_epilogue_half<MOOEE>(p0, np, size_t(x0 + j) * hl + sp, sp, acc);
+      if constexpr (sizeof(T) == 4) n2 = dhop_mooee_epilogue<MOOEE>(p0, p.x5, np, size_t(x0 + j) * hl + sp, sp, acc);
+      else n2 = dhop_mooee_epilogue_half<MOOEE>(p0, p.x5, p.x5_norms, np, size_t(x0 + j) * hl + sp, sp, acc);
       nsum = double(n2.x) + double(n2.y);
     } else {
       PairIO<T>::store(p.out, reinterpret_cast<float2*>(p.out_norms), np, size_t(x0 + j) * hl + sp, acc);
@@ -749,8 +754,7 @@ template <class T, bool DAG, bool RECON, int MOOEE = 0> static int launch_dhop_p
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
     configured.store(true);
   }
-  dhop_pair_kernel<T, DAG, RECON, MOOEE>
-      <<<dim3(unsigned(s.blocks), s.ychunks, p.in2 ? 2u : 1u), dim3(s.threads), smem, op->stream>>>(p);
+  launch_pdl(dhop_pair_kernel<T, DAG, RECON, MOOEE>, dim3(unsigned(s.blocks), s.ychunks, p.in2 ? 2u : 1u), dim3(s.threads), smem, op->stream, p);
   GB_CHECK_CUDA(cudaGetLastError());
   return GB_OK;
 }

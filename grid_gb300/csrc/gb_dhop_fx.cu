@@ -283,9 +283,10 @@ __device__ __forceinline__ void fx_pad(const FxParams& p, double2* out, int64_t 
 // site.  A pass of its own: each site is read by eight outputs, and converting it eight times
 // there took more instructions than the SU(3) products.
 __global__ void __launch_bounds__(256) fx_convert_kernel(const __grid_constant__ FxParams p) {
+  pdl_wait();
   const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= p.n5) return;
-  const double2* in = static_cast<const double2*>(p.in[blockIdx.z]);
+  const double2* in = after_wait(static_cast<const double2*>(p.in[blockIdx.z]));
   longlong2* out = p.fxin[blockIdx.z];
   Spinor<double> f;
   SpinorIO<double>::load(in, nullptr, p.n5, i, f);
@@ -314,10 +315,8 @@ __global__ void __launch_bounds__(128, 4) dhop_fx_kernel(const __grid_constant__
   int4* slink = reinterpret_cast<int4*>(dyn_smem);  // k4 * kFxLinkStride
   __shared__ __align__(8) uint64_t bar;
   const int side = blockIdx.z;
-  const double2* in = static_cast<const double2*>(p.in[side]);
   double2* out = static_cast<double2*>(p.out[side]);
   const int* nbr = p.nbr[side];
-  const int* exps = p.exps[side];
   const int t = threadIdx.x;
   const int64_t x0 = int64_t(blockIdx.x) * p.k4;
   const int nsite = int(min(int64_t(p.k4), p.n4h - x0));
@@ -329,6 +328,11 @@ __global__ void __launch_bounds__(128, 4) dhop_fx_kernel(const __grid_constant__
     mbar_expect_tx(&bar, uint32_t(nsite) * 1152u);
     for (int k = 0; k < nsite; k++) bulk_g2s(slink + k * kFxLinkStride, p.links[side] + (x0 + k) * 72, 1152u, &bar);
   }
+  pdl_wait();  // the field; links and neighbour tables were there before
+  const double2* in = after_wait(static_cast<const double2*>(p.in[side]));
+  const double2* z = after_wait(p.z[side]);
+  const longlong2* fxin = after_wait(p.fxin[side]);
+  const int* exps = after_wait(p.exps[side]);
   if (!mbar_wait_bounded(&bar, 0)) {  // every thread waits; the error flag as in gb_dhop.cu
     atomicExch(p.err, 1);
     return;
@@ -338,15 +342,15 @@ __global__ void __launch_bounds__(128, 4) dhop_fx_kernel(const __grid_constant__
   fx_pad(p, out, x, s);
   const int Ea = fx_site_exponent(exps, nbr, p.L5, x, s);
   if (Ea == fx::kBad) {
-    fx_site_fp64(in, out, p.z[side], p.c0, p.c1, p.links_d[side], nbr, p.n5, p.L5, x, s, p.dag);
+    fx_site_fp64(in, out, z, p.c0, p.c1, p.links_d[side], nbr, p.n5, p.L5, x, s, p.dag);
     return;
   }
   FxAcc acc;
-  fx_legs(p, p.fxin[side], exps, nbr, slink + j * kFxLinkStride, 1, x, s, 0, 4, Ea, acc);
+  fx_legs(p, fxin, exps, nbr, slink + j * kFxLinkStride, 1, x, s, 0, 4, Ea, acc);
   const int e = fx::result_exponent(Ea, p.link_exp);
   const size_t i = size_t(x) * p.L5 + s;
 #pragma unroll
-  for (int k = 0; k < 12; k++) fx_store<AXPY>(p, p.z[side], out, size_t(k) * p.n5 + i, fx_value(acc.re[k], e), fx_value(acc.im[k], e));
+  for (int k = 0; k < 12; k++) fx_store<AXPY>(p, z, out, size_t(k) * p.n5 + i, fx_value(acc.re[k], e), fx_value(acc.im[k], e));
 }
 
 // Four warps share 32 output sites, one direction (its forward and backward leg) each, and add
@@ -360,18 +364,21 @@ __global__ void __launch_bounds__(128, 4) dhop_fx_split_kernel(const __grid_cons
   __shared__ long long part[4][24][32];
   const int side = blockIdx.z;
   const int lane = threadIdx.x & 31, mu = threadIdx.x >> 5;
-  const double2* in = static_cast<const double2*>(p.in[side]);
   double2* out = static_cast<double2*>(p.out[side]);
   const int* nbr = p.nbr[side];
-  const int* exps = p.exps[side];
   const int64_t g = int64_t(blockIdx.x) * 32 + lane;
   const bool active = g < p.n4h * p.L5a;
   const int64_t x = active ? g / p.L5a : 0;
   const int s = active ? int(g - x * p.L5a) : 0;
+  pdl_wait();
+  const double2* in = after_wait(static_cast<const double2*>(p.in[side]));
+  const double2* z = after_wait(p.z[side]);
+  const longlong2* fxin = after_wait(p.fxin[side]);
+  const int* exps = after_wait(p.exps[side]);
   const int Ea = fx_site_exponent(exps, nbr, p.L5, x, s);
   if (Ea != fx::kBad) {
     FxAcc acc;
-    fx_legs(p, p.fxin[side], exps, nbr, SOA ? p.links[side] + x : p.links[side] + x * 72, SOA ? size_t(p.n4h) : size_t(1),
+    fx_legs(p, fxin, exps, nbr, SOA ? p.links[side] + x : p.links[side] + x * 72, SOA ? size_t(p.n4h) : size_t(1),
             x, s, mu, 1, Ea, acc);
 #pragma unroll
     for (int k = 0; k < 12; k++) { part[mu][2 * k][lane] = acc.re[k]; part[mu][2 * k + 1][lane] = acc.im[k]; }
@@ -380,7 +387,7 @@ __global__ void __launch_bounds__(128, 4) dhop_fx_split_kernel(const __grid_cons
   if (!active) return;
   if (mu == 0) fx_pad(p, out, x, s);
   if (Ea == fx::kBad) {
-    if (mu == 0) fx_site_fp64(in, out, p.z[side], p.c0, p.c1, p.links_d[side], nbr, p.n5, p.L5, x, s, p.dag);
+    if (mu == 0) fx_site_fp64(in, out, z, p.c0, p.c1, p.links_d[side], nbr, p.n5, p.L5, x, s, p.dag);
     return;
   }
   const int e = fx::result_exponent(Ea, p.link_exp);
@@ -392,7 +399,7 @@ __global__ void __launch_bounds__(128, 4) dhop_fx_split_kernel(const __grid_cons
 #pragma unroll
     for (int c = 0; c < 2; c++)
       v[c] = (part[0][2 * k + c][lane] + part[1][2 * k + c][lane]) + (part[2][2 * k + c][lane] + part[3][2 * k + c][lane]);
-    fx_store<AXPY>(p, p.z[side], out, size_t(k) * p.n5 + i, fx_value(v[0], e), fx_value(v[1], e));
+    fx_store<AXPY>(p, z, out, size_t(k) * p.n5 + i, fx_value(v[0], e), fx_value(v[1], e));
   }
 }
 
@@ -669,20 +676,20 @@ int launch_dhop_fx(Op* op, HalfView in, HalfView out, int out_parity, const Half
   p.link_exp = op->fx_exp;
   p.dag = dag;
   p.err = op->d_err;
-  fx_convert_kernel<<<dim3(unsigned((p.n5 + 255) / 256), 1, in2 ? 2u : 1u), 256, 0, op->stream>>>(p);
+  launch_pdl(fx_convert_kernel, dim3(unsigned((p.n5 + 255) / 256), 1, in2 ? 2u : 1u), 256, 0, op->stream, p);
   const bool soa = fx_soa(op);
   void (*kernel)(const FxParams);
   if (soa || p.n4h * p.L5a * (in2 ? 2 : 1) <= kFxSplitSites) {
     if (soa) kernel = axpy ? dhop_fx_split_kernel<true, true> : dhop_fx_split_kernel<true, false>;
     else kernel = axpy ? dhop_fx_split_kernel<false, true> : dhop_fx_split_kernel<false, false>;
-    kernel<<<dim3(unsigned((p.n4h * p.L5a + 31) / 32), 1, in2 ? 2u : 1u), 128, 0, op->stream>>>(p);
+    launch_pdl(kernel, dim3(unsigned((p.n4h * p.L5a + 31) / 32), 1, in2 ? 2u : 1u), 128, 0, op->stream, p);
   } else {
     kernel = axpy ? dhop_fx_kernel<true> : dhop_fx_kernel<false>;
     p.L5c = p.L5a > 128 ? 128 : p.L5a;
     p.k4 = 128 / p.L5c;
     const dim3 grid(unsigned((p.n4h + p.k4 - 1) / p.k4), unsigned((p.L5a + p.L5c - 1) / p.L5c), in2 ? 2u : 1u);
     const unsigned threads = unsigned((p.k4 * p.L5c + 31) / 32 * 32);
-    kernel<<<grid, threads, size_t(p.k4) * kFxLinkStride * sizeof(int4), op->stream>>>(p);
+    launch_pdl(kernel, grid, threads, size_t(p.k4) * kFxLinkStride * sizeof(int4), op->stream, p);
   }
   GB_CHECK_CUDA(cudaGetLastError());
   return GB_OK;
@@ -703,7 +710,7 @@ int launch_deriv_fx(Op* op, HalfView A, HalfView B, int out_parity, int dag, dou
     p.exps[z] = c.exps[z];
   }
   c.n5 = p.n5 = op->n5();
-  fx_convert_kernel<<<dim3(unsigned((c.n5 + 255) / 256), 1, 2), 256, 0, op->stream>>>(c);
+  launch_pdl(fx_convert_kernel, dim3(unsigned((c.n5 + 255) / 256), 1, 2), 256, 0, op->stream, c);
   p.links = static_cast<const double*>(op->links[out_parity]);
   p.nbr = op->nbr[out_parity];
   p.mat = reinterpret_cast<double2*>(mat);

@@ -165,6 +165,7 @@ __device__ __forceinline__ void ms_post(MSState* st, const double* partial, int 
 // partial: <x, y> and <x, x> (real parts).  MID: the last CTA to finish runs ms_mid.
 template <class V, bool MID>
 __global__ void __launch_bounds__(256) ms_dot_kernel(const V* x, const V* y, size_t nw, double* partial, MSState* st) {
+  pdl_wait();
   if (MID && st->frozen) return;
   double s1 = 0, s2 = 0;
 #pragma unroll 4
@@ -181,6 +182,7 @@ __global__ void __launch_bounds__(256) ms_dot_kernel(const V* x, const V* y, siz
 template <class V, bool POST>
 __global__ void __launch_bounds__(256) ms_r_kernel(V* r, const V* mmp, const V* p, size_t nw, MSState* st,
                                                    double* partial) {
+  pdl_wait();
   using R = typename Word<V>::R;
   if (st->frozen) return;
   const R b = R(st->b), bm = R(st->b * st->m0);
@@ -201,6 +203,7 @@ __global__ void __launch_bounds__(256) ms_r_kernel(V* r, const V* mmp, const V* 
 template <class V>
 __global__ void __launch_bounds__(256) ms_update_kernel(V* p, const V* r, const MSFields f, size_t nw,
                                                         const MSState* st, int do_p) {
+  pdl_wait();
   using R = typename Word<V>::R;
   if (st->frozen) return;
   const int ns = st->nshift;
@@ -295,8 +298,8 @@ template <class V> struct MS {
   int dot(const Field* x, const Field* y, bool mid = false) {
     const V* a = static_cast<const V*>(x->data);
     const V* b = static_cast<const V*>(y->data);
-    if (mid) ms_dot_kernel<V, true><<<blocks(), 256, 0, op->stream>>>(a, b, nw, partial, st);
-    else ms_dot_kernel<V, false><<<blocks(), 256, 0, op->stream>>>(a, b, nw, partial, st);
+    if (mid) launch_pdl(ms_dot_kernel<V, true>, blocks(), 256, 0, op->stream, a, b, nw, partial, st);
+    else launch_pdl(ms_dot_kernel<V, false>, blocks(), 256, 0, op->stream, a, b, nw, partial, st);
     GB_CHECK_CUDA(cudaGetLastError());
     return GB_OK;
   }
@@ -304,13 +307,13 @@ template <class V> struct MS {
     V* a = static_cast<V*>(r->data);
     const V* b = static_cast<const V*>(mmp->data);
     const V* c = static_cast<const V*>(p->data);
-    if (post) ms_r_kernel<V, true><<<blocks(), 256, 0, op->stream>>>(a, b, c, nw, st, partial);
-    else ms_r_kernel<V, false><<<blocks(), 256, 0, op->stream>>>(a, b, c, nw, st, partial);
+    if (post) launch_pdl(ms_r_kernel<V, true>, blocks(), 256, 0, op->stream, a, b, c, nw, st, partial);
+    else launch_pdl(ms_r_kernel<V, false>, blocks(), 256, 0, op->stream, a, b, c, nw, st, partial);
     GB_CHECK_CUDA(cudaGetLastError());
     return GB_OK;
   }
   int update(Field* p, const Field* r, const MSFields& f, int do_p) {
-    ms_update_kernel<V><<<update_blocks(), 256, 0, op->stream>>>(static_cast<V*>(p->data), static_cast<const V*>(r->data), f,
+    launch_pdl(ms_update_kernel<V>, update_blocks(), 256, 0, op->stream, static_cast<V*>(p->data), static_cast<const V*>(r->data), f,
                                                          nw, st, do_p);
     GB_CHECK_CUDA(cudaGetLastError());
     return GB_OK;

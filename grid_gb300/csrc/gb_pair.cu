@@ -110,7 +110,12 @@ template <class R> struct Coef5p {
 // NORM: a grid-stride loop (blockDim a multiple of L5/2) whose CTAs also sum |chi|^2 as
 // stored per right-hand side, in a fixed order (block_reduce_pairs)
 template <class T, bool DAG, bool ZTERM, bool SAME, bool NORM>
-__global__ void __launch_bounds__(512) m5d_pair_kernel(const M5PairParams p, const Coef5p<float> c) {
+__global__ void __launch_bounds__(512) m5d_pair_kernel(const M5PairParams p0, const Coef5p<float> c) {
+  M5PairParams p = p0;
+  pdl_wait();
+  p.psi = after_wait(p.psi); p.psi_n = after_wait(p.psi_n);
+  p.phi = after_wait(p.phi); p.phi_n = after_wait(p.phi_n);
+  p.z = after_wait(p.z); p.z_n = after_wait(p.z_n);
   double nv0[1] = {0.0}, nv1[1] = {0.0};
   const size_t stride = NORM ? size_t(gridDim.x) * blockDim.x : p.np;
   for (size_t q = size_t(blockIdx.x) * blockDim.x + threadIdx.x; q < p.np; q += stride) {
@@ -184,14 +189,14 @@ static void m5d_pair_go(Op* op, const M5PairParams& p, const Coef5p<float>& c, b
       int g = 1, B = 256;
       m5d_norm_grid(op, p.np, &g, &B);
       const size_t smem = size_t(op->nrhs == 1 ? 32 : 2 * B) * sizeof(double);
-      if (same) m5d_pair_kernel<T, DAG, Z, true, true><<<g, B, smem, op->stream>>>(p, c);
-      else m5d_pair_kernel<T, DAG, Z, false, true><<<g, B, smem, op->stream>>>(p, c);
+      if (same) launch_pdl(m5d_pair_kernel<T, DAG, Z, true, true>, g, B, smem, op->stream, p, c);
+      else launch_pdl(m5d_pair_kernel<T, DAG, Z, false, true>, g, B, smem, op->stream, p, c);
       return;
     }
   }
   const unsigned blocks = unsigned((p.np + 255) / 256);
-  if (same) m5d_pair_kernel<T, DAG, Z, true, false><<<blocks, 256, 0, op->stream>>>(p, c);
-  else m5d_pair_kernel<T, DAG, Z, false, false><<<blocks, 256, 0, op->stream>>>(p, c);
+  if (same) launch_pdl(m5d_pair_kernel<T, DAG, Z, true, false>, blocks, 256, 0, op->stream, p, c);
+  else launch_pdl(m5d_pair_kernel<T, DAG, Z, false, false>, blocks, 256, 0, op->stream, p, c);
 }
 
 int launch_m5d_pair(Op* op, HalfView psi, HalfView phi, HalfView chi, const double* lower, const double* diag,
@@ -237,8 +242,9 @@ __global__ void __launch_bounds__(512) reduce_pair_kernel(const PairShape sh, co
                                                           double a, const CGScalars* cg, size_t np, double* partial,
                                                           const CGFinish fin) {
   constexpr int NV = KIND == 1 ? 2 : 1;
-  x = half_at<T>(x, np); xn = norms_at(xn, np);
-  y = half_at<T>(y, np); yn = norms_at(yn, np);
+  pdl_wait();
+  x = after_wait(half_at<T>(x, np)); xn = after_wait(norms_at(xn, np));
+  y = after_wait(half_at<T>(y, np)); yn = after_wait(norms_at(yn, np));
   z = half_at<T>(z, np); zn = norms_at(zn, np);
   const double* const all = partial;
   partial += size_t(blockIdx.y) * gridDim.x * sh.nrhs * NV;
@@ -319,7 +325,7 @@ static int reduce_pair_t(Op* op, HalfView x, HalfView y, HalfView z, double a, s
   PairShape sh{op->L5, op->Ls, op->nrhs};
   const int NV = KIND == 1 ? 2 : 1;
   const size_t smem = size_t(NV) * (op->nrhs == 1 ? 32 : 2 * B) * sizeof(double);
-  reduce_pair_kernel<T, KIND><<<dim3(g, halves), B, smem, op->stream>>>(
+  launch_pdl(reduce_pair_kernel<T, KIND>, dim3(g, halves), B, smem, op->stream, 
       sh, x.data, reinterpret_cast<const float2*>(x.norms), y.data, reinterpret_cast<const float2*>(y.norms), z.data,
       reinterpret_cast<float2*>(z.norms), a, op->d_cg, np, partial, CGFinish{op->d_cg, op->d_all_done, finish});
   GB_CHECK_CUDA(cudaGetLastError());
@@ -344,10 +350,11 @@ int launch_reduce_pair(Op* op, int kind, HalfView x, HalfView y, HalfView z, dou
 template <class T>
 __global__ void __launch_bounds__(256) cg_p_pair_kernel(const PairShape sh, void* p, float2* pn, const void* r,
                                                         const float2* rn, const CGScalars* cg, size_t np) {
+  pdl_wait();
   const size_t q = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (q >= np) return;
-  p = half_at<T>(p, np); pn = norms_at(pn, np);
-  r = half_at<T>(r, np); rn = norms_at(rn, np);
+  p = after_wait(half_at<T>(p, np)); pn = after_wait(norms_at(pn, np));
+  r = after_wait(half_at<T>(r, np)); rn = after_wait(norms_at(rn, np));
   const int s5 = int((2 * q) % sh.L5);
   const float2 b = make_float2(float(cg[s5 / sh.Ls].b), float(cg[(s5 + 1) / sh.Ls].b));
   Pair12 fp, fr;
@@ -366,10 +373,10 @@ int launch_cg_p_pair(Op* op, HalfView p, HalfView r, size_t n5, int halves) {
   const size_t np = n5 >> 1;
   const dim3 blocks(unsigned((np + 255) / 256), halves);
   if (p.prec == GB_F32)
-    cg_p_pair_kernel<float><<<blocks, 256, 0, op->stream>>>(sh, p.data, reinterpret_cast<float2*>(p.norms), r.data,
+    launch_pdl(cg_p_pair_kernel<float>, blocks, 256, 0, op->stream, sh, p.data, reinterpret_cast<float2*>(p.norms), r.data,
                                                             reinterpret_cast<const float2*>(r.norms), op->d_cg, np);
   else
-    cg_p_pair_kernel<__half><<<blocks, 256, 0, op->stream>>>(sh, p.data, reinterpret_cast<float2*>(p.norms), r.data,
+    launch_pdl(cg_p_pair_kernel<__half>, blocks, 256, 0, op->stream, sh, p.data, reinterpret_cast<float2*>(p.norms), r.data,
                                                              reinterpret_cast<const float2*>(r.norms), op->d_cg, np);
   GB_CHECK_CUDA(cudaGetLastError());
   return GB_OK;
@@ -381,11 +388,12 @@ template <class T, class TS, bool PUPD>
 __global__ void __launch_bounds__(256) cg_xp_pair_kernel(const PairShape sh, void* psi, float2* psin, void* p, float2* pn,
                                                          const void* r, const float2* rn, const CGScalars* cg,
                                                          size_t np) {
+  pdl_wait();
   const size_t q = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (q >= np) return;
-  p = half_at<T>(p, np); pn = norms_at(pn, np);
-  r = half_at<T>(r, np); rn = norms_at(rn, np);
-  psi = half_at<TS>(psi, np); psin = norms_at(psin, np);
+  p = after_wait(half_at<T>(p, np)); pn = after_wait(norms_at(pn, np));
+  r = after_wait(half_at<T>(r, np)); rn = after_wait(norms_at(rn, np));
+  psi = after_wait(half_at<TS>(psi, np)); psin = after_wait(norms_at(psin, np));
   const int s5 = int((2 * q) % sh.L5);
   const CGScalars& c0 = cg[s5 / sh.Ls];
   const CGScalars& c1 = cg[(s5 + 1) / sh.Ls];
@@ -412,6 +420,28 @@ __global__ void __launch_bounds__(256) cg_xp_pair_kernel(const PairShape sh, voi
   }
 }
 
+// The same on FP32 fields, one 16-byte vector per thread (blockIdx.y: the plane, over both
+// checkerboards of a full field): all loads of a thread are in flight before its first store.
+// With a site pair per thread the loads of r came after the stores of psi.
+template <bool PUPD>
+__global__ void __launch_bounds__(256) cg_xp_vector_kernel(const PairShape sh, float4* psi, float4* p, const float4* r,
+                                                           const CGScalars* cg, size_t np) {
+  pdl_wait();
+  const size_t q = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (q >= np) return;
+  int r0 = 0, r1 = 0;
+  if (sh.nrhs > 1) {
+    const int s5 = int((2 * q) % sh.L5);
+    r0 = s5 / sh.Ls;
+    r1 = (s5 + 1) / sh.Ls;
+  }
+  const size_t w = size_t(blockIdx.y) * np + q;
+  const float4 vp = p[w], vs = psi[w], vr = PUPD ? r[w] : make_float4(0.f, 0.f, 0.f, 0.f);
+  const float a0 = float(cg[r0].a), a1 = float(cg[r1].a), b0 = float(cg[r0].b), b1 = float(cg[r1].b);
+  psi[w] = make_float4(fmaf(a0, vp.x, vs.x), fmaf(a1, vp.y, vs.y), fmaf(a0, vp.z, vs.z), fmaf(a1, vp.w, vs.w));
+  if (PUPD) p[w] = make_float4(fmaf(b0, vp.x, vr.x), fmaf(b1, vp.y, vr.y), fmaf(b0, vp.z, vr.z), fmaf(b1, vp.w, vr.w));
+}
+
 template <class T, class TS>
 static void cg_xp_pair_go(Op* op, HalfView psi, HalfView p, HalfView r, size_t np, bool pupd, int halves) {
   PairShape sh{op->L5, op->Ls, op->nrhs};
@@ -420,14 +450,19 @@ static void cg_xp_pair_go(Op* op, HalfView psi, HalfView p, HalfView r, size_t n
   auto* pn = reinterpret_cast<float2*>(p.norms);
   auto* rn = reinterpret_cast<const float2*>(r.norms);
   if (pupd)
-    cg_xp_pair_kernel<T, TS, true><<<blocks, 256, 0, op->stream>>>(sh, psi.data, psin, p.data, pn, r.data, rn, op->d_cg, np);
+    launch_pdl(cg_xp_pair_kernel<T, TS, true>, blocks, 256, 0, op->stream, sh, psi.data, psin, p.data, pn, r.data, rn, op->d_cg, np);
   else
-    cg_xp_pair_kernel<T, TS, false><<<blocks, 256, 0, op->stream>>>(sh, psi.data, psin, p.data, pn, r.data, rn, op->d_cg, np);
+    launch_pdl(cg_xp_pair_kernel<T, TS, false>, blocks, 256, 0, op->stream, sh, psi.data, psin, p.data, pn, r.data, rn, op->d_cg, np);
 }
 
 int launch_cg_xp_pair(Op* op, HalfView psi, HalfView p, HalfView r, size_t n5, int update_p, int halves) {
   const size_t np = n5 >> 1;
-  if (p.prec == GB_F32 && psi.prec == GB_F32) cg_xp_pair_go<float, float>(op, psi, p, r, np, update_p != 0, halves);
+  if (p.prec == GB_F32 && psi.prec == GB_F32) {
+    PairShape sh{op->L5, op->Ls, op->nrhs};
+    const dim3 grid(unsigned((np + 255) / 256), 12 * halves);
+    launch_pdl(update_p ? cg_xp_vector_kernel<true> : cg_xp_vector_kernel<false>, grid, 256, 0, op->stream, sh,
+               static_cast<float4*>(psi.data), static_cast<float4*>(p.data), static_cast<const float4*>(r.data), op->d_cg, np);
+  }
   else if (p.prec == GB_F16 && psi.prec == GB_F32) cg_xp_pair_go<__half, float>(op, psi, p, r, np, update_p != 0, halves);
   else if (p.prec == GB_F16 && psi.prec == GB_F16) cg_xp_pair_go<__half, __half>(op, psi, p, r, np, update_p != 0, halves);
   else {
@@ -442,10 +477,11 @@ template <class T>
 __global__ void __launch_bounds__(256) axpby_pair_kernel(void* z, float2* zn, float a, const void* x, const float2* xn,
                                                          float b, const void* y, const float2* yn, size_t np,
                                                          int use_y) {
+  pdl_wait();
   const size_t q = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (q >= np) return;
-  x = half_at<T>(x, np); xn = norms_at(xn, np);
-  y = half_at<T>(y, np); yn = norms_at(yn, np);
+  x = after_wait(half_at<T>(x, np)); xn = after_wait(norms_at(xn, np));
+  y = after_wait(half_at<T>(y, np)); yn = after_wait(norms_at(yn, np));
   z = half_at<T>(z, np); zn = norms_at(zn, np);
   Pair12 fx, o;
   PairIO<T>::load(x, xn, np, q, fx);
@@ -470,11 +506,11 @@ int launch_axpby_pair(Op* op, HalfView z, double a, HalfView x, double b, HalfVi
   const size_t np = n5 >> 1;
   const dim3 blocks(unsigned((np + 255) / 256), halves);
   if (z.prec == GB_F32)
-    axpby_pair_kernel<float><<<blocks, 256, 0, op->stream>>>(z.data, reinterpret_cast<float2*>(z.norms), float(a), x.data,
+    launch_pdl(axpby_pair_kernel<float>, blocks, 256, 0, op->stream, z.data, reinterpret_cast<float2*>(z.norms), float(a), x.data,
                                                              reinterpret_cast<const float2*>(x.norms), float(b), y.data,
                                                              reinterpret_cast<const float2*>(y.norms), np, use_y);
   else
-    axpby_pair_kernel<__half><<<blocks, 256, 0, op->stream>>>(z.data, reinterpret_cast<float2*>(z.norms), float(a),
+    launch_pdl(axpby_pair_kernel<__half>, blocks, 256, 0, op->stream, z.data, reinterpret_cast<float2*>(z.norms), float(a),
                                                               x.data, reinterpret_cast<const float2*>(x.norms), float(b),
                                                               y.data, reinterpret_cast<const float2*>(y.norms), np, use_y);
   GB_CHECK_CUDA(cudaGetLastError());
