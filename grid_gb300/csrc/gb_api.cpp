@@ -420,12 +420,14 @@ static int op_dhop_full_axpy(Op* op, Field* in, Field* z, Field* out, double c0,
   GB_TRY(op_dhop_full(op, in, out, dag));
   return field_axpby(out, c1, c0, out, z);
 }
-int op_dhop_cb_axpy(Op* op, Field* in, Field* z, Field* out, double c0, double c1, int dag) {
+int op_dhop_cb_axpy(Op* op, Field* in, Field* z, Field* out, double c0, double c1, int dag, int* parts, Field* r) {
+  if (parts) *parts = 0;
   if (in->full() || out->full()) { set_error("DhopEO/OE: half fields expected"); return GB_ERR_BAD_PARITY; }
   int done = 0;
+  HalfView rv = r ? half_view(r, 0) : HalfView{};
   const int p = in->subset;
   const DhopAxpy a{{half_view(z, 0), half_view(z, 0)}, c0, c1};
-  GB_TRY(launch_dhop_axpy(op, half_view(in, 0), half_view(out, 0), 1 - p, dag, a, &done));
+  GB_TRY(launch_dhop_axpy(op, half_view(in, 0), half_view(out, 0), 1 - p, dag, a, &done, parts, r ? &rv : nullptr));
   out->subset = 1 - p;
   if (done) return GB_OK;
   GB_TRY(op_dhop_cb(op, in, out, dag));
@@ -518,7 +520,8 @@ int op_mooee_inv(Op* op, Field* in, Field* out, int dag) {
 
 // SchurDiagMooeeOperator::Mpc / MpcDag (LinearOperator.h:330-349).  With norm_parts (Mpc
 // of a FP32 / FP16 Moebius operator) the last kernel also reduces |out|^2 per right-hand
-// side (see launch_m5d_pair).  With r_upd (MpcDag of a FP32 / FP16 Moebius operator whose
+// side (see launch_m5d_pair; Wilson: launch_dhop_axpy).  With r_upd (MpcDag of a FP32 / FP16 Wilson
+// operator, or Moebius operator whose
 // right-hand-side count divides 16) the last kernel applies r -= a out for the CG instead
 // of storing out (see launch_col).
 int op_mpc(Op* op, Field* in, Field* out, int dag, int* norm_parts, Field* r_upd, int* r_parts) {
@@ -532,7 +535,7 @@ int op_mpc(Op* op, Field* in, Field* out, int dag, int* norm_parts, Field* r_upd
     // out = d in - (1/d) DhopOE DhopEO in
     te1->subset = GB_EVEN;
     GB_TRY(op_dhop_cb(op, in, te1, dag));
-    return op_dhop_cb_axpy(op, te1, in, out, op->diag_mass, -1.0 / op->diag_mass, dag);
+    return op_dhop_cb_axpy(op, te1, in, out, op->diag_mass, -1.0 / op->diag_mass, dag, r_upd ? r_parts : norm_parts, r_upd);
   }
   GB_TRY(ws_get(op, GB_EVEN, in->prec, WS_MPC_E2, &te2));
   GB_TRY(ws_get(op, GB_ODD, in->prec, WS_MPC_O, &to));
@@ -811,10 +814,10 @@ static int op_create(int kind, const int dims[4], int Ls, double mass, double M5
     alloc(reinterpret_cast<void**>(&op->nbr[p]), size_t(op->half4) * 8 * sizeof(int));
   }
   alloc(reinterpret_cast<void**>(&op->d_err), sizeof(int));
-  // the reductions' [2 halves][kRedBlocks][nrhs][2]; an FP32 Moebius Dhop with the Mooee
-  // epilogue writes nrhs sums per CTA
+  // the reductions' [2 halves][kRedBlocks][nrhs][2]; an FP32 or FP16 Dhop with a summing epilogue
+  // writes nrhs sums per CTA
   op->partial_doubles = size_t(2) * kRedBlocks * nrhs * 2;
-  if (op->prec != GB_F64 && op->kind == 1)
+  if (op->prec != GB_F64)
     op->partial_doubles = std::max(op->partial_doubles, dhop_pair_ctas(op) * nrhs);
   alloc(reinterpret_cast<void**>(&op->d_partial), op->partial_doubles * sizeof(double));
   alloc(reinterpret_cast<void**>(&op->d_result), size_t(nrhs) * 8 * sizeof(double));

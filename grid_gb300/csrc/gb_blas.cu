@@ -325,6 +325,19 @@ __global__ void __launch_bounds__(1024) cg_alpha_kernel(CGScalars* cg, const dou
   if (threadIdx.x == 0) cg_alpha_update(cg[r], d);
 }
 
+__global__ void __launch_bounds__(1024) cg_beta_kernel(CGScalars* cg, const double* partial, int nparts, int nrhs,
+                                                      int* flags) {
+  pdl_wait();
+  const int r = blockIdx.x;
+  const double cp = cta_sum_fixed(partial, nparts, nrhs, r);
+  if (threadIdx.x == 0) {
+    CGScalars s = cg[r];
+    cg_beta_update(s, cp);
+    cg[r] = s;
+  }
+  if (last_cta(flags + kCGTicket, nrhs) && threadIdx.x == 0) cg_set_flags(cg, nrhs, flags);
+}
+
 __global__ void cg_relup_reset_kernel(CGScalars* cg, const double* cp_true, int nrhs) {
   const int r = threadIdx.x;
   if (r >= nrhs) return;
@@ -350,6 +363,11 @@ int launch_cg_init(Op* op, const double* d_ssq, const double* d_cp, double tol, 
 static inline int sum_threads(int nparts) { return nparts > 2048 ? 1024 : 256; }
 int launch_cg_alpha(Op* op, const double* partial, int nparts) {
   launch_pdl(cg_alpha_kernel, op->nrhs, sum_threads(nparts), 0, op->stream, op->d_cg, partial, nparts, op->nrhs);
+  GB_CHECK_CUDA(cudaGetLastError());
+  return GB_OK;
+}
+int launch_cg_beta(Op* op, const double* partial, int nparts) {
+  launch_pdl(cg_beta_kernel, op->nrhs, sum_threads(nparts), 0, op->stream, op->d_cg, partial, nparts, op->nrhs, op->d_all_done);
   GB_CHECK_CUDA(cudaGetLastError());
   return GB_OK;
 }

@@ -475,6 +475,18 @@ __device__ __forceinline__ void cg_beta_update(CGScalars& s, double cp) {
   else if (cp < s.delta * s.maxres) s.relup = 1;
 }
 
+// flags[0]: every right-hand side has converged, flags[1]: those that want a reliable update
+__device__ __forceinline__ void cg_set_flags(const CGScalars* cg, int nrhs, int* flags) {
+  int nd = 0, nr = 0;
+  for (int k = 0; k < nrhs; k++) {
+    const int done = __ldcg(&cg[k].done);
+    nd += done;
+    nr += __ldcg(&cg[k].relup) && !done;
+  }
+  flags[0] = nd == nrhs;
+  flags[1] = nr;
+}
+
 // Called by every thread of every CTA of a reduction with partial sums [nparts][nrhs], after they are
 // written.  One (full) warp sums a right-hand side: strided sums of its lanes, then shuffles.
 __device__ __forceinline__ void cg_finish(const CGFinish& f, const double* partial, int nparts, int nrhs, int ctas) {
@@ -494,17 +506,9 @@ __device__ __forceinline__ void cg_finish(const CGFinish& f, const double* parti
     }
   }
   if (f.mode != CG_FINISH_BETA) return;
+  __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int nd = 0, nr = 0;
-    for (int k = 0; k < nrhs; k++) {
-      const int done = f.cg[k].done;
-      nd += done;
-      nr += f.cg[k].relup && !done;
-    }
-    f.flags[0] = nd == nrhs;
-    f.flags[1] = nr;
-  }
+  if (threadIdx.x == 0) cg_set_flags(f.cg, nrhs, f.flags);
 }
 
 }  // namespace gb

@@ -61,6 +61,10 @@ struct DhopParams {
   const void* x5b;
   const float* x5b_norms;
   float c0, c1;
+  // AXPY with the residual update: r -= a out per right-hand side instead of storing out
+  void* r;
+  float* r_norms;
+  const CGScalars* cg;
   double* dpart;
   int Ls, nrhs;
   float md[kMaxLs], ml[kMaxLs], mu[kMaxLs];
@@ -590,13 +594,60 @@ __device__ __forceinline__ void dhop_axpy_epilogue(const DhopParams& p, size_t n
   }
 }
 
+// The CG's residual update of a Wilson operator (whose slots are the right-hand sides): r -= a out on
+// the thread's site pair, out in acc; returns |r|^2 per lane, from the values before FP16 encoding
+// (as the separate update pass sums it).
+template <class T>
+__device__ __forceinline__ float2 dhop_r_update(const DhopParams& p, void* r, float* rn, size_t np, size_t q, int sp,
+                                                const Pair12& acc) {
+  Pair12 v;
+  PairIO<T>::load(r, reinterpret_cast<const float2*>(rn), np, q, v);
+  const float2 ma = make_float2(-float(p.cg[2 * sp].a), -float(p.cg[2 * sp + 1].a));
+  float2 n2 = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int k = 0; k < 12; k++) {
+    v.re[k] = __ffma2_rn(ma, acc.re[k], v.re[k]);
+    v.im[k] = __ffma2_rn(ma, acc.im[k], v.im[k]);
+    n2 = __ffma2_rn(v.re[k], v.re[k], __ffma2_rn(v.im[k], v.im[k], n2));
+  }
+  PairIO<T>::store(r, reinterpret_cast<float2*>(rn), np, q, v);
+  return n2;
+}
+
+// Per-slot sums over the CTA's sites of each thread's n2 (lane 0 its slot 2 sp, lane 1 the next), in
+// a fixed order, into part[CTA][nrhs]: where whole sites fill a warp the lanes of a slot first add by
+// shuffles, then one thread per slot adds what is left.
+__device__ __forceinline__ void dhop_slot_sums(float2 n2, int hc, int k4, int slot0, int L5, double* part) {
+  __shared__ double red[2 * GB_DHOP_THREADS];
+  const int t = threadIdx.x;
+  double a = n2.x, b = n2.y;
+  const bool fold = (32 % hc) == 0 && (blockDim.x & 31) == 0;
+  if (fold)
+    for (int off = 16; off >= hc; off >>= 1) {
+      a += __shfl_down_sync(0xffffffffu, a, off);
+      b += __shfl_down_sync(0xffffffffu, b, off);
+    }
+  red[2 * t] = a;
+  red[2 * t + 1] = b;
+  __syncthreads();
+  // rows of 2 hc sums: one per site, or the first of each warp
+  const int rows = fold ? int(blockDim.x) >> 5 : k4, stride = fold ? 64 : 2 * hc;
+  for (int s = t; s < 2 * hc && slot0 + s < L5; s += blockDim.x) {
+    double sum = 0.0;
+    for (int j = 0; j < rows; j++) sum += red[j * stride + s];
+    part[size_t(blockIdx.x) * L5 + slot0 + s] = sum;
+  }
+}
+
 // CTA = k4 4D sites x hc pair threads.  Thread (j, sp) computes the 5D sites
 // (2 sp, 2 sp + 1) of 4D site x0 + j: eight legs, +mu and -mu back to back.  MOOEE (1: one
 // right-hand side, 2: several, with CTAs over 8-pair chunks that each touch at most two
 // right-hand sides): the result goes through dhop_mooee_epilogue, and the CTA writes the
 // sums of |out|^2, nrhs of them for MOOEE 2 (zero for the right-hand sides it does not touch).
 // MOOEE 3: the AXPY epilogue, where the separate pass (read, read, write) cost 91 us beside a
-// Dhop of 138 us at 24^3 x 32 with 12 Wilson right-hand sides.
+// Dhop of 138 us at 24^3 x 32 with 12 Wilson right-hand sides.  Wilson operators in the CG: 4 also
+// sums |out|^2 per right-hand side (177 us there, the norm's own pass 45), 5 applies r -= a out in
+// place of storing out and sums |r|^2 (200 us, the update's own pass 110).
 template <class T, bool DAG, bool RECON, int MOOEE = 0>
 __global__ void __launch_bounds__(GB_DHOP_THREADS, GB_DHOP_MINB) dhop_pair_kernel(const __grid_constant__ DhopParams p0) {
   DhopParams p = dhop_side(p0);
@@ -637,6 +688,7 @@ __global__ void __launch_bounds__(GB_DHOP_THREADS, GB_DHOP_MINB) dhop_pair_kerne
   p.in_norms = after_wait(p.in_norms);
   p.x5 = after_wait(p.x5);
   p.x5_norms = after_wait(p.x5_norms);
+  if (MOOEE == 5) { p.r = after_wait(p.r); p.r_norms = after_wait(p.r_norms); }
   // every thread waits for the links before it leaves.  If the bounded wait gives up,
   // the copy may still be in flight when the CTA exits: the error flag is raised and the
   // host then refuses further Dhops on this operator (Op::poisoned)
@@ -651,6 +703,7 @@ __global__ void __launch_bounds__(GB_DHOP_THREADS, GB_DHOP_MINB) dhop_pair_kerne
   }
   if (!ok) return;  // every thread of the CTA sees the same wait result
   if ((MOOEE == 0 || MOOEE == 3) && !active) return;
+  float2 slot_n2 = make_float2(0.f, 0.f);  // MOOEE 4, 5: this thread's sums
   const size_t np = p.n5 >> 1;
   double nsum = 0.0;  // MOOEE: this thread's |out|^2
   if (active) {
@@ -662,16 +715,21 @@ __global__ void __launch_bounds__(GB_DHOP_THREADS, GB_DHOP_MINB) dhop_pair_kerne
       PairIO<T>::load_raw(p.in, reinterpret_cast<const float2*>(p.in_norms), np, size_t(nb[kLegOrder[i]]) * hl + sp,
                           buf[i]);
     dhop_pair_step<T, DAG, GB_DHOP_PF, 0>(p, nb, sp, np, hl, U, buf, acc);
-    if constexpr (MOOEE == 3) dhop_axpy_epilogue<T>(p, np, size_t(x0 + j) * hl + sp, acc);
+    if constexpr (MOOEE >= 3) dhop_axpy_epilogue<T>(p, np, size_t(x0 + j) * hl + sp, acc);
     if constexpr (MOOEE == 1 || MOOEE == 2) {
       float2 n2;
       if constexpr (sizeof(T) == 4) n2 = dhop_mooee_epilogue<MOOEE>(p0, p.x5, np, size_t(x0 + j) * hl + sp, sp, acc);
       else n2 = dhop_mooee_epilogue_half<MOOEE>(p0, p.x5, p.x5_norms, np, size_t(x0 + j) * hl + sp, sp, acc);
       nsum = double(n2.x) + double(n2.y);
+    } else if constexpr (MOOEE == 4) {
+      slot_n2 = PairIO<T>::store_n2(p.out, reinterpret_cast<float2*>(p.out_norms), np, size_t(x0 + j) * hl + sp, acc);
+    } else if constexpr (MOOEE == 5) {
+      slot_n2 = dhop_r_update<T>(p, p.r, p.r_norms, np, size_t(x0 + j) * hl + sp, sp, acc);
     } else {
       PairIO<T>::store(p.out, reinterpret_cast<float2*>(p.out_norms), np, size_t(x0 + j) * hl + sp, acc);
     }
   }
+  if constexpr (MOOEE >= 4) dhop_slot_sums(slot_n2, hc, p.k4, 2 * int(blockIdx.y) * hc, p.L5, p.dpart);
   if constexpr (MOOEE == 1) {  // fixed-order CTA sum: warp shuffles, then the warps in order
     __shared__ double wsum[GB_DHOP_THREADS / 32];
 #pragma unroll
@@ -832,6 +890,9 @@ static void fill_dhop_params(Op* op, HalfView in, HalfView out, int out_parity, 
   p.x5 = p.x5b = nullptr;
   p.x5_norms = p.x5b_norms = nullptr;
   p.c0 = p.c1 = 0.f;
+  p.r = nullptr;
+  p.r_norms = nullptr;
+  p.cg = op->d_cg;
   p.dpart = nullptr;
   p.Ls = op->Ls;
   p.nrhs = op->nrhs;
@@ -881,8 +942,9 @@ int launch_dhop_mooee(Op* op, HalfView in, HalfView x5, HalfView out, int out_pa
 }
 
 static int dhop_axpy_sides(Op* op, HalfView in, HalfView out, int out_parity, const HalfView* in2, const HalfView* out2,
-                           int dag, const DhopAxpy& a, int* done) {
+                           int dag, const DhopAxpy& a, int* done, int* parts = nullptr, HalfView* r = nullptr) {
   *done = 0;
+  if (parts) *parts = 0;
   if (op->recon12 || (op->prec == GB_F64 && !op->fx_ready)) return GB_OK;
   GB_TRY(dhop_checks(op, in, out, in2, out2));
   if (a.z[0].prec != op->prec || a.z[1].prec != op->prec) {
@@ -899,13 +961,27 @@ static int dhop_axpy_sides(Op* op, HalfView in, HalfView out, int out_parity, co
   p.x5b_norms = a.z[1].norms;
   p.c0 = float(a.c0);
   p.c1 = float(a.c1);
-  if (op->prec == GB_F32)
-    return dag ? launch_dhop_pair_t<float, true, false, 3>(op, p) : launch_dhop_pair_t<float, false, false, 3>(op, p);
+  const bool f = op->prec == GB_F32;
+  const PairShapeDhop s = dhop_pair_shape(op->L5, op->half4);
+  if (parts && op->Ls == 1 && !in2 && size_t(s.blocks) * op->nrhs <= op->partial_doubles && (!r || r->prec == op->prec)) {
+    p.dpart = op->d_partial;
+    *parts = int(s.blocks);
+    if (r) {
+      p.r = r->data;
+      p.r_norms = r->norms;
+      if (f) return dag ? launch_dhop_pair_t<float, true, false, 5>(op, p) : launch_dhop_pair_t<float, false, false, 5>(op, p);
+      return dag ? launch_dhop_pair_t<__half, true, false, 5>(op, p) : launch_dhop_pair_t<__half, false, false, 5>(op, p);
+    }
+    if (f) return dag ? launch_dhop_pair_t<float, true, false, 4>(op, p) : launch_dhop_pair_t<float, false, false, 4>(op, p);
+    return dag ? launch_dhop_pair_t<__half, true, false, 4>(op, p) : launch_dhop_pair_t<__half, false, false, 4>(op, p);
+  }
+  if (f) return dag ? launch_dhop_pair_t<float, true, false, 3>(op, p) : launch_dhop_pair_t<float, false, false, 3>(op, p);
   return dag ? launch_dhop_pair_t<__half, true, false, 3>(op, p) : launch_dhop_pair_t<__half, false, false, 3>(op, p);
 }
 
-int launch_dhop_axpy(Op* op, HalfView in, HalfView out, int out_parity, int dag, const DhopAxpy& a, int* done) {
-  return dhop_axpy_sides(op, in, out, out_parity, nullptr, nullptr, dag, a, done);
+int launch_dhop_axpy(Op* op, HalfView in, HalfView out, int out_parity, int dag, const DhopAxpy& a, int* done, int* parts,
+                     HalfView* r) {
+  return dhop_axpy_sides(op, in, out, out_parity, nullptr, nullptr, dag, a, done, parts, r);
 }
 int launch_dhop_full_axpy(Op* op, HalfView in_odd, HalfView out_even, HalfView in_even, HalfView out_odd, int dag,
                           const DhopAxpy& a, int* done) {

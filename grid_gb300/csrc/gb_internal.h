@@ -184,7 +184,11 @@ struct DhopAxpy {
   HalfView z[2];
   double c0, c1;
 };
-int launch_dhop_axpy(Op* op, HalfView in, HalfView out, int out_parity, int dag, const DhopAxpy& a, int* done);
+// parts (the CG on FP32 / FP16 Wilson operators): the launch also writes sums of |out|^2, or with r
+// applies r -= a out (a: the CG scalars) in place of storing out and writes sums of |r|^2, into
+// op->d_partial [*parts][nrhs]; *parts = 0 where it did neither and only stored out.
+int launch_dhop_axpy(Op* op, HalfView in, HalfView out, int out_parity, int dag, const DhopAxpy& a, int* done,
+                     int* parts = nullptr, HalfView* r = nullptr);
 int launch_dhop_full_axpy(Op* op, HalfView in_odd, HalfView out_even, HalfView in_even, HalfView out_odd, int dag,
                           const DhopAxpy& a, int* done);
 // FP32 / FP16: out = M5D(x5) - DhopEO/OE(in) in one launch (M5D with the given coefficients:
@@ -308,6 +312,8 @@ int build_neighbours(Op* op);
 int launch_cg_init(Op* op, const double* d_ssq, const double* d_cp, double tol, double delta);
 // a = c / d per rhs, d from the partial sums [nparts][nrhs] of a kernel that does not finish them
 int launch_cg_alpha(Op* op, const double* partial, int nparts);
+// the same for |r|^2: b and the convergence flags
+int launch_cg_beta(Op* op, const double* partial, int nparts);
 // r -= a mmp ; |r|^2 -> b and the convergence flags
 int launch_cg_r_update(Op* op, HalfView r, HalfView mmp, size_t n5, double* partial, int halves = 1);
 // psi += a p ; with update_p also p = b p + r

@@ -46,7 +46,9 @@ int op_meooe5d(Op* op, Field* in, Field* out, int dag);
 int op_dhop_cb(Op* op, Field* in, Field* out, int dag);
 int op_dhop_full(Op* op, Field* in, Field* out, int dag);
 // out = c0 z + c1 Dhop(in) on half fields, z on the output's checkerboard
-int op_dhop_cb_axpy(Op* op, Field* in, Field* z, Field* out, double c0, double c1, int dag);
+// (parts, r: see launch_dhop_axpy)
+int op_dhop_cb_axpy(Op* op, Field* in, Field* z, Field* out, double c0, double c1, int dag, int* parts = nullptr,
+                    Field* r = nullptr);
 // out = z - Meooe in
 int op_meooe_from(Op* op, Field* in, Field* z, Field* out);
 int op_meooe(Op* op, Field* in, Field* out, int dag);

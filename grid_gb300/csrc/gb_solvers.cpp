@@ -69,7 +69,7 @@ int cg_matrix_step(Op* op, int kind, Field* p, Field* mmp, Field* r) {
     else GB_TRY(cg_alpha_norm(op, z));
     GB_TRY(op_mpc(op, z, mmp, 1, nullptr, r, &rparts));
   }
-  if (rparts > 0) return GB_OK;  // r, |r|^2 and b are done
+  if (rparts > 0) return op->kind == 0 ? launch_cg_beta(op, op->d_partial, rparts) : GB_OK;  // (Moebius: b is done too)
   return cg_r_update(op, r, mmp);
 }
 // psi += a p ; with update_p also p = b p + r
