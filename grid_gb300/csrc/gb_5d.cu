@@ -30,7 +30,8 @@ struct M5Params {
   int L5, Ls;
 };
 
-template <class T, bool DAG, bool ZTERM>
+// UNIT: the diagonal is 1 (one FP64 operation per value instead of two)
+template <class T, bool DAG, bool ZTERM, bool UNIT = false>
 __global__ void __launch_bounds__(256) m5d_kernel(const M5Params p0, const Coef5<typename Arith<T>::type> c) {
   using R = typename Arith<T>::type;
   M5Params p = p0;
@@ -56,13 +57,13 @@ __global__ void __launch_bounds__(256) m5d_kernel(const M5Params p0, const Coef5
   Spinor<R> o;
 #pragma unroll
   for (int k = 0; k < 6; k++) {
-    o.re[k] = fma(cu, a.re[k], d * f.re[k]);
-    o.im[k] = fma(cu, a.im[k], d * f.im[k]);
+    o.re[k] = fma(cu, a.re[k], UNIT ? f.re[k] : d * f.re[k]);
+    o.im[k] = fma(cu, a.im[k], UNIT ? f.im[k] : d * f.im[k]);
   }
 #pragma unroll
   for (int k = 6; k < 12; k++) {
-    o.re[k] = fma(cl, a.re[k], d * f.re[k]);
-    o.im[k] = fma(cl, a.im[k], d * f.im[k]);
+    o.re[k] = fma(cl, a.re[k], UNIT ? f.re[k] : d * f.re[k]);
+    o.im[k] = fma(cl, a.im[k], UNIT ? f.im[k] : d * f.im[k]);
   }
   if (ZTERM) {
     Spinor<R> z;
@@ -435,6 +436,197 @@ int launch_mooee_inv(Op* op, HalfView in, HalfView out, int dag, size_t n4) {
   const unsigned blocks = unsigned((p.nq + 127) / 128);
   if (dag) mooee_inv_half_kernel<true><<<blocks, 128, 0, op->stream>>>(p, c);
   else mooee_inv_half_kernel<false><<<blocks, 128, 0, op->stream>>>(p, c);
+  GB_CHECK_CUDA(cudaGetLastError());
+  return GB_OK;
+}
+
+// ---------------------------------------------------------------------------------------
+// The 5D steps of the FP64 Mpc / MpcDag (LinearOperator.h:330-349).  FP64 issue bounds them, so
+// their constant factors are taken out: with M5D' = Meooe5D / b (unit diagonal, b = bs the same for
+// every s) and MooeeInv' = MooeeInv / D (D = 1 / dee the same below s = Ls - 1), one operation per
+// value less each,
+//   Mpc    = Mooee    - K Dhop M5D' MooeeInv' Dhop M5D',                K = b^2 D,
+//   MpcDag = MooeeDag - K M5D'^dag Dhop^dag MooeeInv'^dag M5D'^dag Dhop^dag,
+// and M5D' MooeeInv' (MooeeInv'^dag M5D'^dag) is one pass.  FP64 operations per 5D site: 24 + 72 + 72
+// and 72 + 96, where the separate passes took 48 + 120 + 72 and 120 + 120.  MpcDagMpc 16^4 x 16
+// with its import and export 1350 -> 1143 us; the two-step column pass 74 us, where MooeeInv and M5D
+// alone took 103 + 50 (16-byte column stores wrote half sectors; here two vectors go at once).
+// ---------------------------------------------------------------------------------------
+struct Mpc64Coef {
+  double e_up[kMaxLs], e_dn[kMaxLs];  // M5D': coefficients of the neighbour for spins 0, 1 and 2, 3
+  double lee[kMaxLs], leem[kMaxLs], uee[kMaxLs], ueem[kMaxLs];
+  double rho;  // the factor of s = Ls - 1 relative to D
+};
+
+// two consecutive 16-byte vectors, 32-byte aligned (a column starts at an even slot of a plane)
+__device__ __forceinline__ void load_two(const double2* p, double2& a, double2& b) {
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(a.x), "=d"(a.y), "=d"(b.x), "=d"(b.y) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void store_two(double2* p, double2 a, double2 b) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a.x), "d"(a.y), "d"(b.x), "d"(b.y) : "memory");
+}
+__device__ __forceinline__ double2 fma_two(double a, double2 x, double2 y) {
+  return make_double2(fma(a, x.x, y.x), fma(a, x.y, y.y));
+}
+
+// One thread per (component, column): M5D'(MooeeInv' x), DAG: MooeeInv'^dag(M5D'^dag x).  The
+// factors of DAG are transposed by the host as for mooee_inv_kernel.
+template <int LS, bool DAG>
+__global__ void __launch_bounds__(128) mpc64_col_kernel(const InvParams p, const Mpc64Coef c) {
+  pdl_wait();
+  const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (t >= p.nq * 12) return;
+  const int k = int(t / p.nq);
+  const size_t q = t - size_t(k) * p.nq;
+  const double2* in = static_cast<const double2*>(p.in) + size_t(k) * p.n5 + q * LS;
+  double2* out = static_cast<double2*>(p.out) + size_t(k) * p.n5 + q * LS;
+  const bool upper = k < 6;
+  const bool first = DAG ? !upper : upper;       // the chirality of the forward sweep
+  const bool from_minus = DAG ? !upper : upper;  // M5D takes s - 1 (else s + 1)
+  const double* e = upper ? c.e_up : c.e_dn;
+  double2 v[LS];
+#pragma unroll
+  for (int m = 0; m < LS; m += 2) load_two(in + m, v[m], v[m + 1]);
+  auto m5d = [&]() {  // in place: v_s += e_s v_{s -+ 1}, from the old values
+    const double2 v0 = v[0], vl = v[LS - 1];
+    if (from_minus) {
+#pragma unroll
+      for (int s = LS - 1; s > 0; s--) v[s] = fma_two(e[s], v[s - 1], v[s]);
+      v[0] = fma_two(e[0], vl, v[0]);
+    } else {
+#pragma unroll
+      for (int s = 0; s < LS - 1; s++) v[s] = fma_two(e[s], v[s + 1], v[s]);
+      v[LS - 1] = fma_two(e[LS - 1], v0, v[LS - 1]);
+    }
+  };
+  if (DAG) m5d();
+  if (first) {
+#pragma unroll
+    for (int s = 1; s < LS; s++) v[s] = fma_two(-c.lee[s - 1], v[s - 1], v[s]);
+  } else {
+#pragma unroll
+    for (int s = 0; s < LS - 1; s++) v[LS - 1] = fma_two(-c.leem[s], v[s], v[LS - 1]);
+  }
+  v[LS - 1].x *= c.rho;
+  v[LS - 1].y *= c.rho;
+  if (first) {
+#pragma unroll
+    for (int s = 0; s < LS - 1; s++) v[s] = fma_two(-c.ueem[s], v[LS - 1], v[s]);
+  } else {
+#pragma unroll
+    for (int s = LS - 2; s >= 0; s--) v[s] = fma_two(-c.uee[s], v[s + 1], v[s]);
+  }
+  if (!DAG) m5d();
+#pragma unroll
+  for (int m = 0; m < LS; m += 2) store_two(out + m, v[m], v[m + 1]);
+}
+
+// out = M5Ddag(x) with the coefficients a, plus zc M5D'^dag(y): the end of MpcDag
+__global__ void __launch_bounds__(256) mpc64_end_kernel(const M5Params p0, const Coef5<double> a, const Mpc64Coef c) {
+  M5Params p = p0;
+  pdl_wait();
+  p.psi = after_wait(p.psi);
+  p.z = after_wait(p.z);
+  const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= p.n5) return;
+  const int s5 = int(i % p.L5);
+  const int s = s5 % p.Ls;
+  const size_t base = i - s;
+  const size_t ip = base + (s + 1 == p.Ls ? 0 : s + 1);
+  const size_t im = base + (s == 0 ? p.Ls - 1 : s - 1);
+  const double2* x = static_cast<const double2*>(p.psi);
+  const double2* y = static_cast<const double2*>(p.z);
+  double2* o = static_cast<double2*>(p.chi);
+  const double d = a.d[s];
+#pragma unroll
+  for (int k = 0; k < 12; k++) {
+    const size_t j = size_t(k) * p.n5, n = j + (k < 6 ? ip : im);  // dag: P+ from s + 1
+    const double cx = k < 6 ? a.u[s] : a.l[s], cy = k < 6 ? c.e_up[s] : c.e_dn[s];
+    const double2 xv = __ldg(x + j + i), xn = __ldg(x + n), yv = __ldg(y + j + i), yn = __ldg(y + n);
+    const double2 w = fma_two(cy, yn, yv);
+    double2 r = make_double2(fma(cx, xn.x, d * xv.x), fma(cx, xn.y, d * xv.y));
+    o[j + i] = fma_two(p.zc, w, r);
+  }
+}
+
+bool mpc64_available(const Op* op, int prec) {
+  if (op->kind != 1 || op->zmobius || prec != GB_F64 || op->bs[0] == 0.0) return false;
+  for (int s = 1; s < op->Ls; s++)
+    if (op->bs[s] != op->bs[0] || (s < op->Ls - 1 && op->dee[s] != op->dee[0])) return false;
+  switch (op->Ls) {
+    case 4: case 6: case 8: case 10: case 12: case 14: case 16: case 18: case 20: case 24: return true;
+  }
+  return false;
+}
+
+double mpc64_factor(const Op* op) { return op->bs[0] * op->bs[0] / op->dee[0]; }
+
+static Mpc64Coef mpc64_coef(const Op* op, const double* lower, const double* upper, int dag) {
+  Mpc64Coef c = {};
+  const std::vector<double>& lee = dag ? op->uee : op->lee;
+  const std::vector<double>& leem = dag ? op->ueem : op->leem;
+  const std::vector<double>& uee = dag ? op->lee : op->uee;
+  const std::vector<double>& ueem = dag ? op->leem : op->ueem;
+  const double b = op->bs[0];
+  for (int s = 0; s < op->Ls; s++) {
+    // spins 0, 1 take s - 1 (dag: s + 1), spins 2, 3 the other side
+    c.e_up[s] = (dag ? upper[s] : lower[s]) / b;
+    c.e_dn[s] = (dag ? lower[s] : upper[s]) / b;
+    c.lee[s] = lee[s]; c.leem[s] = leem[s]; c.uee[s] = uee[s]; c.ueem[s] = ueem[s];
+  }
+  c.rho = op->dee[0] / op->dee[op->Ls - 1];
+  return c;
+}
+
+int launch_mpc64_m5d(Op* op, HalfView in, HalfView out, const double* lower, const double* upper) {
+  M5Params p = {};
+  p.psi = p.phi = in.data;
+  p.chi = out.data;
+  p.n5 = op->n5();
+  p.L5 = op->L5;
+  p.Ls = op->Ls;
+  Coef5<double> c;
+  for (int s = 0; s < op->Ls; s++) { c.d[s] = 1.0; c.u[s] = upper[s] / op->bs[0]; c.l[s] = lower[s] / op->bs[0]; }
+  launch_pdl(m5d_kernel<double, false, false, true>, unsigned((p.n5 + 255) / 256), 256, 0, op->stream, p, c);
+  GB_CHECK_CUDA(cudaGetLastError());
+  return GB_OK;
+}
+
+int launch_mpc64_col(Op* op, HalfView in, HalfView out, const double* lower, const double* upper, int dag) {
+  const Mpc64Coef c = mpc64_coef(op, lower, upper, dag);
+  InvParams p = {};
+  p.in = in.data;
+  p.out = out.data;
+  p.n5 = op->n5();
+  p.nq = size_t(op->half4) * op->nrhs;
+  const unsigned blocks = unsigned((p.nq * 12 + 127) / 128);
+  switch (op->Ls) {
+#define GB_MPC64(L)                                                                                       \
+  case L:                                                                                                 \
+    launch_pdl(dag ? mpc64_col_kernel<L, true> : mpc64_col_kernel<L, false>, blocks, 128, 0, op->stream, p, c); \
+    break;
+    GB_MPC64(4) GB_MPC64(6) GB_MPC64(8) GB_MPC64(10) GB_MPC64(12) GB_MPC64(14) GB_MPC64(16) GB_MPC64(18)
+    GB_MPC64(20) GB_MPC64(24)
+#undef GB_MPC64
+    default: set_error("FP64 column kernel: Ls = %d not instantiated", op->Ls); return GB_ERR_UNSUPPORTED;
+  }
+  GB_CHECK_CUDA(cudaGetLastError());
+  return GB_OK;
+}
+
+int launch_mpc64_end(Op* op, HalfView x, HalfView y, HalfView out, const double* xl, const double* xd, const double* xu,
+                     const double* yl, const double* yu, double zc) {
+  M5Params p = {};
+  p.psi = x.data;
+  p.z = y.data;
+  p.chi = out.data;
+  p.zc = zc;
+  p.n5 = op->n5();
+  p.L5 = op->L5;
+  p.Ls = op->Ls;
+  Coef5<double> a;
+  for (int s = 0; s < op->Ls; s++) { a.d[s] = xd[s]; a.u[s] = xu[s]; a.l[s] = xl[s]; }
+  launch_pdl(mpc64_end_kernel, unsigned((p.n5 + 255) / 256), 256, 0, op->stream, p, a, mpc64_coef(op, yl, yu, 1));
   GB_CHECK_CUDA(cudaGetLastError());
   return GB_OK;
 }

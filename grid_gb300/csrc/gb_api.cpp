@@ -576,6 +576,26 @@ int op_mpc(Op* op, Field* in, Field* out, int dag, int* norm_parts, Field* r_upd
     h.l2 = meo.l1; h.d2 = meo.d1; h.u2 = meo.u1;
     return col_field(op, COL_M5D, COLB_M5D, 1, in, to, out, -1.0, h, r_upd, r_parts);
   }
+  if (mpc64_available(op, in->prec)) {
+    te1->subset = te2->subset = GB_EVEN;
+    to->subset = out->subset = GB_ODD;
+    std::vector<double> l, d, u, ml, md, mu;
+    coeffs_meooe5d(op, dag, l, d, u);
+    coeffs_mooee(op, dag, ml, md, mu);
+    const double K = mpc64_factor(op);
+    if (!dag) {
+      GB_TRY(launch_mpc64_m5d(op, half_view(in, 0), half_view(to, 0), l.data(), u.data()));
+      GB_TRY(op_dhop_cb(op, to, te1, 0));
+      GB_TRY(launch_mpc64_col(op, half_view(te1, 0), half_view(te2, 0), l.data(), u.data(), 0));
+      GB_TRY(op_dhop_cb(op, te2, to, 0));
+      return m5d_field(op, in, in, out, ml, md, mu, 0, to, -K);
+    }
+    GB_TRY(op_dhop_cb(op, in, te1, 1));
+    GB_TRY(launch_mpc64_col(op, half_view(te1, 0), half_view(te2, 0), l.data(), u.data(), 1));
+    GB_TRY(op_dhop_cb(op, te2, to, 1));
+    return launch_mpc64_end(op, half_view(in, 0), half_view(to, 0), half_view(out, 0), ml.data(), md.data(), mu.data(),
+                            l.data(), u.data(), -K);
+  }
   GB_TRY(op_meooe(op, in, te1, dag));
   GB_TRY(op_mooee_inv(op, te1, te2, dag));
   GB_TRY(op_meooe(op, te2, to, dag));

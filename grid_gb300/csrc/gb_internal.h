@@ -218,6 +218,14 @@ int launch_deriv_fx(Op* op, HalfView A, HalfView B, int out_parity, int dag, dou
 int launch_m5d(Op* op, HalfView psi, HalfView phi, HalfView chi, const double* lower, const double* diag,
                const double* upper, int dag, size_t n5);
 int launch_mooee_inv(Op* op, HalfView in, HalfView out, int dag, size_t n4);
+// the 5D steps of the FP64 Mpc / MpcDag with their constant factors taken out (gb_5d.cu): lower,
+// upper are the Meooe5D coefficients of the same dagger; Mpc = Mooee - mpc64_factor() (the rest)
+bool mpc64_available(const Op* op, int prec);
+double mpc64_factor(const Op* op);
+int launch_mpc64_m5d(Op* op, HalfView in, HalfView out, const double* lower, const double* upper);
+int launch_mpc64_col(Op* op, HalfView in, HalfView out, const double* lower, const double* upper, int dag);
+int launch_mpc64_end(Op* op, HalfView x, HalfView y, HalfView out, const double* xl, const double* xd, const double* xu,
+                     const double* yl, const double* yu, double zc);
 // The field kernels below take one checkerboard, or with halves = 2 both of a full field in one
 // launch (the views of its first, even half; the odd one follows it in memory).
 // z = a*x + b*y (host scalars); x or y may alias z
