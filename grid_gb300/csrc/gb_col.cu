@@ -11,7 +11,7 @@
 // largest |re|, |im| of each 5D site) on the way out.
 //
 // Programs: out = A(x) + zc * B(y) with
-//   A in {M5D, INV, M5D(INV(x)), INV(M5D(x))},  B in {none, y, M5D(y)},
+//   A in {M5D, INV, M5D(INV(x)), INV(M5D(x))},  B in {none, M5D(y)},
 // one dagger flag for the whole program.  They fuse the steps of
 // SchurDiagMooeeOperator::Mpc / MpcDag (LinearOperator.h:330-349) that touch no
 // neighbour in 4D: Mpc = Mooee - DhopOE M5D MooeeInv DhopEO M5D, and
@@ -23,10 +23,8 @@
 
 namespace gb {
 
-// columns per CTA and the shared-memory slot of one column (an odd number of float4, so
-// the column reads of a quarter warp fall on distinct banks)
-// (with two input tiles 16 columns, so that several CTAs fit an SM's shared memory)
-template <int LS, int NIN = 1> __host__ __device__ constexpr int col_q() { return (LS >= 16 || NIN > 1) ? 16 : 32; }
+// the shared-memory slot of one column: an odd number of float4, so the column reads of a quarter
+// warp fall on distinct banks
 template <int LS> __host__ __device__ constexpr int col_stride() { return (LS / 2) % 2 == 0 ? LS / 2 + 1 : LS / 2; }
 
 template <int LS> struct ColCoef {
@@ -56,59 +54,9 @@ struct ColParams {
   CGFinish fin;  // RUPD: the last CTA updates the CG's b and convergence flags
 };
 
-// stage one input into the [12][Q][ST] float4 tile: FP32 copies the vectors, FP16 decodes
-// the two components of each vector with the norms of the pair's sites
-template <class T, int LS, int Q> struct ColIO;
-template <int LS, int Q> struct ColIO<float, LS, Q> {
-  static __device__ __forceinline__ void load(const void* src, const float*, float*, float4* tile, size_t np, size_t q0,
-                                              int nv) {
-    constexpr int H = LS / 2, ST = col_stride<LS>();
-    const float4* x = static_cast<const float4*>(src);
-#pragma unroll 4
-    for (int e = threadIdx.x; e < 12 * Q * H; e += 12 * Q) {
-      const int k = e / (Q * H), r = e - k * (Q * H);
-      if (r < nv) {
-        const int qq = r / H, m = r - qq * H;
-        tile[(k * Q + qq) * ST + m] = __ldg(x + size_t(k) * np + q0 * H + r);
-      }
-    }
-  }
-  static __device__ __forceinline__ void store(void* dst, float*, float*, float4* tile, size_t np, size_t q0, int nv) {
-    constexpr int H = LS / 2, ST = col_stride<LS>();
-    float4* o = static_cast<float4*>(dst);
-#pragma unroll 4
-    for (int e = threadIdx.x; e < 12 * Q * H; e += 12 * Q) {
-      const int k = e / (Q * H), r = e - k * (Q * H);
-      if (r < nv) {
-        const int qq = r / H, m = r - qq * H;
-        o[size_t(k) * np + q0 * H + r] = tile[(k * Q + qq) * ST + m];
-      }
-    }
-  }
-};
-template <int LS, int Q> struct ColIO<__half, LS, Q> {
-  // snorm: Q * LS floats of shared memory for the CTA's site norms
-  static __device__ __forceinline__ void load(const void* src, const float* norms, float* snorm, float4* tile,
-                                              size_t np, size_t q0, int nv) {
-    constexpr int H = LS / 2, ST = col_stride<LS>();
-    for (int e = threadIdx.x; e < 2 * nv; e += 12 * Q) snorm[e] = __ldg(norms + q0 * LS + e);
-    __syncthreads();
-    const uint4* x = static_cast<const uint4*>(src);
-    for (int e = threadIdx.x; e < 6 * Q * H; e += 12 * Q) {
-      const int g = e / (Q * H), r = e - g * (Q * H);
-      if (r < nv) {
-        const int qq = r / H, m = r - qq * H;
-        const uint4 v = __ldg(x + size_t(g) * np + q0 * H + r);
-        const __half2* h = reinterpret_cast<const __half2*>(&v);
-        const float n0 = snorm[qq * LS + 2 * m], n1 = snorm[qq * LS + 2 * m + 1];
-        const float2 a = __half22float2(h[0]), b = __half22float2(h[1]), c = __half22float2(h[2]),
-                     d = __half22float2(h[3]);
-        tile[((2 * g) * Q + qq) * ST + m] = make_float4(a.x * n0, a.y * n1, b.x * n0, b.y * n1);
-        tile[((2 * g + 1) * Q + qq) * ST + m] = make_float4(c.x * n0, c.y * n1, d.x * n0, d.y * n1);
-      }
-    }
-    __syncthreads();  // snorm is reused by the next input
-  }
+// a [12][Q][ST] float tile out as FP16 vectors with fresh norms (the largest |re|, |im| of each 5D
+// site); snorm: Q * LS floats of shared memory
+template <int LS, int Q> struct ColHalfIO {
   static __device__ __forceinline__ void store(void* dst, float* norms, float* snorm, float4* tile, size_t np,
                                                size_t q0, int nv) {
     constexpr int H = LS / 2, ST = col_stride<LS>();
@@ -239,27 +187,6 @@ __device__ __forceinline__ void col_run(float4* slot, const float4* yslot, float
   }
 #pragma unroll
   for (int m = 0; m < H; m++) slot[m] = make_float4(orr[2 * m], orr[2 * m + 1], oi[2 * m], oi[2 * m + 1]);
-}
-
-template <class T, int LS, bool DAG, int OPA, int OPB>
-__global__ void __launch_bounds__(12 * col_q<LS, OPB != COLB_NONE ? 2 : 1>()) col_kernel(const ColParams p,
-                                                                                        const ColCoef<LS> c) {
-  constexpr int Q = col_q<LS, OPB != COLB_NONE ? 2 : 1>(), H = LS / 2, ST = col_stride<LS>();
-  extern __shared__ float4 col_tile[];  // [inputs][12][Q][ST], then Q * LS norms (FP16)
-  float4* tx = col_tile;
-  float4* ty = col_tile + 12 * Q * ST;
-  float* snorm = reinterpret_cast<float*>(col_tile + (OPB != COLB_NONE ? 2 : 1) * 12 * Q * ST);
-  const int t = threadIdx.x;
-  const size_t q0 = size_t(blockIdx.x) * Q;
-  const int qn = p.nq - q0 < size_t(Q) ? int(p.nq - q0) : Q;
-  const int nv = qn * H;  // vectors of one plane in this CTA
-  ColIO<T, LS, Q>::load(p.x, p.xn, snorm, tx, p.np, q0, nv);
-  if (OPB != COLB_NONE) ColIO<T, LS, Q>::load(p.y, p.yn, snorm, ty, p.np, q0, nv);
-  __syncthreads();
-  const int k = t / Q, qq = t - k * Q;
-  if (qq < qn) col_run<LS, DAG, OPA, OPB>(tx + (k * Q + qq) * ST, ty + (k * Q + qq) * ST, p.zc, c, k < 6);
-  __syncthreads();
-  ColIO<T, LS, Q>::store(p.out, p.outn, snorm, tx, p.np, q0, nv);
 }
 
 // FP32 programs as a persistent kernel: each CTA walks its tiles of 16 columns with the
@@ -510,9 +437,9 @@ __global__ void __launch_bounds__(12 * kColPipeQ) col_pipe_half_kernel(const Col
           for (int m = 0; m < H; m++) s += cn[(kk * Q + t) * H + m];
         colacc += double(s);
       }
-      ColIO<__half, LS, Q>::store(p.r, p.rn, snorm, rt, p.np, tile * Q, nv);
+      ColHalfIO<LS, Q>::store(p.r, p.rn, snorm, rt, p.np, tile * Q, nv);
     } else {
-      ColIO<__half, LS, Q>::store(p.out, p.outn, snorm, ftile, p.np, tile * Q, nv);
+      ColHalfIO<LS, Q>::store(p.out, p.outn, snorm, ftile, p.np, tile * Q, nv);
     }
     __syncthreads();  // the float tile and this stage are read out before they are reused
   }
@@ -547,10 +474,6 @@ template <int LS> static void fill_col(const Op* op, int dag, const ColCoefsHost
     c.dinv[s] = float(1.0 / op->dee[s]);
   }
 }
-
-#ifndef GB_COL_PIPE
-#define GB_COL_PIPE 1
-#endif
 
 template <int LS, bool DAG, int OPA, int OPB, bool RUPD = false>
 static int col_pipe_go(Op* op, const ColParams& p, const ColCoef<LS>& c, int* r_parts = nullptr) {
@@ -610,21 +533,8 @@ static int col_pipe_half_go(Op* op, const ColParams& p, const ColCoef<LS>& c, in
 
 template <class T, int LS, bool DAG, int OPA, int OPB>
 static int col_go(Op* op, const ColParams& p, const ColCoef<LS>& c) {
-  if (GB_COL_PIPE && sizeof(T) == 4) return col_pipe_go<LS, DAG, OPA, OPB>(op, p, c);
-  if (GB_COL_PIPE && sizeof(T) == 2) return col_pipe_half_go<LS, DAG, OPA, OPB>(op, p, c);
-  constexpr int Q = col_q<LS, OPB != COLB_NONE ? 2 : 1>();
-  const size_t smem = size_t(OPB != COLB_NONE ? 2 : 1) * 12 * Q * col_stride<LS>() * sizeof(float4) +
-                      (sizeof(T) == 2 ? size_t(Q) * LS * sizeof(float) : 0);
-  static std::atomic<bool> configured{false};
-  if (!configured.load()) {
-    GB_CHECK_CUDA(cudaFuncSetAttribute(col_kernel<T, LS, DAG, OPA, OPB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       int(smem)));
-    configured.store(true);
-  }
-  const unsigned blocks = unsigned((p.nq + Q - 1) / Q);
-  col_kernel<T, LS, DAG, OPA, OPB><<<blocks, 12 * Q, smem, op->stream>>>(p, c);
-  GB_CHECK_CUDA(cudaGetLastError());
-  return GB_OK;
+  if constexpr (sizeof(T) == 4) return col_pipe_go<LS, DAG, OPA, OPB>(op, p, c);
+  else return col_pipe_half_go<LS, DAG, OPA, OPB>(op, p, c);
 }
 
 // the programs the operators use; the others are not instantiated
@@ -632,16 +542,12 @@ template <class T, int LS>
 static int col_ls(Op* op, int opa, int opb, int dag, const ColParams& p, const ColCoefsHost& h, int* r_parts) {
   ColCoef<LS> c;
   fill_col<LS>(op, dag, h, c);
-  if (GB_COL_PIPE && p.r && dag && opa == COL_M5D && opb == COLB_M5D) {
-    if (sizeof(T) == 4) return col_pipe_go<LS, true, COL_M5D, COLB_M5D, true>(op, p, c, r_parts);
-    return col_pipe_half_go<LS, true, COL_M5D, COLB_M5D, true>(op, p, c, r_parts);
+  if (p.r && dag && opa == COL_M5D && opb == COLB_M5D) {
+    if constexpr (sizeof(T) == 4) return col_pipe_go<LS, true, COL_M5D, COLB_M5D, true>(op, p, c, r_parts);
+    else return col_pipe_half_go<LS, true, COL_M5D, COLB_M5D, true>(op, p, c, r_parts);
   }
   const int key = (dag ? 100 : 0) + opa * 10 + opb;
   switch (key) {
-    case 0 + COL_M5D * 10 + COLB_NONE: return col_go<T, LS, false, COL_M5D, COLB_NONE>(op, p, c);
-    case 100 + COL_M5D * 10 + COLB_NONE: return col_go<T, LS, true, COL_M5D, COLB_NONE>(op, p, c);
-    case 0 + COL_M5D * 10 + COLB_IDENT: return col_go<T, LS, false, COL_M5D, COLB_IDENT>(op, p, c);
-    case 100 + COL_M5D * 10 + COLB_IDENT: return col_go<T, LS, true, COL_M5D, COLB_IDENT>(op, p, c);
     case 0 + COL_INV * 10 + COLB_NONE: return col_go<T, LS, false, COL_INV, COLB_NONE>(op, p, c);
     case 100 + COL_INV * 10 + COLB_NONE: return col_go<T, LS, true, COL_INV, COLB_NONE>(op, p, c);
     case 0 + COL_INV_M5D * 10 + COLB_NONE: return col_go<T, LS, false, COL_INV_M5D, COLB_NONE>(op, p, c);
@@ -652,10 +558,14 @@ static int col_ls(Op* op, int opa, int opb, int dag, const ColParams& p, const C
   return GB_ERR_UNSUPPORTED;
 }
 
+// Every even Ls from 4 to 24: with the column programs MpcDagMpc takes 319 us instead of 409 with the
+// separate M5D and MooeeInv kernels at 20 x 18 x 14 x 22 x 14 FP32, 252 instead of 475 at 16^4 x 18,
+// and 181 instead of 598 at 16^4 x 14 FP16 (whose MooeeInv without a column runs per site).  Above
+// 24 a thread's column and its result no longer fit the registers.
 bool col_available(const Op* op, int prec) {
   if (op->kind != 1 || op->zmobius || (prec != GB_F32 && prec != GB_F16)) return false;
   switch (op->Ls) {
-    case 4: case 6: case 8: case 10: case 12: case 16: case 20: case 24: return true;
+    case 4: case 6: case 8: case 10: case 12: case 14: case 16: case 18: case 20: case 22: case 24: return true;
   }
   return false;
 }
@@ -686,7 +596,8 @@ int launch_col(Op* op, int opa, int opb, int dag, HalfView x, HalfView y, HalfVi
   switch (op->Ls) {
 #define GB_COL_LS(L) \
   case L: return half ? col_ls<__half, L>(op, opa, opb, dag, p, h, parts) : col_ls<float, L>(op, opa, opb, dag, p, h, parts);
-    GB_COL_LS(4) GB_COL_LS(6) GB_COL_LS(8) GB_COL_LS(10) GB_COL_LS(12) GB_COL_LS(16) GB_COL_LS(20) GB_COL_LS(24)
+    GB_COL_LS(4) GB_COL_LS(6) GB_COL_LS(8) GB_COL_LS(10) GB_COL_LS(12) GB_COL_LS(14) GB_COL_LS(16) GB_COL_LS(18)
+    GB_COL_LS(20) GB_COL_LS(22) GB_COL_LS(24)
 #undef GB_COL_LS
   }
   set_error("column kernel: Ls = %d not instantiated", op->Ls);

@@ -266,7 +266,7 @@ inline int red_parts(Op* op, int prec) {
 // fused s-column programs of the Cayley 5D operators (gb_col.cu, FP32 Moebius):
 // out = A(x) + zc * B(y), one dagger flag for the program
 enum { COL_M5D = 0, COL_INV = 1, COL_INV_M5D = 2, COL_M5D_INV = 3 };  // A: M5D, INV, M5D(INV x), INV(M5D x)
-enum { COLB_NONE = 0, COLB_IDENT = 1, COLB_M5D = 2 };                 // B: -, y, M5D(y)
+enum { COLB_NONE = 0, COLB_M5D = 2 };                                 // B: -, M5D(y)
 struct ColCoefsHost {
   std::vector<double> l1, d1, u1;  // M5D of A (lower, diagonal, upper per s)
   std::vector<double> l2, d2, u2;  // M5D of B
