@@ -13,8 +13,8 @@
 //                         output site.  The multiply-add pipe is its bound (70 % busy); four
 //                         CTAs of 128 threads at 128 registers beat three at 168
 //   dhop_fx_split_kernel  the same with a site's directions over four warps
-// DhopEO, dhop_kernel<double> -> these: 16^4 x 16 820 -> 185 us, 16^4 x 12 599 -> 153 us,
-// 24^3 x 32 x 12 right-hand sides 3847 -> 955 us, Wilson 24^3 x 32 345 -> 138 us, 8^4 33 -> 12 us.
+// DhopEO, dhop_kernel<double> -> these: 16^4 x 16 820 -> 185 us, 16^4 x 12 599 -> 144 us,
+// 24^3 x 32 x 12 right-hand sides 3847 -> 931 us, Wilson 24^3 x 32 345 -> 138 us, 8^4 33 -> 12 us.
 //
 // A site whose values the fixed-point range does not hold (infinities, NaN, magnitudes outside
 // 2^(fx::kEmin - 1023) .. 2^(fx::kEmax - 1022)) is marked, and the outputs next to it are
@@ -651,6 +651,17 @@ static int* fx_exps(const Op* op, int z) {
   return reinterpret_cast<int*>(static_cast<longlong2*>(op->fx_field) + 24 * op->n5()) + size_t(z) * op->n5();
 }
 
+// Output sites per CTA of dhop_fx_kernel for L5c slots a site: of CTAs of up to 128 and up to 96
+// threads, the one that leaves fewer lanes of its warps idle, the larger one when equal (12 slots
+// fill 120 of 128 lanes or 96 of 96; 16 fill both).  Measured, always 128 -> this rule: 12 slots
+// 16^4 149 -> 144 us and 24^3 x 32 964 -> 931 us, 19 slots 240 -> 232 us, 22 slots 278 -> 267 us;
+// 96 threads at 16 slots: 186 against 182 us.
+static int fx_cta_sites(int L5c) {
+  const int large = 128 / L5c, small = 96 / L5c;
+  const auto lanes = [&](int sites) { return (sites * L5c + 31) / 32 * 32; };
+  return small * lanes(large) > large * lanes(small) ? small : large;
+}
+
 int launch_dhop_fx(Op* op, HalfView in, HalfView out, int out_parity, const HalfView* in2, const HalfView* out2, int dag,
                    const DhopAxpy* axpy) {
   FxParams p;
@@ -686,7 +697,7 @@ int launch_dhop_fx(Op* op, HalfView in, HalfView out, int out_parity, const Half
   } else {
     kernel = axpy ? dhop_fx_kernel<true> : dhop_fx_kernel<false>;
     p.L5c = p.L5a > 128 ? 128 : p.L5a;
-    p.k4 = 128 / p.L5c;
+    p.k4 = fx_cta_sites(p.L5c);
     const dim3 grid(unsigned((p.n4h + p.k4 - 1) / p.k4), unsigned((p.L5a + p.L5c - 1) / p.L5c), in2 ? 2u : 1u);
     const unsigned threads = unsigned((p.k4 * p.L5c + 31) / 32 * 32);
     launch_pdl(kernel, grid, threads, size_t(p.k4) * kFxLinkStride * sizeof(int4), op->stream, p);

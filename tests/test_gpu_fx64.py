@@ -54,6 +54,13 @@ def test_fixed_point_dhop(gpu_available, kind, dims, Ls, nrhs):
             assert o.rel_l2(y[r], ref.apply(code, np.ascontiguousarray(x.reshape(nrhs, -1)[r]))) < TOL, (dag, r)
 
 
+@pytest.mark.parametrize("dims,Ls,nrhs", [
+    ((8, 8, 6, 18), 1, 13), ((8, 8, 6, 12), 1, 19), ((8, 6, 10, 10), 12, 3), ((6, 10, 12, 10), 12, 1)])
+def test_cta_sizes(gpu_available, dims, Ls, nrhs):
+    """CTAs of 96 threads (12, 13 and 19 slots per site; 36 fill 128 better), 7 and 5 sites each with a remainder."""
+    test_fixed_point_dhop(gpu_available, "wilson" if Ls == 1 else "mobius", dims, Ls, nrhs)
+
+
 @pytest.mark.parametrize("power", [-1060, -1000, -920, -300, 300, 870, 890, 1010])
 def test_magnitudes(gpu_available, power):
     """The hopping term of 2^power x is 2^power times that of x, through the ends of the
