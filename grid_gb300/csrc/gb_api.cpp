@@ -411,11 +411,15 @@ int op_dhop_full(Op* op, Field* in, Field* out, int dag) {
 }
 
 // out = c0 z + c1 Dhop(in): one launch where the operator's kernel has the form, else two
-static int op_dhop_full_axpy(Op* op, Field* in, Field* z, Field* out, double c0, double c1, int dag) {
+static int op_dhop_full_axpy(Op* op, Field* in, Field* z, Field* out, double c0, double c1, int dag, int* parts = nullptr,
+                             Field* r = nullptr) {
+  if (parts) *parts = 0;
   if (!in->full() || !out->full()) { set_error("Dhop: full fields expected"); return GB_ERR_BAD_PARITY; }
   int done = 0;
-  const DhopAxpy a{{half_view(z, 0), half_view(z, 1)}, c0, c1};
-  GB_TRY(launch_dhop_full_axpy(op, half_view(in, 1), half_view(out, 0), half_view(in, 0), half_view(out, 1), dag, a, &done));
+  DhopAxpy a{{half_view(z, 0), half_view(z, 1)}, c0, c1};
+  if (r) { a.r[0] = half_view(r, 0); a.r[1] = half_view(r, 1); }
+  GB_TRY(launch_dhop_full_axpy(op, half_view(in, 1), half_view(out, 0), half_view(in, 0), half_view(out, 1), dag, a, &done,
+                               parts));
   if (done) return GB_OK;
   GB_TRY(op_dhop_full(op, in, out, dag));
   return field_axpby(out, c1, c0, out, z);
@@ -424,10 +428,10 @@ int op_dhop_cb_axpy(Op* op, Field* in, Field* z, Field* out, double c0, double c
   if (parts) *parts = 0;
   if (in->full() || out->full()) { set_error("DhopEO/OE: half fields expected"); return GB_ERR_BAD_PARITY; }
   int done = 0;
-  HalfView rv = r ? half_view(r, 0) : HalfView{};
   const int p = in->subset;
-  const DhopAxpy a{{half_view(z, 0), half_view(z, 0)}, c0, c1};
-  GB_TRY(launch_dhop_axpy(op, half_view(in, 0), half_view(out, 0), 1 - p, dag, a, &done, parts, r ? &rv : nullptr));
+  DhopAxpy a{{half_view(z, 0), half_view(z, 0)}, c0, c1};
+  if (r) a.r[0] = half_view(r, 0);
+  GB_TRY(launch_dhop_axpy(op, half_view(in, 0), half_view(out, 0), 1 - p, dag, a, &done, parts));
   out->subset = 1 - p;
   if (done) return GB_OK;
   GB_TRY(op_dhop_cb(op, in, out, dag));
@@ -520,10 +524,9 @@ int op_mooee_inv(Op* op, Field* in, Field* out, int dag) {
 
 // SchurDiagMooeeOperator::Mpc / MpcDag (LinearOperator.h:330-349).  With norm_parts (Mpc
 // of a FP32 / FP16 Moebius operator) the last kernel also reduces |out|^2 per right-hand
-// side (see launch_m5d_pair; Wilson: launch_dhop_axpy).  With r_upd (MpcDag of a FP32 / FP16 Wilson
-// operator, or Moebius operator whose
-// right-hand-side count divides 16) the last kernel applies r -= a out for the CG instead
-// of storing out (see launch_col).
+// side (see launch_m5d_pair; Wilson: launch_dhop_axpy).  With r_upd (MpcDag of a Wilson operator,
+// or of a FP32 / FP16 Moebius operator whose right-hand-side count divides 16) the last kernel
+// applies r -= a out for the CG instead of storing out (see launch_col).
 int op_mpc(Op* op, Field* in, Field* out, int dag, int* norm_parts, Field* r_upd, int* r_parts) {
   if (norm_parts) *norm_parts = 0;
   if (r_parts) *r_parts = 0;
@@ -611,10 +614,11 @@ int op_mpcdagmpc(Op* op, Field* in, Field* out) {
 
 // M / Mdag on full fields (WilsonFermionImplementation.h:113-127,
 // CayleyFermion5DImplementation.h:272-306)
-int op_m(Op* op, Field* in, Field* out, int dag) {
+int op_m(Op* op, Field* in, Field* out, int dag, int* norm_parts, Field* r_upd) {
+  if (norm_parts) *norm_parts = 0;
   if (!in->full() || !out->full()) { set_error("M: full fields expected"); return GB_ERR_BAD_PARITY; }
   if (op->kind == 0) {
-    if (!op->tm) return op_dhop_full_axpy(op, in, in, out, op->diag_mass, 1.0, dag);
+    if (!op->tm) return op_dhop_full_axpy(op, in, in, out, op->diag_mass, 1.0, dag, norm_parts, r_upd);
     GB_TRY(op_dhop_full(op, in, out, dag));
     return tm_diag(op, in, out, dag, 0, out, 1.0);  // out = Mooee in + Dhop in
   }
@@ -634,11 +638,10 @@ int op_m(Op* op, Field* in, Field* out, int dag) {
   return m5d_field(op, in, Din, out, l, d, u, 1, in, 1.0);  // out = M5Ddag(psi, Din) + psi
 }
 
-int op_mdagm(Op* op, Field* in, Field* out, Field** m_in) {
+int op_mdagm(Op* op, Field* in, Field* out) {
   Field* t;
   GB_TRY(ws_get(op, GB_FULL, in->prec, WS_MDAGM, &t));
   GB_TRY(op_m(op, in, t, 0));
-  if (m_in) *m_in = t;
   return op_m(op, t, out, 1);
 }
 
@@ -835,10 +838,12 @@ static int op_create(int kind, const int dims[4], int Ls, double mass, double M5
   }
   alloc(reinterpret_cast<void**>(&op->d_err), sizeof(int));
   // the reductions' [2 halves][kRedBlocks][nrhs][2]; an FP32 or FP16 Dhop with a summing epilogue
-  // writes nrhs sums per CTA
+  // writes nrhs sums per CTA, the FP64 one a sum per 32 sites of both checkerboards
   op->partial_doubles = size_t(2) * kRedBlocks * nrhs * 2;
   if (op->prec != GB_F64)
     op->partial_doubles = std::max(op->partial_doubles, dhop_pair_ctas(op) * nrhs);
+  else if (op->Ls == 1 && op->nrhs_user == 1)
+    op->partial_doubles = std::max(op->partial_doubles, size_t((op->half4 + 31) / 32) * 2);
   alloc(reinterpret_cast<void**>(&op->d_partial), op->partial_doubles * sizeof(double));
   alloc(reinterpret_cast<void**>(&op->d_result), size_t(nrhs) * 8 * sizeof(double));
   alloc(reinterpret_cast<void**>(&op->d_cg), size_t(nrhs) * sizeof(CGScalars));

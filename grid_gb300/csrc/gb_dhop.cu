@@ -942,17 +942,19 @@ int launch_dhop_mooee(Op* op, HalfView in, HalfView x5, HalfView out, int out_pa
 }
 
 static int dhop_axpy_sides(Op* op, HalfView in, HalfView out, int out_parity, const HalfView* in2, const HalfView* out2,
-                           int dag, const DhopAxpy& a, int* done, int* parts = nullptr, HalfView* r = nullptr) {
+                           int dag, const DhopAxpy& a, int* done, int* parts) {
   *done = 0;
   if (parts) *parts = 0;
   if (op->recon12 || (op->prec == GB_F64 && !op->fx_ready)) return GB_OK;
   GB_TRY(dhop_checks(op, in, out, in2, out2));
+  const HalfView* r = a.r[0].data ? a.r : nullptr;
   if (a.z[0].prec != op->prec || a.z[1].prec != op->prec) {
     set_error("Dhop: field precision differs from the operator's");
     return GB_ERR_BAD_ARG;
   }
   *done = 1;
-  if (op->prec == GB_F64) return launch_dhop_fx(op, in, out, out_parity, in2, out2, dag, &a);
+  if (op->prec == GB_F64)
+    return launch_dhop_fx(op, in, out, out_parity, in2, out2, dag, &a, r && r->prec != op->prec ? nullptr : parts);
   DhopParams p;
   fill_dhop_params(op, in, out, out_parity, in2, out2, p);
   p.x5 = a.z[0].data;
@@ -979,13 +981,12 @@ static int dhop_axpy_sides(Op* op, HalfView in, HalfView out, int out_parity, co
   return dag ? launch_dhop_pair_t<__half, true, false, 3>(op, p) : launch_dhop_pair_t<__half, false, false, 3>(op, p);
 }
 
-int launch_dhop_axpy(Op* op, HalfView in, HalfView out, int out_parity, int dag, const DhopAxpy& a, int* done, int* parts,
-                     HalfView* r) {
-  return dhop_axpy_sides(op, in, out, out_parity, nullptr, nullptr, dag, a, done, parts, r);
+int launch_dhop_axpy(Op* op, HalfView in, HalfView out, int out_parity, int dag, const DhopAxpy& a, int* done, int* parts) {
+  return dhop_axpy_sides(op, in, out, out_parity, nullptr, nullptr, dag, a, done, parts);
 }
 int launch_dhop_full_axpy(Op* op, HalfView in_odd, HalfView out_even, HalfView in_even, HalfView out_odd, int dag,
-                          const DhopAxpy& a, int* done) {
-  return dhop_axpy_sides(op, in_odd, out_even, 0, &in_even, &out_odd, dag, a, done);
+                          const DhopAxpy& a, int* done, int* parts) {
+  return dhop_axpy_sides(op, in_odd, out_even, 0, &in_even, &out_odd, dag, a, done, parts);
 }
 
 int launch_dhop(Op* op, HalfView in, HalfView out, int out_parity, int dag) {

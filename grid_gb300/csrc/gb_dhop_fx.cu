@@ -50,6 +50,9 @@ struct FxParams {
   int link_exp;          // k of gb_fx64.cuh
   int dag;
   int* err;
+  double2* r[2];  // the CG forms of the split kernel: the residual, the CTAs' sums, what the last CTA does
+  double* partial;
+  CGFinish fin;
 };
 
 constexpr int kFxLinkStride = 73;  // int4 per staged site: 72 and one of padding
@@ -202,13 +205,13 @@ __device__ __forceinline__ void fp64_legs(const double2* in, const double* links
 }
 // one output component: the Dhop's value, or (AXPY) c0 z + c1 of it
 template <bool AXPY>
-__device__ __forceinline__ void fx_store(const FxParams& p, const double2* z, double2* out, size_t w, double re, double im) {
+__device__ __forceinline__ double2 fx_result(const FxParams& p, const double2* z, size_t w, double re, double im) {
   if (AXPY) {
     const double2 v = __ldg(z + w);
     re = fma(p.c1, re, p.c0 * v.x);
     im = fma(p.c1, im, p.c0 * v.y);
   }
-  out[w] = make_double2(re, im);
+  return make_double2(re, im);
 }
 
 // the integer (units of 2^e) as a double, rounded once; 0 stays 0
@@ -350,7 +353,52 @@ __global__ void __launch_bounds__(128, 4) dhop_fx_kernel(const __grid_constant__
   const int e = fx::result_exponent(Ea, p.link_exp);
   const size_t i = size_t(x) * p.L5 + s;
 #pragma unroll
-  for (int k = 0; k < 12; k++) fx_store<AXPY>(p, z, out, size_t(k) * p.n5 + i, fx_value(acc.re[k], e), fx_value(acc.im[k], e));
+  for (int k = 0; k < 12; k++) {
+    const size_t w = size_t(k) * p.n5 + i;
+    out[w] = fx_result<AXPY>(p, z, w, fx_value(acc.re[k], e), fx_value(acc.im[k], e));
+  }
+}
+
+// |v|^2 into sum; UPDATE: of r - a v, which replaces r
+template <bool UPDATE>
+__device__ __forceinline__ void fx_cg_term(double2* r, double a, double2 v, double& sum) {
+  if (UPDATE) {
+    const double2 o = *r;
+    v = make_double2(fma(-a, v.x, o.x), fma(-a, v.y, o.y));
+    *r = v;
+  }
+  sum = fma(v.x, v.x, fma(v.y, v.y, sum));
+}
+
+// The end of a CG form for one right-hand side, by every thread of every CTA of 128: the CTA's sum, and in
+// the last CTA all of them in a fixed order and the CG's scalars from it.  The padding's scalars stay as
+// cg_init_kernel set them (done, a = b = 0).
+__device__ __forceinline__ void fx_cg_finish(const FxParams& p, double sum) {
+  __shared__ double ws[4];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const auto cta_sum = [&](double v) {  // in thread 0
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if (lane == 0) ws[warp] = v;
+    __syncthreads();
+    return (ws[0] + ws[1]) + (ws[2] + ws[3]);
+  };
+  const int ctas = int(gridDim.x * gridDim.z);
+  sum = cta_sum(sum);
+  if (threadIdx.x == 0) p.partial[blockIdx.z * gridDim.x + blockIdx.x] = sum;
+  if (!last_cta(p.fin.flags + kCGTicket, ctas)) return;
+  sum = 0.0;
+#pragma unroll 8
+  for (int b = threadIdx.x; b < ctas; b += 128) sum += __ldcg(p.partial + b);
+  sum = cta_sum(sum);
+  if (threadIdx.x != 0) return;
+  CGScalars c = *p.fin.cg;
+  if (p.fin.mode == CG_FINISH_ALPHA) cg_alpha_update(c, sum);
+  else cg_beta_update(c, sum);
+  *p.fin.cg = c;
+  if (p.fin.mode != CG_FINISH_BETA) return;
+  __threadfence();
+  cg_set_flags(p.fin.cg, p.L5, p.fin.flags);
 }
 
 // Four warps share 32 output sites, one direction (its forward and backward leg) each, and add
@@ -359,7 +407,12 @@ __global__ void __launch_bounds__(128, 4) dhop_fx_kernel(const __grid_constant__
 // chain is the launch's time (8^4: 12.4 us, one thread per site 20.0), and with sites in lanes
 // the extra warps keep more of the links' 1152 bytes per site in flight (24^3 x 32: 138 us, one
 // thread per site 153).  SOA: the links' sites-in-lanes layout.
-template <bool SOA, bool AXPY>
+// CG (one right-hand side): the CG's next reduction rides on the launch.  CG_FINISH_ALPHA stores
+// out and sums |out|^2, CG_FINISH_BETA applies r -= a out in place of storing out and sums |r|^2,
+// and the last CTA turns the sum into the CG's a or b.  Separate passes -> this, us per CG
+// iteration on MdagM: 8^4 42.4 -> 33.7, 12^4 75.3 -> 70.2, 16^4 164 -> 155, 24^3 x 32 932 -> 894,
+// 32^4 2137 -> 2109; with more right-hand sides the passes stay.
+template <bool SOA, bool AXPY, int CG = CG_FINISH_NONE>
 __global__ void __launch_bounds__(128, 4) dhop_fx_split_kernel(const __grid_constant__ FxParams p) {
   __shared__ long long part[4][24][32];
   const int side = blockIdx.z;
@@ -384,23 +437,34 @@ __global__ void __launch_bounds__(128, 4) dhop_fx_split_kernel(const __grid_cons
     for (int k = 0; k < 12; k++) { part[mu][2 * k][lane] = acc.re[k]; part[mu][2 * k + 1][lane] = acc.im[k]; }
   }
   __syncthreads();
-  if (!active) return;
-  if (mu == 0) fx_pad(p, out, x, s);
-  if (Ea == fx::kBad) {
-    if (mu == 0) fx_site_fp64(in, out, z, p.c0, p.c1, p.links_d[side], nbr, p.n5, p.L5, x, s, p.dag);
-    return;
-  }
-  const int e = fx::result_exponent(Ea, p.link_exp);
   const size_t i = size_t(x) * p.L5 + s;
-#pragma unroll
-  for (int m = 0; m < 3; m++) {  // warp mu finishes components 3 mu .. 3 mu + 2
-    const int k = 3 * mu + m;
-    long long v[2];
-#pragma unroll
-    for (int c = 0; c < 2; c++)
-      v[c] = (part[0][2 * k + c][lane] + part[1][2 * k + c][lane]) + (part[2][2 * k + c][lane] + part[3][2 * k + c][lane]);
-    fx_store<AXPY>(p, z, out, size_t(k) * p.n5 + i, fx_value(v[0], e), fx_value(v[1], e));
+  double2* const r = CG == CG_FINISH_BETA ? p.r[side] + i : nullptr;
+  const double a = CG == CG_FINISH_BETA ? __ldcg(&p.fin.cg->a) : 0.0;
+  double sum = 0.0;
+  if (active && mu == 0) {
+    fx_pad(p, out, x, s);
+    if (Ea == fx::kBad) {
+      fx_site_fp64(in, out, z, p.c0, p.c1, p.links_d[side], nbr, p.n5, p.L5, x, s, p.dag);
+      if (CG != CG_FINISH_NONE)
+        for (int k = 0; k < 12; k++) fx_cg_term<CG == CG_FINISH_BETA>(r + size_t(k) * p.n5, a, out[size_t(k) * p.n5 + i], sum);
+    }
   }
+  if (active && Ea != fx::kBad) {
+    const int e = fx::result_exponent(Ea, p.link_exp);
+#pragma unroll
+    for (int m = 0; m < 3; m++) {  // warp mu finishes components 3 mu .. 3 mu + 2
+      const int k = 3 * mu + m;
+      long long v[2];
+#pragma unroll
+      for (int c = 0; c < 2; c++)
+        v[c] = (part[0][2 * k + c][lane] + part[1][2 * k + c][lane]) + (part[2][2 * k + c][lane] + part[3][2 * k + c][lane]);
+      const size_t w = size_t(k) * p.n5 + i;
+      const double2 d = fx_result<AXPY>(p, z, w, fx_value(v[0], e), fx_value(v[1], e));
+      if (CG != CG_FINISH_BETA) out[w] = d;
+      if (CG != CG_FINISH_NONE) fx_cg_term<CG == CG_FINISH_BETA>(r + size_t(k) * p.n5, a, d, sum);
+    }
+  }
+  if (CG != CG_FINISH_NONE) fx_cg_finish(p, sum);
 }
 
 // ---- force term (gb_dhop.cu's deriv_kernel: mat = U W, W = sum_s h conj(g)^T) in fixed point ----
@@ -663,7 +727,7 @@ static int fx_cta_sites(int L5c) {
 }
 
 int launch_dhop_fx(Op* op, HalfView in, HalfView out, int out_parity, const HalfView* in2, const HalfView* out2, int dag,
-                   const DhopAxpy* axpy) {
+                   const DhopAxpy* axpy, int* parts) {
   FxParams p;
   const HalfView* ins[2] = {&in, in2};
   const HalfView* outs[2] = {&out, out2};
@@ -690,6 +754,18 @@ int launch_dhop_fx(Op* op, HalfView in, HalfView out, int out_parity, const Half
   launch_pdl(fx_convert_kernel, dim3(unsigned((p.n5 + 255) / 256), 1, in2 ? 2u : 1u), 256, 0, op->stream, p);
   const bool soa = fx_soa(op);
   void (*kernel)(const FxParams);
+  const size_t ctas = size_t((p.n4h * p.L5a + 31) / 32) * (in2 ? 2 : 1);
+  if (parts && axpy && op->Ls == 1 && op->nrhs_user == 1 && ctas <= op->partial_doubles) {
+    const bool beta = axpy->r[0].data != nullptr;
+    for (int z = 0; z < 2; z++) p.r[z] = static_cast<double2*>(axpy->r[z].data);
+    p.partial = op->d_partial;
+    p.fin = CGFinish{op->d_cg, op->d_all_done, beta ? CG_FINISH_BETA : CG_FINISH_ALPHA};
+    *parts = -1;
+    launch_pdl(beta ? dhop_fx_split_kernel<true, true, CG_FINISH_BETA> : dhop_fx_split_kernel<true, true, CG_FINISH_ALPHA>,
+               dim3(unsigned((p.n4h + 31) / 32), 1, in2 ? 2u : 1u), 128, 0, op->stream, p);
+    GB_CHECK_CUDA(cudaGetLastError());
+    return GB_OK;
+  }
   if (soa || p.n4h * p.L5a * (in2 ? 2 : 1) <= kFxSplitSites) {
     if (soa) kernel = axpy ? dhop_fx_split_kernel<true, true> : dhop_fx_split_kernel<true, false>;
     else kernel = axpy ? dhop_fx_split_kernel<false, true> : dhop_fx_split_kernel<false, false>;

@@ -105,7 +105,7 @@ struct Op {
 
   // reduction scratch
   double* d_partial = nullptr;  // per-CTA partial sums, partial_doubles of them
-  size_t partial_doubles = 0;    // 4 kRedBlocks nrhs, or a single-checkerboard Dhop's CTAs x nrhs if more
+  size_t partial_doubles = 0;    // 4 kRedBlocks nrhs, or the sums of a Dhop with a summing end if more
   double* d_result = nullptr;   // nrhs * 4
   double* h_result = nullptr;   // pinned, nrhs * 4
   // canonical FP64 staging buffer for import/export (device)
@@ -183,14 +183,16 @@ int launch_dhop(Op* op, HalfView in, HalfView out, int out_parity, int dag);
 struct DhopAxpy {
   HalfView z[2];
   double c0, c1;
+  HalfView r[2] = {};
 };
-// parts (the CG on FP32 / FP16 Wilson operators): the launch also writes sums of |out|^2, or with r
-// applies r -= a out (a: the CG scalars) in place of storing out and writes sums of |r|^2, into
-// op->d_partial [*parts][nrhs]; *parts = 0 where it did neither and only stored out.
+// parts (the CG on Wilson operators): the launch also sums |out|^2, or with r.data
+// applies r -= a out (a: the CG scalars) in place of storing out and sums |r|^2.
+// *parts > 0: the sums are in op->d_partial [*parts][nrhs] (FP32 / FP16 half fields); < 0: the CG's a (with r: b) is
+// computed from them too (FP64, one right-hand side); 0: it did neither and only stored out.
 int launch_dhop_axpy(Op* op, HalfView in, HalfView out, int out_parity, int dag, const DhopAxpy& a, int* done,
-                     int* parts = nullptr, HalfView* r = nullptr);
+                     int* parts = nullptr);
 int launch_dhop_full_axpy(Op* op, HalfView in_odd, HalfView out_even, HalfView in_even, HalfView out_odd, int dag,
-                          const DhopAxpy& a, int* done);
+                          const DhopAxpy& a, int* done, int* parts = nullptr);
 // FP32 / FP16: out = M5D(x5) - DhopEO/OE(in) in one launch (M5D with the given coefficients:
 // Mooee for the end of Mpc), |out|^2 per CTA and right-hand side into op->d_partial
 // ([CTA][nrhs], the norm partials' layout) and the CTA count into *parts.  Cases: one
@@ -204,9 +206,8 @@ size_t dhop_pair_ctas(const Op* op);
 // copies, and one launch (in2, out2: the second checkerboard of a full-lattice Dhop)
 bool fx_wanted(const Op* op);
 int fx_import_links(Op* op);
-struct DhopAxpy;
 int launch_dhop_fx(Op* op, HalfView in, HalfView out, int out_parity, const HalfView* in2, const HalfView* out2, int dag,
-                   const DhopAxpy* axpy = nullptr);
+                   const DhopAxpy* axpy = nullptr, int* parts = nullptr);
 int launch_dhop_full(Op* op, HalfView in_odd, HalfView out_even, HalfView in_even, HalfView out_odd, int dag);
 // force term of the output parity's sites into mat (FP64 canonical gauge layout, indexed
 // by x_cb when half_out, else by the lexicographic site); A has the output parity

@@ -56,17 +56,18 @@ int op_mooee(Op* op, Field* in, Field* out, int dag, Field* z, double zc, int* n
 int op_mooee_inv(Op* op, Field* in, Field* out, int dag);
 // norm_parts (Mpc only): when non-null, the last kernel may also reduce |out|^2 into
 // op->d_partial ([CTA][nrhs], the layout of the norm partials) and sets *norm_parts to the
-// number of CTA sums written, or to 0 when it did not.
+// number of CTA sums written, to 0 when it did not, or below 0 when it has updated the CG's a too.
 // r_upd, r_parts (MpcDag only, for the CG): when both are non-null, the last kernel may
 // instead of storing out apply r_upd -= a out (a: the CG scalars of op) and reduce
-// |r_upd|^2, from which it updates the CG's b and convergence flags; *r_parts is the number of CTA
-// sums, or 0 when it stored out and left r_upd and the scalars alone
+// |r_upd|^2, from which it updates the CG's b and convergence flags (a FP32 / FP16 Wilson operator's
+// leaves those to launch_cg_beta); *r_parts is the number of CTA
+// sums, below 0 without sums to read, or 0 when it stored out and left r_upd and the scalars alone
 int op_mpc(Op* op, Field* in, Field* out, int dag, int* norm_parts = nullptr, Field* r_upd = nullptr,
            int* r_parts = nullptr);
 int op_mpcdagmpc(Op* op, Field* in, Field* out);
-int op_m(Op* op, Field* in, Field* out, int dag);
-// m_in: the workspace field that holds M in afterwards
-int op_mdagm(Op* op, Field* in, Field* out, Field** m_in = nullptr);
+// norm_parts, r_upd (for the CG): as norm_parts and r_parts of op_mpc, *norm_parts either 0 or < 0
+int op_m(Op* op, Field* in, Field* out, int dag, int* norm_parts = nullptr, Field* r_upd = nullptr);
+int op_mdagm(Op* op, Field* in, Field* out);
 int op_dminus(Op* op, Field* in, Field* out, int dag);
 // flops of one application of MdagM (kind 0) or MpcDagMpc (kind 1) in Grid's model
 double hermop_flops(const Op* op, int kind);

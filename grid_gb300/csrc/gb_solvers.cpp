@@ -51,26 +51,22 @@ int cg_r_update(Op* op, Field* r, Field* mmp) {
   return launch_cg_r_update(op, half_view(r, 0), half_view(mmp, 0), r->n5, op->d_partial, P.halves);
 }
 // One CG matrix step on p: A = MdagM (kind 0) or MpcDagMpc (kind 1) with d = |M p|^2
-// (|Mpc p|^2) -> a, then r -= a A p, cp = |r|^2 -> b.  For a FP32 / FP16 Moebius Schur
-// operator the norm comes from the kernel that stores Mpc p, and MpcDag's last kernel
-// updates r in place of storing A p (mmp is then not written).
+// (|Mpc p|^2) -> a, then r -= a A p, cp = |r|^2 -> b.  For a Wilson operator (FP64: one
+// right-hand side; FP32 / FP16: Schur) and a FP32 / FP16 Moebius Schur operator the norm comes from
+// the kernel that stores M p, and the dagger's last kernel updates r in place of storing A p
+// (mmp is then not written, or only in part).
 int cg_matrix_step(Op* op, int kind, Field* p, Field* mmp, Field* r) {
-  int rparts = 0;
-  if (kind == 0) {
-    Field* mp = nullptr;
-    GB_TRY(op_mdagm(op, p, mmp, &mp));
-    GB_TRY(cg_alpha_norm(op, mp));
-  } else {
-    Field* z;
-    GB_TRY(ws_get(op, GB_ODD, p->prec, WS_MPCDAGMPC, &z));
-    int dparts = 0;
-    GB_TRY(op_mpc(op, p, z, 0, &dparts));
-    if (dparts > 0) GB_TRY(launch_cg_alpha(op, op->d_partial, dparts));
-    else GB_TRY(cg_alpha_norm(op, z));
-    GB_TRY(op_mpc(op, z, mmp, 1, nullptr, r, &rparts));
-  }
-  if (rparts > 0) return op->kind == 0 ? launch_cg_beta(op, op->d_partial, rparts) : GB_OK;  // (Moebius: b is done too)
-  return cg_r_update(op, r, mmp);
+  Field* z;
+  GB_TRY(ws_get(op, kind == 0 ? GB_FULL : GB_ODD, p->prec, kind == 0 ? WS_MDAGM : WS_MPCDAGMPC, &z));
+  int dparts = 0, rparts = 0;
+  if (kind == 0) GB_TRY(op_m(op, p, z, 0, &dparts));
+  else GB_TRY(op_mpc(op, p, z, 0, &dparts));
+  if (dparts > 0) GB_TRY(launch_cg_alpha(op, op->d_partial, dparts));
+  else if (dparts == 0) GB_TRY(cg_alpha_norm(op, z));
+  if (kind == 0) GB_TRY(op_m(op, z, mmp, 1, &rparts, r));
+  else GB_TRY(op_mpc(op, z, mmp, 1, nullptr, r, &rparts));
+  if (rparts == 0) return cg_r_update(op, r, mmp);
+  return rparts > 0 && op->kind == 0 ? launch_cg_beta(op, op->d_partial, rparts) : GB_OK;  // (otherwise b is done too)
 }
 // psi += a p ; with update_p also p = b p + r
 int cg_xp_update(Op* op, Field* psi, Field* p, Field* r, int update_p) {

@@ -120,3 +120,29 @@ def test_links_of_any_size_and_reimport(gpu_available):
         op.ImportGauge(U * scale)
         op.DhopEO(fi, fo, 0)
         assert np.abs(fo.export() - scale * one).max() <= 4e-15 * scale * np.abs(one).max()
+
+
+@pytest.mark.parametrize("dims", [(2, 2, 2, 2), (4, 4, 4, 6), (6, 2, 4, 10), (8, 8, 8, 8)])
+@pytest.mark.parametrize("tiny", [False, True])
+@pytest.mark.parametrize("schur", [False, True])
+def test_cg_sums_in_the_hopping_term(gpu_available, dims, tiny, schur):
+    """One right-hand side takes the CG's sums and residual update in the hopping term's launch, two
+    the separate passes: the same solution and iterations.  tiny: a point source and values
+    below the fixed-point range elsewhere, so that both kinds of site end in a sum.  Bound: both
+    true residuals are below 1e-10, the condition number of M^dag M (mass 0.5) below 1000."""
+    U = g.random_gauge(dims, 0.5, 17)
+    n = int(np.prod(dims)) // (2 if schur else 1) * 12
+    x = fermion(n // 12, 1, 18)
+    if tiny:
+        x = x.copy()
+        x[12:] *= 2.0 ** -940
+    got = []
+    for nrhs in (1, 2):
+        op = g.WilsonFermion(U, dims, 0.5, nrhs=nrhs)
+        new = (lambda: op.FermionRedBlackField(g.ODD)) if schur else op.FermionField
+        src, sol = new().import_(np.concatenate([x] * nrhs)), new().import_(np.zeros(n * nrhs, complex))
+        cg = g.ConjugateGradient(1e-10, 500, check_every=1)
+        cg(g.SchurDiagMooeeOperator(op) if schur else g.MdagMLinearOperator(op), src, sol)
+        got.append((sol.export().reshape(nrhs, -1)[0], cg.IterationsToComplete))
+    assert abs(got[0][1] - got[1][1]) <= 1
+    assert o.rel_l2(got[0][0], got[1][0]) < 2e-7
