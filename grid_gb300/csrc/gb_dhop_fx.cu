@@ -14,7 +14,7 @@
 //                         CTAs of 128 threads at 128 registers beat three at 168
 //   dhop_fx_split_kernel  the same with a site's directions over four warps
 // DhopEO, dhop_kernel<double> -> these: 16^4 x 16 820 -> 185 us, 16^4 x 12 599 -> 144 us,
-// 24^3 x 32 x 12 right-hand sides 3847 -> 931 us, Wilson 24^3 x 32 345 -> 138 us, 8^4 33 -> 12 us.
+// 24^3 x 32 x 12 right-hand sides 3847 -> 931 us, Wilson 24^3 x 32 345 -> 125 us, 8^4 33 -> 8 us.
 //
 // A site whose values the fixed-point range does not hold (infinities, NaN, magnitudes outside
 // 2^(fx::kEmin - 1023) .. 2^(fx::kEmax - 1022)) is marked, and the outputs next to it are
@@ -36,7 +36,7 @@ namespace {
 
 struct FxParams {
   const void* in[2];    // [z]: the checkerboards of a full-lattice Dhop, one per blockIdx.z
-  longlong2* fxin[2];   // their fixed-point copies: 12 planes, then an exponent per 5D site
+  longlong2* fxin[2];   // their fixed-point copies, without padding slots: 12 planes of [x_cb][L5a]
   int* exps[2];
   void* out[2];
   const double2* z[2];  // out = c0 z + c1 Dhop when given, else the Dhop
@@ -45,7 +45,7 @@ struct FxParams {
   const double* links_d[2];  // the FP64 links, for sites that leave the fixed-point range
   const int* nbr[2];
   int64_t n4h;
-  size_t n5;
+  size_t n5, nfx;  // 5D sites with and without padding slots
   int L5, L5a, L5c, k4;  // as DhopParams (gb_dhop.cu)
   int link_exp;          // k of gb_fx64.cuh
   int dag;
@@ -239,14 +239,14 @@ __device__ __noinline__ void fx_site_fp64(const double2* in, double2* out, const
 }
 
 // the largest exponent of a site's eight neighbours (kBad is above every other)
-__device__ __forceinline__ int fx_site_exponent(const int* exps, const int* nbr, int L5, int64_t x, int s) {
+__device__ __forceinline__ int fx_site_exponent(const int* exps, const int* nbr, int L5a, int64_t x, int s) {
   const int4* nb = reinterpret_cast<const int4*>(nbr + x * 8);
   const int4 a = __ldg(nb), b = __ldg(nb + 1);
   const int* e = exps + s;
-  const int e0 = max(__ldg(e + size_t(a.x) * L5), __ldg(e + size_t(a.y) * L5));
-  const int e1 = max(__ldg(e + size_t(a.z) * L5), __ldg(e + size_t(a.w) * L5));
-  const int e2 = max(__ldg(e + size_t(b.x) * L5), __ldg(e + size_t(b.y) * L5));
-  const int e3 = max(__ldg(e + size_t(b.z) * L5), __ldg(e + size_t(b.w) * L5));
+  const int e0 = max(__ldg(e + size_t(a.x) * L5a), __ldg(e + size_t(a.y) * L5a));
+  const int e1 = max(__ldg(e + size_t(a.z) * L5a), __ldg(e + size_t(a.w) * L5a));
+  const int e2 = max(__ldg(e + size_t(b.x) * L5a), __ldg(e + size_t(b.y) * L5a));
+  const int e3 = max(__ldg(e + size_t(b.z) * L5a), __ldg(e + size_t(b.w) * L5a));
   return max(max(e0, e1), max(e2, e3));
 }
 
@@ -266,8 +266,8 @@ __device__ __forceinline__ void fx_legs(const FxParams& p, const longlong2* in, 
   for (int m = 0; m < 2 * n; m++) {
     if (m == n) fx_negate_lower(acc);
     const int leg = m < n ? leg0 + m : leg0 + 4 + m - n;
-    const size_t j = size_t(__ldg(nbr + x * 8 + leg)) * p.L5 + s;
-    fx_leg(2 * (leg & 3) + ((leg >= 4) != (p.dag != 0) ? 1 : 0), in, p.n5, j, min(Ea - __ldg(exps + j), 63),
+    const size_t j = size_t(__ldg(nbr + x * 8 + leg)) * p.L5a + s;
+    fx_leg(2 * (leg & 3) + ((leg >= 4) != (p.dag != 0) ? 1 : 0), in, p.nfx, j, min(Ea - __ldg(exps + j), 63),
            U + size_t(leg) * 9 * ustride, ustride, acc);
   }
   if (p.dag) fx_negate_lower(acc);
@@ -284,15 +284,19 @@ __device__ __forceinline__ void fx_pad(const FxParams& p, double2* out, int64_t 
 
 // The fixed-point copy of one checkerboard of a field (both with blockIdx.z), one thread per 5D
 // site.  A pass of its own: each site is read by eight outputs, and converting it eight times
-// there took more instructions than the SU(3) products.
+// there took more instructions than the SU(3) products.  The copies have no padding slots: with
+// one right-hand side those are half of the field (DhopEO 24^3 x 32 137 -> 125 us, 16^4 22.9 -> 20.1 us,
+// CG iteration on MdagM of 24^3 x 32 894 -> 840 us).
 __global__ void __launch_bounds__(256) fx_convert_kernel(const __grid_constant__ FxParams p) {
   pdl_wait();
   const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= p.n5) return;
+  if (i >= p.nfx) return;
   const double2* in = after_wait(static_cast<const double2*>(p.in[blockIdx.z]));
   longlong2* out = p.fxin[blockIdx.z];
+  size_t j = i;
+  if (p.L5a != p.L5) j += i / unsigned(p.L5a) * unsigned(p.L5 - p.L5a);
   Spinor<double> f;
-  SpinorIO<double>::load(in, nullptr, p.n5, i, f);
+  SpinorIO<double>::load(in, nullptr, p.n5, j, f);
   uint32_t amax = 0, low = 0;
 #pragma unroll
   for (int k = 0; k < 12; k++) {
@@ -308,7 +312,7 @@ __global__ void __launch_bounds__(256) fx_convert_kernel(const __grid_constant__
     longlong2 v;
     v.x = fx::from_words(uint32_t(__double2hiint(f.re[k])), uint32_t(__double2loint(f.re[k])), E);
     v.y = fx::from_words(uint32_t(__double2hiint(f.im[k])), uint32_t(__double2loint(f.im[k])), E);
-    out[size_t(k) * p.n5 + i] = v;
+    out[size_t(k) * p.nfx + i] = v;
   }
 }
 
@@ -343,7 +347,7 @@ __global__ void __launch_bounds__(128, 4) dhop_fx_kernel(const __grid_constant__
   if (j >= nsite || s >= p.L5a) return;
   const int64_t x = x0 + j;
   fx_pad(p, out, x, s);
-  const int Ea = fx_site_exponent(exps, nbr, p.L5, x, s);
+  const int Ea = fx_site_exponent(exps, nbr, p.L5a, x, s);
   if (Ea == fx::kBad) {
     fx_site_fp64(in, out, z, p.c0, p.c1, p.links_d[side], nbr, p.n5, p.L5, x, s, p.dag);
     return;
@@ -411,7 +415,7 @@ __device__ __forceinline__ void fx_cg_finish(const FxParams& p, double sum) {
 // out and sums |out|^2, CG_FINISH_BETA applies r -= a out in place of storing out and sums |r|^2,
 // and the last CTA turns the sum into the CG's a or b.  Separate passes -> this, us per CG
 // iteration on MdagM: 8^4 42.4 -> 33.7, 12^4 75.3 -> 70.2, 16^4 164 -> 155, 24^3 x 32 932 -> 894,
-// 32^4 2137 -> 2109; with more right-hand sides the passes stay.
+// 32^4 2137 -> 2109 (the fixed-point copies then still held padding); with more right-hand sides the passes stay.
 template <bool SOA, bool AXPY, int CG = CG_FINISH_NONE>
 __global__ void __launch_bounds__(128, 4) dhop_fx_split_kernel(const __grid_constant__ FxParams p) {
   __shared__ long long part[4][24][32];
@@ -428,7 +432,7 @@ __global__ void __launch_bounds__(128, 4) dhop_fx_split_kernel(const __grid_cons
   const double2* z = after_wait(p.z[side]);
   const longlong2* fxin = after_wait(p.fxin[side]);
   const int* exps = after_wait(p.exps[side]);
-  const int Ea = fx_site_exponent(exps, nbr, p.L5, x, s);
+  const int Ea = fx_site_exponent(exps, nbr, p.L5a, x, s);
   if (Ea != fx::kBad) {
     FxAcc acc;
     fx_legs(p, fxin, exps, nbr, SOA ? p.links[side] + x : p.links[side] + x * 72, SOA ? size_t(p.n4h) : size_t(1),
@@ -487,7 +491,7 @@ struct FxDerivParams {
   const double* links;
   const int* nbr;
   double2* mat;
-  size_t n5;
+  size_t n5, nfx;
   int64_t n4h;
   int L5, L5a, bits;
   int half_out, dag, parity;
@@ -509,11 +513,11 @@ __device__ __forceinline__ void deriv_project(const longlong2 (&f)[12], bool plu
 }
 
 // the limbs of the two-spinor of one site, in the site's units shifted down by sh
-__device__ __forceinline__ void deriv_limbs(int mu, bool plus, const longlong2* __restrict__ in, size_t n5, size_t i, int sh,
+__device__ __forceinline__ void deriv_limbs(int mu, bool plus, const longlong2* __restrict__ in, size_t nfx, size_t i, int sh,
                                             int (&rh)[6], int (&rl)[6], int (&ih)[6], int (&il)[6]) {
   longlong2 f[12];
 #pragma unroll
-  for (int k = 0; k < 12; k++) f[k] = __ldg(in + size_t(k) * n5 + i);
+  for (int k = 0; k < 12; k++) f[k] = __ldg(in + size_t(k) * nfx + i);
   long long hr[6], hi[6];
   switch (mu) {
     case 0: deriv_project<0>(f, plus, hr, hi); break;
@@ -561,8 +565,8 @@ __global__ void __launch_bounds__(128, 3) deriv_fx_kernel(const __grid_constant_
   const int64_t x = int64_t(blockIdx.x) * 16 + (threadIdx.x >> 1);
   const bool active = x < p.n4h;
   const int64_t nb = active ? p.nbr[size_t(x) * 8 + mu] : 0;
-  const int* ea = p.exps[0] + size_t(x) * p.L5;
-  const int* eb = p.exps[1] + size_t(nb) * p.L5;
+  const int* ea = p.exps[0] + size_t(x) * p.L5a;
+  const int* eb = p.exps[1] + size_t(nb) * p.L5a;
   int EA = 0, EB = 0;
   if (active)
     for (int s = g; s < p.L5a; s += 2) { EA = max(EA, __ldg(ea + s)); EB = max(EB, __ldg(eb + s)); }
@@ -591,8 +595,8 @@ __global__ void __launch_bounds__(128, 3) deriv_fx_kernel(const __grid_constant_
 #pragma unroll 1
     for (int s = g; s < p.L5a; s += 2) {
       int hrh[6], hrl[6], hih[6], hil[6], grh[6], grl[6], gih[6], gil[6];
-      deriv_limbs(mu, plus, p.fxin[1], p.n5, size_t(nb) * p.L5 + s, min(EB - __ldg(eb + s) + drop, 63), hrh, hrl, hih, hil);
-      deriv_limbs(mu, plus, p.fxin[0], p.n5, size_t(x) * p.L5 + s, min(EA - __ldg(ea + s) + drop, 63), grh, grl, gih, gil);
+      deriv_limbs(mu, plus, p.fxin[1], p.nfx, size_t(nb) * p.L5a + s, min(EB - __ldg(eb + s) + drop, 63), hrh, hrl, hih, hil);
+      deriv_limbs(mu, plus, p.fxin[0], p.nfx, size_t(x) * p.L5a + s, min(EA - __ldg(ea + s) + drop, 63), grh, grl, gih, gil);
 #pragma unroll
       for (int j = 0; j < 2; j++)
 #pragma unroll
@@ -662,6 +666,9 @@ __global__ void __launch_bounds__(256) fx_links_kernel(const double* links, int4
 // 12-real links (rebuilt per CTA in FP64) and GB_FLAG_DF64 chooses its own.
 bool fx_wanted(const Op* op) { return op->prec == GB_F64 && !op->recon12 && !op->df64; }
 
+// 5D sites of one checkerboard without padding slots
+static size_t fx_sites(const Op* op) { return size_t(op->half4) * op->Ls * op->nrhs_user; }
+
 // The links' layout: sites in lanes below 8 slots per site (a CTA of 128 threads then stages 16
 // sites at most, 18.7 KB, and four CTAs stay resident).
 static bool fx_soa(const Op* op) { return op->Ls * op->nrhs_user < 8; }
@@ -687,7 +694,7 @@ int fx_import_links(Op* op) {
   while (double(top) > 1.5 * std::ldexp(1.0, k)) k++;
   op->fx_exp = k;
   const size_t n = size_t(op->half4) * 72;
-  const size_t field = op->n5() * 2 * (12 * sizeof(longlong2) + sizeof(int));
+  const size_t field = fx_sites(op) * 2 * (12 * sizeof(longlong2) + sizeof(int));
   void** bufs[3] = {&op->links_fx[0], &op->links_fx[1], &op->fx_field};
   for (int i = 0; i < 3; i++) {
     if (*bufs[i]) continue;  // kept from an earlier import
@@ -710,9 +717,9 @@ int fx_import_links(Op* op) {
   return GB_OK;
 }
 
-static longlong2* fx_planes(const Op* op, int z) { return static_cast<longlong2*>(op->fx_field) + size_t(z) * 12 * op->n5(); }
+static longlong2* fx_planes(const Op* op, int z) { return static_cast<longlong2*>(op->fx_field) + size_t(z) * 12 * fx_sites(op); }
 static int* fx_exps(const Op* op, int z) {
-  return reinterpret_cast<int*>(static_cast<longlong2*>(op->fx_field) + 24 * op->n5()) + size_t(z) * op->n5();
+  return reinterpret_cast<int*>(static_cast<longlong2*>(op->fx_field) + 24 * fx_sites(op)) + size_t(z) * fx_sites(op);
 }
 
 // Output sites per CTA of dhop_fx_kernel for L5c slots a site: of CTAs of up to 128 and up to 96
@@ -744,6 +751,7 @@ int launch_dhop_fx(Op* op, HalfView in, HalfView out, int out_parity, const Half
   }
   p.n4h = op->half4;
   p.n5 = op->n5();
+  p.nfx = fx_sites(op);
   p.L5 = op->L5;
   p.L5a = op->Ls * op->nrhs_user;
   p.c0 = axpy ? axpy->c0 : 0.0;
@@ -751,7 +759,7 @@ int launch_dhop_fx(Op* op, HalfView in, HalfView out, int out_parity, const Half
   p.link_exp = op->fx_exp;
   p.dag = dag;
   p.err = op->d_err;
-  launch_pdl(fx_convert_kernel, dim3(unsigned((p.n5 + 255) / 256), 1, in2 ? 2u : 1u), 256, 0, op->stream, p);
+  launch_pdl(fx_convert_kernel, dim3(unsigned((p.nfx + 255) / 256), 1, in2 ? 2u : 1u), 256, 0, op->stream, p);
   const bool soa = fx_soa(op);
   void (*kernel)(const FxParams);
   const size_t ctas = size_t((p.n4h * p.L5a + 31) / 32) * (in2 ? 2 : 1);
@@ -797,13 +805,14 @@ int launch_deriv_fx(Op* op, HalfView A, HalfView B, int out_parity, int dag, dou
     p.exps[z] = c.exps[z];
   }
   c.n5 = p.n5 = op->n5();
-  launch_pdl(fx_convert_kernel, dim3(unsigned((c.n5 + 255) / 256), 1, 2), 256, 0, op->stream, c);
+  c.nfx = p.nfx = fx_sites(op);
+  c.L5 = p.L5 = op->L5;
+  c.L5a = p.L5a = op->Ls * op->nrhs_user;
+  launch_pdl(fx_convert_kernel, dim3(unsigned((c.nfx + 255) / 256), 1, 2), 256, 0, op->stream, c);
   p.links = static_cast<const double*>(op->links[out_parity]);
   p.nbr = op->nbr[out_parity];
   p.mat = reinterpret_cast<double2*>(mat);
   p.n4h = op->half4;
-  p.L5 = op->L5;
-  p.L5a = op->Ls * op->nrhs_user;
   p.bits = p.L5a <= 16 ? 57 : p.L5a <= 32 ? 56 : 55;
   p.half_out = half_out;
   p.dag = dag;
