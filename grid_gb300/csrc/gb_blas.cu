@@ -3,8 +3,8 @@
 // Reductions follow Grid's rankInnerProduct / sumD / axpy_norm
 // (Grid/lattice/Lattice_reduction.h:202-372): per-site products in the field's
 // precision, accumulation over sites in FP64, one result per right-hand side.  The
-// partial sums of a fixed grid of CTAs are combined in a fixed order by a second kernel,
-// so a reduction is bit-reproducible from run to run.
+// partial sums of a fixed grid of CTAs are combined in a fixed order by a second kernel, or in
+// a CG by the reduction's last CTA, so a reduction is bit-reproducible from run to run.
 #include <cuda_fp16.h>
 
 #include "gb_device.cuh"

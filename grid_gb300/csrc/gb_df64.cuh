@@ -1,7 +1,9 @@
 // Double-float ("df64") arithmetic: a value is hi + lo, two floats, about 48 significant
-// bits.  The FP64 hopping term can run in it on the FP32 pipes, which GB300 issues at 64
-// times its FP64 rate, while the fields keep their FP64 storage: each double is split
-// into (hi, lo) on load and hi + lo is rounded back to a double on store.
+// bits.  The FP64 hopping term of an operator created with GB_FLAG_DF64 runs in it on the FP32
+// pipes, which GB300 issues at 64 times its FP64 rate, while the fields keep their FP64
+// storage: each double is split into (hi, lo) on load and hi + lo is rounded back to a double
+// on store.  (Other FP64 operators use the fixed-point form of gb_fx64.cuh, which is exact and
+// faster.)
 //
 // The split and the widening use integer operations only, so no FP64 instruction is
 // spent on them.  Error-free transformations (Knuth's TwoSum, Dekker's FastTwoSum and the

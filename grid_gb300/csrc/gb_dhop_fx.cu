@@ -410,7 +410,7 @@ __device__ __forceinline__ void fx_cg_finish(const FxParams& p, double sum) {
 // kernel ran.  A site is a chain of about 4600 instructions for one thread: with few sites that
 // chain is the launch's time (8^4: 12.4 us, one thread per site 20.0), and with sites in lanes
 // the extra warps keep more of the links' 1152 bytes per site in flight (24^3 x 32: 138 us, one
-// thread per site 153).  SOA: the links' sites-in-lanes layout.
+// thread per site 153; measured with plain launches and padding in the fixed-point copies).  SOA: the links' sites-in-lanes layout.
 // CG (one right-hand side): the CG's next reduction rides on the launch.  CG_FINISH_ALPHA stores
 // out and sums |out|^2, CG_FINISH_BETA applies r -= a out in place of storing out and sums |r|^2,
 // and the last CTA turns the sum into the CG's a or b.  Separate passes -> this, us per CG

@@ -5,8 +5,10 @@
 //   c = cp ; mmp = A p ; d = <p|mmp> ; a = c/d ; r -= a mmp ; cp = |r|^2 ; b = cp/c ;
 //   psi += a p ; p = b p + r ; stop when cp <= tol^2 |src|^2
 // with A = Mdag M or MpcDag Mpc, d = <p|A p> is reduced as |M p|^2 (|Mpc p|^2): the same
-// number, from the intermediate field, by the kernel that writes it where it can.  As in
-// Grid, psi and p are updated in one pass after the residual.
+// number, from the intermediate field, by the kernel that writes it where it can, and r is
+// updated by the operator's last kernel where it can (cg_matrix_step).  The last CTA of a
+// reduction computes the scalars.  As in Grid, psi and p are updated in one pass after the
+// residual.
 // All scalars live on the device (one set per right-hand side); the host only polls the
 // "all converged" flag every check_every iterations, so an iteration issues no host
 // synchronisation.  A right-hand side that converges freezes (a = b = 0) while the
