@@ -412,12 +412,13 @@ int op_dhop_full(Op* op, Field* in, Field* out, int dag) {
 
 // out = c0 z + c1 Dhop(in): one launch where the operator's kernel has the form, else two
 static int op_dhop_full_axpy(Op* op, Field* in, Field* z, Field* out, double c0, double c1, int dag, int* parts = nullptr,
-                             Field* r = nullptr) {
+                             Field* r = nullptr, bool fx_given = false) {
   if (parts) *parts = 0;
   if (!in->full() || !out->full()) { set_error("Dhop: full fields expected"); return GB_ERR_BAD_PARITY; }
   int done = 0;
   DhopAxpy a{{half_view(z, 0), half_view(z, 1)}, c0, c1};
   if (r) { a.r[0] = half_view(r, 0); a.r[1] = half_view(r, 1); }
+  a.fx_given = fx_given;
   GB_TRY(launch_dhop_full_axpy(op, half_view(in, 1), half_view(out, 0), half_view(in, 0), half_view(out, 1), dag, a, &done,
                                parts));
   if (done) return GB_OK;
@@ -527,7 +528,7 @@ int op_mooee_inv(Op* op, Field* in, Field* out, int dag) {
 // side (see launch_m5d_pair; Wilson: launch_dhop_axpy).  With r_upd (MpcDag of a Wilson operator,
 // or of a FP32 / FP16 Moebius operator whose right-hand-side count divides 16) the last kernel
 // applies r -= a out for the CG instead of storing out (see launch_col).
-int op_mpc(Op* op, Field* in, Field* out, int dag, int* norm_parts, Field* r_upd, int* r_parts) {
+int op_mpc(Op* op, Field* in, Field* out, int dag, int* norm_parts, Field* r_upd, int* r_parts, bool fx_given) {
   if (norm_parts) *norm_parts = 0;
   if (r_parts) *r_parts = 0;
   if (in->subset != GB_ODD) { set_error("Mpc: odd checkerboard expected"); return GB_ERR_BAD_PARITY; }
@@ -537,7 +538,8 @@ int op_mpc(Op* op, Field* in, Field* out, int dag, int* norm_parts, Field* r_upd
     // Wilson: Mooee = d and MooeeInv = 1/d are numbers, which ride on the second Dhop:
     // out = d in - (1/d) DhopOE DhopEO in
     te1->subset = GB_EVEN;
-    GB_TRY(op_dhop_cb(op, in, te1, dag));
+    if (fx_given) GB_TRY(launch_dhop_given(op, half_view(in, 0), half_view(te1, 0), GB_EVEN, dag));
+    else GB_TRY(op_dhop_cb(op, in, te1, dag));
     return op_dhop_cb_axpy(op, te1, in, out, op->diag_mass, -1.0 / op->diag_mass, dag, r_upd ? r_parts : norm_parts, r_upd);
   }
   GB_TRY(ws_get(op, GB_EVEN, in->prec, WS_MPC_E2, &te2));
@@ -614,11 +616,11 @@ int op_mpcdagmpc(Op* op, Field* in, Field* out) {
 
 // M / Mdag on full fields (WilsonFermionImplementation.h:113-127,
 // CayleyFermion5DImplementation.h:272-306)
-int op_m(Op* op, Field* in, Field* out, int dag, int* norm_parts, Field* r_upd) {
+int op_m(Op* op, Field* in, Field* out, int dag, int* norm_parts, Field* r_upd, bool fx_given) {
   if (norm_parts) *norm_parts = 0;
   if (!in->full() || !out->full()) { set_error("M: full fields expected"); return GB_ERR_BAD_PARITY; }
   if (op->kind == 0) {
-    if (!op->tm) return op_dhop_full_axpy(op, in, in, out, op->diag_mass, 1.0, dag, norm_parts, r_upd);
+    if (!op->tm) return op_dhop_full_axpy(op, in, in, out, op->diag_mass, 1.0, dag, norm_parts, r_upd, fx_given);
     GB_TRY(op_dhop_full(op, in, out, dag));
     return tm_diag(op, in, out, dag, 0, out, 1.0);  // out = Mooee in + Dhop in
   }

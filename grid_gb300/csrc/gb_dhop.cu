@@ -957,7 +957,8 @@ static int dhop_axpy_sides(Op* op, HalfView in, HalfView out, int out_parity, co
   }
   *done = 1;
   if (op->prec == GB_F64)
-    return launch_dhop_fx(op, in, out, out_parity, in2, out2, dag, &a, r && r->prec != op->prec ? nullptr : parts);
+    return launch_dhop_fx(op, in, out, out_parity, in2, out2, dag, &a, r && r->prec != op->prec ? nullptr : parts,
+                          a.fx_given);
   DhopParams p;
   fill_dhop_params(op, in, out, out_parity, in2, out2, p);
   p.x5 = a.z[0].data;
@@ -994,6 +995,11 @@ int launch_dhop_full_axpy(Op* op, HalfView in_odd, HalfView out_even, HalfView i
 
 int launch_dhop(Op* op, HalfView in, HalfView out, int out_parity, int dag) {
   return launch_dhop_sides(op, in, out, out_parity, nullptr, nullptr, dag);
+}
+
+int launch_dhop_given(Op* op, HalfView in, HalfView out, int out_parity, int dag) {
+  GB_TRY(dhop_checks(op, in, out, nullptr, nullptr));
+  return launch_dhop_fx(op, in, out, out_parity, nullptr, nullptr, dag, nullptr, nullptr, true);
 }
 
 int launch_dhop_full(Op* op, HalfView in_odd, HalfView out_even, HalfView in_even, HalfView out_odd, int dag) {

@@ -50,6 +50,8 @@ struct FxParams {
   int link_exp;          // k of gb_fx64.cuh
   int dag;
   int* err;
+  longlong2* fxout[2];  // CG_FINISH_ALPHA: the fixed-point copy of out, as fxin and exps
+  int* expout[2];
   double2* r[2];  // the CG forms of the split kernel: the residual, the CTAs' sums, what the last CTA does
   double* partial;
   CGFinish fin;
@@ -282,6 +284,26 @@ __device__ __forceinline__ void fx_pad(const FxParams& p, double2* out, int64_t 
   for (int z = p.L5a; z < p.L5; z++) SpinorIO<double>::store(out, nullptr, p.n5, size_t(x) * p.L5 + z, zero);
 }
 
+// what the exponent of a site's fixed-point copy is taken from
+struct FxRange {
+  uint32_t amax = 0, low = 0;  // the largest upper word without its sign, the lower words' bits
+  __device__ __forceinline__ void add(double2 v) {
+    amax = max(amax, max(uint32_t(__double2hiint(v.x)) & 0x7fffffffu, uint32_t(__double2hiint(v.y)) & 0x7fffffffu));
+    low |= uint32_t(__double2loint(v.x)) | uint32_t(__double2loint(v.y));
+  }
+  __device__ __forceinline__ bool ok() const { return int(amax >> 20) >= fx::kEmin && int(amax >> 20) <= fx::kEmax; }
+  __device__ __forceinline__ int exponent() const { return (amax | low) == 0 ? 0 : ok() ? int(amax >> 20) : fx::kBad; }
+  // of the integers: values of zero and marked sites become zeros, or are not read
+  __device__ __forceinline__ int scale() const { return ok() ? int(amax >> 20) : fx::kEmax; }
+};
+
+__device__ __forceinline__ longlong2 fx_words(double2 v, int E) {
+  longlong2 w;
+  w.x = fx::from_words(uint32_t(__double2hiint(v.x)), uint32_t(__double2loint(v.x)), E);
+  w.y = fx::from_words(uint32_t(__double2hiint(v.y)), uint32_t(__double2loint(v.y)), E);
+  return w;
+}
+
 // The fixed-point copy of one checkerboard of a field (both with blockIdx.z), one thread per 5D
 // site.  A pass of its own: each site is read by eight outputs, and converting it eight times
 // there took more instructions than the SU(3) products.  The copies have no padding slots: with
@@ -297,23 +319,13 @@ __global__ void __launch_bounds__(256) fx_convert_kernel(const __grid_constant__
   if (p.L5a != p.L5) j += i / unsigned(p.L5a) * unsigned(p.L5 - p.L5a);
   Spinor<double> f;
   SpinorIO<double>::load(in, nullptr, p.n5, j, f);
-  uint32_t amax = 0, low = 0;
+  FxRange m;
 #pragma unroll
-  for (int k = 0; k < 12; k++) {
-    amax = max(amax, max(uint32_t(__double2hiint(f.re[k])) & 0x7fffffffu, uint32_t(__double2hiint(f.im[k])) & 0x7fffffffu));
-    low |= uint32_t(__double2loint(f.re[k])) | uint32_t(__double2loint(f.im[k]));
-  }
-  int E = int(amax >> 20);
-  const bool zero = (amax | low) == 0, ok = E >= fx::kEmin && E <= fx::kEmax;
-  p.exps[blockIdx.z][i] = zero ? 0 : ok ? E : fx::kBad;
-  E = ok ? E : fx::kEmax;  // values of zero and marked sites: zeros, or not read
+  for (int k = 0; k < 12; k++) m.add(make_double2(f.re[k], f.im[k]));
+  const int E = m.scale();
+  p.exps[blockIdx.z][i] = m.exponent();
 #pragma unroll
-  for (int k = 0; k < 12; k++) {
-    longlong2 v;
-    v.x = fx::from_words(uint32_t(__double2hiint(f.re[k])), uint32_t(__double2loint(f.re[k])), E);
-    v.y = fx::from_words(uint32_t(__double2hiint(f.im[k])), uint32_t(__double2loint(f.im[k])), E);
-    out[size_t(k) * p.nfx + i] = v;
-  }
+  for (int k = 0; k < 12; k++) out[size_t(k) * p.nfx + i] = fx_words(make_double2(f.re[k], f.im[k]), E);
 }
 
 template <bool AXPY>
@@ -412,12 +424,15 @@ __device__ __forceinline__ void fx_cg_finish(const FxParams& p, double sum) {
 // the extra warps keep more of the links' 1152 bytes per site in flight (24^3 x 32: 138 us, one
 // thread per site 153; measured with plain launches and padding in the fixed-point copies).  SOA: the links' sites-in-lanes layout.
 // CG (one right-hand side): the CG's next reduction rides on the launch.  CG_FINISH_ALPHA stores
-// out and sums |out|^2, CG_FINISH_BETA applies r -= a out in place of storing out and sums |r|^2,
-// and the last CTA turns the sum into the CG's a or b.  Separate passes -> this, us per CG
-// iteration on MdagM: 8^4 42.4 -> 33.7, 12^4 75.3 -> 70.2, 16^4 164 -> 155, 24^3 x 32 932 -> 894,
-// 32^4 2137 -> 2109 (the fixed-point copies then still held padding); with more right-hand sides the passes stay.
+// out, also as the fixed-point copy that the dagger's launch reads, and sums |out|^2;
+// CG_FINISH_BETA applies r -= a out in place of storing out and sums |r|^2,
+// and the last CTA turns the sum into the CG's a or b.  us per CG iteration on MdagM, separate passes ->
+// sums here: 8^4 42.4 -> 33.7, 24^3 x 32 932 -> 894, 32^4 2137 -> 2109 (with padding in the copies);
+// then with the copy left for the dagger: 8^4 33.7 -> 30.9, 24^3 x 32 840 -> 812, 32^4 1957 -> 1899.
+// With more right-hand sides the passes stay.
 template <bool SOA, bool AXPY, int CG = CG_FINISH_NONE>
 __global__ void __launch_bounds__(128, 4) dhop_fx_split_kernel(const __grid_constant__ FxParams p) {
+  constexpr bool LEAVE = CG == CG_FINISH_ALPHA;
   __shared__ long long part[4][24][32];
   const int side = blockIdx.z;
   const int lane = threadIdx.x & 31, mu = threadIdx.x >> 5;
@@ -451,8 +466,15 @@ __global__ void __launch_bounds__(128, 4) dhop_fx_split_kernel(const __grid_cons
       fx_site_fp64(in, out, z, p.c0, p.c1, p.links_d[side], nbr, p.n5, p.L5, x, s, p.dag);
       if (CG != CG_FINISH_NONE)
         for (int k = 0; k < 12; k++) fx_cg_term<CG == CG_FINISH_BETA>(r + size_t(k) * p.n5, a, out[size_t(k) * p.n5 + i], sum);
+      if (LEAVE) {
+        FxRange m;
+        for (int k = 0; k < 12; k++) m.add(out[size_t(k) * p.n5 + i]);
+        p.expout[side][g] = m.exponent();
+        for (int k = 0; k < 12; k++) p.fxout[side][size_t(k) * p.nfx + g] = fx_words(out[size_t(k) * p.n5 + i], m.scale());
+      }
     }
   }
+  double2 kept[3];
   if (active && Ea != fx::kBad) {
     const int e = fx::result_exponent(Ea, p.link_exp);
 #pragma unroll
@@ -466,6 +488,25 @@ __global__ void __launch_bounds__(128, 4) dhop_fx_split_kernel(const __grid_cons
       const double2 d = fx_result<AXPY>(p, z, w, fx_value(v[0], e), fx_value(v[1], e));
       if (CG != CG_FINISH_BETA) out[w] = d;
       if (CG != CG_FINISH_NONE) fx_cg_term<CG == CG_FINISH_BETA>(r + size_t(k) * p.n5, a, d, sum);
+      kept[m] = d;
+    }
+  }
+  if (LEAVE) {  // the site's range is that of its four warps' components
+    __shared__ uint2 range[4][32];
+    FxRange m;
+    if (active && Ea != fx::kBad)
+      for (int k = 0; k < 3; k++) m.add(kept[k]);
+    range[mu][lane] = make_uint2(m.amax, m.low);
+    __syncthreads();
+    if (active && Ea != fx::kBad) {
+#pragma unroll
+      for (int w = 0; w < 4; w++) {
+        m.amax = max(m.amax, range[w][lane].x);
+        m.low |= range[w][lane].y;
+      }
+      if (mu == 0) p.expout[side][g] = m.exponent();
+#pragma unroll
+      for (int k = 0; k < 3; k++) p.fxout[side][size_t(3 * mu + k) * p.nfx + g] = fx_words(kept[k], m.scale());
     }
   }
   if (CG != CG_FINISH_NONE) fx_cg_finish(p, sum);
@@ -668,6 +709,8 @@ bool fx_wanted(const Op* op) { return op->prec == GB_F64 && !op->recon12 && !op-
 
 // 5D sites of one checkerboard without padding slots
 static size_t fx_sites(const Op* op) { return size_t(op->half4) * op->Ls * op->nrhs_user; }
+// fixed-point copies the operator holds: the inputs of a launch, and what the CG form leaves for the next
+static int fx_sets(const Op* op) { return op->Ls == 1 && op->nrhs_user == 1 ? 4 : 2; }
 
 // The links' layout: sites in lanes below 8 slots per site (a CTA of 128 threads then stages 16
 // sites at most, 18.7 KB, and four CTAs stay resident).
@@ -694,7 +737,7 @@ int fx_import_links(Op* op) {
   while (double(top) > 1.5 * std::ldexp(1.0, k)) k++;
   op->fx_exp = k;
   const size_t n = size_t(op->half4) * 72;
-  const size_t field = fx_sites(op) * 2 * (12 * sizeof(longlong2) + sizeof(int));
+  const size_t field = fx_sites(op) * fx_sets(op) * (12 * sizeof(longlong2) + sizeof(int));
   void** bufs[3] = {&op->links_fx[0], &op->links_fx[1], &op->fx_field};
   for (int i = 0; i < 3; i++) {
     if (*bufs[i]) continue;  // kept from an earlier import
@@ -719,7 +762,7 @@ int fx_import_links(Op* op) {
 
 static longlong2* fx_planes(const Op* op, int z) { return static_cast<longlong2*>(op->fx_field) + size_t(z) * 12 * fx_sites(op); }
 static int* fx_exps(const Op* op, int z) {
-  return reinterpret_cast<int*>(static_cast<longlong2*>(op->fx_field) + 24 * fx_sites(op)) + size_t(z) * fx_sites(op);
+  return reinterpret_cast<int*>(static_cast<longlong2*>(op->fx_field) + fx_sets(op) * 12 * fx_sites(op)) + size_t(z) * fx_sites(op);
 }
 
 // Output sites per CTA of dhop_fx_kernel for L5c slots a site: of CTAs of up to 128 and up to 96
@@ -734,7 +777,7 @@ static int fx_cta_sites(int L5c) {
 }
 
 int launch_dhop_fx(Op* op, HalfView in, HalfView out, int out_parity, const HalfView* in2, const HalfView* out2, int dag,
-                   const DhopAxpy* axpy, int* parts) {
+                   const DhopAxpy* axpy, int* parts, bool given) {
   FxParams p;
   const HalfView* ins[2] = {&in, in2};
   const HalfView* outs[2] = {&out, out2};
@@ -746,8 +789,6 @@ int launch_dhop_fx(Op* op, HalfView in, HalfView out, int out_parity, const Half
     p.links[z] = static_cast<const int4*>(op->links_fx[par]);
     p.links_d[z] = static_cast<const double*>(op->links[par]);
     p.nbr[z] = op->nbr[par];
-    p.fxin[z] = fx_planes(op, z);
-    p.exps[z] = fx_exps(op, z);
   }
   p.n4h = op->half4;
   p.n5 = op->n5();
@@ -759,13 +800,23 @@ int launch_dhop_fx(Op* op, HalfView in, HalfView out, int out_parity, const Half
   p.link_exp = op->fx_exp;
   p.dag = dag;
   p.err = op->d_err;
-  launch_pdl(fx_convert_kernel, dim3(unsigned((p.nfx + 255) / 256), 1, in2 ? 2u : 1u), 256, 0, op->stream, p);
+  for (int z = 0; z < 2; z++) {  // the sets 2, 3 hold what the CG form's blockIdx.z 0, 1 left
+    const int set = given ? (in2 ? 3 - z : 2 + z) : z;
+    p.fxin[z] = fx_planes(op, set);
+    p.exps[z] = fx_exps(op, set);
+  }
+  if (!given)
+    launch_pdl(fx_convert_kernel, dim3(unsigned((p.nfx + 255) / 256), 1, in2 ? 2u : 1u), 256, 0, op->stream, p);
   const bool soa = fx_soa(op);
   void (*kernel)(const FxParams);
   const size_t ctas = size_t((p.n4h * p.L5a + 31) / 32) * (in2 ? 2 : 1);
   if (parts && axpy && op->Ls == 1 && op->nrhs_user == 1 && ctas <= op->partial_doubles) {
     const bool beta = axpy->r[0].data != nullptr;
-    for (int z = 0; z < 2; z++) p.r[z] = static_cast<double2*>(axpy->r[z].data);
+    for (int z = 0; z < 2; z++) {
+      p.r[z] = static_cast<double2*>(axpy->r[z].data);
+      p.fxout[z] = fx_planes(op, 2 + z);
+      p.expout[z] = fx_exps(op, 2 + z);
+    }
     p.partial = op->d_partial;
     p.fin = CGFinish{op->d_cg, op->d_all_done, beta ? CG_FINISH_BETA : CG_FINISH_ALPHA};
     *parts = -1;

@@ -184,6 +184,7 @@ struct DhopAxpy {
   HalfView z[2];
   double c0, c1;
   HalfView r[2] = {};
+  bool fx_given = false;  // the launch before summed |in|^2 with *parts < 0: its fixed-point copy of in is there
 };
 // parts (the CG on Wilson operators): the launch also sums |out|^2, or with r.data
 // applies r -= a out (a: the CG scalars) in place of storing out and sums |r|^2.
@@ -207,7 +208,9 @@ size_t dhop_pair_ctas(const Op* op);
 bool fx_wanted(const Op* op);
 int fx_import_links(Op* op);
 int launch_dhop_fx(Op* op, HalfView in, HalfView out, int out_parity, const HalfView* in2, const HalfView* out2, int dag,
-                   const DhopAxpy* axpy = nullptr, int* parts = nullptr);
+                   const DhopAxpy* axpy = nullptr, int* parts = nullptr, bool given = false);
+// DhopEO/OE of a field whose fixed-point copy the last launch left (see fx_given)
+int launch_dhop_given(Op* op, HalfView in, HalfView out, int out_parity, int dag);
 int launch_dhop_full(Op* op, HalfView in_odd, HalfView out_even, HalfView in_even, HalfView out_odd, int dag);
 // force term of the output parity's sites into mat (FP64 canonical gauge layout, indexed
 // by x_cb when half_out, else by the lexicographic site); A has the output parity

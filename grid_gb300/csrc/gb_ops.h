@@ -62,11 +62,12 @@ int op_mooee_inv(Op* op, Field* in, Field* out, int dag);
 // |r_upd|^2, from which it updates the CG's b and convergence flags (a FP32 / FP16 Wilson operator's
 // leaves those to launch_cg_beta); *r_parts is the number of CTA
 // sums, below 0 without sums to read, or 0 when it stored out and left r_upd and the scalars alone
+// fx_given: in is the out of the last launch, which set *norm_parts below 0
 int op_mpc(Op* op, Field* in, Field* out, int dag, int* norm_parts = nullptr, Field* r_upd = nullptr,
-           int* r_parts = nullptr);
+           int* r_parts = nullptr, bool fx_given = false);
 int op_mpcdagmpc(Op* op, Field* in, Field* out);
 // norm_parts, r_upd (for the CG): as norm_parts and r_parts of op_mpc, *norm_parts either 0 or < 0
-int op_m(Op* op, Field* in, Field* out, int dag, int* norm_parts = nullptr, Field* r_upd = nullptr);
+int op_m(Op* op, Field* in, Field* out, int dag, int* norm_parts = nullptr, Field* r_upd = nullptr, bool fx_given = false);
 int op_mdagm(Op* op, Field* in, Field* out);
 int op_dminus(Op* op, Field* in, Field* out, int dag);
 // flops of one application of MdagM (kind 0) or MpcDagMpc (kind 1) in Grid's model

@@ -65,8 +65,8 @@ int cg_matrix_step(Op* op, int kind, Field* p, Field* mmp, Field* r) {
   else GB_TRY(op_mpc(op, p, z, 0, &dparts));
   if (dparts > 0) GB_TRY(launch_cg_alpha(op, op->d_partial, dparts));
   else if (dparts == 0) GB_TRY(cg_alpha_norm(op, z));
-  if (kind == 0) GB_TRY(op_m(op, z, mmp, 1, &rparts, r));
-  else GB_TRY(op_mpc(op, z, mmp, 1, nullptr, r, &rparts));
+  if (kind == 0) GB_TRY(op_m(op, z, mmp, 1, &rparts, r, dparts < 0));
+  else GB_TRY(op_mpc(op, z, mmp, 1, nullptr, r, &rparts, dparts < 0));
   if (rparts == 0) return cg_r_update(op, r, mmp);
   return rparts > 0 && op->kind == 0 ? launch_cg_beta(op, op->d_partial, rparts) : GB_OK;  // (otherwise b is done too)
 }
