@@ -9,8 +9,8 @@
 //                         instructions per output site and was slower for every Moebius size
 //   dhop_fx_kernel        projections, SU(3) products and sums over legs and spins as exact
 //                         integer arithmetic, each result rounded to a double once; 1728 wide
-//                         multiply-adds (32 lanes per clock and SM) of 4600 instructions per
-//                         output site.  The multiply-add pipe is its bound (70 % busy); four
+//                         multiply-adds (32 lanes per clock and SM) of 4500 instructions per
+//                         output site.  The multiply-add pipe is its bound (74 % busy); four
 //                         CTAs of 128 threads at 128 registers beat three at 168
 //   dhop_fx_split_kernel  the same with a site's directions over four warps
 // DhopEO, dhop_kernel<double> -> these: 16^4 x 16 820 -> 185 us, 16^4 x 12 599 -> 144 us,
