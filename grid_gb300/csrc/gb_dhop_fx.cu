@@ -12,9 +12,9 @@
 //                         multiply-adds (32 lanes per clock and SM) of 4500 instructions per
 //                         output site.  The multiply-add pipe is its bound (74 % busy); four
 //                         CTAs of 128 threads at 128 registers beat three at 168
-//   dhop_fx_split_kernel  the same with a site's directions over four warps
+//   dhop_fx_split_kernel  the same with a site's directions over two or four warps
 // DhopEO, dhop_kernel<double> -> these: 16^4 x 16 820 -> 185 us, 16^4 x 12 599 -> 144 us,
-// 24^3 x 32 x 12 right-hand sides 3847 -> 931 us, Wilson 24^3 x 32 345 -> 125 us, 8^4 33 -> 8 us.
+// 24^3 x 32 x 12 right-hand sides 3847 -> 931 us, Wilson 24^3 x 32 345 -> 116 us, 8^4 33 -> 8 us.
 //
 // A site whose values the fixed-point range does not hold (infinities, NaN, magnitudes outside
 // 2^(fx::kEmin - 1023) .. 2^(fx::kEmax - 1022)) is marked, and the outputs next to it are
@@ -62,6 +62,13 @@ constexpr int kFxLinkStride = 73;  // int4 per staged site: 72 and one of paddin
 // equal at 32768 sites (8^3 x 16 x 8: 22.3 against 22.7 us), 15.5 against 19.3 us at 16384, and
 // 232 against 185 us at 524288, where the shared staging of the links counts.
 constexpr int64_t kFxSplitSites = 40000;
+// Above this many CTAs of the split kernel (608 are resident with four warps each), two warps share a
+// site's directions in place of four: half of the partial sums through shared memory, and no second
+// wave that is nearly empty.  Four -> two warps: DhopEO 8^3 x 16 x 8 (1024 CTAs) 19.2 -> 18.4 us,
+// Wilson 24^3 x 32 (6912) 125 -> 116 us, with 3 right-hand sides 319 -> 289 us, CG iteration on MpcDagMpc
+// of 16^4 (1024) 133 -> 125 us; 8^4 x 12 (768) 16.1 and 16.1 us, 8^4 x 10 (640) 15.4 -> 15.8 us,
+// Wilson 12^4 (324) 10.8 -> 13.2 us.
+constexpr size_t kFxTwoWarps = 800;
 
 // f of the leg's two-spinor h = (1 + S gamma_MU) f as integers
 template <int MU, int S>
@@ -386,18 +393,19 @@ __device__ __forceinline__ void fx_cg_term(double2* r, double a, double2 v, doub
   sum = fma(v.x, v.x, fma(v.y, v.y, sum));
 }
 
-// The end of a CG form for one right-hand side, by every thread of every CTA of 128: the CTA's sum, and in
+// The end of a CG form for one right-hand side, by every thread of every CTA of W warps: the CTA's sum, and in
 // the last CTA all of them in a fixed order and the CG's scalars from it.  The padding's scalars stay as
 // cg_init_kernel set them (done, a = b = 0).
+template <int W>
 __device__ __forceinline__ void fx_cg_finish(const FxParams& p, double sum) {
-  __shared__ double ws[4];
+  __shared__ double ws[W];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const auto cta_sum = [&](double v) {  // in thread 0
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     if (lane == 0) ws[warp] = v;
     __syncthreads();
-    return (ws[0] + ws[1]) + (ws[2] + ws[3]);
+    return W == 4 ? (ws[0] + ws[1]) + (ws[W - 2] + ws[W - 1]) : ws[0] + ws[1];
   };
   const int ctas = int(gridDim.x * gridDim.z);
   sum = cta_sum(sum);
@@ -405,7 +413,7 @@ __device__ __forceinline__ void fx_cg_finish(const FxParams& p, double sum) {
   if (!last_cta(p.fin.flags + kCGTicket, ctas)) return;
   sum = 0.0;
 #pragma unroll 8
-  for (int b = threadIdx.x; b < ctas; b += 128) sum += __ldcg(p.partial + b);
+  for (int b = threadIdx.x; b < ctas; b += 32 * W) sum += __ldcg(p.partial + b);
   sum = cta_sum(sum);
   if (threadIdx.x != 0) return;
   CGScalars c = *p.fin.cg;
@@ -417,23 +425,27 @@ __device__ __forceinline__ void fx_cg_finish(const FxParams& p, double sum) {
   cg_set_flags(p.fin.cg, p.L5, p.fin.flags);
 }
 
-// Four warps share 32 output sites, one direction (its forward and backward leg) each, and add
-// their integer sums through shared memory: exactly, so the result does not depend on which
+// W = 4 warps share 32 output sites, one direction (its forward and backward leg) each, or W = 2 with
+// two directions each (kFxTwoWarps), and add their integer sums through shared memory: exactly, so the result does not depend on which
 // kernel ran.  A site is a chain of about 4600 instructions for one thread: with few sites that
 // chain is the launch's time (8^4: 12.4 us, one thread per site 20.0), and with sites in lanes
 // the extra warps keep more of the links' 1152 bytes per site in flight (24^3 x 32: 138 us, one
-// thread per site 153; measured with plain launches and padding in the fixed-point copies).  SOA: the links' sites-in-lanes layout.
+// thread per site 153; measured with plain launches and padding in the fixed-point copies).
+// SOA: the links' sites-in-lanes layout.
 // CG (one right-hand side): the CG's next reduction rides on the launch.  CG_FINISH_ALPHA stores
 // out, also as the fixed-point copy that the dagger's launch reads, and sums |out|^2;
 // CG_FINISH_BETA applies r -= a out in place of storing out and sums |r|^2,
 // and the last CTA turns the sum into the CG's a or b.  us per CG iteration on MdagM, separate passes ->
 // sums here: 8^4 42.4 -> 33.7, 24^3 x 32 932 -> 894, 32^4 2137 -> 2109 (with padding in the copies);
-// then with the copy left for the dagger: 8^4 33.7 -> 30.9, 24^3 x 32 840 -> 812, 32^4 1957 -> 1899.
+// then with the copy left for the dagger: 8^4 33.7 -> 30.9, 24^3 x 32 840 -> 812, 32^4 1957 -> 1899; with
+// two warps 24^3 x 32 753, 32^4 1753.
 // With more right-hand sides the passes stay.
-template <bool SOA, bool AXPY, int CG = CG_FINISH_NONE>
-__global__ void __launch_bounds__(128, 4) dhop_fx_split_kernel(const __grid_constant__ FxParams p) {
+template <bool SOA, bool AXPY, int W, int CG = CG_FINISH_NONE>
+__global__ void __launch_bounds__(32 * W, 16 / W) dhop_fx_split_kernel(const __grid_constant__ FxParams p) {
   constexpr bool LEAVE = CG == CG_FINISH_ALPHA;
-  __shared__ long long part[4][24][32];
+  static_assert(W == 4 || W == 2, "a site's four directions over four or two warps");
+  constexpr int K = 12 / W;  // components that a warp finishes
+  __shared__ long long part[W][24][32];
   const int side = blockIdx.z;
   const int lane = threadIdx.x & 31, mu = threadIdx.x >> 5;
   double2* out = static_cast<double2*>(p.out[side]);
@@ -451,7 +463,7 @@ __global__ void __launch_bounds__(128, 4) dhop_fx_split_kernel(const __grid_cons
   if (Ea != fx::kBad) {
     FxAcc acc;
     fx_legs(p, fxin, exps, nbr, SOA ? p.links[side] + x : p.links[side] + x * 72, SOA ? size_t(p.n4h) : size_t(1),
-            x, s, mu, 1, Ea, acc);
+            x, s, mu * (4 / W), 4 / W, Ea, acc);
 #pragma unroll
     for (int k = 0; k < 12; k++) { part[mu][2 * k][lane] = acc.re[k]; part[mu][2 * k + 1][lane] = acc.im[k]; }
   }
@@ -474,16 +486,18 @@ __global__ void __launch_bounds__(128, 4) dhop_fx_split_kernel(const __grid_cons
       }
     }
   }
-  double2 kept[3];
+  double2 kept[K];
   if (active && Ea != fx::kBad) {
     const int e = fx::result_exponent(Ea, p.link_exp);
 #pragma unroll
-    for (int m = 0; m < 3; m++) {  // warp mu finishes components 3 mu .. 3 mu + 2
-      const int k = 3 * mu + m;
+    for (int m = 0; m < K; m++) {  // warp mu finishes components K mu .. K mu + K - 1
+      const int k = K * mu + m;
       long long v[2];
 #pragma unroll
-      for (int c = 0; c < 2; c++)
-        v[c] = (part[0][2 * k + c][lane] + part[1][2 * k + c][lane]) + (part[2][2 * k + c][lane] + part[3][2 * k + c][lane]);
+      for (int c = 0; c < 2; c++) {
+        v[c] = part[0][2 * k + c][lane] + part[1][2 * k + c][lane];
+        if (W == 4) v[c] += part[W - 2][2 * k + c][lane] + part[W - 1][2 * k + c][lane];
+      }
       const size_t w = size_t(k) * p.n5 + i;
       const double2 d = fx_result<AXPY>(p, z, w, fx_value(v[0], e), fx_value(v[1], e));
       if (CG != CG_FINISH_BETA) out[w] = d;
@@ -491,25 +505,25 @@ __global__ void __launch_bounds__(128, 4) dhop_fx_split_kernel(const __grid_cons
       kept[m] = d;
     }
   }
-  if (LEAVE) {  // the site's range is that of its four warps' components
-    __shared__ uint2 range[4][32];
+  if (LEAVE) {  // the site's range is that of its warps' components
+    __shared__ uint2 range[W][32];
     FxRange m;
     if (active && Ea != fx::kBad)
-      for (int k = 0; k < 3; k++) m.add(kept[k]);
+      for (int k = 0; k < K; k++) m.add(kept[k]);
     range[mu][lane] = make_uint2(m.amax, m.low);
     __syncthreads();
     if (active && Ea != fx::kBad) {
 #pragma unroll
-      for (int w = 0; w < 4; w++) {
+      for (int w = 0; w < W; w++) {
         m.amax = max(m.amax, range[w][lane].x);
         m.low |= range[w][lane].y;
       }
       if (mu == 0) p.expout[side][g] = m.exponent();
 #pragma unroll
-      for (int k = 0; k < 3; k++) p.fxout[side][size_t(3 * mu + k) * p.nfx + g] = fx_words(kept[k], m.scale());
+      for (int k = 0; k < K; k++) p.fxout[side][size_t(K * mu + k) * p.nfx + g] = fx_words(kept[k], m.scale());
     }
   }
-  if (CG != CG_FINISH_NONE) fx_cg_finish(p, sum);
+  if (CG != CG_FINISH_NONE) fx_cg_finish<W>(p, sum);
 }
 
 // ---- force term (gb_dhop.cu's deriv_kernel: mat = U W, W = sum_s h conj(g)^T) in fixed point ----
@@ -810,6 +824,7 @@ int launch_dhop_fx(Op* op, HalfView in, HalfView out, int out_parity, const Half
   const bool soa = fx_soa(op);
   void (*kernel)(const FxParams);
   const size_t ctas = size_t((p.n4h * p.L5a + 31) / 32) * (in2 ? 2 : 1);
+  const bool two = ctas > kFxTwoWarps;
   if (parts && axpy && op->Ls == 1 && op->nrhs_user == 1 && ctas <= op->partial_doubles) {
     const bool beta = axpy->r[0].data != nullptr;
     for (int z = 0; z < 2; z++) {
@@ -820,15 +835,18 @@ int launch_dhop_fx(Op* op, HalfView in, HalfView out, int out_parity, const Half
     p.partial = op->d_partial;
     p.fin = CGFinish{op->d_cg, op->d_all_done, beta ? CG_FINISH_BETA : CG_FINISH_ALPHA};
     *parts = -1;
-    launch_pdl(beta ? dhop_fx_split_kernel<true, true, CG_FINISH_BETA> : dhop_fx_split_kernel<true, true, CG_FINISH_ALPHA>,
-               dim3(unsigned((p.n4h + 31) / 32), 1, in2 ? 2u : 1u), 128, 0, op->stream, p);
+    if (two) kernel = beta ? dhop_fx_split_kernel<true, true, 2, CG_FINISH_BETA> : dhop_fx_split_kernel<true, true, 2, CG_FINISH_ALPHA>;
+    else kernel = beta ? dhop_fx_split_kernel<true, true, 4, CG_FINISH_BETA> : dhop_fx_split_kernel<true, true, 4, CG_FINISH_ALPHA>;
+    launch_pdl(kernel, dim3(unsigned((p.n4h + 31) / 32), 1, in2 ? 2u : 1u), two ? 64u : 128u, 0, op->stream, p);
     GB_CHECK_CUDA(cudaGetLastError());
     return GB_OK;
   }
   if (soa || p.n4h * p.L5a * (in2 ? 2 : 1) <= kFxSplitSites) {
-    if (soa) kernel = axpy ? dhop_fx_split_kernel<true, true> : dhop_fx_split_kernel<true, false>;
-    else kernel = axpy ? dhop_fx_split_kernel<false, true> : dhop_fx_split_kernel<false, false>;
-    launch_pdl(kernel, dim3(unsigned((p.n4h * p.L5a + 31) / 32), 1, in2 ? 2u : 1u), 128, 0, op->stream, p);
+    if (soa && two) kernel = axpy ? dhop_fx_split_kernel<true, true, 2> : dhop_fx_split_kernel<true, false, 2>;
+    else if (soa) kernel = axpy ? dhop_fx_split_kernel<true, true, 4> : dhop_fx_split_kernel<true, false, 4>;
+    else if (two) kernel = axpy ? dhop_fx_split_kernel<false, true, 2> : dhop_fx_split_kernel<false, false, 2>;
+    else kernel = axpy ? dhop_fx_split_kernel<false, true, 4> : dhop_fx_split_kernel<false, false, 4>;
+    launch_pdl(kernel, dim3(unsigned((p.n4h * p.L5a + 31) / 32), 1, in2 ? 2u : 1u), two ? 64u : 128u, 0, op->stream, p);
   } else {
     kernel = axpy ? dhop_fx_kernel<true> : dhop_fx_kernel<false>;
     p.L5c = p.L5a > 128 ? 128 : p.L5a;

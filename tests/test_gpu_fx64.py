@@ -61,6 +61,12 @@ def test_cta_sizes(gpu_available, dims, Ls, nrhs):
     test_fixed_point_dhop(gpu_available, "wilson" if Ls == 1 else "mobius", dims, Ls, nrhs)
 
 
+@pytest.mark.parametrize("dims,Ls,nrhs", [((10, 14, 18, 22), 1, 1), ((6, 10, 14, 22), 1, 3), ((6, 10, 10, 10), 10, 1)])
+def test_two_warps_per_site(gpu_available, dims, Ls, nrhs):
+    """Above 800 CTAs of 32 sites the split kernel runs two warps; the last CTA is not full."""
+    test_fixed_point_dhop(gpu_available, "wilson" if Ls == 1 else "mobius", dims, Ls, nrhs)
+
+
 @pytest.mark.parametrize("power", [-1060, -1000, -920, -300, 300, 870, 890, 1010])
 def test_magnitudes(gpu_available, power):
     """The hopping term of 2^power x is 2^power times that of x, through the ends of the
@@ -122,7 +128,7 @@ def test_links_of_any_size_and_reimport(gpu_available):
         assert np.abs(fo.export() - scale * one).max() <= 4e-15 * scale * np.abs(one).max()
 
 
-@pytest.mark.parametrize("dims", [(2, 2, 2, 2), (4, 4, 4, 6), (6, 2, 4, 10), (8, 8, 8, 8)])
+@pytest.mark.parametrize("dims", [(2, 2, 2, 2), (4, 4, 4, 6), (6, 2, 4, 10), (8, 8, 8, 8), (10, 14, 18, 22)])
 @pytest.mark.parametrize("tiny", [False, True])
 @pytest.mark.parametrize("schur", [False, True])
 def test_cg_sums_in_the_hopping_term(gpu_available, dims, tiny, schur):
