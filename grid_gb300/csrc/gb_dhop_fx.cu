@@ -530,11 +530,13 @@ __global__ void __launch_bounds__(32 * W, 16 / W) dhop_fx_split_kernel(const __g
 //
 // What bounds the FP64 kernel is its 96 FP64 operations per (site, direction, s).  Here A (on the
 // output's checkerboard) and B come as the fixed-point copies of fx_convert_kernel, and the sum over
-// s of the two-spinors' products is exact integer arithmetic: the two-spinors are shifted to the
-// units of their site's largest s and to b bits, b = 57 for up to 16 slots and one less for each
-// doubling, cut into limbs of 29 and b - 29 bits, so that a lane's sums (2 slots' products of
-// 2^b each, half of the slots) stay below 2^63; products of two lower limbs, 2^-57 of the
-// largest, are dropped.  Above 64 slots b would fall below a double's 53 bits and more.
+// s of the two-spinors' products is exact integer arithmetic: the two-spinors are cut to b bits, b = 57
+// for up to 16 slots and one less for each doubling, in limbs of 29 and b - 29 bits, so that a lane's
+// sums (2 slots' products of 2^b each, half of the slots) stay below 2^63; products of two lower
+// limbs, 2^-57 of the largest, are dropped.  The sum's unit is that of its largest product, taken over s as the
+// largest sum of the two exponents: B stays in the units of its own slot and A is shifted for both, so that factors
+// which peak at different s (the two walls of the fifth dimension) keep their bits.  Above 64 slots b
+// would fall below a double's 53 bits and more.
 // U W runs in FP64.  Same lanes, warps and CTAs as deriv_kernel.  MDeriv 16^4 x 12:
 // 708 -> 418 us, of which Meooe5D is 80 and the conversions 94 (two or four CTAs per SM: 466, 463).
 constexpr int kDerivSlots = 64;
@@ -622,14 +624,18 @@ __global__ void __launch_bounds__(128, 3) deriv_fx_kernel(const __grid_constant_
   const int64_t nb = active ? p.nbr[size_t(x) * 8 + mu] : 0;
   const int* ea = p.exps[0] + size_t(x) * p.L5a;
   const int* eb = p.exps[1] + size_t(nb) * p.L5a;
-  int EA = 0, EB = 0;
+  int EAB = 0, worst = 0;  // of the largest product (0: all are zero), and of any factor
   if (active)
-    for (int s = g; s < p.L5a; s += 2) { EA = max(EA, __ldg(ea + s)); EB = max(EB, __ldg(eb + s)); }
-  EA = max(EA, __shfl_xor_sync(0xffffffffu, EA, 1));  // the same for both lanes of a site
-  EB = max(EB, __shfl_xor_sync(0xffffffffu, EB, 1));
+    for (int s = g; s < p.L5a; s += 2) {
+      const int a = __ldg(ea + s), b = __ldg(eb + s);
+      worst = max(worst, max(a, b));
+      if (a != 0 && b != 0) EAB = max(EAB, a + b);
+    }
+  EAB = max(EAB, __shfl_xor_sync(0xffffffffu, EAB, 1));  // the same for both lanes of a site
+  worst = max(worst, __shfl_xor_sync(0xffffffffu, worst, 1));
   // a factor outside the range, or a product whose double could over- or underflow
-  const bool zero = EA == 0 || EB == 0;
-  const bool bad = EA == fx::kBad || EB == fx::kBad || (!zero && (EA + EB < 1146 || EA + EB > 2946));
+  const bool zero = EAB == 0;
+  const bool bad = worst == fx::kBad || (!zero && (EAB < 1146 || EAB > 2946));
   double wr[9], wi[9];
 #pragma unroll
   for (int e = 0; e < 9; e++) { wr[e] = 0.0; wi[e] = 0.0; }
@@ -650,8 +656,10 @@ __global__ void __launch_bounds__(128, 3) deriv_fx_kernel(const __grid_constant_
 #pragma unroll 1
     for (int s = g; s < p.L5a; s += 2) {
       int hrh[6], hrl[6], hih[6], hil[6], grh[6], grl[6], gih[6], gil[6];
-      deriv_limbs(mu, plus, p.fxin[1], p.nfx, size_t(nb) * p.L5a + s, min(EB - __ldg(eb + s) + drop, 63), hrh, hrl, hih, hil);
-      deriv_limbs(mu, plus, p.fxin[0], p.nfx, size_t(x) * p.L5a + s, min(EA - __ldg(ea + s) + drop, 63), grh, grl, gih, gil);
+      const int a = __ldg(ea + s), b = __ldg(eb + s);
+      if (a == 0 || b == 0) continue;
+      deriv_limbs(mu, plus, p.fxin[1], p.nfx, size_t(nb) * p.L5a + s, drop, hrh, hrl, hih, hil);
+      deriv_limbs(mu, plus, p.fxin[0], p.nfx, size_t(x) * p.L5a + s, min(EAB - a - b + drop, 63), grh, grl, gih, gil);
 #pragma unroll
       for (int j = 0; j < 2; j++)
 #pragma unroll
@@ -668,7 +676,7 @@ __global__ void __launch_bounds__(128, 3) deriv_fx_kernel(const __grid_constant_
             im[e] = fx::mad(nh, gil[k], fx::mad(nl, gih[k], im[e]));
           }
     }
-    const int e2 = 58 + EA + EB - 2042 - 2 * p.bits;
+    const int e2 = 58 + EAB - 2042 - 2 * p.bits;
     const unsigned pair = 3u << (threadIdx.x & 30);
 #pragma unroll
     for (int e = 0; e < 9; e++) {
