@@ -304,6 +304,20 @@ struct FxRange {
   __device__ __forceinline__ int scale() const { return ok() ? int(amax >> 20) : fx::kEmax; }
 };
 
+// A site as a factor of the force: its exponent, and for each of the four pairs of spins that a projection
+// adds how far (in powers of two, up to 31) the smallest colour of the pair lies below it.
+__device__ __forceinline__ uint32_t fx_force_word(const Spinor<double>& f, int E) {
+  int e[12];
+#pragma unroll
+  for (int k = 0; k < 12; k++)
+    e[k] = int(max(uint32_t(__double2hiint(f.re[k])) & 0x7fffffffu, uint32_t(__double2hiint(f.im[k])) & 0x7fffffffu) >> 20);
+  const auto below = [&](int i, int j) {
+    const int least = min(max(e[3 * i], e[3 * j]), min(max(e[3 * i + 1], e[3 * j + 1]), max(e[3 * i + 2], e[3 * j + 2])));
+    return uint32_t(min(E - least, 31));
+  };
+  return uint32_t(E) << 20 | below(0, 3) << 15 | below(1, 2) << 10 | below(0, 2) << 5 | below(1, 3);
+}
+
 __device__ __forceinline__ longlong2 fx_words(double2 v, int E) {
   longlong2 w;
   w.x = fx::from_words(uint32_t(__double2hiint(v.x)), uint32_t(__double2loint(v.x)), E);
@@ -316,6 +330,8 @@ __device__ __forceinline__ longlong2 fx_words(double2 v, int E) {
 // there took more instructions than the SU(3) products.  The copies have no padding slots: with
 // one right-hand side those are half of the field (DhopEO 24^3 x 32 137 -> 125 us, 16^4 22.9 -> 20.1 us,
 // CG iteration on MdagM of 24^3 x 32 894 -> 840 us).
+// FORCE: the exponents carry what deriv_fx_kernel asks of its factors (fx_force_word).
+template <bool FORCE>
 __global__ void __launch_bounds__(256) fx_convert_kernel(const __grid_constant__ FxParams p) {
   pdl_wait();
   const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -330,7 +346,7 @@ __global__ void __launch_bounds__(256) fx_convert_kernel(const __grid_constant__
 #pragma unroll
   for (int k = 0; k < 12; k++) m.add(make_double2(f.re[k], f.im[k]));
   const int E = m.scale();
-  p.exps[blockIdx.z][i] = m.exponent();
+  p.exps[blockIdx.z][i] = FORCE ? int(fx_force_word(f, m.exponent())) : m.exponent();
 #pragma unroll
   for (int k = 0; k < 12; k++) out[size_t(k) * p.nfx + i] = fx_words(make_double2(f.re[k], f.im[k]), E);
 }
@@ -530,13 +546,21 @@ __global__ void __launch_bounds__(32 * W, 16 / W) dhop_fx_split_kernel(const __g
 //
 // What bounds the FP64 kernel is its 96 FP64 operations per (site, direction, s).  Here A (on the
 // output's checkerboard) and B come as the fixed-point copies of fx_convert_kernel, and the sum over
-// s of the two-spinors' products is exact integer arithmetic: the two-spinors are cut to b bits, b = 57
-// for up to 16 slots and one less for each doubling, in limbs of 29 and b - 29 bits, so that a lane's
-// sums (2 slots' products of 2^b each, half of the slots) stay below 2^63; products of two lower
-// limbs, 2^-57 of the largest, are dropped.  The sum's unit is that of its largest product, taken over s as the
+// s of the two-spinors' products is exact integer arithmetic: the two-spinors are cut to b bits, b = 59
+// for one slot, 58 for up to 4, 57 for up to 16 and one less for each doubling, in limbs of 29 and b - 29 bits, so
+// that the sums over a lane's slots (8 products of 2^(b - 1) each in the middle, 4 of 2^(2 b - 58) on top) and over
+// the two lanes stay below 2^63; products of two lower limbs, below 2^-57 of the largest, are dropped.  The sum's unit is that of its largest product, taken over s as the
 // largest sum of the two exponents: B stays in the units of its own slot and A is shifted for both, so that factors
 // which peak at different s (the two walls of the fifth dimension) keep their bits.  Above 64 slots b
 // would fall below a double's 53 bits and more.
+//
+// The error is a fixed part of that unit, 2^(58 - 2 b) of it and a few 2^-59, where FP64's is one of each sum's own
+// terms.  So each lane also adds up a lower bound of every colour pair's sum of |h_c| |g_b| (per slot and j, the
+// smallest colour of either two-spinor's pair of spins), and where that is below 2^(2 (58 - b) - 4) of the unit, as for colours
+// that the links keep apart and that differ in size, the site is summed in FP64.  At that bound the error is
+// at most 4 times FP64's rounding (integer model on the host: 3.3e-16 against 8.3e-17 of the sum of the terms'
+// magnitudes; with terms of one size 1e-17 to 4e-17 against 5e-17 to 7e-17).  Gaussian factors stay above it by 4 to 24:
+// none of 2e5 sites falls below with up to 32 slots, 0.6 % with 33.
 // U W runs in FP64.  Same lanes, warps and CTAs as deriv_kernel.  MDeriv 16^4 x 12:
 // 708 -> 418 us, of which Meooe5D is 80 and the conversions 94 (two or four CTAs per SM: 466, 463).
 constexpr int kDerivSlots = 64;
@@ -627,7 +651,7 @@ __global__ void __launch_bounds__(128, 3) deriv_fx_kernel(const __grid_constant_
   int EAB = 0, worst = 0;  // of the largest product (0: all are zero), and of any factor
   if (active)
     for (int s = g; s < p.L5a; s += 2) {
-      const int a = __ldg(ea + s), b = __ldg(eb + s);
+      const int a = int(uint32_t(__ldg(ea + s)) >> 20), b = int(uint32_t(__ldg(eb + s)) >> 20);
       worst = max(worst, max(a, b));
       if (a != 0 && b != 0) EAB = max(EAB, a + b);
     }
@@ -635,31 +659,28 @@ __global__ void __launch_bounds__(128, 3) deriv_fx_kernel(const __grid_constant_
   worst = max(worst, __shfl_xor_sync(0xffffffffu, worst, 1));
   // a factor outside the range, or a product whose double could over- or underflow
   const bool zero = EAB == 0;
-  const bool bad = worst == fx::kBad || (!zero && (EAB < 1146 || EAB > 2946));
+  bool bad = worst == fx::kBad || (!zero && (EAB < 1146 || EAB > 2946));
   double wr[9], wi[9];
 #pragma unroll
   for (int e = 0; e < 9; e++) { wr[e] = 0.0; wi[e] = 0.0; }
-  if (bad) {
-    deriv_site_fp64(p, x, nb, mu, g, wr, wi);
-#pragma unroll
-    for (int e = 0; e < 9; e++) {  // the two lanes of a site are here together
-      const unsigned pair = 3u << (threadIdx.x & 30);
-      wr[e] += __shfl_xor_sync(pair, wr[e], 1);
-      wi[e] += __shfl_xor_sync(pair, wi[e], 1);
-    }
-  } else if (!zero) {
+  if (!bad && !zero) {
     long long rh[9], rm[9], ih[9], im[9];
 #pragma unroll
     for (int e = 0; e < 9; e++) { rh[e] = 0; rm[e] = 0; ih[e] = 0; im[e] = 0; }
     const int drop = 61 - p.bits;
     const bool plus = p.dag != 0;
+    uint32_t least = 0;  // the lower bound of the sums' terms, 2^24 for one of the unit
 #pragma unroll 1
     for (int s = g; s < p.L5a; s += 2) {
       int hrh[6], hrl[6], hih[6], hil[6], grh[6], grl[6], gih[6], gil[6];
-      const int a = __ldg(ea + s), b = __ldg(eb + s);
+      const uint32_t a = uint32_t(__ldg(ea + s)), b = uint32_t(__ldg(eb + s));
       if (a == 0 || b == 0) continue;
+      const int sh = EAB - int(a >> 20) - int(b >> 20);
+      const uint32_t ab = mu < 2 ? a >> 10 : a, bb = mu < 2 ? b >> 10 : b;
+      least += ((1u << 24) >> min(uint32_t(sh) + (ab >> 5 & 31) + (bb >> 5 & 31), 31u)) +
+               ((1u << 24) >> min(uint32_t(sh) + (ab & 31) + (bb & 31), 31u));
       deriv_limbs(mu, plus, p.fxin[1], p.nfx, size_t(nb) * p.L5a + s, drop, hrh, hrl, hih, hil);
-      deriv_limbs(mu, plus, p.fxin[0], p.nfx, size_t(x) * p.L5a + s, min(EAB - a - b + drop, 63), grh, grl, gih, gil);
+      deriv_limbs(mu, plus, p.fxin[0], p.nfx, size_t(x) * p.L5a + s, min(sh + drop, 63), grh, grl, gih, gil);
 #pragma unroll
       for (int j = 0; j < 2; j++)
 #pragma unroll
@@ -685,6 +706,21 @@ __global__ void __launch_bounds__(128, 3) deriv_fx_kernel(const __grid_constant_
       imv += __shfl_xor_sync(pair, imv, 1);
       wr[e] = fx_value(re, e2);
       wi[e] = fx_value(imv, e2);
+    }
+    least += __shfl_xor_sync(pair, least, 1);
+    bad = least < 1u << (136 - 2 * p.bits);
+    if (bad) {
+#pragma unroll
+      for (int e = 0; e < 9; e++) { wr[e] = 0.0; wi[e] = 0.0; }
+    }
+  }
+  if (bad) {
+    deriv_site_fp64(p, x, nb, mu, g, wr, wi);
+#pragma unroll
+    for (int e = 0; e < 9; e++) {  // the two lanes of a site are here together
+      const unsigned pair = 3u << (threadIdx.x & 30);
+      wr[e] += __shfl_xor_sync(pair, wr[e], 1);
+      wi[e] += __shfl_xor_sync(pair, wi[e], 1);
     }
   }
   if (!active) return;
@@ -828,7 +864,7 @@ int launch_dhop_fx(Op* op, HalfView in, HalfView out, int out_parity, const Half
     p.exps[z] = fx_exps(op, set);
   }
   if (!given)
-    launch_pdl(fx_convert_kernel, dim3(unsigned((p.nfx + 255) / 256), 1, in2 ? 2u : 1u), 256, 0, op->stream, p);
+    launch_pdl(fx_convert_kernel<false>, dim3(unsigned((p.nfx + 255) / 256), 1, in2 ? 2u : 1u), 256, 0, op->stream, p);
   const bool soa = fx_soa(op);
   void (*kernel)(const FxParams);
   const size_t ctas = size_t((p.n4h * p.L5a + 31) / 32) * (in2 ? 2 : 1);
@@ -885,12 +921,12 @@ int launch_deriv_fx(Op* op, HalfView A, HalfView B, int out_parity, int dag, dou
   c.nfx = p.nfx = fx_sites(op);
   c.L5 = p.L5 = op->L5;
   c.L5a = p.L5a = op->Ls * op->nrhs_user;
-  launch_pdl(fx_convert_kernel, dim3(unsigned((c.nfx + 255) / 256), 1, 2), 256, 0, op->stream, c);
+  launch_pdl(fx_convert_kernel<true>, dim3(unsigned((c.nfx + 255) / 256), 1, 2), 256, 0, op->stream, c);
   p.links = static_cast<const double*>(op->links[out_parity]);
   p.nbr = op->nbr[out_parity];
   p.mat = reinterpret_cast<double2*>(mat);
   p.n4h = op->half4;
-  p.bits = p.L5a <= 16 ? 57 : p.L5a <= 32 ? 56 : 55;
+  p.bits = p.L5a == 1 ? 59 : p.L5a <= 4 ? 58 : p.L5a <= 16 ? 57 : p.L5a <= 32 ? 56 : 55;
   p.half_out = half_out;
   p.dag = dag;
   p.parity = out_parity;
