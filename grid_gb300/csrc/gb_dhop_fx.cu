@@ -27,6 +27,7 @@
 //   sites in lanes  [leg][9][x_cb] int4, read coalesced by each thread, below 8 slots per site:
 //                   staging 1152 bytes for each few threads would leave an SM one or two CTAs
 #include <cmath>
+#include <cstring>
 
 #include "gb_dhop_site.cuh"
 #include "gb_fx64.cuh"
@@ -57,6 +58,7 @@ struct FxParams {
   CGFinish fin;
 };
 
+constexpr float kFxLinkRatio = 4.f;  // of the largest and smallest link row (see fx_import_links)
 constexpr int kFxLinkStride = 73;  // int4 per staged site: 72 and one of padding
 // Up to this many output sites in a launch the split kernel takes the slots-in-CTAs layout too:
 // equal at 32768 sites (8^3 x 16 x 8: 22.3 against 22.7 us), 15.5 against 19.3 us at 16384, and
@@ -732,10 +734,10 @@ __global__ void __launch_bounds__(128, 3) deriv_fx_kernel(const __grid_constant_
   deriv_rows<2, double>(Ul, wr, wi, g, p.mat + (size_t(idx) * 4 + mu) * 9);
 }
 
-// the largest row sum of absolute values over one parity's links, as the bits of a float
-// rounded up (infinity for anything not finite)
+// The largest row sum of absolute values over one parity's links as the bits of a float
+// rounded up (infinity for anything not finite), and the complement of the smallest's, rounded down.
 __global__ void __launch_bounds__(256) fx_row_sum_kernel(const double* links, size_t rows, unsigned* out) {
-  float m = 0.f;
+  float m = 0.f, least = __int_as_float(0x7f800000);
   for (size_t r = size_t(blockIdx.x) * blockDim.x + threadIdx.x; r < rows; r += size_t(gridDim.x) * blockDim.x) {
     double s = 0.0;
 #pragma unroll
@@ -743,9 +745,14 @@ __global__ void __launch_bounds__(256) fx_row_sum_kernel(const double* links, si
     const float f = __double2float_ru(s);
     m = f <= 3.0e38f ? fmaxf(m, f) : __int_as_float(0x7f800000);
     if (!(f <= 3.0e38f)) break;
+    least = fminf(least, __double2float_rd(s));
   }
   m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
-  if ((threadIdx.x & 31) == 0) atomicMax(out, __float_as_uint(m));
+  least = __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(least)));
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(out, __float_as_uint(m));
+    atomicMax(out + 1, ~__float_as_uint(least));
+  }
 }
 
 // fixed-point copy of one parity's links (k = exponent), AoS [x][leg][9] or SoA [leg][9][x]
@@ -776,21 +783,30 @@ static bool fx_soa(const Op* op) { return op->Ls * op->nrhs_user < 8; }
 
 // Fixed-point copies of op->links, and the scratch of fx_convert_kernel (both checkerboards of
 // a field and their exponents): allocated here so that a launch allocates nothing.  Links that
-// are all zero, not finite or of extreme magnitude, and a device without the memory, leave
-// op->fx_ready off and the hopping term on the FP64 kernel.
+// are not finite or of extreme magnitude, and a device without the memory, leave op->fx_ready off and
+// the hopping term on the FP64 kernel.  So do links whose rows differ in size: they all share one unit, that
+// of the largest, and an output whose own links are small would lose the bits that FP64 keeps.  The sums of
+// absolute values of unitary rows differ by sqrt(6) at most, so a factor of 4 takes every gauge field of unitary
+// links (also times one number, and smeared ones that have not been projected back, nearly so) and costs two bits
+// of the five that the links have beyond a double's; a row of zeros is refused too.
 int fx_import_links(Op* op) {
   op->fx_ready = false;
   if (!fx_wanted(op)) return GB_OK;
   unsigned* d_max = reinterpret_cast<unsigned*>(op->d_result);
-  GB_CHECK_CUDA(cudaMemsetAsync(d_max, 0, sizeof(unsigned), op->stream));
+  GB_CHECK_CUDA(cudaMemsetAsync(d_max, 0, 2 * sizeof(unsigned), op->stream));
   for (int p = 0; p < 2; p++)
     fx_row_sum_kernel<<<kRedBlocks, 256, 0, op->stream>>>(static_cast<const double*>(op->links[p]), size_t(op->half4) * 24,
                                                           d_max);
   GB_CHECK_CUDA(cudaGetLastError());
-  GB_CHECK_CUDA(cudaMemcpyAsync(op->h_result, d_max, sizeof(float), cudaMemcpyDeviceToHost, op->stream));
+  GB_CHECK_CUDA(cudaMemcpyAsync(op->h_result, d_max, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, op->stream));
   GB_CHECK_CUDA(cudaStreamSynchronize(op->stream));
-  const float top = *reinterpret_cast<const float*>(op->h_result);
-  if (!(top > 1e-9f && top < 1e9f)) return GB_OK;
+  unsigned sums[2];
+  std::memcpy(sums, op->h_result, sizeof(sums));
+  sums[1] = ~sums[1];
+  float top, least;
+  std::memcpy(&top, &sums[0], sizeof(top));
+  std::memcpy(&least, &sums[1], sizeof(least));
+  if (!(top > 1e-9f && top < 1e9f && top <= kFxLinkRatio * least)) return GB_OK;
   int k = -32;
   while (double(top) > 1.5 * std::ldexp(1.0, k)) k++;
   op->fx_exp = k;
