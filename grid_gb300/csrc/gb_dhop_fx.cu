@@ -249,16 +249,32 @@ __device__ __noinline__ void fx_site_fp64(const double2* in, double2* out, const
   }
 }
 
-// the largest exponent of a site's eight neighbours (kBad is above every other)
+// The largest exponent of a site's eight neighbours, and kBad (above every other) where one is marked or where
+// the output cannot be left to their common unit.  The error is a fixed part of that unit, while FP64's is one of
+// the terms of each output component.  A component takes from each neighbour one pair of spins in every
+// colour, and a link's row has no smaller sum than another's by more than kFxLinkRatio: its terms add up to the
+// unit's size if the neighbours' smallest pairs do, to 2^-kFxSpread of it.  At that bound the error is 1.6
+// times FP64's rounding (integer model on the host: 2.3e-16 against 1.4e-16 of the sum of the terms'
+// magnitudes with all of it in one neighbour; eight of 2^-3 each 3e-17 against 4.5e-17).  Colours that the links keep
+// apart and that differ in size by more than 2^4 are below it; ordinary fields are not: of a Gaussian
+// field one pair of one neighbour is enough everywhere, of the smallest pole's solution on 8^3 x 16 x 8 in all but 3e-5 of the
+// sites, and the sum there.  (Without the sum those few sites, 10 us each for the thread that takes them in FP64,
+// made that multishift solve 52 -> 67 ms.)
+constexpr int kFxSpread = 3;
 __device__ __forceinline__ int fx_site_exponent(const int* exps, const int* nbr, int L5a, int64_t x, int s) {
   const int4* nb = reinterpret_cast<const int4*>(nbr + x * 8);
   const int4 a = __ldg(nb), b = __ldg(nb + 1);
-  const int* e = exps + s;
-  const int e0 = max(__ldg(e + size_t(a.x) * L5a), __ldg(e + size_t(a.y) * L5a));
-  const int e1 = max(__ldg(e + size_t(a.z) * L5a), __ldg(e + size_t(a.w) * L5a));
-  const int e2 = max(__ldg(e + size_t(b.x) * L5a), __ldg(e + size_t(b.y) * L5a));
-  const int e3 = max(__ldg(e + size_t(b.z) * L5a), __ldg(e + size_t(b.w) * L5a));
-  return max(max(e0, e1), max(e2, e3));
+  const unsigned* e = reinterpret_cast<const unsigned*>(exps) + s;
+  const unsigned e0 = __vmaxu2(__ldg(e + size_t(a.x) * L5a), __ldg(e + size_t(a.y) * L5a));
+  const unsigned e1 = __vmaxu2(__ldg(e + size_t(a.z) * L5a), __ldg(e + size_t(a.w) * L5a));
+  const unsigned e2 = __vmaxu2(__ldg(e + size_t(b.x) * L5a), __ldg(e + size_t(b.y) * L5a));
+  const unsigned e3 = __vmaxu2(__ldg(e + size_t(b.z) * L5a), __ldg(e + size_t(b.w) * L5a));
+  const unsigned m = __vmaxu2(__vmaxu2(e0, e1), __vmaxu2(e2, e3));
+  const int E = int(m >> 16);
+  if (E - int(m & 0xffffu) <= kFxSpread || E == fx::kBad) return E;
+  unsigned sum = 0;
+  for (int k = 0; k < 8; k++) sum += 256u >> min(E - int(__ldg(e + size_t(__ldg(nbr + x * 8 + k)) * L5a) & 0xffffu), 31);
+  return sum >= 256u >> kFxSpread ? E : fx::kBad;
 }
 
 __device__ __forceinline__ void fx_negate_lower(FxAcc& acc) {
@@ -278,7 +294,7 @@ __device__ __forceinline__ void fx_legs(const FxParams& p, const longlong2* in, 
     if (m == n) fx_negate_lower(acc);
     const int leg = m < n ? leg0 + m : leg0 + 4 + m - n;
     const size_t j = size_t(__ldg(nbr + x * 8 + leg)) * p.L5a + s;
-    fx_leg(2 * (leg & 3) + ((leg >= 4) != (p.dag != 0) ? 1 : 0), in, p.nfx, j, min(Ea - __ldg(exps + j), 63),
+    fx_leg(2 * (leg & 3) + ((leg >= 4) != (p.dag != 0) ? 1 : 0), in, p.nfx, j, min(Ea - (__ldg(exps + j) >> 16), 63),
            U + size_t(leg) * 9 * ustride, ustride, acc);
   }
   if (p.dag) fx_negate_lower(acc);
@@ -293,17 +309,30 @@ __device__ __forceinline__ void fx_pad(const FxParams& p, double2* out, int64_t 
   for (int z = p.L5a; z < p.L5; z++) SpinorIO<double>::store(out, nullptr, p.n5, size_t(x) * p.L5 + z, zero);
 }
 
-// what the exponent of a site's fixed-point copy is taken from
+// The upper word of the larger of a component's |re|, |im|; its lowest bit stands for the lower words.
+__device__ __forceinline__ uint32_t fx_size(double2 v) {
+  const uint32_t hi = max(uint32_t(__double2hiint(v.x)) & 0x7fffffffu, uint32_t(__double2hiint(v.y)) & 0x7fffffffu);
+  return hi | uint32_t((__double2loint(v.x) | __double2loint(v.y)) != 0);
+}
+
+// What the exponents of a site's fixed-point copy are taken from: the sizes of its 12 components.
 struct FxRange {
-  uint32_t amax = 0, low = 0;  // the largest upper word without its sign, the lower words' bits
-  __device__ __forceinline__ void add(double2 v) {
-    amax = max(amax, max(uint32_t(__double2hiint(v.x)) & 0x7fffffffu, uint32_t(__double2hiint(v.y)) & 0x7fffffffu));
-    low |= uint32_t(__double2loint(v.x)) | uint32_t(__double2loint(v.y));
+  uint32_t top, least;  // the largest, and the smallest over the colours and the pairs of spins that a projection adds
+  // size(k): of component k = 3 spin + colour.  The pairs are those of a spin 0, 1 with a spin 2, 3.
+  template <class F> __device__ __forceinline__ explicit FxRange(const F& size) : top(0), least(0xffffffffu) {
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const uint32_t a = size(c), b = size(3 + c), d = size(6 + c), e = size(9 + c);
+      top = max(top, max(max(a, b), max(d, e)));
+      least = min(least, max(min(a, b), min(d, e)));  // = the smallest of max(a, d), max(a, e), max(b, d), max(b, e)
+    }
   }
-  __device__ __forceinline__ bool ok() const { return int(amax >> 20) >= fx::kEmin && int(amax >> 20) <= fx::kEmax; }
-  __device__ __forceinline__ int exponent() const { return (amax | low) == 0 ? 0 : ok() ? int(amax >> 20) : fx::kBad; }
+  __device__ __forceinline__ bool ok() const { return int(top >> 20) >= fx::kEmin && int(top >> 20) <= fx::kEmax; }
+  __device__ __forceinline__ int exponent() const { return top == 0 ? 0 : ok() ? int(top >> 20) : fx::kBad; }
+  // the exponents as one word: that of the site above, that of its smallest pair below
+  __device__ __forceinline__ int word() const { return exponent() << 16 | int(least >> 20); }
   // of the integers: values of zero and marked sites become zeros, or are not read
-  __device__ __forceinline__ int scale() const { return ok() ? int(amax >> 20) : fx::kEmax; }
+  __device__ __forceinline__ int scale() const { return ok() ? int(top >> 20) : fx::kEmax; }
 };
 
 // A site as a factor of the force: its exponent, and for each of the four pairs of spins that a projection
@@ -344,11 +373,9 @@ __global__ void __launch_bounds__(256) fx_convert_kernel(const __grid_constant__
   if (p.L5a != p.L5) j += i / unsigned(p.L5a) * unsigned(p.L5 - p.L5a);
   Spinor<double> f;
   SpinorIO<double>::load(in, nullptr, p.n5, j, f);
-  FxRange m;
-#pragma unroll
-  for (int k = 0; k < 12; k++) m.add(make_double2(f.re[k], f.im[k]));
+  const FxRange m([&](int k) { return fx_size(make_double2(f.re[k], f.im[k])); });
   const int E = m.scale();
-  p.exps[blockIdx.z][i] = FORCE ? int(fx_force_word(f, m.exponent())) : m.exponent();
+  p.exps[blockIdx.z][i] = FORCE ? int(fx_force_word(f, m.exponent())) : m.word();
 #pragma unroll
   for (int k = 0; k < 12; k++) out[size_t(k) * p.nfx + i] = fx_words(make_double2(f.re[k], f.im[k]), E);
 }
@@ -497,14 +524,13 @@ __global__ void __launch_bounds__(32 * W, 16 / W) dhop_fx_split_kernel(const __g
       if (CG != CG_FINISH_NONE)
         for (int k = 0; k < 12; k++) fx_cg_term<CG == CG_FINISH_BETA>(r + size_t(k) * p.n5, a, out[size_t(k) * p.n5 + i], sum);
       if (LEAVE) {
-        FxRange m;
-        for (int k = 0; k < 12; k++) m.add(out[size_t(k) * p.n5 + i]);
-        p.expout[side][g] = m.exponent();
+        const FxRange m([&](int k) { return fx_size(out[size_t(k) * p.n5 + i]); });
+        p.expout[side][g] = m.word();
         for (int k = 0; k < 12; k++) p.fxout[side][size_t(k) * p.nfx + g] = fx_words(out[size_t(k) * p.n5 + i], m.scale());
       }
     }
   }
-  double2 kept[K];
+  double2 kept[K] = {};
   if (active && Ea != fx::kBad) {
     const int e = fx::result_exponent(Ea, p.link_exp);
 #pragma unroll
@@ -524,19 +550,13 @@ __global__ void __launch_bounds__(32 * W, 16 / W) dhop_fx_split_kernel(const __g
     }
   }
   if (LEAVE) {  // the site's range is that of its warps' components
-    __shared__ uint2 range[W][32];
-    FxRange m;
-    if (active && Ea != fx::kBad)
-      for (int k = 0; k < K; k++) m.add(kept[k]);
-    range[mu][lane] = make_uint2(m.amax, m.low);
+    __shared__ uint32_t size[12][32];
+#pragma unroll
+    for (int m = 0; m < K; m++) size[K * mu + m][lane] = fx_size(kept[m]);
     __syncthreads();
     if (active && Ea != fx::kBad) {
-#pragma unroll
-      for (int w = 0; w < W; w++) {
-        m.amax = max(m.amax, range[w][lane].x);
-        m.low |= range[w][lane].y;
-      }
-      if (mu == 0) p.expout[side][g] = m.exponent();
+      const FxRange m([&](int k) { return size[k][lane]; });
+      if (mu == 0) p.expout[side][g] = m.word();
 #pragma unroll
       for (int k = 0; k < K; k++) p.fxout[side][size_t(K * mu + k) * p.nfx + g] = fx_words(kept[k], m.scale());
     }
