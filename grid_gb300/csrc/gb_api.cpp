@@ -87,6 +87,22 @@ static cudaError_t dev_alloc(void** p, size_t n, cudaStream_t s) { return cudaMa
 static void dev_free(void* p, cudaStream_t s) {
   if (p) cudaFreeAsync(p, s);
 }
+// Memory of an operator's fields and staging.  Where there is no more, the fixed-point copies of its
+// links and fields go first: the hopping term can do without them.
+static cudaError_t op_alloc(Op* op, void** p, size_t n) {
+  cudaError_t e = dev_alloc(p, n, op->stream);
+  for (Op* o : {op, op->fx_lender}) {
+    if (e != cudaErrorMemoryAllocation || !o || !fx_release(o)) continue;
+    cudaStreamSynchronize(o->stream);
+    cudaMemPool_t pool;
+    int device = 0;
+    if (cudaGetDevice(&device) == cudaSuccess && cudaDeviceGetMemPool(&pool, device) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
+    cudaGetLastError();
+    e = dev_alloc(p, n, op->stream);
+  }
+  if (e != cudaSuccess) cudaGetLastError();  // reported here: the next launch's check is not to find it
+  return e;
+}
 
 namespace {
 struct PinnedPool {
@@ -132,7 +148,7 @@ int field_alloc(Op* op, int subset, int prec, Field** out) {
   f->prec = prec;
   f->n5 = op->n5();
   const size_t halves = subset == GB_FULL ? 2 : 1;
-  cudaError_t e = dev_alloc(&f->data, halves * f->half_bytes(), op->stream);
+  cudaError_t e = op_alloc(op, &f->data, halves * f->half_bytes());
   if (e != cudaSuccess) {
     delete static_cast<gb_field_s*>(f);
     set_error("device allocation of %zu bytes failed: %s", halves * f->n5 * spinor_bytes(prec), cudaGetErrorString(e));
@@ -143,7 +159,7 @@ int field_alloc(Op* op, int subset, int prec, Field** out) {
   // have written the (lazily allocated) field
   cudaMemsetAsync(f->data, 0, halves * f->half_bytes(), op->stream);
   if (prec == GB_F16) {
-    e = dev_alloc(reinterpret_cast<void**>(&f->norms), halves * f->n5 * sizeof(float), op->stream);
+    e = op_alloc(op, reinterpret_cast<void**>(&f->norms), halves * f->n5 * sizeof(float));
     if (e != cudaSuccess) {
       dev_free(f->data, op->stream);
       delete static_cast<gb_field_s*>(f);
@@ -763,10 +779,9 @@ static void op_release(Op* op) {
   op->ws.clear();
   for (int p = 0; p < 2; p++) {
     dev_free(op->links[p], op->stream);
-    dev_free(op->links_fx[p], op->stream);
     dev_free(op->nbr[p], op->stream);
   }
-  dev_free(op->fx_field, op->stream);
+  dev_free(op->links_fx[0], op->stream);
   dev_free(op->d_err, op->stream);
   dev_free(op->d_partial, op->stream);
   dev_free(op->d_result, op->stream);
@@ -878,7 +893,7 @@ int ensure_stage(Op* op, size_t bytes) {
   dev_free(op->d_stage, op->stream);
   op->d_stage = nullptr;
   op->stage_bytes = 0;
-  if (dev_alloc(reinterpret_cast<void**>(&op->d_stage), bytes, op->stream) != cudaSuccess) {
+  if (op_alloc(op, reinterpret_cast<void**>(&op->d_stage), bytes) != cudaSuccess) {
     set_error("device allocation of %zu staging bytes failed", bytes);
     return GB_ERR_OOM;
   }
@@ -1329,7 +1344,7 @@ static int deriv_entry(gb_op_t op, gb_field_t A, gb_field_t B, int dag, double* 
   if (!ops_conformable(A->op, op)) { set_error("field is not conformable to the operator"); return GB_ERR_BAD_ARG; }
   const size_t bytes = size_t(A->full() ? op->vol4 : op->half4) * 36 * 16;
   double* d = mat;
-  if (!on_device) GB_CHECK_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&d), bytes, op->stream));
+  if (!on_device) GB_CHECK_CUDA(op_alloc(op, reinterpret_cast<void**>(&d), bytes));
   struct Free { double* p; cudaStream_t s; ~Free() { if (p) cudaFreeAsync(p, s); } } guard{on_device ? nullptr : d, op->stream};
   Field* a = A;
   Field* b = B;

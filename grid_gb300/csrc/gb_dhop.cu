@@ -999,6 +999,7 @@ int launch_dhop(Op* op, HalfView in, HalfView out, int out_parity, int dag) {
 
 int launch_dhop_given(Op* op, HalfView in, HalfView out, int out_parity, int dag) {
   GB_TRY(dhop_checks(op, in, out, nullptr, nullptr));
+  if (!op->fx_ready) return launch_dhop(op, in, out, out_parity, dag);  // the copies were given back since
   return launch_dhop_fx(op, in, out, out_parity, nullptr, nullptr, dag, nullptr, nullptr, true);
 }
 

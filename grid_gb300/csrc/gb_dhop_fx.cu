@@ -832,18 +832,15 @@ int fx_import_links(Op* op) {
   op->fx_exp = k;
   const size_t n = size_t(op->half4) * 72;
   const size_t field = fx_sites(op) * fx_sets(op) * (12 * sizeof(longlong2) + sizeof(int));
-  void** bufs[3] = {&op->links_fx[0], &op->links_fx[1], &op->fx_field};
-  for (int i = 0; i < 3; i++) {
-    if (*bufs[i]) continue;  // kept from an earlier import
-    if (cudaMallocAsync(bufs[i], i < 2 ? n * sizeof(int4) : field, op->stream) != cudaSuccess) {
+  if (!op->links_fx[0]) {  // (else kept from an earlier import)
+    char* block = nullptr;  // one, so that it comes back as one
+    if (cudaMallocAsync(reinterpret_cast<void**>(&block), 2 * n * sizeof(int4) + field, op->stream) != cudaSuccess) {
       cudaGetLastError();
-      for (int j = 0; j < i; j++) {
-        cudaFreeAsync(*bufs[j], op->stream);
-        *bufs[j] = nullptr;
-      }
-      *bufs[i] = nullptr;
       return GB_OK;
     }
+    op->links_fx[0] = block;
+    op->links_fx[1] = block + n * sizeof(int4);
+    op->fx_field = block + 2 * n * sizeof(int4);
   }
   for (int p = 0; p < 2; p++)
     fx_links_kernel<<<unsigned((n + 255) / 256), 256, 0, op->stream>>>(static_cast<const double*>(op->links[p]),
@@ -852,6 +849,25 @@ int fx_import_links(Op* op) {
   GB_CHECK_CUDA(cudaGetLastError());
   op->fx_ready = true;
   return GB_OK;
+}
+
+bool fx_release(Op* op) {
+  if (!op->links_fx[0] || op->fx_captured || op->own_graphs > 0) return false;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (op->stream && (cudaStreamIsCapturing(op->stream, &status) != cudaSuccess || status != cudaStreamCaptureStatusNone))
+    return false;
+  op->fx_ready = false;
+  cudaFreeAsync(op->links_fx[0], op->stream);
+  op->links_fx[0] = op->links_fx[1] = op->fx_field = nullptr;
+  return true;
+}
+
+// before each launch on the copies (see Op::fx_captured)
+static void fx_note_capture(Op* op) {
+  if (!op->stream || op->fx_captured || op->own_graphs > 0) return;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(op->stream, &status) != cudaSuccess) cudaGetLastError();
+  else op->fx_captured = status != cudaStreamCaptureStatusNone;
 }
 
 static longlong2* fx_planes(const Op* op, int z) { return static_cast<longlong2*>(op->fx_field) + size_t(z) * 12 * fx_sites(op); }
@@ -872,6 +888,7 @@ static int fx_cta_sites(int L5c) {
 
 int launch_dhop_fx(Op* op, HalfView in, HalfView out, int out_parity, const HalfView* in2, const HalfView* out2, int dag,
                    const DhopAxpy* axpy, int* parts, bool given) {
+  fx_note_capture(op);
   FxParams p;
   const HalfView* ins[2] = {&in, in2};
   const HalfView* outs[2] = {&out, out2};
@@ -942,6 +959,7 @@ int launch_dhop_fx(Op* op, HalfView in, HalfView out, int out_parity, const Half
 bool fx_deriv_ok(const Op* op) { return op->Ls * op->nrhs_user <= kDerivSlots; }
 
 int launch_deriv_fx(Op* op, HalfView A, HalfView B, int out_parity, int dag, double* mat, int half_out) {
+  fx_note_capture(op);
   FxParams c = {};  // the conversion of both factors: one launch, one per blockIdx.z
   FxDerivParams p;
   const HalfView* f[2] = {&A, &B};

@@ -81,10 +81,16 @@ struct Op {
   int* nbr[2] = {nullptr, nullptr};
   // fixed-point copies of FP64 links for the hopping term (gb_dhop_fx.cu): made at the gauge
   // import, with the exponent of their units; fx_ready is off where the FP64 kernel is used
-  void* links_fx[2] = {nullptr, nullptr};
-  void* fx_field = nullptr;  // the input field of a launch in fixed point
+  void* links_fx[2] = {nullptr, nullptr};  // one block with fx_field, from links_fx[0]
+  void* fx_field = nullptr;                // the input field of a launch in fixed point
   int fx_exp = 0;
   bool fx_ready = false;
+  // The copies are given back (fx_release) when an allocation of this operator, or of one whose solve it is part
+  // of (fx_lender there), finds no memory: not while a graph of a solve is alive, and never once
+  // a launch on them was captured into a graph of the caller's.
+  bool fx_captured = false;
+  int own_graphs = 0;
+  Op* fx_lender = nullptr;
   int* d_err = nullptr;                 // device error flag of bounded waits
   // Set when the host finds d_err raised.  A Dhop CTA whose bounded wait for its TMA copy
   // gave up returns while that copy may still be writing into shared memory that the
@@ -207,6 +213,7 @@ size_t dhop_pair_ctas(const Op* op);
 // copies, and one launch (in2, out2: the second checkerboard of a full-lattice Dhop)
 bool fx_wanted(const Op* op);
 int fx_import_links(Op* op);
+bool fx_release(Op* op);  // false: nothing was given back
 int launch_dhop_fx(Op* op, HalfView in, HalfView out, int out_parity, const HalfView* in2, const HalfView* out2, int dag,
                    const DhopAxpy* axpy = nullptr, int* parts = nullptr, bool given = false);
 // DhopEO/OE of a field whose fixed-point copy the last launch left (see fx_given)

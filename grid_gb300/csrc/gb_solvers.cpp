@@ -133,12 +133,18 @@ struct ChunkRunner {
   int chunk;
   bool graphs;
   int runs = 0;
+  bool counted = false;  // in op->own_graphs
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   // use_graphs == 2: the loop graph, WHILE (condition) { chunk iterations; check }
   cudaGraph_t lgraph = nullptr;
   cudaGraphExec_t lexec = nullptr;
+  void count() {
+    if (!counted) op->own_graphs++;
+    counted = true;
+  }
   ~ChunkRunner() {
+    if (counted) op->own_graphs--;
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
     if (lexec) cudaGraphExecDestroy(lexec);
@@ -151,6 +157,7 @@ struct ChunkRunner {
   // which every right-hand side converged or a reliable update became due
   int loop(int max_chunks) {
     if (!lexec) {
+      count();
       GB_CHECK_CUDA(cudaGraphCreate(&lgraph, 0));
       cudaGraphConditionalHandle h;
       GB_CHECK_CUDA(cudaGraphConditionalHandleCreate(&h, lgraph, 1, cudaGraphCondAssignDefault));
@@ -190,6 +197,7 @@ struct ChunkRunner {
     runs++;
     if (!use) return launch(m);
     if (!exec) {
+      count();
       GB_CHECK_CUDA(cudaStreamBeginCapture(op->stream, cudaStreamCaptureModeThreadLocal));
       const int rc = launch(m);
       cudaGraph_t g = nullptr;
@@ -212,7 +220,12 @@ struct SolveStream {
   Op* ops[4] = {nullptr, nullptr, nullptr, nullptr};
   cudaStream_t saved[4] = {nullptr, nullptr, nullptr, nullptr};
   cudaStream_t own = nullptr;
+  Op* lent = nullptr;  // the inner operator, which may take back the outer one's fixed-point copies
   SolveStream(Op* a, Op* b, Field* f0, Field* f1, bool want) {
+    if (b && b != a) {
+      lent = b;
+      lent->fx_lender = a;
+    }
     Op* cand[4] = {a, b, f0 ? f0->op : nullptr, f1 ? f1->op : nullptr};
     int n = 0;
     for (Op* o : cand) {
@@ -226,6 +239,7 @@ struct SolveStream {
     for (Op* o : ops) if (o) o->stream = own;
   }
   ~SolveStream() {
+    if (lent) lent->fx_lender = nullptr;
     if (!own) return;
     cudaStreamSynchronize(own);
     for (int i = 0; i < 4; i++) if (ops[i]) ops[i]->stream = saved[i];
