@@ -790,7 +790,7 @@ __global__ void __launch_bounds__(256) fx_links_kernel(const double* links, int4
 
 // Operators whose FP64 hopping term runs in fixed point: the native FP64 arithmetic stays for
 // 12-real links (rebuilt per CTA in FP64) and GB_FLAG_DF64 chooses its own.
-bool fx_wanted(const Op* op) { return op->prec == GB_F64 && !op->recon12 && !op->df64; }
+bool fx_wanted(const Op* op) { return op->prec == GB_F64 && !op->recon12 && !op->df64 && !op->fx_off; }
 
 // 5D sites of one checkerboard without padding slots
 static size_t fx_sites(const Op* op) { return size_t(op->half4) * op->Ls * op->nrhs_user; }

@@ -89,6 +89,7 @@ struct Op {
   // of (fx_lender there), finds no memory: not while a graph of a solve is alive, and never once
   // a launch on them was captured into a graph of the caller's.
   bool fx_captured = false;
+  bool fx_off = false;  // set before the import: no copies
   int own_graphs = 0;
   Op* fx_lender = nullptr;
   int* d_err = nullptr;                 // device error flag of bounded waits

@@ -180,17 +180,27 @@ struct gb_server_s {
 
 namespace {
 
-// device bytes a Moebius mixed-precision Schur solve of nsrc sources holds (operators,
-// gauge staging, FP64 and inner-precision workspace); an upper estimate
-size_t request_bytes(const gb_request& r, int nsrc) {
+int64_t request_vol(const gb_request& r) {
   int64_t vol = 1;
   for (int k = 0; k < 4; k++) vol *= r.dims[k];
-  const int64_t n5 = vol / 2 * r.Ls * (nsrc + ((r.Ls * nsrc) & 1));
+  return vol;
+}
+// 5D sites of a checkerboard with nsrc sources
+int64_t request_n5(const gb_request& r, int nsrc) {
+  return request_vol(r) / 2 * r.Ls * (nsrc + ((r.Ls * nsrc) & 1));
+}
+
+// device bytes a Moebius mixed-precision Schur solve of nsrc sources needs (operators,
+// gauge staging, FP64 and inner-precision workspace); an upper estimate
+size_t request_bytes(const gb_request& r, int nsrc) {
   const size_t lo = r.inner_precision == GB_F16 ? 52 : 96;
-  // FP64 + fixed-point + FP32 links, neighbours, FP64 gauge staging
-  const size_t per_site4 = 1152 + 1152 + 576 + 64 + 576;
-  // work fields, and both checkerboards of the FP64 hopping term's fixed-point input
-  return size_t(vol) * per_site4 + size_t(n5) * (26 * 192 + 2 * 196 + 12 * lo);
+  const size_t per_site4 = 1152 + 576 + 64 + 576;  // FP64 + FP32 links, neighbours, FP64 gauge staging
+  return size_t(request_vol(r)) * per_site4 + size_t(request_n5(r, nsrc)) * (26 * 192 + 12 * lo);
+}
+// what the FP64 operator takes on top for its hopping term in fixed point: the links, and both
+// checkerboards of an input.  A request is admitted without them where the budget has no room for them.
+size_t copies_bytes(const gb_request& r, int nsrc) {
+  return size_t(request_vol(r)) * 1152 + size_t(request_n5(r, nsrc)) * 2 * 196;
 }
 
 // work of one CG iteration (the shortest-first key): 4D volume x Ls x sources
@@ -208,7 +218,8 @@ int fitting_chunk(const gb_server_s* S, const gb_request& r) {
 // The queue position to admit now, or -1 (under mu).  Default: the first in arrival order
 // that fits what is left of the budget; FIFO (flags bit 2), or once the oldest has waited
 // age_limit: only the oldest; shortest first (bit 3): the least work among those allowed.
-int pick(gb_server_s* S, size_t* need, int* chunk) {
+// *copies: the budget has room for its fixed-point copies too, which *need then includes.
+int pick(gb_server_s* S, size_t* need, int* chunk, bool* copies) {
   const int n = int(S->queue.size());
   if (n == 0) return -1;
   const bool only_head = (S->flags & 4) || S->now() - S->queue.front().second.t_submit >= S->age_limit;
@@ -223,15 +234,16 @@ int pick(gb_server_s* S, size_t* need, int* chunk) {
     if (best < 0 || ((S->flags & 8) && w < best_work)) {
       best = i;
       best_work = w;
-      *need = nb;
       *chunk = c;
+      *copies = S->used + nb + copies_bytes(r, c) <= S->budget;
+      *need = *copies ? nb + copies_bytes(r, c) : nb;
       if (!(S->flags & 8)) break;
     }
   }
   return best;
 }
 
-int solve_request(gb_server_s* S, const gb_request& rq, int nsrc, uint64_t src_seed_offset, cudaStream_t st,
+int solve_request(gb_server_s* S, const gb_request& rq, int nsrc, bool copies, uint64_t src_seed_offset, cudaStream_t st,
                   gb_request_result* out, double* sol_host, size_t sol_offset) {
   gb_op_t od = nullptr, of = nullptr;
   gb_field_t src = nullptr, sol = nullptr;
@@ -244,6 +256,7 @@ int solve_request(gb_server_s* S, const gb_request& rq, int nsrc, uint64_t src_s
   const size_t ncomplex = size_t(vol) * rq.Ls * 12 * nsrc;
   do {
     if ((rc = gb_mobius_create(rq.dims, rq.Ls, rq.mf, rq.M5, rq.b, rq.c, ph, GB_F64, nsrc, st, 0, &od))) break;
+    od->fx_off = !copies;
     if ((rc = gb_mobius_create(rq.dims, rq.Ls, rq.mf, rq.M5, rq.b, rq.c, ph, rq.inner_precision, nsrc, st, 0, &of))) break;
     if (cudaMallocAsync(reinterpret_cast<void**>(&dU), size_t(vol) * 36 * 16, st) != cudaSuccess) { rc = GB_ERR_OOM; break; }
     const int64_t nl = vol * 4;
@@ -312,6 +325,7 @@ void worker(gb_server_s* S) {
     std::pair<int64_t, gb_request> item;
     size_t need = 0;
     int chunk = 0;
+    bool copies = false;
     {
       std::unique_lock<std::mutex> lk(S->mu);
       int at = -1;
@@ -323,7 +337,7 @@ void worker(gb_server_s* S) {
           if (st) cudaStreamDestroy(st);
           return;
         }
-        if ((at = pick(S, &need, &chunk)) >= 0) break;
+        if ((at = pick(S, &need, &chunk, &copies)) >= 0) break;
         // wake at least when the oldest request reaches its age bound
         S->cv.wait_for(lk, std::chrono::milliseconds(50));
       }
@@ -354,7 +368,7 @@ void worker(gb_server_s* S) {
         const int n = std::min(chunk, rq.nsrc - first);
         int64_t vol = 1;
         for (int k = 0; k < 4; k++) vol *= rq.dims[k];
-        rc = solve_request(S, rq, n, uint64_t(first) * 0x100000001ull, st, &res, rq.solution,
+        rc = solve_request(S, rq, n, copies, uint64_t(first) * 0x100000001ull, st, &res, rq.solution,
                            size_t(first) * size_t(vol) * rq.Ls * 24);
       }
       cudaEventRecord(e1, st);

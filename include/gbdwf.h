@@ -573,7 +573,7 @@ int gb_server_wait(gb_server_t s, int64_t finished_count, double timeout_s);
 int gb_server_results(gb_server_t s, gb_request_result* out, int max, int* n);
 int gb_server_stats(gb_server_t s, gb_server_stats_t* st);
 int gb_server_destroy(gb_server_t s);
-int gb_request_bytes(const gb_request* r, size_t* bytes); /* the admission estimate */
+int gb_request_bytes(const gb_request* r, size_t* bytes); /* the least admission estimate */
 int gb_server_set_age_limit(gb_server_t s, double seconds);
 /* Sheds every request still queued (not admitted): each finishes with GB_ERR_CANCELLED;
  * *n = how many.  Requests already running complete. */
