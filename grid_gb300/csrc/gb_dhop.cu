@@ -969,17 +969,17 @@ static int dhop_axpy_sides(Op* op, HalfView in, HalfView out, int out_parity, co
   p.c1 = float(a.c1);
   const bool f = op->prec == GB_F32;
   const PairShapeDhop s = dhop_pair_shape(op->L5, op->half4);
-  if (parts && op->Ls == 1 && !in2 && size_t(s.blocks) * op->nrhs <= op->partial_doubles && (!r || r->prec == op->prec)) {
+  // (the CG asks for |out|^2 without the dagger and for the update of r with it)
+  if (parts && op->Ls == 1 && !in2 && size_t(s.blocks) * op->nrhs <= op->partial_doubles &&
+      (r ? dag && r->prec == op->prec : !dag)) {
     p.dpart = op->d_partial;
     *parts = int(s.blocks);
     if (r) {
       p.r = r->data;
       p.r_norms = r->norms;
-      if (f) return dag ? launch_dhop_pair_t<float, true, false, 5>(op, p) : launch_dhop_pair_t<float, false, false, 5>(op, p);
-      return dag ? launch_dhop_pair_t<__half, true, false, 5>(op, p) : launch_dhop_pair_t<__half, false, false, 5>(op, p);
+      return f ? launch_dhop_pair_t<float, true, false, 5>(op, p) : launch_dhop_pair_t<__half, true, false, 5>(op, p);
     }
-    if (f) return dag ? launch_dhop_pair_t<float, true, false, 4>(op, p) : launch_dhop_pair_t<float, false, false, 4>(op, p);
-    return dag ? launch_dhop_pair_t<__half, true, false, 4>(op, p) : launch_dhop_pair_t<__half, false, false, 4>(op, p);
+    return f ? launch_dhop_pair_t<float, false, false, 4>(op, p) : launch_dhop_pair_t<__half, false, false, 4>(op, p);
   }
   if (f) return dag ? launch_dhop_pair_t<float, true, false, 3>(op, p) : launch_dhop_pair_t<float, false, false, 3>(op, p);
   return dag ? launch_dhop_pair_t<__half, true, false, 3>(op, p) : launch_dhop_pair_t<__half, false, false, 3>(op, p);
