@@ -1237,6 +1237,7 @@ int gb_field_axpy_norm(gb_field_t z, double a, gb_field_t x, gb_field_t y, doubl
   GB_TRY(check_conf(z, x));
   GB_TRY(check_conf(z, y));
   if (x->subset != y->subset) { set_error("axpy_norm: checkerboard mismatch"); return GB_ERR_BAD_PARITY; }
+  if (!z->full() && x->full()) { set_error("axpy_norm: full/half mismatch"); return GB_ERR_BAD_PARITY; }
   Op* op = z->op;
   z->subset = x->subset;
   const int g = red_parts(op, z->prec);
