@@ -2,7 +2,7 @@
 // bits.  The FP64 hopping term of an operator created with GB_FLAG_DF64 runs in it on the FP32
 // pipes, which GB300 issues at 64 times its FP64 rate, while the fields keep their FP64
 // storage: each double is split into (hi, lo) on load and hi + lo is rounded back to a double
-// on store.  (Other FP64 operators use the fixed-point form of gb_fx64.cuh, which is exact and
+// on store.  (Other FP64 operators use the fixed-point form of gb_fx64.cuh, which is more accurate and
 // faster.)
 //
 // The split and the widening use integer operations only, so no FP64 instruction is

@@ -18,7 +18,8 @@
 //    time boundary is already folded into the stored links, as in Grid's DoubleStore).
 //
 // FP64 operators run gb_dhop_fx.cu instead.  dhop_kernel<double> here serves those with 12-real
-// links or without memory for the fixed-point links, and the double-float form of GB_FLAG_DF64.
+// links, with links that differ in size or without memory for the fixed-point copies, and the double-float form of
+// GB_FLAG_DF64.
 #include <cuda_fp16.h>
 
 #include <atomic>

@@ -3,11 +3,12 @@
 // The same sum as gb_dhop.cu's dhop_kernel<double> (DhopEO / DhopOE and their daggers,
 // WilsonKernelsImplementation.h:113-163) on the same FP64 fields.  What bounds that kernel is
 // the FP64 pipe, 2 lanes per clock and SM for 860 operations per output site.  Here:
-//   fx_convert_kernel     the input checkerboard as integers with one exponent per 5D site: a
+//   fx_convert_kernel     the input checkerboard as integers with one exponent per 5D site (and that of its smallest
+//                         pair of spins): a
 //                         pass over the field (22 us for 75 MB in, 77 MB out, at HBM rate).
 //                         Converting inside the legs, eight times per site, took 1700 of 6200
 //                         instructions per output site and was slower for every Moebius size
-//   dhop_fx_kernel        projections, SU(3) products and sums over legs and spins as exact
+//   dhop_fx_kernel        projections, SU(3) products and sums over legs and spins in
 //                         integer arithmetic, each result rounded to a double once; 1728 wide
 //                         multiply-adds (32 lanes per clock and SM) of 4500 instructions per
 //                         output site.  The multiply-add pipe is its bound (74 % busy); four
@@ -18,7 +19,8 @@
 //
 // A site whose values the fixed-point range does not hold (infinities, NaN, magnitudes outside
 // 2^(fx::kEmin - 1023) .. 2^(fx::kEmax - 1022)) is marked, and the outputs next to it are
-// computed by fx_site_fp64 in FP64.
+// computed by fx_site_fp64 in FP64; so are outputs whose terms are all small (fx_site_exponent).  With every
+// output on that path, a field of one colour on unit links, DhopEO takes 847 us at 16^4 x 16.
 //
 // Links: fixed-point copies made at the gauge import, in one of two layouts.
 //   slots in CTAs   [x_cb][leg][9] int4, staged per CTA in shared memory by TMA bulk copies, one
@@ -60,9 +62,11 @@ struct FxParams {
 
 constexpr float kFxLinkRatio = 4.f;  // of the largest and smallest link row (see fx_import_links)
 constexpr int kFxLinkStride = 73;  // int4 per staged site: 72 and one of padding
-// Up to this many output sites in a launch the split kernel takes the slots-in-CTAs layout too:
-// equal at 32768 sites (8^3 x 16 x 8: 22.3 against 22.7 us), 15.5 against 19.3 us at 16384, and
-// 232 against 185 us at 524288, where the shared staging of the links counts.
+// Up to this many output sites in a launch the split kernel takes the slots-in-CTAs layout too.  Split against
+// one thread per site, DhopEO: 16384 sites 11.8 / 15.5 us (8 slots), 24576 15.7 / 18.2 (12), 32768 18.1 / 18.9 (8) and 18.0 /
+// 18.3 (16), 40960 25.1 / 25.2 (8) and 25.0 / 24.7 (20), 49152 25.9 / 25.1 (16), 65536 30.1 / 30.6 (8) and 29.9 / 30.1 (16),
+// 73728 32.6 / 36.1 (12), 71680 32.2 / 29.6 (20), 124416 55.1 / 49.7 (12), 131072 58.5 / 52.0 (8), 262144 112 / 98.7 (8): within
+// 4 % of one another from 32768 to 65536 but for single waves, and from there the shared staging of the links counts.
 constexpr int64_t kFxSplitSites = 40000;
 // Above this many CTAs of the split kernel (608 are resident with four warps each), two warps share a
 // site's directions in place of four: half of the partial sums through shared memory, and no second
@@ -584,7 +588,8 @@ __global__ void __launch_bounds__(32 * W, 16 / W) dhop_fx_split_kernel(const __g
 // magnitudes; with terms of one size 1e-17 to 4e-17 against 5e-17 to 7e-17).  Gaussian factors stay above it by 4 to 24:
 // none of 2e5 sites falls below with up to 32 slots, 0.6 % with 33.
 // U W runs in FP64.  Same lanes, warps and CTAs as deriv_kernel.  MDeriv 16^4 x 12:
-// 708 -> 418 us, of which Meooe5D is 80 and the conversions 94 (two or four CTAs per SM: 466, 463).
+// 708 -> 421 us, of which Meooe5D is 80 and the conversions 94 (two or four CTAs per SM: 466, 463; the lower
+// bound of the terms 9).
 constexpr int kDerivSlots = 64;
 
 struct FxDerivParams {
@@ -798,7 +803,10 @@ static size_t fx_sites(const Op* op) { return size_t(op->half4) * op->Ls * op->n
 static int fx_sets(const Op* op) { return op->Ls == 1 && op->nrhs_user == 1 ? 4 : 2; }
 
 // The links' layout: sites in lanes below 8 slots per site (a CTA of 128 threads then stages 16
-// sites at most, 18.7 KB, and four CTAs stay resident).
+// sites at most, 18.7 KB, and four CTAs stay resident).  Wilson DhopEO, slots in CTAs against sites in lanes, us: 12^3 x 16
+// with 6 / 7 / 8 / 9 slots 42.3 / 44.0 / 43.0 / 53.3 against 37.1 / 40.3 / 45.7 / 55.0; 16^4 79.5 / 94.9 / 98.9 / 118 against
+// 83.5 / 99.0 / 108 / 124; 24^3 x 32 469 / 574 / 606 / 733 against 531 / 633 / 700 / 812: 4 to 7 slots on large
+// lattices would be up to 12 % faster the other way, which no rule takes yet.
 static bool fx_soa(const Op* op) { return op->Ls * op->nrhs_user < 8; }
 
 // Fixed-point copies of op->links, and the scratch of fx_convert_kernel (both checkerboards of

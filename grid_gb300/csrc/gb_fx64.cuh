@@ -20,8 +20,10 @@
 // sum |lo_u hi_h| <= 6 2^31 2^29 = 6 2^60, so |mid| < 7.6 2^60 < 2^63; |hh| <= 1.5 2^58 and
 // eight legs stay below 2^62.
 //
-// The rounding of one site is below the FP64 kernel's (tests/cpp/test_fx64.cpp measures both
-// against long double): sums are exact, where FP64 rounds each of them at 2^-53.
+// The error is a fixed part of the unit, where FP64's is one of each sum's own terms.  With terms of the unit's
+// size it is below the FP64 kernel's (tests/cpp/test_fx64.cpp measures both against long double): sums are
+// exact, where FP64 rounds each of them at 2^-53.  A sum of terms far below the unit would keep fewer bits than a
+// double: kernels find those (fx_site_exponent, deriv_fx_kernel in gb_dhop_fx.cu) and take them in FP64.
 #pragma once
 
 #include <stdint.h>

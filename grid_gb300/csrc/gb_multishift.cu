@@ -135,7 +135,7 @@ __device__ __forceinline__ void ms_mid(MSState* st, const double* partial, int n
 // first warp per shift (kMaxShift = 32).  The other CTAs are done and this one's chain of FP64
 // divisions and loads is what the launch still takes: q = znew / zold comes from the one division
 // that znew needs, the state is loaded before the sums, and a CTA sums only the values that
-// are used (8^3 x 16 x 8 solve with 6 poles 52.9 -> 50.8 ms).
+// are used (8^3 x 16 x 8 solve with 6 poles, both in turn: 52.9 -> 50.8 ms; from box to box the solve takes 50.8 to 55.4).
 __device__ __forceinline__ void ms_post(MSState* st, const double* partial, int nparts) {
   // the state is on its way while the sums are taken
   const int s = threadIdx.x & 31, ns = st->nshift;
