@@ -326,6 +326,7 @@ void worker(gb_server_s* S) {
     size_t need = 0;
     int chunk = 0;
     bool copies = false;
+    double started = 0.0;
     {
       std::unique_lock<std::mutex> lk(S->mu);
       int at = -1;
@@ -343,6 +344,7 @@ void worker(gb_server_s* S) {
       }
       item = S->queue[at];
       S->queue.erase(S->queue.begin() + at);
+      started = S->now();  // under the lock: start times follow the order of admission
       S->used += need;
       S->peak_used = std::max(S->peak_used, S->used);
       S->running++;
@@ -354,7 +356,7 @@ void worker(gb_server_s* S) {
     std::memset(&res, 0, sizeof(res));
     res.id = item.first;
     res.t_submit = rq.t_submit;
-    res.t_start = S->now();
+    res.t_start = started;
     res.nsrc = rq.nsrc;
     res.chunk = chunk;
     res.dev_start = res.dev_end = -1.0;
