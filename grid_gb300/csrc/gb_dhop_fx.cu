@@ -259,7 +259,8 @@ __device__ __noinline__ void fx_site_fp64(const double2* in, double2* out, const
 // colour, and a link's row has no smaller sum than another's by more than kFxLinkRatio: its terms add up to the
 // unit's size if the neighbours' smallest pairs do, to 2^-kFxSpread of it.  At that bound the error is 1.6
 // times FP64's rounding (integer model on the host: 2.3e-16 against 1.4e-16 of the sum of the terms'
-// magnitudes with all of it in one neighbour; eight of 2^-3 each 3e-17 against 4.5e-17).  Colours that the links keep
+// magnitudes with all of it in one neighbour; eight of 2^-3 each 3e-17 against 4.5e-17; unitary links, with
+// rows at kFxLinkRatio up to 2.7 times that).  Colours that the links keep
 // apart and that differ in size by more than 2^4 are below it; ordinary fields are not: of a Gaussian
 // field one pair of one neighbour is enough everywhere, of the smallest pole's solution on 8^3 x 16 x 8 in all but 3e-5 of the
 // sites, and the sum there.  (Without the sum those few sites, 10 us each for the thread that takes them in FP64,

@@ -80,8 +80,8 @@ int gb_device_count(int* n);
  * once.  Its relative L2 error is below IEEE double arithmetic's (5e-17 against 1.4e-16 per
  * site, Gaussian fields).  Outputs whose terms are all well below that unit, sites outside its range
  * and gauge fields whose links differ in size are computed in IEEE double, so that the error
- * of a component stays within twice double's rounding of its terms (of |f| of the two spins
- * that a projection adds).  It is faster; the flag remains for callers that chose its arithmetic.
+ * of a component stays within about twice double's rounding of its terms (of |f| of the two spins
+ * that a projection adds; four times where the links' row sums differ by 4, the most that is taken).  It is faster; the flag remains for callers that chose its arithmetic.
  */
 #define GB_FLAG_RECON12 1u
 #define GB_FLAG_DF64 2u
